@@ -1,10 +1,10 @@
 """Build libpicgb.so (the CUDA step library) in-tree for sm_103a.
 
 Each translation unit is compiled by nvcc in parallel and linked into a
-shared library next to this file.  pgb_fields.cu is compiled with
---fmad=false so that its FP64 multigrid performs the reference's operations
-one at a time (no fused multiply-add), which keeps it bit-identical to the
-reference's Mglin for the same right-hand side.
+shared library next to this file.  pgb_fields.cu and pgb_mg.cu are compiled
+with --fmad=false so that the FP64 right-hand side and multigrid round as the
+reference's operations do (no contraction), which keeps the potential
+bit-identical to the reference's Mglin for the same right-hand side.
 """
 from __future__ import annotations
 
@@ -29,6 +29,7 @@ UNITS = {
     "pgb_particles.cu": [],
     "pgb_walls.cu": [],
     "pgb_fields.cu": ["--fmad=false"],
+    "pgb_mg.cu": ["--fmad=false"],
     "pgb_sort.cu": [],
     "pgb_reduce.cu": [],
     "pgb_graphs.cu": [],

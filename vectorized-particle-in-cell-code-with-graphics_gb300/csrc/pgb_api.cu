@@ -442,7 +442,6 @@ extern "C" int pgb_destroy(pgb_run* r) {
     cudaFree(r->rho); cudaFree(r->phi); cudaFree(r->ex); cudaFree(r->ey); cudaFree(r->exy);
     cudaFree(r->prob_cx);
     for (int j = 0; j < r->ng; ++j) { cudaFree(r->mg_u[j]); cudaFree(r->mg_f[j]); cudaFree(r->mg_v[j]); cudaFree(r->mg_r[j]); }
-    cudaFree(r->mg_tab);
     pgb_mg_free(r);
     for (int w = 0; w < 2; ++w) cudaFree(r->neut[w]);
     if (r->h_stage) cudaFreeHost(r->h_stage);

@@ -30,9 +30,7 @@
 #define PGB_ITEMS (PGB_TILE / PGB_PUSH_THREADS)
 #define PGB_FIX_SCALE 524288.0      /* deposit fixed point: 2^19 per unit weight */
 #define PGB_FIX_SCALE_F 524288.0f
-#define PGB_MG_SMALL 65        /* levels with n <= 65 are solved by one CTA  */
 #define PGB_CX_TILE 2048       /* ions per charge-exchange tile sum            */
-#define PGB_MG_SMALL64 33      /* the same for the FP64 multigrid            */
 #define PGB_MAX_LEVELS 16
 #define PGB_BIN 32             /* bin edge in cells (spatial sort)            */
 #define PGB_HALO 8             /* deposit window halo around a bin, cells     */
@@ -132,8 +130,6 @@ struct pgb_run {
     int ng = 0;
     int mg_n[PGB_MAX_LEVELS];
     double *mg_u[PGB_MAX_LEVELS], *mg_f[PGB_MAX_LEVELS], *mg_v[PGB_MAX_LEVELS], *mg_r[PGB_MAX_LEVELS];
-    double** mg_tab = nullptr;                       /* device table of the level pointers */
-    float** mg32_tab = nullptr;
     double *dc_u = nullptr, *dc_u2 = nullptr;       /* FP32_DC: FP64 solution, two buffers */
     /* DST_DC: sine-transform scratch ((N-1) rows of N floats), twiddles, s_k */
     float* dst_t = nullptr;
@@ -144,8 +140,8 @@ struct pgb_run {
     double* dst_wc = nullptr;
     double* dst_wr = nullptr;
     float *mg32_u[PGB_MAX_LEVELS], *mg32_f[PGB_MAX_LEVELS], *mg32_v[PGB_MAX_LEVELS], *mg32_r[PGB_MAX_LEVELS];
-    /* the pre-smoothing result of each level (the tiled smoother reads one
-     * buffer and writes another: blocks never see a neighbour's update)  */
+    /* the pre-smoothing result of each level (the tiles read one buffer and
+     * write another: none sees a neighbour's update)                     */
     double* mg_w[PGB_MAX_LEVELS] = {};
     float* mg32_w[PGB_MAX_LEVELS] = {};
     /* event lists: per tile 32 ballot words (slot order) and a count, then
@@ -307,6 +303,12 @@ int pgb_launch_dump_offsets(pgb_run* r, int s);
 int pgb_launch_dump(pgb_run* r, int s, double* d_out, unsigned int* d_ids, long long cap, int t0, int t1);
 int pgb_mg_setup(pgb_run* r);
 void pgb_mg_free(pgb_run* r);
+/* multigrid (pgb_mg.cu): full multigrid from f[top] into u[top]; one FP32
+ * V-cycle from 0 on the right-hand side r[top] into v[top]              */
+int pgb_mg_attributes(pgb_run* r);
+int pgb_mg_fmg64(pgb_run* r);
+int pgb_mg_fmg32(pgb_run* r);
+int pgb_mg_vcycle32(pgb_run* r);
 /* FP32 sine-transform Poisson solver (pgb_dst.cu) */
 int pgb_dst_setup(pgb_run* r);
 void pgb_dst_free(pgb_run* r);
