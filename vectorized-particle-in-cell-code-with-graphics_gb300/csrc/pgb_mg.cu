@@ -20,10 +20,9 @@
  *     interpolated or corrected before a sweep that starts with red;
  *   - a correction starts at 0, so its first red sweep is (0 - h^2 f)/4.
  *
- * Who works on a level:
- *   n <= 33         one CTA, every level in shared memory; n <= 17 on 128
- *                   threads (one warp per scheduler, barrier of 21 clocks)
- *   n = 65, 129     a cluster of 16 CTAs in the same launch, a band of rows
+ * Who works on a level (Cfg):
+ *   n <= 17 (FP64), 33 (FP32)   one CTA, every level in shared memory
+ *   up to n = 129   a cluster of 16 CTAs in the same launch, a band of rows
  *                   per CTA with the halo that makes one exchange (through
  *                   L2, a cluster barrier of 380 clocks) enough for
  *                   smoothing, residual and restriction, and one for
@@ -43,10 +42,12 @@ template <int K>
 __device__ __forceinline__ double down_pow2(double x) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
     const unsigned a = (unsigned)hi & 0x7fffffffu;
-    /* normal before and after: the exponent field drops by K */
-    if (a - ((unsigned)(K + 1) << 20) < 0x7ff00000u - ((unsigned)(K + 1) << 20)) return __hiloint2double(hi - (K << 20), lo);
-    if ((a | (unsigned)lo) == 0u) return x;
-    return x * (1.0 / (1 << K));   /* subnormal results, infinities, NaN */
+    /* normal before and after: the exponent field drops by K; +-0 stays */
+    const bool normal = a - ((unsigned)(K + 1) << 20) < 0x7ff00000u - ((unsigned)(K + 1) << 20);
+    const bool zero = (a | (unsigned)lo) == 0u;
+    double r = __hiloint2double(normal ? hi - (K << 20) : hi, lo);
+    if (!(normal || zero)) r = x * (1.0 / (1 << K));   /* subnormal results, infinities, NaN */
+    return r;
 }
 template <int K>
 __device__ __forceinline__ float down_pow2(float x) { return x * (1.0f / (1 << K)); }
@@ -82,214 +83,232 @@ __device__ __forceinline__ void black_pair(int i, int j, int nc, int& k1, int& k
 /* how a V-cycle's first smoothing starts */
 enum { FROM_ZERO = 0, FROM_U = 1, FROM_COARSE = 2 };
 
-/* --------------------------------------------- levels in one CTA (n <= 33) */
-/* level l has n_l = 2^(l+1) + 1 nodes a side; SM_TOP is the level of 33 */
-constexpr int SM_TOP = 4;
-constexpr int SM_THREADS = 512;
-constexpr int SM_TEAM = 128;   /* threads on levels of 17 nodes and fewer */
+/* a correction's first red value (0 - g)/4: +0 for g = +-0, else -g/4 */
+__device__ __forceinline__ double red_from_zero(double g) {
+    const int hi = __double2hiint(g), lo = __double2loint(g);
+    const unsigned a = (unsigned)hi & 0x7fffffffu;
+    const bool normal = a - (3u << 20) < 0x7ff00000u - (3u << 20), zero = (a | (unsigned)lo) == 0u;
+    double r = __hiloint2double(normal ? (hi ^ (int)0x80000000) - (2 << 20) : 0, lo);
+    if (!(normal || zero)) r = (0.0 - g) * 0.25;
+    return r;
+}
+__device__ __forceinline__ float red_from_zero(float g) { return (0.0f - g) * 0.25f; }
+
+/* A level's h^2 and 1/h^2, rounded as the reference rounds them, from the
+ * host: a division in FP64 is a chain of some ten operations of 64 clocks */
+template <class T>
+struct MgConst {
+    T h2[PGB_MAX_LEVELS], h2i[PGB_MAX_LEVELS];
+    T c0;   /* -h * h of the 3x3 grid */
+};
+
+/* level l has n_l = 2^(l+1) + 1 nodes a side */
 __host__ __device__ constexpr int sm_n(int l) { return (2 << l) + 1; }
 __host__ __device__ constexpr int sm_below(int l) { return l == 0 ? 0 : sm_below(l - 1) + sm_n(l - 1) * sm_n(l - 1); }
-/* shared image: U, F, G = h^2 F of levels 0..SM_TOP (a V-cycle's top), V,
- * R, GR = h^2 R of levels 0..SM_TOP-1 (below its top), one residual plane */
-constexpr int SM_A = sm_below(SM_TOP + 1), SM_B = sm_below(SM_TOP);
-constexpr int SM_WORDS = 3 * SM_A + 3 * SM_B + sm_n(SM_TOP) * sm_n(SM_TOP);
+
+/* the finest level that one CTA solves, and the threads of a CTA.  FP64:
+ * 17 nodes (a level of 33 nodes takes 7.3 us in one CTA, bound by its FP64
+ * pipe, and 2.9 us on the cluster); FP32: 33 nodes (1.0 us in one CTA)   */
+template <class T>
+struct Cfg;
+template <>
+struct Cfg<double> { static constexpr int TOP = 3, THREADS = 256; };
+template <>
+struct Cfg<float> { static constexpr int TOP = 4, THREADS = 512; };
+
+/* ----------------------------------------------------- levels in one CTA */
+/* shared image: U, F, G = h^2 F of levels 0..TOP (a V-cycle's top), V, R,
+ * GR = h^2 R of levels 0..TOP-1 (below its top), one residual plane      */
+template <class T>
+struct Sm {
+    static constexpr int TOP = Cfg<T>::TOP, A = sm_below(TOP + 1), B = sm_below(TOP);
+    static constexpr int WORDS = 3 * A + 3 * B + sm_n(TOP) * sm_n(TOP);
+};
 
 extern __shared__ __align__(16) unsigned char mg_smem[];
+template <class T>
+__device__ __forceinline__ T* smem() { return reinterpret_cast<T*>(mg_smem); }
 
 template <class T, int L, bool TOP>
 struct Arr {
-    static constexpr int n = sm_n(L), per = 1 << L;   /* nodes a side, slots a row */
-    static constexpr int o = sm_below(L);
-    static __device__ __forceinline__ T* u() { return reinterpret_cast<T*>(mg_smem) + (TOP ? o : 3 * SM_A + o); }
-    static __device__ __forceinline__ T* f() { return reinterpret_cast<T*>(mg_smem) + (TOP ? SM_A + o : 3 * SM_A + SM_B + o); }
-    static __device__ __forceinline__ T* g() { return reinterpret_cast<T*>(mg_smem) + (TOP ? 2 * SM_A + o : 3 * SM_A + 2 * SM_B + o); }
+    static constexpr int A = Sm<T>::A, B = Sm<T>::B, o = sm_below(L);
+    static __device__ __forceinline__ T* u() { return smem<T>() + (TOP ? o : 3 * A + o); }
+    static __device__ __forceinline__ T* f() { return smem<T>() + (TOP ? A + o : 3 * A + B + o); }
+    static __device__ __forceinline__ T* g() { return smem<T>() + (TOP ? 2 * A + o : 3 * A + 2 * B + o); }
 };
 template <class T>
-__device__ __forceinline__ T* sm_res() { return reinterpret_cast<T*>(mg_smem) + 3 * SM_A + 3 * SM_B; }
+__device__ __forceinline__ T* sm_res() { return smem<T>() + 3 * Sm<T>::A + 3 * Sm<T>::B; }
 
+/* who works on a level: one warp for n <= 9, 128 threads for n = 17, 512
+ * for n = 33.  Every point is updated by the same arithmetic whichever team
+ * updates it.                                                            */
 template <int L>
-__device__ __forceinline__ void team_sync() {
-    if (L >= SM_TOP) __syncthreads();
-    else asm volatile("bar.sync 1, %0;" ::"n"(SM_TEAM) : "memory");
-}
-template <int L>
-__device__ __forceinline__ constexpr int team_size() { return L >= SM_TOP ? SM_THREADS : SM_TEAM; }
-
-/* one colour of a sweep (0 red, 1 black): a row has 2^L slots */
-template <class T, int L, bool TOP>
-__device__ __forceinline__ void sm_sweep(int color) {
-    using A = Arr<T, L, TOP>;
-    constexpr int n = A::n;
-    T* const u = A::u();
-    const T* const g = A::g();
-#pragma unroll 1
-    for (int t = threadIdx.x; t < (n - 2) * A::per; t += team_size<L>()) {
-        const int i = (t >> L) + 1, j = 1 + ((i + 1 + color) & 1) + 2 * (t & (A::per - 1));
-        if (j <= n - 2) {
-            const int k = i * n + j;
-            u[k] = gs_value(u[k + n], u[k - n], u[k + 1], u[k - 1], g[k]);
-        }
+struct Team {
+    static constexpr int size = L <= 2 ? 32 : L == 3 ? 128 : 512;
+    static __device__ __forceinline__ void sync() {
+        if (L <= 2) __syncwarp();
+        else if (L == 3) asm volatile("bar.sync 1, 128;" ::: "memory");
+        else __syncthreads();
     }
-    team_sync<L>();
-}
+};
 
-/* the points of a level below the top start at 0: red points (0 - g)/4
- * (written by whoever produced g), then the black sweep                  */
-template <class T>
-__device__ __forceinline__ T red_from_zero(T g) { return down_pow2<2>((T)0 - g); }
-
+/* One V-cycle's work on level L.  A thread keeps its red and its black
+ * point (each colour has at most one point per thread) and the shared
+ * index arithmetic is done once.                                         */
 template <class T, int L, bool TOP, int START>
-__device__ __forceinline__ void sm_down(T length) {
+__device__ __forceinline__ void sm_level_down(const MgConst<T>& c, int kr, int kb, bool hr, bool hb, int b1, int b0) {
     using A = Arr<T, L, TOP>;
     using C = Arr<T, L - 1, false>;
-    constexpr int n = A::n, nc = C::n, per = A::per;
+    constexpr int n = sm_n(L), nc = sm_n(L - 1), per = 1 << L, S = Team<L>::size;
     T* const u = A::u();
     const T* const f = A::f();
-    const T h = length / (T)(n - 1), h2i = (T)1.0 / (h * h);
+    const T* const g = A::g();
+    const T h2i = c.h2i[L];
     if (START == FROM_COARSE) {
         const T* const uc = Arr<T, L - 1, true>::u();
-#pragma unroll 1
-        for (int t = threadIdx.x; t < (n - 2) * per; t += team_size<L>()) {
-            const int i = (t >> L) + 1, j = 1 + (i & 1) + 2 * (t & (per - 1));
-            if (j <= n - 2) {
-                int k1, k0;
-                black_pair(i, j, nc, k1, k0);
-                u[i * n + j] = down_pow2<1>(uc[k1] + uc[k0]);
-            }
-        }
-        team_sync<L>();
+        if (hb) u[kb] = down_pow2<1>(uc[b1] + uc[b0]);
+        Team<L>::sync();
     }
-    if (START != FROM_ZERO) sm_sweep<T, L, TOP>(0);   /* else the red points are there */
-    sm_sweep<T, L, TOP>(1);
+    if (START != FROM_ZERO) {   /* else the red points are there */
+        if (hr) u[kr] = gs_value(u[kr + n], u[kr - n], u[kr + 1], u[kr - 1], g[kr]);
+        Team<L>::sync();
+    }
+    if (hb) u[kb] = gs_value(u[kb + n], u[kb - n], u[kb + 1], u[kb - 1], g[kb]);
+    Team<L>::sync();
     /* residuals where the restriction reads them: all points of even rows,
-     * the black points (even j) of odd rows                              */
+     * the black points (even columns) of odd rows                        */
     T* const res = sm_res<T>();
-    constexpr int na = (per - 1) * 2 * per, nb = per * per;
-#pragma unroll 1
-    for (int t = threadIdx.x; t < na + nb; t += team_size<L>()) {
-        const int s = t - na;
+    constexpr int na = (per - 1) * 2 * per, nb = per * per, trips = (na + nb + S - 1) / S;
+    T rv[trips];
+    int rk[trips];
+#pragma unroll
+    for (int q = 0; q < trips; ++q) {
+        const int t = threadIdx.x + q * S, s = t - na;
         const int i = s < 0 ? 2 * (t >> (L + 1)) + 2 : 2 * (s >> L) + 1;
         const int j = s < 0 ? 1 + (t & (2 * per - 1)) : 2 * (s & (per - 1)) + 2;
-        if (j <= n - 2) {
-            const int k = i * n + j;
-            res[k] = resid_value(u[k + n], u[k - n], u[k + 1], u[k - 1], u[k], f[k], h2i);
-        }
+        const bool ok = t < na + nb && j <= n - 2;
+        const int k = ok ? i * n + j : n + 1;
+        rv[q] = resid_value(u[k + n], u[k - n], u[k + 1], u[k - 1], u[k], f[k], h2i);
+        rk[q] = ok ? k : -1;
     }
-    team_sync<L>();
+#pragma unroll
+    for (int q = 0; q < trips; ++q)
+        if (rk[q] >= 0) res[rk[q]] = rv[q];
+    Team<L>::sync();
     /* half weighting; the coarse red points get their first value here */
-    const T hc = length / (T)(nc - 1), h2c = hc * hc;
-    T* const rc = C::f();
-    T* const gc = C::g();
-    T* const vc = C::u();
-#pragma unroll 1
-    for (int t = threadIdx.x; t < (nc - 2) * per; t += team_size<L>()) {
-        const int ic = (t >> L) + 1, jc = 1 + (t & (per - 1));
-        if (jc <= nc - 2) {
-            const int k = 2 * ic * n + 2 * jc, kc = ic * nc + jc;
-            const T r = half_weight(res[k], res[k + n], res[k - n], res[k + 1], res[k - 1]);
-            const T g = h2c * r;
-            rc[kc] = r;
-            gc[kc] = g;
-            if (((ic + jc) & 1) == 0) vc[kc] = red_from_zero(g);
-        }
+    const T h2c = c.h2[L - 1];
+    const int t = threadIdx.x, ic = (t >> L) + 1, jc = 1 + (t & (per - 1));
+    if (t < (nc - 2) * per && jc <= nc - 2) {
+        const int k = 2 * ic * n + 2 * jc, kc = ic * nc + jc;
+        const T r = half_weight(res[k], res[k + n], res[k - n], res[k + 1], res[k - 1]);
+        const T gg = h2c * r;
+        C::f()[kc] = r;
+        C::g()[kc] = gg;
+        if (((ic + jc) & 1) == 0) C::u()[kc] = red_from_zero(gg);
     }
-    team_sync<L>();
+    Team<L>::sync();
 }
-/* the correction of the black points, then a sweep */
 template <class T, int L, bool TOP>
-__device__ __forceinline__ void sm_up() {
-    using A = Arr<T, L, TOP>;
-    constexpr int n = A::n, per = A::per, nc = sm_n(L - 1);
-    T* const u = A::u();
+__device__ __forceinline__ void sm_level_up(int kr, int kb, bool hr, bool hb, int b1, int b0) {
+    constexpr int n = sm_n(L);
+    T* const u = Arr<T, L, TOP>::u();
+    const T* const g = Arr<T, L, TOP>::g();
     const T* const vc = Arr<T, L - 1, false>::u();
-#pragma unroll 1
-    for (int t = threadIdx.x; t < (n - 2) * per; t += team_size<L>()) {
-        const int i = (t >> L) + 1, j = 1 + (i & 1) + 2 * (t & (per - 1));
-        if (j <= n - 2) {
-            int k1, k0;
-            black_pair(i, j, nc, k1, k0);
-            u[i * n + j] = fma_t((T)0.5, vc[k1] + vc[k0], u[i * n + j]);
-        }
-    }
-    team_sync<L>();
-    sm_sweep<T, L, TOP>(0);
-    sm_sweep<T, L, TOP>(1);
+    if (hb) u[kb] = fma_t((T)0.5, vc[b1] + vc[b0], u[kb]);
+    Team<L>::sync();
+    if (hr) u[kr] = gs_value(u[kr + n], u[kr - n], u[kr + 1], u[kr - 1], g[kr]);
+    Team<L>::sync();
+    if (hb) u[kb] = gs_value(u[kb + n], u[kb - n], u[kb + 1], u[kb - 1], g[kb]);
+    Team<L>::sync();
 }
 /* V-cycle with top L; entered by the team of level L */
 template <class T, int L, bool TOP, int START>
 struct SmV {
-    static __device__ __noinline__ void run(T length) {
-        sm_down<T, L, TOP, START>(length);
-        if (L == SM_TOP) {
-            if (threadIdx.x < SM_TEAM) SmV<T, L - 1, false, FROM_ZERO>::run(length);
-            __syncthreads();
+    static __device__ __noinline__ void run(const MgConst<T>& mc) {
+        constexpr int n = sm_n(L), per = 1 << L;
+        static_assert((n - 2) * per <= Team<L>::size, "one point of a colour per thread");
+        const int t = threadIdx.x, i = (t >> L) + 1, c = 2 * (t & (per - 1)) + 1;
+        const int jr = c + ((i + 1) & 1), jb = c + (i & 1);
+        const bool in = i <= n - 2, hr = in && jr <= n - 2, hb = in && jb <= n - 2;
+        int b1 = 0, b0 = 0;
+        if (hb) black_pair(i, jb, sm_n(L - 1), b1, b0);
+        sm_level_down<T, L, TOP, START>(mc, i * n + jr, i * n + jb, hr, hb, b1, b0);
+        if (Team<L - 1>::size < Team<L>::size) {
+            if (threadIdx.x < Team<L - 1>::size) SmV<T, L - 1, false, FROM_ZERO>::run(mc);
+            Team<L>::sync();
         } else {
-            SmV<T, L - 1, false, FROM_ZERO>::run(length);
+            SmV<T, L - 1, false, FROM_ZERO>::run(mc);
         }
-        sm_up<T, L, TOP>();
+        sm_level_up<T, L, TOP>(i * n + jr, i * n + jb, hr, hb, b1, b0);
     }
 };
 /* the 3x3 grid: u = -h^2 f / 4 (mglin.cpp:103-110) */
 template <class T, bool TOP, int START>
 struct SmV<T, 0, TOP, START> {
-    static __device__ __forceinline__ void run(T length) {
-        if (threadIdx.x == 0) {
-            const T h = (T)0.5 * length;
-            Arr<T, 0, TOP>::u()[4] = -h * h * Arr<T, 0, TOP>::f()[4] / (T)4.0;
-        }
-        team_sync<0>();
+    static __device__ __forceinline__ void run(const MgConst<T>& mc) {
+        if (threadIdx.x == 0) Arr<T, 0, TOP>::u()[4] = down_pow2<2>(mc.c0 * Arr<T, 0, TOP>::f()[4]);
+        Team<0>::sync();
     }
 };
 
-/* all shared words to 0: the walls of every level stay 0 */
-template <class T>
-__device__ __forceinline__ void sm_clear() {
-    T* const s = reinterpret_cast<T*>(mg_smem);
-    for (int k = threadIdx.x; k < SM_WORDS; k += SM_THREADS) s[k] = (T)0;
-    __syncthreads();
+/* zero walls of U and V (the other arrays' walls are not read) */
+template <class T, int L, bool TOP>
+__device__ __forceinline__ void sm_walls(int t) {
+    constexpr int n = sm_n(L);
+    T* const u = Arr<T, L, TOP>::u();
+    if (t >= 0 && t < n) u[t] = u[(n - 1) * n + t] = u[t * n] = u[t * n + n - 1] = (T)0;
+    if constexpr (L > 0) sm_walls<T, L - 1, TOP>(t - n);
 }
-
 /* F of level L (and G) from a global right-hand side with the same nodes */
 template <class T, int L>
-__device__ __forceinline__ void sm_load_f(const T* gf, T length, bool red) {
+__device__ __forceinline__ void sm_load_f(const T* gf, const MgConst<T>& mc, bool red) {
     using A = Arr<T, L, true>;
-    constexpr int n = A::n;
-    const T h = length / (T)(n - 1), h2 = h * h;
-    for (int k = threadIdx.x; k < n * n; k += SM_THREADS) {
-        const int i = k / n, j = k - i * n;
-        if (i > 0 && j > 0 && i < n - 1 && j < n - 1) {
-            const T f = __ldcg(gf + k), g = h2 * f;
-            A::f()[k] = f;
-            A::g()[k] = g;
-            if (red && ((i + j) & 1) == 0) A::u()[k] = red_from_zero(g);
+    constexpr int n = sm_n(L), W = 2 << L, trips = (W * W + Cfg<T>::THREADS - 1) / Cfg<T>::THREADS;
+    const T h2 = mc.h2[L];
+    T v[trips];
+#pragma unroll
+    for (int q = 0; q < trips; ++q) {
+        const int t = threadIdx.x + q * Cfg<T>::THREADS, i = t >> (L + 1), j = t & (W - 1);
+        v[q] = (i > 0 && j > 0 && i < W) ? __ldcg(gf + i * n + j) : (T)0;
+    }
+    sm_walls<T, L, true>(threadIdx.x);
+    if constexpr (L > 0) sm_walls<T, L - 1, false>((int)threadIdx.x - Cfg<T>::THREADS / 2);
+#pragma unroll
+    for (int q = 0; q < trips; ++q) {
+        const int t = threadIdx.x + q * Cfg<T>::THREADS, i = t >> (L + 1), j = t & (W - 1);
+        if (i > 0 && j > 0 && i < W) {
+            const T g = h2 * v[q];
+            A::f()[i * n + j] = v[q];
+            A::g()[i * n + j] = g;
+            if (red && ((i + j) & 1) == 0) A::u()[i * n + j] = red_from_zero(g);
         }
     }
     __syncthreads();
 }
 template <class T, int L>
 __device__ __forceinline__ void sm_store_u(T* gu) {
-    using A = Arr<T, L, true>;
-    constexpr int n = A::n;
-    for (int k = threadIdx.x; k < n * n; k += SM_THREADS) {
-        const int i = k / n, j = k - i * n;
-        if (i > 0 && j > 0 && i < n - 1 && j < n - 1) gu[k] = A::u()[k];
+    constexpr int n = sm_n(L), W = 2 << L;
+#pragma unroll
+    for (int t = threadIdx.x; t < W * W; t += Cfg<T>::THREADS) {
+        const int i = t >> (L + 1), j = t & (W - 1);
+        if (i > 0 && j > 0) gu[i * n + j] = Arr<T, L, true>::u()[i * n + j];
     }
     __syncthreads();
 }
 /* F of level L from F of level L+1 (interior) */
 template <class T, int L>
-__device__ __forceinline__ void sm_restrict_f(T length) {
+__device__ __forceinline__ void sm_restrict_f(const MgConst<T>& mc) {
     using A = Arr<T, L, true>;
-    constexpr int n = A::n, nf = sm_n(L + 1);
-    const T h = length / (T)(n - 1), h2 = h * h;
+    constexpr int n = sm_n(L), nf = sm_n(L + 1), W = 2 << L;
+    const T h2 = mc.h2[L];
     const T* const ff = Arr<T, L + 1, true>::f();
-    for (int k = threadIdx.x; k < n * n; k += SM_THREADS) {
-        const int i = k / n, j = k - i * n;
-        if (i > 0 && j > 0 && i < n - 1 && j < n - 1) {
+    for (int t = threadIdx.x; t < W * W; t += Cfg<T>::THREADS) {
+        const int i = t >> (L + 1), j = t & (W - 1);
+        if (i > 0 && j > 0) {
             const int q = 2 * i * nf + 2 * j;
             const T f = half_weight(ff[q], ff[q + nf], ff[q - nf], ff[q + 1], ff[q - 1]);
-            A::f()[k] = f;
-            A::g()[k] = h2 * f;
+            A::f()[i * n + j] = f;
+            A::g()[i * n + j] = h2 * f;
         }
     }
     __syncthreads();
@@ -297,47 +316,41 @@ __device__ __forceinline__ void sm_restrict_f(T length) {
 /* F of the levels below L, then the full multigrid up to level L */
 template <class T, int L>
 struct SmF {
-    static __device__ __forceinline__ void restrict_all(T length) {
-        sm_restrict_f<T, L - 1>(length);
-        SmF<T, L - 1>::restrict_all(length);
+    static __device__ __forceinline__ void restrict_all(const MgConst<T>& mc) {
+        sm_restrict_f<T, L - 1>(mc);
+        SmF<T, L - 1>::restrict_all(mc);
     }
-    static __device__ __forceinline__ void solve(T length) {
-        SmF<T, L - 1>::solve(length);
-        if (L >= SM_TOP) __syncthreads();
-        if (L >= SM_TOP || threadIdx.x < SM_TEAM) {
-            SmV<T, L, true, FROM_COARSE>::run(length);
-            SmV<T, L, true, FROM_U>::run(length);
+    static __device__ __forceinline__ void solve(const MgConst<T>& mc) {
+        SmF<T, L - 1>::solve(mc);
+        __syncthreads();
+        if (threadIdx.x < Team<L>::size) {
+            SmV<T, L, true, FROM_COARSE>::run(mc);
+            SmV<T, L, true, FROM_U>::run(mc);
         }
     }
 };
 template <class T>
 struct SmF<T, 0> {
-    static __device__ __forceinline__ void restrict_all(T) {}
-    static __device__ __forceinline__ void solve(T length) {
-        if (threadIdx.x < SM_TEAM) SmV<T, 0, true, FROM_U>::run(length);
+    static __device__ __forceinline__ void restrict_all(const MgConst<T>&) {}
+    static __device__ __forceinline__ void solve(const MgConst<T>& mc) {
+        if (threadIdx.x < Team<0>::size) SmV<T, 0, true, FROM_U>::run(mc);
     }
 };
 /* full multigrid at level L, right-hand side f, into u (one CTA) */
 template <class T, int L>
-__device__ __forceinline__ void sm_fmg(const T* f, T* u, T length) {
-    sm_clear<T>();
-    sm_load_f<T, L>(f, length, false);
-    SmF<T, L>::restrict_all(length);
-    SmF<T, L>::solve(length);
+__device__ __forceinline__ void sm_fmg(const T* f, T* u, const MgConst<T>& mc) {
+    sm_load_f<T, L>(f, mc, false);
+    SmF<T, L>::restrict_all(mc);
+    SmF<T, L>::solve(mc);
     __syncthreads();
     sm_store_u<T, L>(u);
 }
 /* one V-cycle from 0 at level L, right-hand side f, into u (one CTA) */
 template <class T, int L>
-__device__ __forceinline__ void sm_vcycle0(const T* f, T* u, T length) {
-    sm_clear<T>();
-    sm_load_f<T, L>(f, length, true);
-    if (L >= SM_TOP) {
-        SmV<T, L, true, FROM_ZERO>::run(length);
-    } else {
-        if (threadIdx.x < SM_TEAM) SmV<T, L, true, FROM_ZERO>::run(length);
-        __syncthreads();
-    }
+__device__ __forceinline__ void sm_vcycle0(const T* f, T* u, const MgConst<T>& mc) {
+    sm_load_f<T, L>(f, mc, true);
+    if (threadIdx.x < Team<L>::size) SmV<T, L, true, FROM_ZERO>::run(mc);
+    __syncthreads();
     sm_store_u<T, L>(u);
 }
 
@@ -360,13 +373,12 @@ struct Tile {
  * from 0) of the tile into w, and the half-weighted residual into rc    */
 template <class T, int M, int N, int START, int THREADS>
 __device__ __forceinline__ void tile_down(const T* u, const T* uc, const T* f, T* w, T* rc, int n, int ic0, int jc0,
-                                          T length) {
+                                          T h2, T h2i) {
     using L = Tile<M, N>;
     T* const su = reinterpret_cast<T*>(mg_smem);
     T* const sf = su + L::UR * L::UC;
     T* const sr = sf + L::FR * L::FC;
     const int nc = n / 2 + 1;
-    const T h = length / (T)(n - 1), h2 = h * h, h2i = (T)1.0 / (h * h);
     const int iu = 2 * ic0 - 4, ju = 2 * jc0 - 4;
     /* black points from their source; walls 0; red points are written below */
 #pragma unroll 2
@@ -445,12 +457,11 @@ __device__ __forceinline__ void tile_down(const T* u, const T* uc, const T* f, T
 
 /* w plus the coarse correction vc, smoothed, into u */
 template <class T, int M, int N, int THREADS>
-__device__ __forceinline__ void tile_up(const T* w, const T* vc, const T* f, T* u, int n, int ic0, int jc0, T length) {
+__device__ __forceinline__ void tile_up(const T* w, const T* vc, const T* f, T* u, int n, int ic0, int jc0, T h2) {
     constexpr int UR = 2 * M + 4, UC = 2 * N + 4, FR = 2 * M + 2, FC = 2 * N + 2;
     T* const su = reinterpret_cast<T*>(mg_smem);
     T* const sf = su + UR * UC;
     const int nc = n / 2 + 1;
-    const T h = length / (T)(n - 1), h2 = h * h;
     const int iu = 2 * ic0 - 3, ju = 2 * jc0 - 3;
 #pragma unroll 2
     for (int t = threadIdx.x; t < UR * UC; t += THREADS) {
@@ -495,14 +506,16 @@ __device__ __forceinline__ void tile_up(const T* w, const T* vc, const T* f, T* 
 #define MG_N 16
 #define MG_THREADS 256
 template <class T, int START>
-__global__ void __launch_bounds__(MG_THREADS) k_mg_down(const T* u, const T* uc, const T* f, T* w, T* rc, int n, T length) {
+__global__ void __launch_bounds__(MG_THREADS) k_mg_down(const T* u, const T* uc, const T* f, T* w, T* rc, int n, T h2,
+                                                        T h2i) {
     pgb_pdl_entry();
-    tile_down<T, MG_M, MG_N, START, MG_THREADS>(u, uc, f, w, rc, n, 1 + MG_M * blockIdx.y, 1 + MG_N * blockIdx.x, length);
+    tile_down<T, MG_M, MG_N, START, MG_THREADS>(u, uc, f, w, rc, n, 1 + MG_M * blockIdx.y, 1 + MG_N * blockIdx.x, h2,
+                                               h2i);
 }
 template <class T>
-__global__ void __launch_bounds__(MG_THREADS) k_mg_up(const T* w, const T* vc, const T* f, T* u, int n, T length) {
+__global__ void __launch_bounds__(MG_THREADS) k_mg_up(const T* w, const T* vc, const T* f, T* u, int n, T h2) {
     pgb_pdl_entry();
-    tile_up<T, MG_M, MG_N, MG_THREADS>(w, vc, f, u, n, 1 + MG_M * blockIdx.y, 1 + MG_N * blockIdx.x, length);
+    tile_up<T, MG_M, MG_N, MG_THREADS>(w, vc, f, u, n, 1 + MG_M * blockIdx.y, 1 + MG_N * blockIdx.x, h2);
 }
 /* right-hand side of the coarser level (interior) */
 template <class T>
@@ -528,6 +541,7 @@ struct MgPtrs {
     T* v[PGB_MAX_LEVELS];
     T* r[PGB_MAX_LEVELS];
     T* w[PGB_MAX_LEVELS];
+    MgConst<T> c;
 };
 
 /* every CTA's global writes before are seen by every CTA's reads after */
@@ -540,90 +554,215 @@ __device__ __forceinline__ int cluster_rank() {
     return (int)r;
 }
 
-/* V-cycle of a cluster level L (5: 65 nodes, 6: 129): CTA c takes the
- * coarse rows from 1 + c M, M = 2^L / 16                                */
+/* The band of a CTA on level L: coarse rows ic0 = 1 + M rank ... and their
+ * fine rows 2 ic0 - 1 ..., whole rows, with the halo that makes the
+ * smoothing, the residual, the restriction and, later, the correction and
+ * its smoothing local.  It stays in shared memory from the way down to the
+ * way up; only the restricted residual, the coarse correction and the
+ * result go through global memory (L2).                                  */
+template <class T, int L>
+struct Band {
+    static constexpr int n = sm_n(L), N = 1 << L, M = N / CL_CTAS;
+    static constexpr int UR = 2 * M + 8;   /* u: rows 2 ic0 - 5 ...       */
+    static constexpr int GR = 2 * M + 6;   /* g: rows 2 ic0 - 4 ...       */
+    static constexpr int FR = 2 * M + 1;   /* f, residual: rows 2 ic0 - 1 ... */
+    static constexpr int WORDS = (UR + GR + 2 * FR) * n;
+    static constexpr int BASE = Sm<T>::WORDS + [] {
+        if constexpr (L > Cfg<T>::TOP + 1) return Band<T, L - 1>::END;
+        else return 0;
+    }();
+    static constexpr int END = BASE - Sm<T>::WORDS + WORDS;
+    static __device__ __forceinline__ T* u() { return smem<T>() + BASE; }
+    static __device__ __forceinline__ T* g() { return u() + UR * n; }
+    static __device__ __forceinline__ T* f() { return g() + GR * n; }
+    static __device__ __forceinline__ T* res() { return f() + FR * n; }
+};
+/* one colour on `rows` band rows from row i0: a row has N slots */
+template <class T, int L>
+__device__ __forceinline__ void band_sweep(int color, int i0, int rows, int iu) {
+    using B = Band<T, L>;
+    constexpr int n = B::n;
+    T* const u = B::u();
+    const T* const g = B::g();
+#pragma unroll 2
+    for (int t = threadIdx.x; t < rows << L; t += Cfg<T>::THREADS) {
+        const int i = i0 + (t >> L), j = 1 + ((i + 1 + color) & 1) + 2 * (t & (B::N - 1));
+        if (i > 0 && i < n - 1 && j < n - 1) {
+            const int k = (i - iu) * n + j;
+            u[k] = gs_value(u[k + n], u[k - n], u[k + 1], u[k - 1], g[k - n]);
+        }
+    }
+    __syncthreads();
+}
+/* V-cycle of level L.  u, f: the level's arrays; uc: the coarser solution
+ * (FROM_COARSE).                                                         */
 template <class T, int L, int START>
-__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* u, const T* f, const T* uc, T length);
+__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* u, const T* f, const T* uc);
 template <class T, int L>
 struct ClLower {
-    static __device__ __forceinline__ void run(const MgPtrs<T>& p, T length) {
-        cl_vcycle<T, L, FROM_ZERO>(p, p.v[L], p.r[L], nullptr, length);
-    }
-};
-template <class T>
-struct ClLower<T, SM_TOP> {
-    static __device__ __forceinline__ void run(const MgPtrs<T>& p, T length) {
-        if (cluster_rank() == 0) sm_vcycle0<T, SM_TOP>(p.r[SM_TOP], p.v[SM_TOP], length);
-        cluster_sync();
+    static __device__ __forceinline__ void run(const MgPtrs<T>& p) {
+        if constexpr (L > Cfg<T>::TOP) {
+            cl_vcycle<T, L, FROM_ZERO>(p, p.v[L], p.r[L], nullptr);
+        } else {
+            if (cluster_rank() == 0) sm_vcycle0<T, L>(p.r[L], p.v[L], p.c);
+            cluster_sync();
+        }
     }
 };
 template <class T, int L, int START>
-__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* u, const T* f, const T* uc, T length) {
-    constexpr int M = (1 << L) / CL_CTAS, N = 1 << L;
-    const int ic0 = 1 + M * cluster_rank();
-    tile_down<T, M, N, START, SM_THREADS>(u, uc, f, p.w[L], p.r[L - 1], sm_n(L), ic0, 1, length);
+__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* gu, const T* gf, const T* uc) {
+    using B = Band<T, L>;
+    constexpr int n = B::n, N = B::N, M = B::M, nc = sm_n(L - 1), TH = Cfg<T>::THREADS;
+    const int ic0 = 1 + M * cluster_rank(), iu = 2 * ic0 - 5;
+    const T h2 = p.c.h2[L], h2i = p.c.h2i[L];
+    T* const su = B::u();
+    T* const sg = B::g();
+    T* const sf = B::f();
+    T* const sr = B::res();
+    /* the walls, then the black points from their source (a correction: 0) */
+    for (int t = threadIdx.x; t < B::UR; t += TH) su[t * n] = su[t * n + n - 1] = (T)0;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < B::UR << L; t += TH) {
+        const int a = t >> L, i = iu + a, c = 2 * (t & (N - 1)) + 1, j = c + (i & 1);
+        T v = (T)0;
+        if (START != FROM_ZERO && i > 0 && i < n - 1 && j < n - 1) {
+            if (START == FROM_U) v = __ldcg(gu + i * n + j);
+            else {
+                int k1, k0;
+                black_pair(i, j, nc, k1, k0);
+                v = down_pow2<1>(__ldcg(uc + k1) + __ldcg(uc + k0));
+            }
+        }
+        if (j < n - 1) su[a * n + j] = v;
+        /* a wall row's red points are read as 0 too */
+        const int jr = c + ((i + 1) & 1);
+        if ((i <= 0 || i >= n - 1) && jr < n - 1) su[a * n + jr] = (T)0;
+    }
+    /* g on the red region, f where residuals are taken; a correction's red
+     * points start from g                                                */
+#pragma unroll 4
+    for (int t = threadIdx.x; t < B::GR << (L + 1); t += TH) {
+        const int a = t >> (L + 1), j = t & (2 * N - 1), i = iu + 1 + a;
+        if (i > 0 && i < n - 1 && j > 0) {
+            const T v = __ldcg(gf + i * n + j), g = h2 * v;
+            sg[a * n + j] = g;
+            const int b = a - 3;
+            if (b >= 0 && b < B::FR) sf[b * n + j] = v;
+            if (START == FROM_ZERO && ((i + j) & 1) == 0) su[(a + 1) * n + j] = red_from_zero(g);
+        }
+    }
+    __syncthreads();
+    if (START != FROM_ZERO) band_sweep<T, L>(0, iu + 1, B::GR, iu);
+    band_sweep<T, L>(1, iu + 2, B::GR - 2, iu);
+    /* residuals: even rows 2 ic0 ... whole, odd rows at even columns */
+#pragma unroll 2
+    for (int t = threadIdx.x; t < (M << (L + 1)) + ((M + 1) << L); t += TH) {
+        const int s = t - (M << (L + 1));
+        const int b = s < 0 ? 2 * (t >> (L + 1)) + 1 : 2 * (s >> L);
+        const int j = s < 0 ? t & (2 * N - 1) : 2 * (s & (N - 1));
+        const int i = iu + 4 + b;
+        if (j > 0 && i < n - 1) {
+            const int k = (b + 4) * n + j;
+            sr[b * n + j] = resid_value(su[k + n], su[k - n], su[k + 1], su[k - 1], su[k], sf[b * n + j], h2i);
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < M << L; t += TH) {
+        const int a = t >> L, jc = t & (N - 1), ic = ic0 + a;
+        if (jc > 0 && ic < nc - 1) {
+            const T* const r = sr + (2 * a + 1) * n + 2 * jc;
+            p.r[L - 1][ic * nc + jc] = half_weight(r[0], r[n], r[-n], r[1], r[-1]);
+        }
+    }
     cluster_sync();
-    ClLower<T, L - 1>::run(p, length);
-    tile_up<T, M, N, SM_THREADS>(p.w[L], p.v[L - 1], f, u, sm_n(L), ic0, 1, length);
+    ClLower<T, L - 1>::run(p);
+    /* the correction of the black points, then a sweep */
+    const T* const vc = p.v[L - 1];
+#pragma unroll 4
+    for (int t = threadIdx.x; t < (2 * M + 4) << L; t += TH) {
+        const int a = t >> L, i = iu + 2 + a, j = 1 + (i & 1) + 2 * (t & (N - 1));
+        if (i > 0 && i < n - 1 && j < n - 1) {
+            int k1, k0;
+            black_pair(i, j, nc, k1, k0);
+            T& x = su[(a + 2) * n + j];
+            x = fma_t((T)0.5, __ldcg(vc + k1) + __ldcg(vc + k0), x);
+        }
+    }
+    __syncthreads();
+    band_sweep<T, L>(0, iu + 3, 2 * M + 2, iu);
+    band_sweep<T, L>(1, iu + 4, 2 * M, iu);
+    for (int t = threadIdx.x; t < (2 * M) << (L + 1); t += TH) {
+        const int a = t >> (L + 1), j = t & (2 * N - 1), i = iu + 4 + a;
+        if (j > 0 && i < n - 1) gu[i * n + j] = su[(a + 4) * n + j];
+    }
     cluster_sync();
 }
-/* right-hand side of level L from level L+1, rows shared out */
+/* right-hand side of level L from level L+1, shared out */
 template <class T, int L>
 __device__ __forceinline__ void cl_restrict(const MgPtrs<T>& p) {
-    constexpr int n = sm_n(L), nf = sm_n(L + 1);
-    for (int k = threadIdx.x + SM_THREADS * cluster_rank(); k < n * n; k += SM_THREADS * CL_CTAS) {
-        const int i = k / n, j = k - i * n;
-        if (i > 0 && j > 0 && i < n - 1 && j < n - 1) {
+    constexpr int n = sm_n(L), nf = sm_n(L + 1), W = 2 << L, TH = Cfg<T>::THREADS;
+    for (int t = threadIdx.x + TH * cluster_rank(); t < W * W; t += TH * CL_CTAS) {
+        const int i = t >> (L + 1), j = t & (W - 1);
+        if (i > 0 && j > 0) {
             const T* const q = p.f[L + 1] + 2 * i * nf + 2 * j;
-            p.f[L][k] = half_weight(__ldcg(q), __ldcg(q + nf), __ldcg(q - nf), __ldcg(q + 1), __ldcg(q - 1));
+            p.f[L][i * n + j] = half_weight(__ldcg(q), __ldcg(q + nf), __ldcg(q - nf), __ldcg(q + 1), __ldcg(q - 1));
         }
     }
     cluster_sync();
 }
 template <class T, int L>
 struct ClF {
-    static __device__ __forceinline__ void run(const MgPtrs<T>& p, T length) {
-        cl_restrict<T, L - 1>(p);
-        ClF<T, L - 1>::run(p, length);
-        cl_vcycle<T, L, FROM_COARSE>(p, p.u[L], p.f[L], p.u[L - 1], length);
-        cl_vcycle<T, L, FROM_U>(p, p.u[L], p.f[L], nullptr, length);
-    }
-};
-template <class T>
-struct ClF<T, SM_TOP> {
-    static __device__ __forceinline__ void run(const MgPtrs<T>& p, T length) {
-        if (cluster_rank() == 0) sm_fmg<T, SM_TOP>(p.f[SM_TOP], p.u[SM_TOP], length);
-        cluster_sync();
+    static __device__ __forceinline__ void run(const MgPtrs<T>& p) {
+        if constexpr (L > Cfg<T>::TOP) {
+            cl_restrict<T, L - 1>(p);
+            ClF<T, L - 1>::run(p);
+            cl_vcycle<T, L, FROM_COARSE>(p, p.u[L], p.f[L], p.u[L - 1]);
+            cl_vcycle<T, L, FROM_U>(p, p.u[L], p.f[L], nullptr);
+        } else {
+            if (cluster_rank() == 0) sm_fmg<T, L>(p.f[L], p.u[L], p.c);
+            cluster_sync();
+        }
     }
 };
 
 /* FMG: full multigrid at level J from f[J] into u[J]; else one V-cycle
  * from 0 at level J on the right-hand side r[J] into v[J].  A cluster of
- * CL_CTAS CTAs for J > SM_TOP, one CTA otherwise.                        */
+ * CL_CTAS CTAs for J > TOP, one CTA otherwise.                           */
 template <class T, int J, bool FMG>
-__global__ void __launch_bounds__(SM_THREADS) k_mg_levels(MgPtrs<T> p, T length) {
+__global__ void __launch_bounds__(Cfg<T>::THREADS) k_mg_levels(const __grid_constant__ MgPtrs<T> p) {
     pgb_pdl_entry();
-    if constexpr (J > SM_TOP) {
-        if constexpr (FMG) ClF<T, J>::run(p, length);
-        else ClLower<T, J>::run(p, length);
+    if constexpr (J > Cfg<T>::TOP) {
+        if constexpr (FMG) ClF<T, J>::run(p);
+        else ClLower<T, J>::run(p);
     } else {
-        if constexpr (FMG) sm_fmg<T, J>(p.f[J], p.u[J], length);
-        else sm_vcycle0<T, J>(p.r[J], p.v[J], length);
+        if constexpr (FMG) sm_fmg<T, J>(p.f[J], p.u[J], p.c);
+        else sm_vcycle0<T, J>(p.r[J], p.v[J], p.c);
     }
 }
 
 /* ====================================================== host side */
 constexpr int CL_TOP = 6;   /* the finest level of k_mg_levels (129 nodes) */
-constexpr int mg_max(int a, int b) { return a > b ? a : b; }
 template <class T, int J>
 constexpr size_t levels_smem() {
-    return sizeof(T) * (J <= SM_TOP ? SM_WORDS
-                        : J == 5 ? mg_max(SM_WORDS, Tile<2, 32>::WORDS)
-                                 : mg_max(SM_WORDS, mg_max(Tile<2, 32>::WORDS, Tile<4, 64>::WORDS)));
+    if constexpr (J > Cfg<T>::TOP) return sizeof(T) * (Sm<T>::WORDS + Band<T, J>::END);
+    else return sizeof(T) * Sm<T>::WORDS;
 }
 template <class T>
 constexpr size_t tile_smem() { return sizeof(T) * Tile<MG_M, MG_N>::WORDS; }
 
+template <class T>
+MgConst<T> mg_const(const pgb_run* r) {
+    MgConst<T> c = {};
+    const T length = (T)r->p.xlength;
+    for (int l = 0; l < r->ng; ++l) {
+        const T h = length / (T)(r->mg_n[l] - 1);
+        c.h2[l] = h * h;
+        c.h2i[l] = (T)1.0 / (h * h);
+    }
+    const T h0 = (T)0.5 * length;
+    c.c0 = -h0 * h0;
+    return c;
+}
 template <class T>
 MgPtrs<T> mg_ptrs(pgb_run* r);
 template <>
@@ -632,6 +771,7 @@ MgPtrs<double> mg_ptrs<double>(pgb_run* r) {
     for (int l = 0; l < PGB_MAX_LEVELS; ++l) {
         p.u[l] = r->mg_u[l]; p.f[l] = r->mg_f[l]; p.v[l] = r->mg_v[l]; p.r[l] = r->mg_r[l]; p.w[l] = r->mg_w[l];
     }
+    p.c = mg_const<double>(r);
     return p;
 }
 template <>
@@ -640,6 +780,7 @@ MgPtrs<float> mg_ptrs<float>(pgb_run* r) {
     for (int l = 0; l < PGB_MAX_LEVELS; ++l) {
         p.u[l] = r->mg32_u[l]; p.f[l] = r->mg32_f[l]; p.v[l] = r->mg32_v[l]; p.r[l] = r->mg32_r[l]; p.w[l] = r->mg32_w[l];
     }
+    p.c = mg_const<float>(r);
     return p;
 }
 
@@ -647,15 +788,15 @@ template <class T, int J, bool FMG>
 cudaError_t levels_attr() {
     cudaError_t e = cudaFuncSetAttribute(k_mg_levels<T, J, FMG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)levels_smem<T, J>());
-    if (e == cudaSuccess && J > SM_TOP)
+    if (e == cudaSuccess && J > Cfg<T>::TOP)
         e = cudaFuncSetAttribute(k_mg_levels<T, J, FMG>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 template <class T, int J, bool FMG>
 int levels_go(pgb_run* r) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(J > SM_TOP ? CL_CTAS : 1);
-    cfg.blockDim = dim3(SM_THREADS);
+    cfg.gridDim = dim3(J > Cfg<T>::TOP ? CL_CTAS : 1);
+    cfg.blockDim = dim3(Cfg<T>::THREADS);
     cfg.dynamicSmemBytes = levels_smem<T, J>();
     cfg.stream = r->stream;
     cudaLaunchAttribute attr[2];
@@ -665,8 +806,8 @@ int levels_go(pgb_run* r) {
     attr[1].val.clusterDim.x = CL_CTAS;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = J > SM_TOP ? 2 : 1;
-    PGB_CK(r, cudaLaunchKernelEx(&cfg, k_mg_levels<T, J, FMG>, mg_ptrs<T>(r), (T)r->p.xlength));
+    cfg.numAttrs = J > Cfg<T>::TOP ? 2 : 1;
+    PGB_CK(r, cudaLaunchKernelEx(&cfg, k_mg_levels<T, J, FMG>, mg_ptrs<T>(r)));
     r->launches++;
     return 0;
 }
@@ -705,9 +846,8 @@ template <class T, int START>
 int vcycle(pgb_run* r, const MgPtrs<T>& p, int j, T* u, const T* f, const T* uc) {
     const int n = r->mg_n[j], nc = r->mg_n[j - 1];
     const dim3 grid((nc - 2 + MG_N - 1) / MG_N, (nc - 2 + MG_M - 1) / MG_M);
-    const T length = (T)r->p.xlength;
     PGB_CK(r, pgb_launch_pdl(k_mg_down<T, START>, grid, dim3(MG_THREADS), tile_smem<T>(), r->stream, (const T*)u, uc, f,
-                             p.w[j], p.r[j - 1], n, length));
+                             p.w[j], p.r[j - 1], n, p.c.h2[j], p.c.h2i[j]));
     r->launches++;
     if (j - 1 > CL_TOP) {
         if (vcycle<T, FROM_ZERO>(r, p, j - 1, p.v[j - 1], p.r[j - 1], nullptr)) return PGB_ERR_CUDA;
@@ -715,7 +855,7 @@ int vcycle(pgb_run* r, const MgPtrs<T>& p, int j, T* u, const T* f, const T* uc)
         return PGB_ERR_CUDA;
     }
     PGB_CK(r, pgb_launch_pdl(k_mg_up<T>, grid, dim3(MG_THREADS), tile_smem<T>(), r->stream, (const T*)p.w[j],
-                             (const T*)p.v[j - 1], f, u, n, length));
+                             (const T*)p.v[j - 1], f, u, n, p.c.h2[j]));
     r->launches++;
     return 0;
 }
