@@ -186,6 +186,7 @@ static int ensure_capacity(pgb_run* r, int s, long long need) {
         PGB_CK(r, cudaStreamSynchronize(r->stream));
         PGB_CK(r, cudaStreamSynchronize(r->copy_stream));
         if (r->side) PGB_CK(r, cudaStreamSynchronize(r->side));
+        if (r->ion) PGB_CK(r, cudaStreamSynchronize(r->ion));
         drop_graphs(r);
     }
     if (need > S.cap) {
@@ -336,18 +337,24 @@ extern "C" int pgb_create(const pgb_params* p, pgb_run** out) {
         }
     r->copy_ev_ok = true;
     if (const char* fa = std::getenv("PGB_FAULT_ALLOC")) r->fault_alloc = std::atoi(fa);
-    /* the side stream only speeds steps up: without it steps run in turn.
-     * It takes the highest priority, so that the field solve's short
-     * kernels get SMs ahead of queued blocks of the run's own stream.     */
-    int prio_lo = 0, prio_hi = 0;
-    if (cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) == cudaSuccess &&
-        cudaStreamCreateWithPriority(&r->side, cudaStreamNonBlocking, prio_hi) == cudaSuccess) {
-        r->prio_hi = prio_hi;
-        if (cudaEventCreateWithFlags(&r->ev_fork, cudaEventDisableTiming) == cudaSuccess) {
-            if (cudaEventCreateWithFlags(&r->ev_join, cudaEventDisableTiming) == cudaSuccess) r->side_ok = true;
-            else cudaEventDestroy(r->ev_fork);
+    /* the side streams only speed steps up: without them steps run in turn.
+     * The field solve's takes the highest priority, so that its short
+     * kernels get SMs ahead of queued blocks of the other two.            */
+    {
+        int prio_lo = 0, prio_hi = 0;
+        cudaEvent_t* const evs[5] = {&r->ev_fork, &r->ev_join, &r->ev_i0, &r->ev_i1, &r->ev_e0};
+        int made = 0;
+        if (cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) == cudaSuccess &&
+            cudaStreamCreateWithPriority(&r->side, cudaStreamNonBlocking, prio_hi) == cudaSuccess &&
+            cudaStreamCreateWithFlags(&r->ion, cudaStreamNonBlocking) == cudaSuccess)
+            while (made < 5 && cudaEventCreateWithFlags(evs[made], cudaEventDisableTiming) == cudaSuccess) ++made;
+        r->side_ok = made == 5;
+        if (!r->side_ok) {
+            for (int k = 0; k < made; ++k) cudaEventDestroy(*evs[k]);
+            if (r->side) cudaStreamDestroy(r->side);
+            if (r->ion) cudaStreamDestroy(r->ion);
+            r->side = r->ion = nullptr;
         }
-        if (!r->side_ok) { cudaStreamDestroy(r->side); r->side = nullptr; }
     }
     cudaGetLastError();
     const size_t G = (size_t)r->nx * r->ny, GE = (size_t)(r->nx + 1) * (r->ny + 1);
@@ -427,6 +434,7 @@ extern "C" int pgb_destroy(pgb_run* r) {
     if (!r) return 0;
     if (r->stream) cudaStreamSynchronize(r->stream);
     if (r->side) cudaStreamSynchronize(r->side);
+    if (r->ion) cudaStreamSynchronize(r->ion);
     drop_graphs(r);
     cudaFree(r->phi_tab);
     if (r->phi_host) cudaFreeHost(r->phi_host);
@@ -454,8 +462,10 @@ extern "C" int pgb_destroy(pgb_run* r) {
         for (int k = 0; k < 13; ++k) cudaEventDestroy(r->prof_ev[k]);
     if (r->copy_ev_ok)
         for (int k = 0; k < PGB_COPY_EVENTS; ++k) cudaEventDestroy(r->copy_ev[k]);
-    if (r->side_ok) { cudaEventDestroy(r->ev_fork); cudaEventDestroy(r->ev_join); }
+    if (r->side_ok)
+        for (cudaEvent_t e : {r->ev_fork, r->ev_join, r->ev_i0, r->ev_i1, r->ev_e0}) cudaEventDestroy(e);
     if (r->side) cudaStreamDestroy(r->side);
+    if (r->ion) cudaStreamDestroy(r->ion);
     if (r->copy_stream) cudaStreamDestroy(r->copy_stream);
     if (r->stream) cudaStreamDestroy(r->stream);
     delete r;
@@ -679,6 +689,7 @@ extern "C" int pgb_boundary(pgb_run* r, int which) {
     /* deposits made by wall events go to the accumulators of the step; in
      * the phase-by-phase form the charge is recomputed by pgb_deposit     */
     if ((rc = set_device_step(r, r->time_step, 1))) return rc;
+    r->charge_dirty = true;
     if ((rc = boundary_phase(r, which))) return rc;
     return sync_state(r);
 }
@@ -689,6 +700,7 @@ extern "C" int pgb_initial_boundary(pgb_run* r) {
     if (rc) return rc;
     /* random streams of the pre-loop boundary pass use step -1 */
     if ((rc = set_device_step(r, -1, 1))) return rc;
+    r->charge_dirty = true;
     rc = boundary_phase(r, PGB_BOUNDARY_IONS);
     if (!rc) rc = boundary_phase(r, PGB_BOUNDARY_ELECTRONS);
     if (rc) return rc;
@@ -748,6 +760,7 @@ extern "C" int pgb_deposit(pgb_run* r, int s) {
     if (!r || s < 0 || s > 1) return fail(r, PGB_ERR_ARG, "pgb_deposit: bad argument");
     int rc = need_particles(r);
     if (rc) return rc;
+    r->charge_dirty = true;
     PGB_CK(r, cudaMemsetAsync(r->qacc[s], 0, sizeof(unsigned long long) * r->nx * r->ny, r->stream));
     if (pgb_launch_deposit(r, s) || pgb_launch_finalize(r, 1 << s, false)) return PGB_ERR_CUDA;
     return sync_state(r);
@@ -776,6 +789,16 @@ extern "C" int pgb_efield(pgb_run* r) {
 }
 
 /* -------------------------------------------------------------- pgb_step */
+/* a step starts from zero charge accumulators and leaves them zero; the
+ * phase-by-phase calls leave their charge in them                        */
+static int clear_charge(pgb_run* r) {
+    if (!r->charge_dirty) return 0;
+    const size_t G = (size_t)r->nx * r->ny;
+    PGB_CK(r, cudaMemsetAsync(r->qacc[0], 0, sizeof(unsigned long long) * G, r->stream));
+    PGB_CK(r, cudaMemsetAsync(r->qacc[1], 0, sizeof(unsigned long long) * G, r->stream));
+    r->charge_dirty = false;
+    return 0;
+}
 /* event k marks the start of section k; event 5 the end of the step */
 #define PROF_MARK(r, k) \
     do { if ((r)->prof_on) PGB_CK((r), cudaEventRecord((r)->prof_ev[k], (r)->stream)); } while (0)
@@ -784,25 +807,63 @@ extern "C" int pgb_efield(pgb_run* r) {
  * (particle phases) and ds->tf (field solve) select the random streams
  * and the right-wall potential, so the same launches can be replayed as
  * CUDA graphs for every step.
- *   step_mcc:       e_collisions::collision (pic.cpp:1071-1075): collision
- *                   tests, scattering and the list of ionization events;
- *                   on an ion step, charge exchange of the ions present
- *                   (ion_collisions::collision, pic.cpp:1102-1104, which
- *                   reads only ions and comes before their push); reads
- *                   no field
- *   step_particles: charge reset, electron push and deposit, ionization
- *                   products, injection, charge exchange of the ions they
- *                   appended, ion push, walls, population control
- *                   (pic.cpp:1080-1141), then ds->t += 1
- *   step_fields:    charge finalisation, grid_rho, grid_potential,
- *                   grid_electric_field (pic.cpp:1143-1161), then ds->tf += 1
+ *   collisions (A):  e_collisions::collision (pic.cpp:1071-1075): collision
+ *                    tests, scattering and the list of ionization events;
+ *                    on an ion step, charge exchange of the ions present
+ *                    (ion_collisions::collision, pic.cpp:1102-1104, which
+ *                    reads only ions and comes before their push); reads
+ *                    no field
+ *   particles (B):   electron push and deposit, ionization products,
+ *                    injection, charge exchange of the ions they appended,
+ *                    ion push, walls, population control
+ *                    (pic.cpp:1080-1141), then ds->t += 1
+ *   fields (F):      charge finalisation (which leaves the accumulators
+ *                    zero for the next step), grid_rho, grid_potential,
+ *                    grid_electric_field (pic.cpp:1143-1161), then
+ *                    ds->tf += 1
  * Run in this order they are the reference's step.  The collisions of step
  * t+1 need the particles after step t's walls, not step t's fields, so the
  * pipelined path (issue_one_step) runs them while step t's field solve is
- * still in flight on the run's side stream.                              */
-static int mcc_part(pgb_run* r, int leave_sms, bool ion_step) {
+ * still in flight on the run's side stream.
+ *
+ * Within A and B the electrons and the ions meet in few places: ionization
+ * products that are stored (appended to both species, ions at their parent
+ * electron's new position), electrons emitted by ion impact (appended
+ * before the electron walls'), and the end of the step.  Everything else
+ * touches one species' particles, counters, lists and charge, so the ions'
+ * kernels run on a stream of their own beside the electrons' (Lanes), with
+ * an event at each of those places: the short kernels between the large
+ * ones, and in small runs the large ones too, then overlap.              */
+struct Lanes {
+    pgb_run* r;
+    cudaStream_t e, i;   /* i == e: one after the other, in the order issued */
+    explicit Lanes(pgb_run* run, bool beside) : r(run), e(run->stream), i(beside ? run->ion : run->stream) {}
+    ~Lanes() { r->stream = e; }
+    void electrons() { r->stream = e; }   /* later launches go to this lane */
+    void ions() { r->stream = i; }
+    /* what is queued on `from` comes before what follows on `to` */
+    int order(cudaStream_t from, cudaStream_t to, cudaEvent_t ev) {
+        if (from == to) return 0;
+        PGB_CK(r, cudaEventRecord(ev, from));
+        PGB_CK(r, cudaStreamWaitEvent(to, ev, 0));
+        return 0;
+    }
+    int fork() { return order(e, i, r->ev_i0); }
+    int join() { return order(i, e, r->ev_i1); }
+    int ions_after_electrons() { return order(e, i, r->ev_e0); }
+};
+/* the ionization products are stored (so the event list is read) only with
+ * steady-state walls or off ion steps: absorbing walls remove them in the
+ * same step, so that else only their number counts                       */
+static bool products_stored(const pgb_run* r, bool ion_step) {
+    return r->p.have_collisions && (r->p.steadystate || !ion_step);
+}
+static int collide_lanes(Lanes& L, int leave_sms, bool ion_step) {
+    pgb_run* const r = L.r;
     if (!r->p.have_collisions) return 0;
-    if (pgb_launch_mcc(r, leave_sms)) return PGB_ERR_CUDA;
+    L.electrons();
+    const bool products = products_stored(r, ion_step);
+    if (pgb_launch_mcc(r, leave_sms, !products)) return PGB_ERR_CUDA;
     PROF_MARK(r, 9);
     /* the field solve beside the collisions ends before the collision test
      * does (0.11 against 0.15 ms at 513^2): the kernels after the test take
@@ -810,74 +871,86 @@ static int mcc_part(pgb_run* r, int leave_sms, bool ion_step) {
      * higher priority, when it has not ended)                             */
     if (pgb_launch_scatter(r, 0)) return PGB_ERR_CUDA;
     PROF_MARK(r, 10);
-    /* the ionization products are stored (so the event list is read) only
-     * with steady-state walls or off ion steps; else only their number is */
-    const bool products = r->p.steadystate || !ion_step;
-    if (pgb_build_list(r, LIST_ION_EV, 0, !products)) return PGB_ERR_CUDA;
+    if (products && pgb_build_list(r, LIST_ION_EV, 0)) return PGB_ERR_CUDA;
     PROF_MARK(r, 11);
+    L.ions();
     if (ion_step && pgb_launch_cx(r, 0, 0)) return PGB_ERR_CUDA;
+    L.electrons();
     PROF_MARK(r, 12);
     return 0;
 }
-static int step_mcc(pgb_run* r, bool ion_step) { return mcc_part(r, 0, ion_step); }
-/* beside a field solve, which needs SMs of its own (r->tune_field_sms) */
-static int step_mcc_beside(pgb_run* r, bool ion_step) { return mcc_part(r, r->tune_field_sms, ion_step); }
 
-static int step_particles(pgb_run* r, bool ion_step) {
-    const bool coll = r->p.have_collisions != 0;
+/* no species can exceed its reduction limit: no host decision in a step */
+static bool no_reduction(const pgb_run* r) {
+    return r->p.steadystate || (r->sp[0].cap <= r->p.size_to_check_e && r->sp[1].cap <= r->p.size_to_check_i);
+}
+
+static int particles_lanes(Lanes& L, bool ion_step) {
+    pgb_run* const r = L.r;
     const size_t G = (size_t)r->nx * r->ny;
-    PGB_CK(r, cudaMemsetAsync(r->qacc[0], 0, sizeof(unsigned long long) * G, r->stream));
-    PGB_CK(r, cudaMemsetAsync(r->qacc[1], 0, sizeof(unsigned long long) * G, r->stream));
+    const bool products = products_stored(r, ion_step), inject = r->p.number_to_inject > 0;
+    /* where the products' number is entered: with the injection, else with
+     * the wall lists (both come before the walls take new ids)            */
+    const int commit_e = r->p.have_collisions && !products ? 1 : 0, commit_i = 2 * commit_e;
     /* get_particle_electric_field + move_particles, charge deposit */
+    L.electrons();
     PROF_MARK(r, 8);
     if (pgb_launch_push(r, 0, true)) return PGB_ERR_CUDA;
     PROF_MARK(r, 7);
-    if (pgb_build_list(r, LIST_OUT_E, 0)) return PGB_ERR_CUDA;
+    if (pgb_build_list(r, LIST_OUT_E, 0, inject ? 0 : commit_e)) return PGB_ERR_CUDA;
     PROF_MARK(r, 1);
-    if (coll) {
+    if (products) {
         /* the ionization products join after the push: an ion takes its
          * parent electron's new position                                */
-        int store_e = r->p.steadystate ? 1 : 0;
-        int store_i = (r->p.steadystate || !ion_step) ? 1 : 0;
-        if (pgb_launch_ionize_appends(r, store_e, store_i)) return PGB_ERR_CUDA;
+        if (pgb_launch_ionize_appends(r, r->p.steadystate ? 1 : 0, 1) || L.ions_after_electrons()) return PGB_ERR_CUDA;
     }
     /* inject_more_particles: electrons are pushed as they are created */
-    if (r->p.number_to_inject > 0 && pgb_launch_inject(r, 3, true)) return PGB_ERR_CUDA;
+    if (inject && pgb_launch_inject(r, 1, true, commit_e)) return PGB_ERR_CUDA;
+    L.ions();
+    if (inject && pgb_launch_inject(r, 2, true, commit_i)) return PGB_ERR_CUDA;
     PROF_MARK(r, 2);
     if (ion_step) {
         /* charge exchange of the ions appended since the collision pass:
          * without steady-state re-insertion only the injected ones (the
          * ionization products of an ion step are not stored), one block  */
-        const bool appended = r->p.number_to_inject > 0 || r->p.steadystate;
+        const bool appended = inject || r->p.steadystate;
         const bool few = !r->p.steadystate && r->p.number_to_inject <= 4096;
-        if (coll && appended && pgb_launch_cx(r, few ? 2 : 1, 0)) return PGB_ERR_CUDA;
+        if (r->p.have_collisions && appended && pgb_launch_cx(r, few ? 2 : 1, 0)) return PGB_ERR_CUDA;
         PROF_MARK(r, 3);
         if (pgb_launch_push(r, 1, true)) return PGB_ERR_CUDA;
-        if (pgb_build_list(r, LIST_OUT_I, 1)) return PGB_ERR_CUDA;
+        if (pgb_build_list(r, LIST_OUT_I, 1, inject ? 0 : commit_i)) return PGB_ERR_CUDA;
         PROF_MARK(r, 4);
+        /* electrons emitted by ion impact join after the injected ones */
+        const bool emits = r->p.species == PGB_ARGON && r->p.ion_impact_see;
+        if (emits) {
+            if (L.join()) return PGB_ERR_CUDA;
+            L.electrons();
+        }
         if (pgb_launch_walls(r, PGB_BOUNDARY_IONS)) return PGB_ERR_CUDA;
-        if (pgb_launch_walls(r, PGB_BOUNDARY_ELECTRONS)) return PGB_ERR_CUDA;
+        if (!emits && L.join()) return PGB_ERR_CUDA;
     } else {
         PROF_MARK(r, 3);
         if (pgb_launch_deposit(r, 1)) return PGB_ERR_CUDA;
         if (r->p.steadystate && (pgb_launch_flag_outside(r, 1) || pgb_build_list(r, LIST_OUT_I, 1))) return PGB_ERR_CUDA;
         PROF_MARK(r, 4);
-        if (pgb_launch_walls(r, PGB_BOUNDARY_ELECTRONS)) return PGB_ERR_CUDA;
+        if (L.join()) return PGB_ERR_CUDA;
     }
+    L.electrons();
+    const bool reduce = !no_reduction(r);
+    if (pgb_launch_walls(r, PGB_BOUNDARY_ELECTRONS, !reduce)) return PGB_ERR_CUDA;
+    if (!reduce) return 0;
     /* contain_particle_growth: only when a species can exceed its limit */
-    if (!r->p.steadystate) {
-        for (int s = 0; s < 2; ++s) {
-            long long lim = s == 0 ? r->p.size_to_check_e : r->p.size_to_check_i;
-            if (r->sp[s].cap > lim) {
-                int rc = sync_state(r);
-                if (rc) return rc;
-                if (r->hs->n[s] - r->hs->dead[s] > lim) {
-                    if ((rc = pgb_launch_reduce(r, s))) return rc;
-                    /* the reduction changes weights: rebuild both charges */
-                    PGB_CK(r, cudaMemsetAsync(r->qacc[0], 0, sizeof(unsigned long long) * G, r->stream));
-                    PGB_CK(r, cudaMemsetAsync(r->qacc[1], 0, sizeof(unsigned long long) * G, r->stream));
-                    if (pgb_launch_deposit(r, 0) || pgb_launch_deposit(r, 1)) return PGB_ERR_CUDA;
-                }
+    for (int s = 0; s < 2; ++s) {
+        long long lim = s == 0 ? r->p.size_to_check_e : r->p.size_to_check_i;
+        if (r->sp[s].cap > lim) {
+            int rc = sync_state(r);
+            if (rc) return rc;
+            if (r->hs->n[s] - r->hs->dead[s] > lim) {
+                if ((rc = pgb_launch_reduce(r, s))) return rc;
+                /* the reduction changes weights: rebuild both charges */
+                PGB_CK(r, cudaMemsetAsync(r->qacc[0], 0, sizeof(unsigned long long) * G, r->stream));
+                PGB_CK(r, cudaMemsetAsync(r->qacc[1], 0, sizeof(unsigned long long) * G, r->stream));
+                if (pgb_launch_deposit(r, 0) || pgb_launch_deposit(r, 1)) return PGB_ERR_CUDA;
             }
         }
     }
@@ -887,19 +960,57 @@ static int step_particles(pgb_run* r, bool ion_step) {
 static int step_fields(pgb_run* r, bool) {
     /* collect_charge edge doubling, grid_rho, grid_potential, grid_electric_field */
     PROF_MARK(r, 5);
-    if (pgb_launch_finalize(r, 3, true)) return PGB_ERR_CUDA;
+    if (pgb_launch_finalize(r, 3, true, true)) return PGB_ERR_CUDA;
     if (pgb_poisson_solve(r)) return PGB_ERR_CUDA;
     if (pgb_launch_efield(r, 1)) return PGB_ERR_CUDA;
     PROF_MARK(r, 6);
     return 0;
 }
 
+/* A and B for capture, the species beside each other */
+static int step_collide(pgb_run* r, bool ion_step) {
+    Lanes L(r, true);
+    return L.fork() || collide_lanes(L, r->tune_field_sms, ion_step) || L.join() ? PGB_ERR_CUDA : 0;
+}
+static int step_particles(pgb_run* r, bool ion_step) {
+    Lanes L(r, true);
+    if (L.fork()) return PGB_ERR_CUDA;
+    return particles_lanes(L, ion_step);
+}
+/* F of the previous step, A and B for capture.  An ion kernel of B waits for
+ * F and for the ions' part of A only.                                    */
+static int step_merged(pgb_run* r, bool ion_step) {
+    Lanes L(r, true);
+    PGB_CK(r, cudaEventRecord(r->ev_fork, L.e));
+    PGB_CK(r, cudaStreamWaitEvent(r->side, r->ev_fork, 0));
+    PGB_CK(r, cudaStreamWaitEvent(L.i, r->ev_fork, 0));
+    r->stream = r->side;
+    if (step_fields(r, ion_step)) return PGB_ERR_CUDA;
+    L.electrons();
+    if (collide_lanes(L, r->tune_field_sms, ion_step)) return PGB_ERR_CUDA;
+    /* the ions' injection takes its ids after the ionization events' */
+    if (r->p.have_collisions && L.ions_after_electrons()) return PGB_ERR_CUDA;
+    PGB_CK(r, cudaEventRecord(r->ev_join, r->side));
+    PGB_CK(r, cudaStreamWaitEvent(L.e, r->ev_join, 0));
+    PGB_CK(r, cudaStreamWaitEvent(L.i, r->ev_join, 0));
+    return particles_lanes(L, ion_step);
+}
+
+/* one after the other: profiling, and steps that may reduce a species */
 static int step_once(pgb_run* r, bool ion_step) {
     PROF_MARK(r, 0);
-    int rc;
-    if ((rc = step_mcc(r, ion_step)) || (rc = step_particles(r, ion_step)) || (rc = step_fields(r, ion_step)))
-        return rc;
-    return 0;
+    {
+        Lanes L(r, false);
+        if (collide_lanes(L, 0, ion_step)) return PGB_ERR_CUDA;
+        const int rc = particles_lanes(L, ion_step);
+        if (rc) return rc;
+    }
+    return step_fields(r, ion_step);
+}
+/* collisions off: no A, so F follows B in the same graph */
+static int step_beside(pgb_run* r, bool ion_step) {
+    if (step_particles(r, ion_step)) return PGB_ERR_CUDA;
+    return step_fields(r, ion_step);
 }
 
 /* add the section times of the step just queued (waits for it) */
@@ -933,25 +1044,18 @@ static void drop_graphs(pgb_run* r) {
         if (r->graph_a[k]) { cudaGraphExecDestroy(r->graph_a[k]); r->graph_a[k] = nullptr; }
         if (r->graph_b[k]) { cudaGraphExecDestroy(r->graph_b[k]); r->graph_b[k] = nullptr; }
         if (r->graph_m[k]) { cudaGraphExecDestroy(r->graph_m[k]); r->graph_m[k] = nullptr; }
-        if (r->tmpl_a[k]) { cudaGraphDestroy(r->tmpl_a[k]); r->tmpl_a[k] = nullptr; }
-        if (r->tmpl_b[k]) { cudaGraphDestroy(r->tmpl_b[k]); r->tmpl_b[k] = nullptr; }
     }
     if (r->graph_f) { cudaGraphExecDestroy(r->graph_f); r->graph_f = nullptr; }
-    if (r->tmpl_f) { cudaGraphDestroy(r->tmpl_f); r->tmpl_f = nullptr; }
 }
 
 /* graphs are usable when no step needs a host decision: no profiling and
  * no species that could reach its reduction limit                       */
 static bool graphs_ok(pgb_run* r) {
-    if (!r->use_graphs || r->prof_on) return false;
-    if (!r->p.steadystate && (r->sp[0].cap > r->p.size_to_check_e || r->sp[1].cap > r->p.size_to_check_i)) return false;
-    return true;
+    return r->use_graphs && !r->prof_on && no_reduction(r);
 }
 
-/* capture fn(r, ion_step) as a graph; -1 if the launches cannot be captured.
- * keep: where to keep the captured template (else it is destroyed)     */
-static int capture(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGraphExec_t* out, long long* nl,
-                   cudaGraph_t* keep = nullptr) {
+/* capture fn(r, ion_step) as a graph; -1 if the launches cannot be captured */
+static int capture(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGraphExec_t* out, long long* nl) {
     cudaGraph_t g = nullptr;
     PGB_CK(r, cudaStreamBeginCapture(r->stream, cudaStreamCaptureModeThreadLocal));
     long long l0 = r->launches;
@@ -966,12 +1070,7 @@ static int capture(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGra
     *nl = r->launches - l0;
     r->launches = l0;
     e = cudaGraphInstantiate(out, g, 0);
-    if (keep && e == cudaSuccess) {
-        if (*keep) cudaGraphDestroy(*keep);
-        *keep = g;
-    } else {
-        cudaGraphDestroy(g);
-    }
+    cudaGraphDestroy(g);
     if (e != cudaSuccess) {
         cudaGetLastError();
         *out = nullptr;
@@ -982,9 +1081,8 @@ static int capture(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGra
 
 /* run fn as graph *slot (captured on first use), or launch it directly
  * when graphs are off or cannot be captured                            */
-static int replay(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGraphExec_t* slot, long long* nl,
-                  cudaGraph_t* keep = nullptr) {
-    if (graphs_ok(r) && !*slot && capture(r, fn, ion_step, slot, nl, keep)) r->use_graphs = 0;
+static int replay(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGraphExec_t* slot, long long* nl) {
+    if (graphs_ok(r) && !*slot && capture(r, fn, ion_step, slot, nl)) r->use_graphs = 0;
     if (!*slot || !graphs_ok(r)) return fn(r, ion_step);
     PGB_CK(r, cudaGraphLaunch(*slot, r->stream));
     r->launches += *nl;
@@ -995,6 +1093,8 @@ static int graph_key(pgb_run* r, bool ion_step) { return (ion_step ? 4 : 0) | (r
 
 static int launch_step(pgb_run* r, bool ion_step) {
     const int key = graph_key(r, ion_step);
+    if (r->side_ok && graphs_ok(r) && !r->p.have_collisions)
+        return replay(r, step_beside, ion_step, &r->graph[key], &r->graph_launches[key]);
     return replay(r, step_once, ion_step, &r->graph[key], &r->graph_launches[key]);
 }
 
@@ -1002,7 +1102,7 @@ static int launch_step(pgb_run* r, bool ion_step) {
 static int flush_fields(pgb_run* r) {
     if (!r->fields_pending) return 0;
     r->fields_pending = false;
-    return replay(r, step_fields, false, &r->graph_f, &r->graph_f_launches, &r->tmpl_f);
+    return replay(r, step_fields, false, &r->graph_f, &r->graph_f_launches);
 }
 
 /* pipelining needs collisions to overlap and graphs to replay the parts */
@@ -1024,55 +1124,13 @@ static bool host_work_due(pgb_run* r) {
     return false;
 }
 
-/* The pipelined step as one graph launch: the previous step's field solve
- * (F, its kernels at the side stream's top priority) beside this step's
- * collisions (A), then the other particle phases (B), built once per key
- * from the captured templates.  0: launched; 1: not available (graphs off
- * or a capture failed), use the separate graphs.                         */
+/* The pipelined step as one graph launch, captured once per key
+ * (step_merged).  0: launched; 1: not available, use the separate graphs. */
 static int launch_merged(pgb_run* r, bool ion_step) {
     const int key = graph_key(r, ion_step);
-    if (!r->graph_m[key]) {
-        if (!r->graph_f && capture(r, step_fields, false, &r->graph_f, &r->graph_f_launches, &r->tmpl_f)) return 1;
-        if (!r->graph_a[key] &&
-            capture(r, step_mcc_beside, ion_step, &r->graph_a[key], &r->graph_a_launches[key], &r->tmpl_a[key]))
-            return 1;
-        if (!r->graph_b[key] &&
-            capture(r, step_particles, ion_step, &r->graph_b[key], &r->graph_b_launches[key], &r->tmpl_b[key]))
-            return 1;
-        if (!r->tmpl_f || !r->tmpl_a[key] || !r->tmpl_b[key]) return 1;
-        /* F's kernels at the top priority, as on the side stream */
-        size_t nn = 0;
-        if (cudaGraphGetNodes(r->tmpl_f, nullptr, &nn) != cudaSuccess) return 1;
-        std::vector<cudaGraphNode_t> nodes(nn);
-        if (nn && cudaGraphGetNodes(r->tmpl_f, nodes.data(), &nn) != cudaSuccess) return 1;
-        for (cudaGraphNode_t nd : nodes) {
-            cudaGraphNodeType t;
-            if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) {
-                cudaLaunchAttributeValue v = {};
-                v.priority = r->prio_hi;
-                cudaGraphKernelNodeSetAttribute(nd, cudaLaunchAttributePriority, &v);
-            }
-        }
-        cudaGetLastError();
-        cudaGraph_t g = nullptr;
-        cudaGraphNode_t nf, na, nb;
-        bool ok = cudaGraphCreate(&g, 0) == cudaSuccess &&
-                  cudaGraphAddChildGraphNode(&nf, g, nullptr, 0, r->tmpl_f) == cudaSuccess &&
-                  cudaGraphAddChildGraphNode(&na, g, nullptr, 0, r->tmpl_a[key]) == cudaSuccess;
-        if (ok) {
-            cudaGraphNode_t deps[2] = {nf, na};
-            ok = cudaGraphAddChildGraphNode(&nb, g, deps, 2, r->tmpl_b[key]) == cudaSuccess &&
-                 cudaGraphInstantiate(&r->graph_m[key], g, 0) == cudaSuccess;
-        }
-        if (g) cudaGraphDestroy(g);
-        if (!ok) {
-            cudaGetLastError();
-            r->graph_m[key] = nullptr;
-            return 1;
-        }
-    }
+    if (!r->graph_m[key] && capture(r, step_merged, ion_step, &r->graph_m[key], &r->graph_m_launches[key])) return 1;
     PGB_CK(r, cudaGraphLaunch(r->graph_m[key], r->stream));
-    r->launches += r->graph_f_launches + r->graph_a_launches[key] + r->graph_b_launches[key];
+    r->launches += r->graph_m_launches[key];
     return 0;
 }
 
@@ -1089,7 +1147,7 @@ static int issue_one_step(pgb_run* r) {
     }
     if (!merged && r->fields_pending) {
         if (pipe && !r->graph_f &&
-            capture(r, step_fields, false, &r->graph_f, &r->graph_f_launches, &r->tmpl_f))
+            capture(r, step_fields, false, &r->graph_f, &r->graph_f_launches))
             r->use_graphs = 0;
         if (pipe && r->graph_f && pipelined(r)) {
             PGB_CK(r, cudaEventRecord(r->ev_fork, r->stream));
@@ -1142,11 +1200,9 @@ static int issue_one_step(pgb_run* r) {
         /* A and B went with F in the step graph */
     } else if (pipe || forked) {
         const int key = graph_key(r, ion_step);
-        if ((rc = replay(r, step_mcc_beside, ion_step, &r->graph_a[key], &r->graph_a_launches[key], &r->tmpl_a[key])))
-            return rc;
+        if ((rc = replay(r, step_collide, ion_step, &r->graph_a[key], &r->graph_a_launches[key]))) return rc;
         if (forked) PGB_CK(r, cudaStreamWaitEvent(r->stream, r->ev_join, 0));
-        if ((rc = replay(r, step_particles, ion_step, &r->graph_b[key], &r->graph_b_launches[key], &r->tmpl_b[key])))
-            return rc;
+        if ((rc = replay(r, step_particles, ion_step, &r->graph_b[key], &r->graph_b_launches[key]))) return rc;
         r->fields_pending = true;
     } else {
         if ((rc = launch_step(r, ion_step))) return rc;
@@ -1171,7 +1227,7 @@ extern "C" int pgb_step(pgb_run* r, int32_t nsteps) {
     int done = 0;
     while (done < nsteps) {
         int chunk = std::min<int>(nsteps - done, (int)r->phi_tab_cap);
-        if ((rc = set_device_step(r, r->time_step, chunk))) return rc;
+        if ((rc = set_device_step(r, r->time_step, chunk)) || (rc = clear_charge(r))) return rc;
         for (int k = 0; k < chunk; ++k)
             if ((rc = issue_one_step(r))) return rc;
         if ((rc = flush_fields(r))) return rc;
@@ -1188,7 +1244,7 @@ extern "C" int pgb_step_async(pgb_run* r, int32_t nsteps) {
     int done = 0;
     while (done < nsteps) {
         int chunk = std::min<int>(nsteps - done, (int)r->phi_tab_cap);
-        if ((rc = set_device_step(r, r->time_step, chunk))) return rc;
+        if ((rc = set_device_step(r, r->time_step, chunk)) || (rc = clear_charge(r))) return rc;
         for (int k = 0; k < chunk; ++k)
             if ((rc = issue_one_step(r))) return rc;
         if ((rc = flush_fields(r))) return rc;
@@ -1225,6 +1281,7 @@ extern "C" int pgb_step_batch(pgb_run* const* runs, int32_t nruns, int32_t nstep
         for (int a = 0; a < nruns; ++a) chunk = std::min<int>(chunk, (int)runs[a]->phi_tab_cap);
         for (int a = 0; a < nruns; ++a) {
             int rc = set_device_step(runs[a], runs[a]->time_step, chunk);
+            if (!rc) rc = clear_charge(runs[a]);
             if (rc) return rc;
         }
         /* one step of every run in turn: each run's work goes to its own

@@ -16,13 +16,14 @@
 
 /* ------------------------------------------------ charge, rho, rhs */
 struct FinalizeArgs {
-    const unsigned long long* acc[2];
+    unsigned long long* acc[2];
     double* q[2];
     double* rho;
     double* f;            /* Poisson right-hand side, or null */
     int nx, ny;
     double qcdxdy[2];     /* qc/(DX*DY) per species */
     int mask;             /* species whose q is rebuilt from acc */
+    int clear;            /* zero acc once read                  */
     double coef;          /* 1/EPSILON */
     double divdxdy;       /* 1/(DX*DY) */
     double phi0x, phi0y, phily;
@@ -56,6 +57,7 @@ __global__ void k_finalize(FinalizeArgs a) {
         for (int s = 0; s < 2; ++s)
             if (a.mask & (1 << s)) {
                 double v = (double)(long long)a.acc[s][k] * (1.0 / PGB_FIX_SCALE);
+                if (a.clear) a.acc[s][k] = 0ull;
                 a.q[s][k] = (v * a.qcdxdy[s]) * ef;
             }
         double rho = a.q[1][k] + a.q[0][k];
@@ -133,6 +135,7 @@ static FinalizeArgs fin_args(pgb_run* r, int mask, bool rhs) {
     a.qcdxdy[0] = r->sp[0].qc / (r->dx * r->dy);
     a.qcdxdy[1] = r->sp[1].qc / (r->dx * r->dy);
     a.mask = mask;
+    a.clear = 0;
     a.coef = 1.0 / 8.854e-12;
     a.divdxdy = 1.0 / (r->dx * r->dy);
     a.phi0x = r->p.phi_left; a.phi0y = r->p.phi_bottom; a.phily = r->p.phi_top;
@@ -140,8 +143,9 @@ static FinalizeArgs fin_args(pgb_run* r, int mask, bool rhs) {
     return a;
 }
 
-int pgb_launch_finalize(pgb_run* r, int mask, bool make_rhs) {
+int pgb_launch_finalize(pgb_run* r, int mask, bool make_rhs, bool clear) {
     FinalizeArgs a = fin_args(r, mask, make_rhs);
+    a.clear = clear;
     int G = r->nx * r->ny;
     PGB_CK(r, pgb_launch_pdl(k_finalize, dim3((G + 255) / 256), dim3(256), 0, r->stream, a));
     r->launches++;

@@ -66,6 +66,8 @@ struct DevState {
                                 potential); trails t while a solve overlaps the next
                                 step's collisions                                      */
     unsigned long long scat_n;   /* scattering events queued by the collision pass */
+    unsigned int ticket;     /* blocks of a wall kernel that are done            */
+    unsigned int pad3;
     long long n_cx;          /* ion slots whose charge exchange was tested before this
                                 step's appends (the rest are tested after them)       */
 };
@@ -175,20 +177,21 @@ struct pgb_run {
      * the side stream while A of step t+1 runs on the run's stream        */
     cudaGraphExec_t graph_a[8] = {}, graph_b[8] = {}, graph_f = nullptr;
     long long graph_a_launches[8] = {}, graph_b_launches[8] = {}, graph_f_launches = 0;
-    /* the captured templates of A, B and F, and per key one step graph
-     * built from them: F of the previous step beside A, then B -- one
-     * launch for a step that needs no host decision                      */
-    cudaGraph_t tmpl_a[8] = {}, tmpl_b[8] = {}, tmpl_f = nullptr;
+    /* per key the whole step as one graph: F of the previous step beside A,
+     * then B -- one launch for a step that needs no host decision         */
     cudaGraphExec_t graph_m[8] = {};
-    int prio_hi = 0;                       /* the side stream's priority      */
+    long long graph_m_launches[8] = {};
     /* launch shapes (pgb_set_launch_config, pgb_autotune): they change no
      * result.  push grid = SMs x tune_push_per_sm; the collision kernels
      * beside a field solve leave it tune_field_sms SMs                   */
     int tune_push_per_sm = 8;
     int tune_field_sms = 32;
     bool fields_pending = false;           /* last step's field solve not yet issued */
+    bool charge_dirty = true;              /* the charge accumulators may not be zero  */
     cudaStream_t side = nullptr;
+    cudaStream_t ion = nullptr;            /* the ions' kernels, beside the electrons' */
     cudaEvent_t ev_fork, ev_join;
+    cudaEvent_t ev_i0, ev_i1, ev_e0;       /* between the electrons' and the ions' kernels */
     bool side_ok = false;
     float* cx_p = nullptr;                 /* per-ion CX probability          */
     float* cx_tile_sum = nullptr;          /* [column][tile] (int64)          */
@@ -282,22 +285,35 @@ inline cudaError_t pgb_launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, si
         if (!pgb_cuda_ok((r), (call), #call)) return PGB_ERR_CUDA; \
     } while (0)
 
+#ifdef __CUDACC__
+/* end of a step's particle phases: the step counter moves on, and the
+ * ionization events are counted from 0 again.  One thread.               */
+__device__ __forceinline__ void pgb_step_end(DevState* ds) {
+    ds->t += 1;
+    ds->list_n[LIST_ION_EV] = 0;
+}
+#endif
+
 /* kernels launched from the host side (defined in the .cu files) */
 struct CollConsts;
 int pgb_launch_push(pgb_run* r, int s, bool deposit);
 int pgb_launch_flag_outside(pgb_run* r, int s);
-/* count_only: the list's length alone (ds->list_n), not the list */
-int pgb_build_list(pgb_run* r, int which, int species_for_tiles, bool count_only = false);
+/* commit: species (1 electrons, 2 ions) whose ionization products, which
+ * are not stored, are entered with the list                              */
+int pgb_build_list(pgb_run* r, int which, int species_for_tiles, int commit = 0);
 int pgb_launch_deposit(pgb_run* r, int s);
-int pgb_launch_finalize(pgb_run* r, int which_species_mask, bool make_rhs);
-int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e);
+/* clear: leave the charge accumulators zero for the next step */
+int pgb_launch_finalize(pgb_run* r, int which_species_mask, bool make_rhs, bool clear = false);
+int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit = 0);
 int pgb_launch_ionize_appends(pgb_run* r, int store_e, int store_i);
-int pgb_launch_mcc(pgb_run* r, int leave_sms);
+/* count_events: ds->list_n[LIST_ION_EV] counts the ionization events (from 0) */
+int pgb_launch_mcc(pgb_run* r, int leave_sms, bool count_events = false);
 int pgb_launch_scatter(pgb_run* r, int leave_sms);
 /* tail 0: the ions present (records their count); 1: those appended since;
  * 2: the same in one block, for a tail of a few thousand ions at most     */
 int pgb_launch_cx(pgb_run* r, int tail, int leave_sms);
-int pgb_launch_walls(pgb_run* r, int which);
+/* advance: the last kernel of the electron (or steady) walls ends the step */
+int pgb_launch_walls(pgb_run* r, int which, bool advance = false);
 int pgb_launch_load(pgb_run* r, int s, const double* d_aos, long long i0, long long i1);
 int pgb_launch_dump_offsets(pgb_run* r, int s);
 int pgb_launch_dump(pgb_run* r, int s, double* d_out, unsigned int* d_ids, long long cap, int t0, int t1);

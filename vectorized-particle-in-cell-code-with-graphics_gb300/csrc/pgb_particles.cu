@@ -44,6 +44,7 @@ struct PushArgs {
     int* tc_out;
     int* tl_ev;                 /* per-tile ionization-event list     */
     int* tc_ev;
+    int count_ev;               /* count the ionization events here (no list is built) */
 };
 
 /* gather (pic.cl:56-92) + push (pic.cl:95-149) of one particle in cell units */
@@ -530,6 +531,7 @@ __global__ void __launch_bounds__(MCC_THREADS, 1) k_mcc(PushArgs a, int* scat) {
             so[lane] = y - d;
             if (lane == 31) {
                 a.tc_ev[tile] = x;
+                if (a.count_ev && x) atomicAdd((unsigned long long*)&a.ds->list_n[LIST_ION_EV], (unsigned long long)x);
                 S.sbase = y ? atomicAdd(&a.ds->scat_n, (unsigned long long)y) : 0ull;
             }
         }
@@ -567,10 +569,11 @@ __global__ void __launch_bounds__(MCC_THREADS, 1) k_scatter(PushArgs a, const in
     }
 }
 
-/* the last kernel of a step's particle phases moves the step counter on */
+/* the last kernel of a step's particle phases moves the step counter on
+ * (where the wall kernels do not, see pgb_launch_walls)                  */
 __global__ void k_step_advance(DevState* ds) {
     pgb_pdl_entry();
-    ds->t += 1;
+    pgb_step_end(ds);
 }
 
 /* ------------------------------------------------------------ scans */
@@ -633,43 +636,93 @@ __global__ void __launch_bounds__(1024) k_scan_small(const int* cnt, int* off, c
     if (threadIdx.x == 0) *total = t;
 }
 
-/* exclusive scan of a list-length array (length read from device memory) */
-__global__ void __launch_bounds__(1024) k_scan_list(const int* cnt, int* off, const long long* m_ptr, long long* total) {
-    pgb_pdl_entry();
-    long long t = block_excl_scan(cnt, off, *m_ptr, 0);
-    if (threadIdx.x == 0) *total = t;
+/* The event count of a step whose ionization products are not stored (see
+ * step_particles): the ids that they would have taken, and their removal,
+ * per species.  One thread.                                              */
+__device__ __forceinline__ void ionize_count_commit(DevState* ds, int species_mask) {
+    const long long m = ds->list_n[LIST_ION_EV];
+    if (species_mask & 1) { ds->next_id[0] += (unsigned int)m; ds->stats[ST_ABS_E] += m; }
+    if (species_mask & 2) { ds->next_id[1] += (unsigned int)m; ds->stats[ST_ABS_I] += m; }
 }
 
-/* gather per-tile lists (32 mask words a tile, see tile_masks) into one
- * dense list in slot order.  A warp per tile, a lane per word: a shuffle
- * scan of the words' counts gives each word's place, then each lane writes
- * the slots of its set bits.                                             */
-__global__ void k_gather_lists(const int* tl, const int* tc, const int* toff, const long long* n_ptr, int* out) {
+/* Per-tile lists (32 mask words a tile, see tile_masks) to one dense list
+ * in slot order, and its length, in one launch.  A block takes a run of
+ * tiles; the entries before its first tile are the sum of the counts
+ * before it, which every block adds up for itself (at 16.4 Ki tiles 32 KB
+ * from L2 on average), so that no block waits for another.  A warp per
+ * tile, a lane per word: a shuffle scan of the words' counts gives each
+ * word's place, then each lane writes the slots of its set bits.
+ * One launch instead of a one-block scan and a gather: at 16.4 Ki tiles
+ * 15.7 + 5.9 us -> 7 us, at 200 tiles 4.1 + 3.6 -> 4 us (ncu).
+ * commit: species whose uncounted ionization products this list's last
+ * block enters (0: none).                                                */
+#define LIST_THREADS 512
+__global__ void __launch_bounds__(LIST_THREADS) k_build_list(const int* tl, const int* tc, DevState* ds, int s, int* out,
+                                                             long long* total, int commit) {
     pgb_pdl_entry();
-    const long long n = *n_ptr;
-    const int ntiles = (int)((n + PGB_TILE - 1) / PGB_TILE);
-    const int lane = threadIdx.x & 31;
-    const int wpb = blockDim.x >> 5;
+    __shared__ int s_sum[LIST_THREADS / 32];
+    __shared__ int s_off[LIST_THREADS];
+    const int ntiles = (int)((ds->n[s] + PGB_TILE - 1) / PGB_TILE);
+    const int per = (ntiles + gridDim.x - 1) / gridDim.x;
+    const int t0 = min((int)blockIdx.x * per, ntiles), t1 = min(t0 + per, ntiles);
+    const bool last = t1 == ntiles && (t0 < t1 || blockIdx.x == 0);
+    if (t0 == t1 && !last) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned* masks = (const unsigned*)tl;
-    for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < ntiles; t += gridDim.x * wpb) {
-        if (tc[t] == 0) continue;   /* the same for every lane */
-        unsigned m = masks[(long long)t * 32 + lane];
-        const int c = __popc(m);
-        int incl = c;
+    int sum = 0;
+    for (int t = threadIdx.x; t < t0; t += LIST_THREADS) sum += tc[t];
+#pragma unroll
+    for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (lane == 0) s_sum[warp] = sum;
+    __syncthreads();
+    int carry = 0;
+#pragma unroll
+    for (int w = 0; w < LIST_THREADS / 32; ++w) carry += s_sum[w];
+    for (int b = t0; b < t1; b += LIST_THREADS) {
+        /* exclusive scan of this run's counts */
+        const int c = b + (int)threadIdx.x < t1 ? tc[b + threadIdx.x] : 0;
+        int x = c;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += y;
+            const int y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
         }
-        int pos = toff[t] + incl - c;
-        /* word lane = k * warps + w holds slots tile*TILE + k*THREADS + w*32 + bit */
-        const int sb = t * PGB_TILE + (lane / (PGB_PUSH_THREADS / 32)) * PGB_PUSH_THREADS +
-                       (lane % (PGB_PUSH_THREADS / 32)) * 32;
-        while (m) {
-            const int b = __ffs(m) - 1;
-            m &= m - 1;
-            out[pos++] = sb + b;
+        __syncthreads();   /* s_sum and s_off of the pass before have been read */
+        if (lane == 31) s_sum[warp] = x;
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < LIST_THREADS / 32; ++w) {
+            if (w < warp) before += s_sum[w];
+            all += s_sum[w];
         }
+        s_off[threadIdx.x] = carry + before + x - c;
+        __syncthreads();
+        const int m1 = min(b + LIST_THREADS, t1);
+        for (int t = b + warp; t < m1; t += LIST_THREADS / 32) {
+            unsigned m = masks[(long long)t * 32 + lane];
+            const int cw = __popc(m);
+            int incl = cw;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += y;
+            }
+            int pos = s_off[t - b] + incl - cw;
+            /* word lane = k * warps + w holds slots tile*TILE + k*THREADS + w*32 + bit */
+            const int sb = t * PGB_TILE + (lane / (PGB_PUSH_THREADS / 32)) * PGB_PUSH_THREADS +
+                           (lane % (PGB_PUSH_THREADS / 32)) * 32;
+            while (m) {
+                const int q = __ffs(m) - 1;
+                m &= m - 1;
+                out[pos++] = sb + q;
+            }
+        }
+        carry += all;
+    }
+    if (last && threadIdx.x == 0) {
+        *total = carry;
+        if (commit) ionize_count_commit(ds, commit);
     }
 }
 
@@ -691,21 +744,15 @@ struct InjectArgs {
     int species_mask;            /* 1 = electrons, 2 = ions                  */
     int* list_out_e;             /* append outside electrons (ordered)       */
     long long list_cap;
-    int* flag;                   /* per new electron: outside after its push */
+    int* flag;                   /* k_inject: per new electron, outside after its push */
 };
-__global__ void k_inject(InjectArgs a) {
-    pgb_pdl_entry();
-    /* one thread per new particle; electrons first, then ions, in id order */
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int total = a.k * ((a.species_mask & 1) + ((a.species_mask >> 1) & 1));
-    if (j >= total) return;
-    const int s = ((a.species_mask & 1) && j < a.k) ? 0 : 1;
-    const int jj = (s == 0 || !(a.species_mask & 1)) ? j : j - a.k;
+/* the j-th new particle of species s: id and slot from the counts before
+ * the injection; true if it left through a wall in its first push        */
+__device__ __forceinline__ bool inject_one(const InjectArgs& a, int s, int jj, long long n0, unsigned int id0) {
     const Species& S = s == 0 ? a.e : a.i;
-    const long long n0 = a.ds->n[s];
     const long long slot = n0 + jj;
-    if (slot >= S.cap) { atomicOr(&a.ds->err, s == 0 ? ERR_CAP_E : ERR_CAP_I); return; }
-    const unsigned int id = a.ds->next_id[s] + (unsigned int)jj;
+    if (slot >= S.cap) { atomicOr(&a.ds->err, s == 0 ? ERR_CAP_E : ERR_CAP_I); return false; }
+    const unsigned int id = id0 + (unsigned int)jj;
     pgb_stream st;
     pgb_stream_init(&st, a.seed, id, (unsigned int)a.ds->t, PGB_STREAM_INJECT, (uint32_t)s);
     double rx = pgb_u01d(pgb_stream_u32(&st));
@@ -727,8 +774,57 @@ __global__ void k_inject(InjectArgs a) {
     S.vz[slot] = vz;
     S.w[slot] = 0.0f;
     S.id[slot] = id;
+    return out;
+}
+__global__ void k_inject(InjectArgs a) {
+    pgb_pdl_entry();
+    /* one thread per new particle; electrons first, then ions, in id order */
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int total = a.k * ((a.species_mask & 1) + ((a.species_mask >> 1) & 1));
+    if (j >= total) return;
+    const int s = ((a.species_mask & 1) && j < a.k) ? 0 : 1;
+    const int jj = (s == 0 || !(a.species_mask & 1)) ? j : j - a.k;
     /* outside electrons join the end of the wall list in slot order */
-    if (out) a.flag[jj] = 1;
+    if (inject_one(a, s, jj, a.ds->n[s], a.ds->next_id[s])) a.flag[jj] = 1;
+}
+
+/* The injection of one species in one block, for NUMBER_TO_INJECT up to
+ * INJECT_BLOCK_MAX: the ids of the step's uncounted ionization products
+ * first (commit), the particles, then the counts and the wall list.  Two
+ * launches and the products' commit kernel in one (6.4 + 4.2 + 2.3 us ->
+ * 6.5 us, ncu); each thread's work is a chain of some 2 us, so more than
+ * four rounds of 1024 are better spread over blocks (k_inject).          */
+#define INJECT_BLOCK_MAX 4096
+__global__ void __launch_bounds__(1024) k_inject_block(InjectArgs a, int s, int commit) {
+    pgb_pdl_entry();
+    __shared__ unsigned s_out[INJECT_BLOCK_MAX / 32];
+    if (commit && threadIdx.x == 0) ionize_count_commit(a.ds, commit);
+    __syncthreads();
+    const Species& S = s == 0 ? a.e : a.i;
+    const long long n0 = a.ds->n[s];
+    const unsigned int id0 = a.ds->next_id[s];
+    for (int j = threadIdx.x; j < ((a.k + 31) & ~31); j += blockDim.x) {
+        const bool out = j < a.k && inject_one(a, s, j, n0, id0);
+        const unsigned m = __ballot_sync(0xffffffffu, out);
+        if ((threadIdx.x & 31) == 0) s_out[j >> 5] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    int k = a.k;
+    if (n0 + k > S.cap) k = (int)(S.cap - n0 > 0 ? S.cap - n0 : 0);
+    if (s == 0 && a.push_e) {
+        long long pos = a.ds->list_n[LIST_OUT_E];
+        for (int w = 0; w < (k + 31) / 32; ++w)
+            for (unsigned m = s_out[w]; m; m &= m - 1) {
+                const int j = 32 * w + __ffs(m) - 1;
+                if (pos < a.list_cap) a.list_out_e[pos++] = (int)(n0 + j);
+                else a.ds->err |= ERR_LIST;
+            }
+        a.ds->list_n[LIST_OUT_E] = pos;
+    }
+    a.ds->n[s] = n0 + k;
+    a.ds->next_id[s] = id0 + (unsigned int)k;
+    a.ds->stats[s == 0 ? ST_INJ_E : ST_INJ_I] += k;
 }
 
 /* after k_inject: counts, ids, and the wall list entries of new electrons */
@@ -824,6 +920,12 @@ __global__ void k_ionize_commit(DevState* ds, int store_e, int store_i, long lon
     else ds->stats[ST_ABS_E] += m;
     if (store_i) { long long v = ds->n[1] + m; ds->n[1] = v < cap_i ? v : cap_i; }
     else ds->stats[ST_ABS_I] += m;
+    ds->list_n[LIST_ION_EV] = 0;   /* k_mcc counts on from 0 where no list is built */
+}
+
+__global__ void k_ionize_count_commit(DevState* ds, int species_mask) {
+    pgb_pdl_entry();
+    ionize_count_commit(ds, species_mask);
 }
 
 /* ------------------------------------------------------------ compaction */
@@ -1042,6 +1144,7 @@ static PushArgs push_args(pgb_run* r, int s) {
     a.tc_out = r->tile_cnt[s == 0 ? LIST_OUT_E : LIST_OUT_I];
     a.tl_ev = r->tile_list[LIST_ION_EV];
     a.tc_ev = r->tile_cnt[LIST_ION_EV];
+    a.count_ev = 0;
     return a;
 }
 
@@ -1081,8 +1184,9 @@ static int mcc_blocks(pgb_run* r, int leave_sms, long long per_block) {
     const long long want = std::max<long long>(1, (n + per_block - 1) / per_block);
     return (int)std::min<long long>(std::max(1, r->sms - leave_sms), want);
 }
-int pgb_launch_mcc(pgb_run* r, int leave_sms) {
+int pgb_launch_mcc(pgb_run* r, int leave_sms, bool count_events) {
     PushArgs a = push_args(r, 0);
+    a.count_ev = count_events;
     const int g = mcc_blocks(r, leave_sms, (long long)MCC_GROUPS * PGB_TILE);
     PGB_CK(r, cudaMemsetAsync(&r->ds->scat_n, 0, sizeof(unsigned long long), r->stream));
     PGB_CK(r, pgb_launch_pdl(k_mcc, dim3(g), dim3(MCC_THREADS), 0, r->stream, a, r->list[LIST_SPARE]));
@@ -1101,13 +1205,9 @@ int pgb_launch_scatter(pgb_run* r, int leave_sms) {
 }
 
 /* per-tile list `which` (tiles of species s) -> dense list + count */
-int pgb_build_list(pgb_run* r, int which, int s, bool count_only) {
-    int* toff = r->aux_j;
-    PGB_CK(r, pgb_launch_pdl(k_scan_small, dim3(1), dim3(1024), 0, r->stream, r->tile_cnt[which], toff, &r->ds->n[s], 0, &r->ds->list_n[which]));
-    r->launches++;
-    if (count_only) return 0;
-    PGB_CK(r, pgb_launch_pdl(k_gather_lists, dim3(grid_for(r, 4)), dim3(256), 0, r->stream, r->tile_list[which], r->tile_cnt[which], toff,
-                                                           &r->ds->n[s], r->list[which]));
+int pgb_build_list(pgb_run* r, int which, int s, int commit) {
+    PGB_CK(r, pgb_launch_pdl(k_build_list, dim3(r->sms), dim3(LIST_THREADS), 0, r->stream, (const int*)r->tile_list[which],
+                             (const int*)r->tile_cnt[which], r->ds, s, r->list[which], &r->ds->list_n[which], commit));
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;
@@ -1120,7 +1220,7 @@ int pgb_launch_deposit(pgb_run* r, int s) {
     return 0;
 }
 
-int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e) {
+int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit) {
     InjectArgs a;
     a.e = r->sp[0]; a.i = r->sp[1]; a.ds = r->ds; a.k = r->p.number_to_inject;
     a.dx = r->dx; a.dy = r->dy; a.xlength = r->p.xlength; a.ylength = r->p.ylength;
@@ -1129,8 +1229,22 @@ int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e) {
     a.push_e = push_e; a.species_mask = species_mask;
     a.list_out_e = r->list[LIST_OUT_E]; a.list_cap = r->list_cap;
     a.flag = r->inject_flag;
-    int tot = 2 * a.k;
-    if (tot <= 0) return 0;
+    if (a.k <= 0) return 0;
+    if (a.k <= INJECT_BLOCK_MAX) {
+        const int threads = std::min(1024, (a.k + 31) & ~31);
+        for (int s = 0; s < 2; ++s)
+            if (species_mask & (1 << s)) {
+                PGB_CK(r, pgb_launch_pdl(k_inject_block, dim3(1), dim3(threads), 0, r->stream, a, s, commit & (1 << s)));
+                r->launches++;
+            }
+        PGB_CK(r, cudaGetLastError());
+        return 0;
+    }
+    const int tot = a.k * ((species_mask & 1) + ((species_mask >> 1) & 1));
+    if (commit) {
+        PGB_CK(r, pgb_launch_pdl(k_ionize_count_commit, dim3(1), dim3(1), 0, r->stream, r->ds, commit));
+        r->launches++;
+    }
     PGB_CK(r, pgb_launch_pdl(k_inject, dim3((tot + 127) / 128), dim3(128), 0, r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_inject_commit, dim3(1), dim3(32), 0, r->stream, a));
     r->launches += 2;
@@ -1145,13 +1259,9 @@ int pgb_launch_ionize_appends(pgb_run* r, int store_e, int store_i) {
     a.dx = r->dx; a.dy = r->dy; a.ps = r->ps;
     a.store_e = store_e;
     a.store_i = store_i;
-    if (store_e || store_i) {   /* else the products are only counted */
-        PGB_CK(r, pgb_launch_pdl(k_ionize_append, dim3(r->sms * 2), dim3(256), 0, r->stream, a));
-        r->launches++;
-        PGB_CK(r, cudaGetLastError());
-    }
+    PGB_CK(r, pgb_launch_pdl(k_ionize_append, dim3(r->sms * 2), dim3(256), 0, r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_ionize_commit, dim3(1), dim3(1), 0, r->stream, r->ds, a.store_e, a.store_i, r->sp[0].cap, r->sp[1].cap));
-    r->launches++;
+    r->launches += 2;
     PGB_CK(r, cudaGetLastError());
     return 0;
 }

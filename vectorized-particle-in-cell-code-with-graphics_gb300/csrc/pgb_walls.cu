@@ -35,7 +35,8 @@ struct WallArgs {
     const int* list_e;
     const int* list_i;
     int* aux;                  /* per list entry: secondary count  */
-    int* off;                  /* exclusive scan of aux            */
+    int* csum;                 /* per WALL_CHUNK entries: their sum */
+    int advance;               /* the last block ends the step     */
     unsigned long long* qacc_e;
     unsigned long long* qacc_i;
     int nx, ny;
@@ -53,6 +54,68 @@ __device__ __forceinline__ void store_particle(const Species& S, long long slot,
                                                double vy, double vz, double dx, double dy, int ps) {
     S.xv[slot] = make_float4(pos_from_m(x, dx, ps), pos_from_m(y, dy, ps), (float)vx, (float)vy);
     S.vz[slot] = (float)vz;
+}
+
+/* New electrons get their slots and ids from an exclusive scan of the list
+ * entries' secondary counts.  Pass 1 (a chunk of WALL_CHUNK entries per
+ * block and round) stores each chunk's sum; in pass 2 a block carries the
+ * sum of all chunks before its own (each chunk's sum is read once by every
+ * block) and scans its chunk, so no scan kernel runs between the passes;
+ * pass 2's last block to finish enters the totals.  Electron walls at 16 Mi
+ * particles: four launches of 10.7 + 34.9 + 9.9 + 2.6 us -> two of 11 + 12
+ * us (ncu).                                                              */
+#define WALL_CHUNK 256
+/* the sum of v over the block (WALL_CHUNK threads) */
+__device__ __forceinline__ int block_sum(int v) {
+    __shared__ int s_w[WALL_CHUNK / 32];
+#pragma unroll
+    for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    __syncthreads();   /* s_w of the call before has been read */
+    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < WALL_CHUNK / 32; ++w) t += s_w[w];
+    return t;
+}
+/* exclusive scan of v over the block */
+__device__ __forceinline__ int block_scan(int v) {
+    __shared__ int s_w[WALL_CHUNK / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) s_w[warp] = x;
+    __syncthreads();
+    int before = 0;
+#pragma unroll
+    for (int w = 0; w < WALL_CHUNK / 32; ++w)
+        if (w < warp) before += s_w[w];
+    return before + x - v;
+}
+/* sum of the chunk sums [c0, c1) */
+__device__ __forceinline__ int chunk_sums(const int* csum, int c0, int c1) {
+    int v = 0;
+    for (int c = c0 + threadIdx.x; c < c1; c += WALL_CHUNK) v += csum[c];
+    return block_sum(v);
+}
+/* true in every thread of the block that is the last of the grid to get
+ * here (its reads then see the other blocks' writes)                     */
+__device__ __forceinline__ bool last_block(DevState* ds) {
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(&ds->ticket, 1u) == gridDim.x - 1;
+        if (s_last) ds->ticket = 0u;
+    }
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last;
 }
 
 /* boundary::secondary_vel (boundary.cpp:427-486) on a particle state */
@@ -102,40 +165,68 @@ __device__ __forceinline__ float ion_yield(const WallArgs& a, float energy) {
     return y;
 }
 
-__global__ void k_iwall1(WallArgs a) {
+/* n, next id and statistics after a wall pass over m list entries that
+ * appended the counted electrons, by the last block to finish            */
+__device__ __forceinline__ void wall_commit(const WallArgs& a, long long m, int which) {
+    if (!last_block(a.ds)) return;
+    const long long t = chunk_sums(a.csum, 0, (int)((m + WALL_CHUNK - 1) / WALL_CHUNK));
+    if (threadIdx.x != 0) return;
+    DevState* const ds = a.ds;
+    const long long v = ds->n[0] + t;
+    ds->n[0] = v < a.e.cap ? v : a.e.cap;
+    ds->next_id[0] += (unsigned int)t;
+    if (which == 0) { ds->stats[ST_ABS_I] += m; ds->dead[1] += m; }
+    ds->stats[which == 0 ? ST_ISEE_EM : ST_SEE_EM] += t;
+    if (a.advance) pgb_step_end(ds);
+}
+
+__global__ void __launch_bounds__(WALL_CHUNK) k_iwall1(WallArgs a) {
     pgb_pdl_entry();
     const long long m = a.ds->list_n[LIST_OUT_I];
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x) {
-        int slot = a.list_i[k];
-        float4 p = a.i.xv[slot];
-        float vx = p.z, vy = p.w, vz = a.i.vz[slot];
-        float energy = (float)((0.5 / PGB_CHARGE) * a.mi) * (vx * vx + vy * vy + vz * vz);
-        float yield = ion_yield(a, energy);
-        pgb_stream st;
-        pgb_stream_init(&st, a.seed, a.i.id[slot], (unsigned int)a.ds->t, PGB_STREAM_IWALL, 1);
-        float R = pgb_u01f(pgb_stream_u32(&st));
-        a.aux[k] = (R < yield) ? (int)floorf(yield) + 1 : 0;
+    for (long long c = blockIdx.x; c * WALL_CHUNK < m; c += gridDim.x) {
+        const long long k = c * WALL_CHUNK + threadIdx.x;
+        int cnt = 0;
+        if (k < m) {
+            int slot = a.list_i[k];
+            float4 p = a.i.xv[slot];
+            float vx = p.z, vy = p.w, vz = a.i.vz[slot];
+            float energy = (float)((0.5 / PGB_CHARGE) * a.mi) * (vx * vx + vy * vy + vz * vz);
+            float yield = ion_yield(a, energy);
+            pgb_stream st;
+            pgb_stream_init(&st, a.seed, a.i.id[slot], (unsigned int)a.ds->t, PGB_STREAM_IWALL, 1);
+            float R = pgb_u01f(pgb_stream_u32(&st));
+            cnt = (R < yield) ? (int)floorf(yield) + 1 : 0;
+            a.aux[k] = cnt;
+        }
+        const int sum = block_sum(cnt);
+        if (threadIdx.x == 0) a.csum[c] = sum;
     }
 }
 
 /* boundary::i_secondary_vel (boundary.cpp:687-756) */
-__global__ void k_iwall2(WallArgs a) {
+__global__ void __launch_bounds__(WALL_CHUNK) k_iwall2(WallArgs a) {
     pgb_pdl_entry();
     const long long m = a.ds->list_n[LIST_OUT_I];
     const long long ne0 = a.ds->n[0];
     const unsigned int id0 = a.ds->next_id[0];
     const double lengthX = a.dx * a.nx, lengthY = a.dy * a.ny;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x) {
+    int carry = 0, c_done = 0;   /* the sum of the chunks before c_done */
+    for (long long ch = blockIdx.x; ch * WALL_CHUNK < m; ch += gridDim.x) {
+        const long long k = ch * WALL_CHUNK + threadIdx.x;
+        carry += chunk_sums(a.csum, c_done, (int)ch);
+        c_done = (int)ch;
+        const int c = k < m ? a.aux[k] : 0;
+        const int off = carry + block_scan(c);
+        if (k >= m) continue;
         int slot = a.list_i[k];
         float4 p = a.i.xv[slot];
-        int c = a.aux[k];
         if (c > 0) {
             double w = a.i.w[slot];
             int jp = pcell(p.x, a.ps), kp = pcell(p.y, a.ps);
             for (int j = 0; j < c; ++j) {
-                long long es = ne0 + a.off[k] + j;
+                long long es = ne0 + off + j;
                 if (es >= a.e.cap) { atomicOr(&a.ds->err, ERR_CAP_E); break; }
-                unsigned int id = id0 + (unsigned int)(a.off[k] + j);
+                unsigned int id = id0 + (unsigned int)(off + j);
                 pgb_stream st;
                 pgb_stream_init(&st, a.seed, id, (unsigned int)a.ds->t, PGB_STREAM_SEE, 0);
                 double x = 0.0, y = 0.0;
@@ -180,6 +271,7 @@ __global__ void k_iwall2(WallArgs a) {
         }
         a.i.xv[slot].x = pos_dead();
     }
+    wall_commit(a, m, 0);
 }
 
 /* ---------------------------------------------------- electron walls */
@@ -242,36 +334,41 @@ __device__ int e_wall_event(const WallArgs& a, pgb_stream* st, double& x, double
     return EW_ABSORB;
 }
 
-__global__ void k_ewall1(WallArgs a) {
+__global__ void __launch_bounds__(WALL_CHUNK) k_ewall1(WallArgs a) {
     pgb_pdl_entry();
     const long long m = a.ds->list_n[LIST_OUT_E];
     int cnt[4] = {0, 0, 0, 0};   /* absorbed, reflected, backscattered, see events */
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x) {
-        int slot = a.list_e[k];
-        float4 p = a.e.xv[slot];
-        double x = pos_m(p.x, a.ps, a.dx), y = pos_m(p.y, a.ps, a.dy);
-        float vx = p.z, vy = p.w, vz = a.e.vz[slot];
-        pgb_stream st;
-        pgb_stream_init(&st, a.seed, a.e.id[slot], (unsigned int)a.ds->t, PGB_STREAM_EWALL, 0);
-        int res = EW_RETRY, nsec = 0, kind = 0;
-        const int jp = pcell(p.x, a.ps), kp = pcell(p.y, a.ps);
-        for (int attempt = 0; attempt < 64 && res == EW_RETRY; ++attempt)
-            res = e_wall_event(a, &st, x, y, vx, vy, vz, jp, kp, nsec, kind);
-        if (res == EW_RETRY) res = EW_ABSORB;
+    for (long long ch = blockIdx.x; ch * WALL_CHUNK < m; ch += gridDim.x) {
+        const long long k = ch * WALL_CHUNK + threadIdx.x;
         int c = 0;
-        if (res == EW_STAY) {
-            store_particle(a.e, slot, x, y, vx, vy, vz, a.dx, a.dy, a.ps);
-            float4 q = a.e.xv[slot];
-            maybe_deposit(a.qacc_e, a.nx, a.ny, a.ps, q.x, q.y, a.e.w[slot]);
-            cnt[kind == ST_REFL ? 1 : 2]++;
-        } else if (res == EW_ABSORB) {
-            a.e.xv[slot].x = pos_dead();
-            cnt[0]++;
-        } else {
-            c = nsec;
-            cnt[3]++;
+        if (k < m) {
+            int slot = a.list_e[k];
+            float4 p = a.e.xv[slot];
+            double x = pos_m(p.x, a.ps, a.dx), y = pos_m(p.y, a.ps, a.dy);
+            float vx = p.z, vy = p.w, vz = a.e.vz[slot];
+            pgb_stream st;
+            pgb_stream_init(&st, a.seed, a.e.id[slot], (unsigned int)a.ds->t, PGB_STREAM_EWALL, 0);
+            int res = EW_RETRY, nsec = 0, kind = 0;
+            const int jp = pcell(p.x, a.ps), kp = pcell(p.y, a.ps);
+            for (int attempt = 0; attempt < 64 && res == EW_RETRY; ++attempt)
+                res = e_wall_event(a, &st, x, y, vx, vy, vz, jp, kp, nsec, kind);
+            if (res == EW_RETRY) res = EW_ABSORB;
+            if (res == EW_STAY) {
+                store_particle(a.e, slot, x, y, vx, vy, vz, a.dx, a.dy, a.ps);
+                float4 q = a.e.xv[slot];
+                maybe_deposit(a.qacc_e, a.nx, a.ny, a.ps, q.x, q.y, a.e.w[slot]);
+                cnt[kind == ST_REFL ? 1 : 2]++;
+            } else if (res == EW_ABSORB) {
+                a.e.xv[slot].x = pos_dead();
+                cnt[0]++;
+            } else {
+                c = nsec;
+                cnt[3]++;
+            }
+            a.aux[k] = c;
         }
-        a.aux[k] = c;
+        const int sum = block_sum(c);
+        if (threadIdx.x == 0) a.csum[ch] = sum;
     }
     const int idx[4] = {ST_ABS_E, ST_REFL, ST_BACK, ST_SEE_EV};
     int dead = cnt[0] + cnt[3];
@@ -285,13 +382,18 @@ __global__ void k_ewall1(WallArgs a) {
 }
 
 /* boundary::secondary_electrons (boundary.cpp:494-529) */
-__global__ void k_ewall2(WallArgs a) {
+__global__ void __launch_bounds__(WALL_CHUNK) k_ewall2(WallArgs a) {
     pgb_pdl_entry();
     const long long m = a.ds->list_n[LIST_OUT_E];
     const long long ne0 = a.ds->n[0];
     const unsigned int id0 = a.ds->next_id[0];
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x) {
-        int c = a.aux[k];
+    int carry = 0, c_done = 0;   /* the sum of the chunks before c_done */
+    for (long long ch = blockIdx.x; ch * WALL_CHUNK < m; ch += gridDim.x) {
+        const long long k = ch * WALL_CHUNK + threadIdx.x;
+        carry += chunk_sums(a.csum, c_done, (int)ch);
+        c_done = (int)ch;
+        const int c = k < m ? a.aux[k] : 0;
+        const int off = carry + block_scan(c);
         if (c == 0) continue;
         int slot = a.list_e[k];
         float4 p = a.e.xv[slot];
@@ -299,9 +401,9 @@ __global__ void k_ewall2(WallArgs a) {
         float w = a.e.w[slot];
         int jpp = pcell(p.x, a.ps);
         for (int j = 0; j < c; ++j) {
-            long long es = ne0 + a.off[k] + j;
+            long long es = ne0 + off + j;
             if (es >= a.e.cap) { atomicOr(&a.ds->err, ERR_CAP_E); break; }
-            unsigned int id = id0 + (unsigned int)(a.off[k] + j);
+            unsigned int id = id0 + (unsigned int)(off + j);
             double x = 0.0, y = 0.0;
             float vx = 0.0f, vy = 0.0f, vz = 0.0f;
             if (jpp < 0 || jpp >= a.nx) x = px;
@@ -322,18 +424,7 @@ __global__ void k_ewall2(WallArgs a) {
         }
         a.e.xv[slot].x = pos_dead();
     }
-}
-
-/* n, next id and statistics after a wall pass that appended `total` electrons */
-__global__ void k_wall_commit(DevState* ds, const long long* total, int which, long long cap_e, int stat_emit) {
-    pgb_pdl_entry();
-    long long t = *total;
-    long long v = ds->n[0] + t;
-    ds->n[0] = v < cap_e ? v : cap_e;
-    ds->next_id[0] += (unsigned int)t;
-    long long m = ds->list_n[which == 0 ? LIST_OUT_I : LIST_OUT_E];
-    if (which == 0) { ds->stats[ST_ABS_I] += m; ds->dead[1] += m; }
-    ds->stats[stat_emit] += t;
+    wall_commit(a, m, 1);
 }
 
 /* ------------------------------------------------- steady-state walls */
@@ -428,7 +519,10 @@ __global__ void __launch_bounds__(1024) k_steady(WallArgs a, int* ion_by_rank) {
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) a.ds->stats[ST_PLOP] += s_plops;
+    if (threadIdx.x == 0) {
+        a.ds->stats[ST_PLOP] += s_plops;
+        if (a.advance) pgb_step_end(a.ds);
+    }
 }
 
 /* ================================================================ CX */
@@ -718,7 +812,7 @@ static WallArgs wall_args(pgb_run* r) {
     WallArgs a;
     a.e = r->sp[0]; a.i = r->sp[1]; a.ds = r->ds;
     a.list_e = r->list[LIST_OUT_E]; a.list_i = r->list[LIST_OUT_I];
-    a.aux = r->aux_i; a.off = r->aux_j;
+    a.aux = r->aux_i; a.csum = r->aux_j; a.advance = 0;
     a.qacc_e = r->qacc[0]; a.qacc_i = r->qacc[1];
     a.nx = r->nx; a.ny = r->ny; a.ps = r->ps; a.dx = r->dx; a.dy = r->dy; a.dt = r->p.dt;
     a.me = r->p.electron_mass; a.mi = r->p.ion_mass;
@@ -731,11 +825,10 @@ static WallArgs wall_args(pgb_run* r) {
     return a;
 }
 
-__global__ void k_scan_list(const int* cnt, int* off, const long long* m_ptr, long long* total);
-
-int pgb_launch_walls(pgb_run* r, int which) {
+int pgb_launch_walls(pgb_run* r, int which, bool advance) {
     WallArgs a = wall_args(r);
-    int g = r->sms * 4;
+    a.advance = advance && which == PGB_BOUNDARY_ELECTRONS;
+    const dim3 g(r->sms * 4), b(WALL_CHUNK);
     if (r->p.steadystate) {
         if (which == PGB_BOUNDARY_ELECTRONS) {
             PGB_CK(r, pgb_launch_pdl(k_steady, dim3(1), dim3(1024), 0, r->stream, a, r->aux_i));
@@ -745,26 +838,13 @@ int pgb_launch_walls(pgb_run* r, int which) {
         return 0;
     }
     if (which == PGB_BOUNDARY_IONS && !a.ion_see) {
-        PGB_CK(r, pgb_launch_pdl(k_iwall_absorb, dim3(g), dim3(256), 0, r->stream, a));
-        r->launches++;
-    } else if (which == PGB_BOUNDARY_IONS) {
-        PGB_CK(r, pgb_launch_pdl(k_iwall1, dim3(g), dim3(256), 0, r->stream, a));
-        r->launches++;
-        PGB_CK(r, pgb_launch_pdl(k_scan_list, dim3(1), dim3(1024), 0, r->stream, r->aux_i, r->aux_j, &r->ds->list_n[LIST_OUT_I], &r->ds->list_n[LIST_SPARE]));
-        r->launches++;
-        PGB_CK(r, pgb_launch_pdl(k_iwall2, dim3(g), dim3(256), 0, r->stream, a));
-        r->launches++;
-        PGB_CK(r, pgb_launch_pdl(k_wall_commit, dim3(1), dim3(1), 0, r->stream, r->ds, &r->ds->list_n[LIST_SPARE], 0, r->sp[0].cap, ST_ISEE_EM));
+        PGB_CK(r, pgb_launch_pdl(k_iwall_absorb, g, b, 0, r->stream, a));
         r->launches++;
     } else {
-        PGB_CK(r, pgb_launch_pdl(k_ewall1, dim3(g), dim3(256), 0, r->stream, a));
-        r->launches++;
-        PGB_CK(r, pgb_launch_pdl(k_scan_list, dim3(1), dim3(1024), 0, r->stream, r->aux_i, r->aux_j, &r->ds->list_n[LIST_OUT_E], &r->ds->list_n[LIST_SPARE]));
-        r->launches++;
-        PGB_CK(r, pgb_launch_pdl(k_ewall2, dim3(g), dim3(256), 0, r->stream, a));
-        r->launches++;
-        PGB_CK(r, pgb_launch_pdl(k_wall_commit, dim3(1), dim3(1), 0, r->stream, r->ds, &r->ds->list_n[LIST_SPARE], 1, r->sp[0].cap, ST_SEE_EM));
-        r->launches++;
+        const bool ions = which == PGB_BOUNDARY_IONS;
+        PGB_CK(r, pgb_launch_pdl(ions ? k_iwall1 : k_ewall1, g, b, 0, r->stream, a));
+        PGB_CK(r, pgb_launch_pdl(ions ? k_iwall2 : k_ewall2, g, b, 0, r->stream, a));
+        r->launches += 2;
     }
     PGB_CK(r, cudaGetLastError());
     return 0;
