@@ -542,6 +542,7 @@ __global__ void __launch_bounds__(1024) k_steady(WallArgs a, int* ion_by_rank) {
  * A probability is at most 2^40, so with 2048 ions a tile neither 32-bit
  * sum can reach 2^32.                                                     */
 #define CX_TILE PGB_CX_TILE
+#define CX_AHEAD 8
 #define CX_ONE (1ll << 40)
 static_assert((long long)CX_TILE << 20 <= (1ll << 31), "32-bit halves of the tile sums must not overflow");
 
@@ -723,23 +724,42 @@ __global__ void __launch_bounds__(256) k_cx_walk(CxArgs a) {
         int first = __ffs(cross) - 1;
         long long before = first ? __shfl_sync(0xffffffffu, ps, first - 1) : 0;
         acc += before;
-        /* scan tile t0+first element by element, then continue after it */
+        /* scan tile t0+first element by element, then continue after it.
+         * The ions of CX_AHEAD batches are in flight together: one batch at
+         * a time, a tile was a chain of 64 loads, 25-50 us for a whole step
+         * in which any column crosses (argon, 257^2, 4 Mi ions: charge
+         * exchange 119 us a step), while the GPU held one warp per column */
         int tt = t0 + first;
-        for (int b = 0; b < CX_TILE; b += 32) {
-            long long i = i0 + (long long)tt * CX_TILE + b + lane;
-            int c = -1;
-            long long pf = 0;
-            if (i < n) pf = cx_prob_fixed(a, a.i.xv[i], a.i.vz[i], c);
-            unsigned match = __ballot_sync(0xffffffffu, c == col && pf > 0);
-            while (match) {
-                int l = __ffs(match) - 1;
-                match &= match - 1;
-                long long v = __shfl_sync(0xffffffffu, pf, l);
-                acc += v;
-                if (acc > CX_ONE) {
-                    acc = 0;
-                    if (lane == l) cx_exchange(a, i);
-                    fired++;
+        for (int b = 0; b < CX_TILE; b += 32 * CX_AHEAD) {
+            float4 p[CX_AHEAD];
+            float vz[CX_AHEAD];
+#pragma unroll
+            for (int q = 0; q < CX_AHEAD; ++q) {
+                const long long i = i0 + (long long)tt * CX_TILE + b + 32 * q + lane;
+                p[q] = make_float4(pos_dead(), 0.f, 0.f, 0.f);
+                vz[q] = 0.f;
+                if (i < n) {
+                    p[q] = a.i.xv[i];
+                    vz[q] = a.i.vz[i];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < CX_AHEAD; ++q) {
+                int c = -1;
+                long long pf = 0;
+                /* a dead or NaN position's cell index is no column */
+                if (pcell(p[q].x, a.ps) == col) pf = cx_prob_fixed(a, p[q], vz[q], c);
+                unsigned match = __ballot_sync(0xffffffffu, c == col && pf > 0);
+                while (match) {
+                    int l = __ffs(match) - 1;
+                    match &= match - 1;
+                    long long v = __shfl_sync(0xffffffffu, pf, l);
+                    acc += v;
+                    if (acc > CX_ONE) {
+                        acc = 0;
+                        if (lane == l) cx_exchange(a, i0 + (long long)tt * CX_TILE + b + 32 * q + lane);
+                        fired++;
+                    }
                 }
             }
         }
