@@ -163,8 +163,8 @@ static void free_lists(pgb_run* r) {
     r->cx_mask = nullptr;
     r->cx_total = nullptr;
     for (int q = 0; q < 2; ++q) {
-        cudaFree(r->tile_bin[q]); cudaFree(r->pieces[q]);
-        r->tile_bin[q] = nullptr; r->pieces[q] = nullptr;
+        cudaFree(r->pieces[q]);
+        r->pieces[q] = nullptr;
     }
     cudaFree(r->sort_counts); cudaFree(r->sort_offs); cudaFree(r->sort_key_total); cudaFree(r->sort_key_start);
     r->sort_counts = r->sort_offs = r->sort_key_total = nullptr;
@@ -251,8 +251,7 @@ static int ensure_capacity(pgb_run* r, int s, long long need) {
         long long nkeys = (long long)nbx * nby + 1;
         r->sort_chunks_cap = (lc + PGB_SORT_CHUNK - 1) / PGB_SORT_CHUNK + 1;
         for (int q = 0; q < 2; ++q) {
-            if (cudaMalloc(&r->tile_bin[q], sizeof(int) * nt) != cudaSuccess ||
-                cudaMalloc(&r->pieces[q], sizeof(int4) * (nt + nkeys + 1)) != cudaSuccess) {
+            if (cudaMalloc(&r->pieces[q], sizeof(int4) * (nt + nkeys + 1)) != cudaSuccess) {
                 cudaGetLastError();
                 return fail(r, PGB_ERR_NOMEM, "device allocation of sort tables failed");
             }
@@ -548,7 +547,7 @@ extern "C" int pgb_footprint(const pgb_params* p, int64_t ne, int64_t ni, int64_
     b += 2 * (16 + 4 + 4 + 4) * (ce + ci);                               /* particles, two copies */
     b += 4 * (4 * nt * 32 + 4 * nt + 4 * lc);                            /* event lists (32 mask words a tile) */
     b += 2 * 4 * std::max(lc, nt);                                        /* aux_i, aux_j */
-    b += 2 * (4 * nt + 16 * (nt + nkeys + 1));                            /* tile bins, pieces */
+    b += 2 * 16 * (nt + nkeys + 1);                                       /* pieces */
     const long long chunks = (lc + PGB_SORT_CHUNK - 1) / PGB_SORT_CHUNK + 1;
     b += 2 * 4 * nkeys * chunks + 4 * nkeys + 8 * (nkeys + 1);            /* sort scratch */
     b += 8 * nx * ((lc + PGB_CX_TILE - 1) / PGB_CX_TILE + 1) + 8 * nx * ((lc + PGB_CX_TILE - 1) / PGB_CX_TILE / 64 + 2); /* CX tile sums, masks */

@@ -36,7 +36,7 @@
 #define PGB_HALO 8             /* deposit window halo around a bin, cells     */
 #define PGB_WIN (PGB_BIN + 2 * PGB_HALO + 1)   /* window edge in nodes         */
 #define PGB_PIECE_TILES 4      /* tiles of one bin per work piece             */
-#define PGB_SORT_CHUNK 2048    /* slots per chunk of the bin sort passes      */
+#define PGB_SORT_CHUNK 4096    /* slots per chunk of the bin sort passes      */
 #define PGB_COPY_CHUNK (1 << 20)   /* particles per host-copy chunk of load/dump */
 #define PGB_COPY_EVENTS 32
 
@@ -65,9 +65,9 @@ struct DevState {
     long long tf;            /* time_step of the field solve being run (its right-wall
                                 potential); trails t while a solve overlaps the next
                                 step's collisions                                      */
-    unsigned long long scat_n;   /* scattering events queued by the collision pass */
     unsigned int ticket;     /* blocks of a wall kernel that are done            */
     unsigned int pad3;
+    unsigned long long scat_n;   /* scattering events queued by the collision pass */
     long long n_cx;          /* ion slots whose charge exchange was tested before this
                                 step's appends (the rest are tested after them)       */
 };
@@ -202,7 +202,6 @@ struct pgb_run {
     long long* cx_total = nullptr;
     int cx_mask_words = 0;
     /* spatial sort */
-    int* tile_bin[2] = {nullptr, nullptr};
     int4* pieces[2] = {nullptr, nullptr};
     int* sort_counts = nullptr;
     int* sort_offs = nullptr;

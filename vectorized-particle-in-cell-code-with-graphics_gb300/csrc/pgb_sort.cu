@@ -14,10 +14,16 @@
  * (charge-exchange accumulation, wall-list order) -- is deterministic.  It
  * also drops removed particles (tombstones).  Passes:
  *   count    per chunk of SORT_CHUNK slots, a shared histogram of bin keys
- *   scan     per bin over chunks, then over bins with tile padding
- *   scatter  one warp per chunk walks its slots in order and writes each
- *            particle to its bin at a running per-bin cursor
- *   pieces   tile -> bin map and work pieces (runs of tiles of one bin)
+ *   scan     per bin over chunks, then over bins with tile padding (and the
+ *            work pieces: runs of tiles of one bin)
+ *   scatter  one CTA per chunk sorts it in shared memory and writes each
+ *            bin's run of particles to its place
+ * Bound by memory traffic: 16 B read by the count, 28 B read and written
+ * by the scatter per particle.  A warp that placed its particles straight
+ * from registers wrote them a few at a time (half a sector of 32 B per
+ * position, an eighth per vz, weight and id): 1.2 ms for 16 Mi particles
+ * loaded in random order.  Sorted in shared memory first, a chunk of 4096
+ * over 257 bins leaves in runs of 16 particles.
  */
 #include <cuda_runtime.h>
 #include "pgb_internal.h"
@@ -32,12 +38,10 @@ struct SortArgs {
     int nx, ny;              /* nodes */
     int ps;                  /* fraction bits of the positions */
     int nbx, nby, nbins;     /* bins; key nbins = not in the deposit region */
-    long long nchunks_cap;
-    int* counts;             /* [key][chunk] */
-    int* offs;               /* [key][chunk] exclusive within the key */
+    int* counts;             /* [chunk][key] */
+    int* offs;               /* [chunk][key] exclusive within the key */
     int* key_total;          /* [key] */
     long long* key_start;    /* [key+1] padded starts */
-    int* tile_bin;           /* [tile] */
     int4* pieces;            /* {first tile, tiles, bin, 0} */
     int piece_tiles;
 };
@@ -50,7 +54,7 @@ __device__ __forceinline__ int bin_key(float4 p, int nx, int ny, int ps, int nbx
     return (kp / PGB_BIN) * nbx + (jp / PGB_BIN);
 }
 
-__global__ void __launch_bounds__(256) k_sort_count(SortArgs a) {
+__global__ void __launch_bounds__(512) k_sort_count(SortArgs a) {
     pgb_pdl_entry();
     extern __shared__ int s_hist[];
     const long long n = a.ds->n[a.s];
@@ -58,14 +62,19 @@ __global__ void __launch_bounds__(256) k_sort_count(SortArgs a) {
     for (int c = blockIdx.x; c < nch; c += gridDim.x) {
         for (int k = threadIdx.x; k <= a.nbins; k += blockDim.x) s_hist[k] = 0;
         __syncthreads();
-        for (int k = threadIdx.x; k < SORT_CHUNK; k += blockDim.x) {
-            long long i = (long long)c * SORT_CHUNK + k;
-            if (i >= n) break;
-            int key = bin_key(a.S.xv[i], a.nx, a.ny, a.ps, a.nbx, a.nbins);
+        float4 p[SORT_CHUNK / 512];
+#pragma unroll
+        for (int q = 0; q < SORT_CHUNK / 512; ++q) {
+            const long long i = (long long)c * SORT_CHUNK + q * 512 + threadIdx.x;
+            p[q] = i < n ? a.S.xv[i] : make_float4(pos_dead(), 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int q = 0; q < SORT_CHUNK / 512; ++q) {
+            const int key = bin_key(p[q], a.nx, a.ny, a.ps, a.nbx, a.nbins);
             if (key >= 0) atomicAdd(&s_hist[key], 1);
         }
         __syncthreads();
-        for (int k = threadIdx.x; k <= a.nbins; k += blockDim.x) a.counts[(long long)k * a.nchunks_cap + c] = s_hist[k];
+        for (int k = threadIdx.x; k <= a.nbins; k += blockDim.x) a.counts[(long long)c * (a.nbins + 1) + k] = s_hist[k];
         __syncthreads();
     }
 }
@@ -96,44 +105,61 @@ __device__ __forceinline__ long long block_excl_scan_ll(long long v, long long* 
     return before + x - v;
 }
 
-/* per key: exclusive scan over the live chunks (one CTA per key) */
+/* per key: exclusive scan over the chunks.  A CTA takes 32 keys (a lane
+ * each), a warp a run of chunks: sums, a scan over the warps, offsets.   */
 __global__ void __launch_bounds__(1024) k_sort_scan_keys(SortArgs a) {
     pgb_pdl_entry();
+    __shared__ int s_sum[32][33];
     const long long n = a.ds->n[a.s];
-    const int nch = (int)((n + SORT_CHUNK - 1) / SORT_CHUNK);
-    __shared__ long long s_w[32];
-    for (int key = blockIdx.x; key <= a.nbins; key += gridDim.x) {
-        const int* row = a.counts + (long long)key * a.nchunks_cap;
-        int* out = a.offs + (long long)key * a.nchunks_cap;
-        long long carry = 0;
-        for (int b = 0; b < nch; b += blockDim.x) {
-            int c = b + threadIdx.x;
-            long long v = c < nch ? row[c] : 0, tot;
-            long long ex = block_excl_scan_ll(v, s_w, tot);
-            if (c < nch) out[c] = (int)(carry + ex);
-            carry += tot;
+    const int nch = (int)((n + SORT_CHUNK - 1) / SORT_CHUNK), nk = a.nbins + 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int key = blockIdx.x * 32 + lane;
+    const int per = (nch + 31) / 32, c0 = min(warp * per, nch), c1 = min(c0 + per, nch);
+    int sum = 0;
+    if (key < nk) {
+#pragma unroll 8
+        for (int c = c0; c < c1; ++c) sum += a.counts[(long long)c * nk + key];
+    }
+    s_sum[warp][lane] = sum;
+    __syncthreads();
+    if (warp == 0) {
+        int acc = 0;
+        for (int w = 0; w < 32; ++w) {
+            const int v = s_sum[w][lane];
+            s_sum[w][lane] = acc;
+            acc += v;
         }
-        if (threadIdx.x == 0) a.key_total[key] = (int)carry;
+        if (key < nk) a.key_total[key] = acc;
+    }
+    __syncthreads();
+    if (key >= nk) return;
+    int acc = s_sum[warp][lane];
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) {
+        const int v = a.counts[(long long)c * nk + key];
+        a.offs[(long long)c * nk + key] = acc;
+        acc += v;
     }
 }
 
 /* over keys: padded starts (each key begins on a tile boundary), pieces.
- * One CTA scans the keys 1024 at a time (tiles and pieces per key), each
- * key's thread writes its pieces, then every tile finds its key by binary
- * search over the starts.                                               */
+ * One CTA scans the keys 1024 at a time (tiles and pieces per key) and
+ * each key's thread writes its pieces.                                   */
 __global__ void __launch_bounds__(1024) k_sort_scan_bins(SortArgs a) {
     pgb_pdl_entry();
     __shared__ long long s_w[32];
-    long long carry_t = 0, carry_p = 0;
+    long long carry_t = 0, carry_p = 0, live = 0;
     for (int base = 0; base <= a.nbins; base += blockDim.x) {
         const int key = base + threadIdx.x;
-        long long tiles = 0, np = 0;
+        long long tiles = 0, np = 0, c = 0;
         if (key <= a.nbins) {
-            long long c = a.key_total[key];
+            c = a.key_total[key];
             tiles = (c + PGB_TILE - 1) / PGB_TILE;
             np = (tiles + a.piece_tiles - 1) / a.piece_tiles;
         }
-        long long tot_t, tot_p;
+        long long tot_t, tot_p, tot_c;
+        (void)block_excl_scan_ll(c, s_w, tot_c);
+        live += tot_c;
         long long t0 = carry_t + block_excl_scan_ll(tiles, s_w, tot_t);
         long long p0 = carry_p + block_excl_scan_ll(np, s_w, tot_p);
         if (key <= a.nbins) {
@@ -152,42 +178,47 @@ __global__ void __launch_bounds__(1024) k_sort_scan_bins(SortArgs a) {
      * tiles.  If they do not fit the capacity, the sort copies the
      * particles in their current order instead (no pieces, no padding) and
      * the step reports the capacity error.                              */
-    __shared__ int s_over;
     if (threadIdx.x == 0) {
         const int over = carry_t * PGB_TILE > a.S.cap ? 1 : 0;
-        s_over = over;
         a.ds->sort_overflow = over;
+        a.ds->list_n[LIST_SPARE] = live;
         a.key_start[a.nbins + 1] = carry_t * PGB_TILE;
         a.ds->n_pieces[a.s] = over ? 0 : (int)carry_p;
         a.ds->sorted_tiles[a.s] = over ? 0 : carry_t;
         if (over) atomicOr(&a.ds->err, a.s == 0 ? ERR_CAP_E : ERR_CAP_I);
     }
-    __syncthreads();
-    if (s_over) return;
-    /* tile -> bin map: the key whose [start, next start) holds the tile */
-    for (long long t = threadIdx.x; t < carry_t; t += blockDim.x) {
-        const long long slot = t * PGB_TILE;
-        int lo = 0, hi = a.nbins;   /* largest key with key_start <= slot */
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (a.key_start[mid] <= slot) lo = mid;
-            else hi = mid - 1;
-        }
-        a.tile_bin[t] = lo < a.nbins ? lo : -1;
-    }
 }
 
-/* one warp per chunk: stable placement at per-key cursors.  Four batches of
- * 32 slots are loaded at once (memory-level parallelism), then placed in
- * slot order.                                                           */
-#define SCATTER_BATCHES 4
-__global__ void __launch_bounds__(256) k_sort_scatter(SortArgs a) {
+/* One CTA per chunk of SORT_CHUNK slots.  A warp takes 256 consecutive
+ * slots, 32 at a time: a particle's rank within its warp is the warp's
+ * running count of its key plus the lanes of the same key before it; the
+ * warps' counts are then scanned per key and the keys over the chunk, which
+ * gives each particle its place in the sorted chunk.  The particles go
+ * there in shared memory and leave from there, bin after bin.            */
+#define SORT_THREADS 512
+#define SORT_WARPS (SORT_THREADS / 32)
+#define SORT_ITEMS (SORT_CHUNK / SORT_THREADS)
+static_assert(SORT_CHUNK <= 65536, "ranks within a chunk are 16 bits");
+/* dynamic shared memory: the staged particles, their keys, the counts per
+ * warp and key, the destination of each key's run                        */
+static size_t sort_smem(int nkeys) {
+    const size_t w = ((size_t)nkeys * SORT_WARPS * sizeof(unsigned short) + 15) & ~(size_t)15;
+    return SORT_CHUNK * (sizeof(float4) + sizeof(unsigned short)) + w + (size_t)nkeys * sizeof(long long);
+}
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SortArgs a) {
     pgb_pdl_entry();
-    extern __shared__ long long s_cur[];   /* [warp][key] */
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const int nk = a.nbins + 1;
+    float4* const s_xv = reinterpret_cast<float4*>(s_raw);
+    unsigned short* const s_key = reinterpret_cast<unsigned short*>(s_raw + SORT_CHUNK * sizeof(float4));
+    unsigned short* const s_cnt = s_key + SORT_CHUNK;   /* [warp][key] */
+    long long* const s_dst = reinterpret_cast<long long*>(
+        s_raw + SORT_CHUNK * (sizeof(float4) + sizeof(unsigned short)) +
+        (((size_t)nk * SORT_WARPS * sizeof(unsigned short) + 15) & ~(size_t)15));
+    __shared__ int s_w[SORT_WARPS];
     const long long n = a.ds->n[a.s];
     const int nch = (int)((n + SORT_CHUNK - 1) / SORT_CHUNK);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    long long* cur = s_cur + (long long)warp * (a.nbins + 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     if (a.ds->sort_overflow) {
         /* the padded layout does not fit: keep the order (and the slots) */
@@ -199,43 +230,109 @@ __global__ void __launch_bounds__(256) k_sort_scatter(SortArgs a) {
         }
         return;
     }
-    for (int c = blockIdx.x * nw + warp; c < nch; c += gridDim.x * nw) {
-        for (int k = lane; k <= a.nbins; k += 32) cur[k] = a.key_start[k] + a.offs[(long long)k * a.nchunks_cap + c];
-        __syncwarp();
-        for (int b = 0; b < SORT_CHUNK; b += 32 * SCATTER_BATCHES) {
-            float4 p[SCATTER_BATCHES];
-            float vz[SCATTER_BATCHES], w[SCATTER_BATCHES];
-            unsigned int id[SCATTER_BATCHES];
-            int key[SCATTER_BATCHES];
+    for (int c = blockIdx.x; c < nch; c += gridDim.x) {
+        const long long base = (long long)c * SORT_CHUNK + warp * (32 * SORT_ITEMS) + lane;
+        float4 p[SORT_ITEMS];
 #pragma unroll
-            for (int u = 0; u < SCATTER_BATCHES; ++u) {
-                long long i = (long long)c * SORT_CHUNK + b + u * 32 + lane;
-                key[u] = -1;
-                if (i < n) {
-                    p[u] = a.S.xv[i];
-                    vz[u] = a.S.vz[i];
-                    w[u] = a.S.w[i];
-                    id[u] = a.S.id[i];
-                    key[u] = bin_key(p[u], a.nx, a.ny, a.ps, a.nbx, a.nbins);
+        for (int q = 0; q < SORT_ITEMS; ++q) {
+            const long long i = base + 32 * q;
+            p[q] = i < n ? a.S.xv[i] : make_float4(pos_dead(), 0.f, 0.f, 0.f);
+        }
+        for (int k = threadIdx.x; k < nk * SORT_WARPS; k += SORT_THREADS) s_cnt[k] = 0;
+        __syncthreads();
+        int key[SORT_ITEMS], pos[SORT_ITEMS];
+        unsigned short* const cnt = s_cnt + warp * nk;
+#pragma unroll
+        for (int q = 0; q < SORT_ITEMS; ++q) {
+            key[q] = bin_key(p[q], a.nx, a.ny, a.ps, a.nbx, a.nbins);
+            const unsigned peers = __match_any_sync(0xffffffffu, key[q]);
+            pos[q] = key[q] >= 0 ? cnt[key[q]] + __popc(peers & lt) : -1;
+            __syncwarp();
+            if (key[q] >= 0 && (peers & lt) == 0) cnt[key[q]] = (unsigned short)(cnt[key[q]] + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        /* per key: exclusive over the warps; over the keys: exclusive */
+        int carry = 0;
+        for (int b = 0; b < nk; b += SORT_THREADS) {
+            const int k = b + threadIdx.x;
+            int tot = 0;
+            if (k < nk)
+                for (int w = 0; w < SORT_WARPS; ++w) {
+                    const int v = s_cnt[w * nk + k];
+                    s_cnt[w * nk + k] = (unsigned short)tot;
+                    tot += v;
                 }
+            int x = tot;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += y;
             }
+            if (lane == 31) s_w[warp] = x;
+            __syncthreads();
+            int before = 0, all = 0;
 #pragma unroll
-            for (int u = 0; u < SCATTER_BATCHES; ++u) {
-                unsigned peers = __match_any_sync(0xffffffffu, key[u]);
-                long long pos = -1;
-                if (key[u] >= 0) pos = cur[key[u]] + __popc(peers & lt);
-                __syncwarp();
-                if (key[u] >= 0 && (peers & lt) == 0) cur[key[u]] += __popc(peers);
-                __syncwarp();
-                if (key[u] >= 0 && pos < a.S.cap) {
-                    a.S.xv2[pos] = p[u];
-                    a.S.vz2[pos] = vz[u];
-                    a.S.w2[pos] = w[u];
-                    a.S.id2[pos] = id[u];
-                }
+            for (int w = 0; w < SORT_WARPS; ++w) {
+                if (w < warp) before += s_w[w];
+                all += s_w[w];
+            }
+            const int start = carry + before + x - tot;   /* of key k in the sorted chunk */
+            if (k < nk) {
+                for (int w = 0; w < SORT_WARPS; ++w) s_cnt[w * nk + k] = (unsigned short)(s_cnt[w * nk + k] + start);
+                s_dst[k] = a.key_start[k] + a.offs[(long long)c * nk + k] - start;
+            }
+            carry += all;
+            __syncthreads();
+        }
+        /* positions and in-plane velocities */
+#pragma unroll
+        for (int q = 0; q < SORT_ITEMS; ++q)
+            if (pos[q] >= 0) {
+                pos[q] += cnt[key[q]];
+                s_xv[pos[q]] = p[q];
+                s_key[pos[q]] = (unsigned short)key[q];
+            }
+        float vz[SORT_ITEMS], wt[SORT_ITEMS];
+        unsigned int id[SORT_ITEMS];
+#pragma unroll
+        for (int q = 0; q < SORT_ITEMS; ++q) {
+            const long long i = base + 32 * q;
+            vz[q] = wt[q] = 0.f;
+            id[q] = 0u;
+            if (pos[q] >= 0) {
+                vz[q] = a.S.vz[i];
+                wt[q] = a.S.w[i];
+                id[q] = a.S.id[i];
             }
         }
-        __syncwarp();
+        __syncthreads();
+        for (int j = threadIdx.x; j < carry; j += SORT_THREADS) {
+            const long long d = j + s_dst[s_key[j]];
+            if (d < a.S.cap) a.S.xv2[d] = s_xv[j];
+        }
+        __syncthreads();
+        /* the other three arrays in the same space */
+        float* const s_vz = reinterpret_cast<float*>(s_raw);
+        float* const s_wt = s_vz + SORT_CHUNK;
+        unsigned int* const s_id = reinterpret_cast<unsigned int*>(s_wt + SORT_CHUNK);
+#pragma unroll
+        for (int q = 0; q < SORT_ITEMS; ++q)
+            if (pos[q] >= 0) {
+                s_vz[pos[q]] = vz[q];
+                s_wt[pos[q]] = wt[q];
+                s_id[pos[q]] = id[q];
+            }
+        __syncthreads();
+        for (int j = threadIdx.x; j < carry; j += SORT_THREADS) {
+            const long long d = j + s_dst[s_key[j]];
+            if (d < a.S.cap) {
+                a.S.vz2[d] = s_vz[j];
+                a.S.w2[d] = s_wt[j];
+                a.S.id2[d] = s_id[j];
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -253,8 +350,7 @@ __global__ void k_sort_pad(SortArgs a) {
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        long long live = 0;
-        for (int key = 0; key <= a.nbins; ++key) live += a.key_total[key];
+        const long long live = a.ds->list_n[LIST_SPARE];
         long long tot = a.key_start[a.nbins + 1];
         a.ds->n[a.s] = tot;
         a.ds->dead[a.s] = tot - live;
@@ -272,22 +368,16 @@ int pgb_launch_sort(pgb_run* r, int s) {
     a.S = r->sp[s]; a.ds = r->ds; a.s = s; a.nx = r->nx; a.ny = r->ny; a.ps = r->ps;
     pgb_bins(r, &a.nbx, &a.nby);
     a.nbins = a.nbx * a.nby;
-    a.nchunks_cap = r->sort_chunks_cap;
     a.counts = r->sort_counts; a.offs = r->sort_offs; a.key_total = r->sort_key_total;
-    a.key_start = r->sort_key_start; a.tile_bin = r->tile_bin[s]; a.pieces = r->pieces[s];
+    a.key_start = r->sort_key_start; a.pieces = r->pieces[s];
     a.piece_tiles = PGB_PIECE_TILES;
-    size_t hist = sizeof(int) * (a.nbins + 1);
-    PGB_CK(r, pgb_launch_pdl(k_sort_count, dim3(r->sms * 4), dim3(256), hist, r->stream, a));
-    r->launches++;
-    PGB_CK(r, pgb_launch_pdl(k_sort_scan_keys, dim3(r->sms * 2), dim3(1024), 0, r->stream, a));
-    r->launches++;
+    const int nk = a.nbins + 1;
+    PGB_CK(r, pgb_launch_pdl(k_sort_count, dim3(r->sms * 4), dim3(512), sizeof(int) * nk, r->stream, a));
+    PGB_CK(r, pgb_launch_pdl(k_sort_scan_keys, dim3((nk + 31) / 32), dim3(1024), 0, r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_sort_scan_bins, dim3(1), dim3(1024), 0, r->stream, a));
-    r->launches++;
-    size_t cur = sizeof(long long) * (a.nbins + 1) * 8;
-    PGB_CK(r, pgb_launch_pdl(k_sort_scatter, dim3(r->sms * 4), dim3(256), cur, r->stream, a));
-    r->launches++;
+    PGB_CK(r, pgb_launch_pdl(k_sort_scatter, dim3(r->sms * 2), dim3(SORT_THREADS), sort_smem(nk), r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_sort_pad, dim3(r->sms), dim3(256), 0, r->stream, a));
-    r->launches++;
+    r->launches += 5;
     PGB_CK(r, cudaGetLastError());
     Species& S = r->sp[s];
     std::swap(S.xv, S.xv2);
@@ -300,10 +390,14 @@ int pgb_launch_sort(pgb_run* r, int s) {
 int pgb_sort_setup(pgb_run* r) {
     int nbx, nby;
     pgb_bins(r, &nbx, &nby);
-    int nbins = nbx * nby;
-    size_t cur = sizeof(long long) * (nbins + 1) * 8;
-    if (cur > 48 * 1024) PGB_CK(r, cudaFuncSetAttribute(k_sort_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cur));
-    size_t hist = sizeof(int) * (nbins + 1);
+    const int nk = nbx * nby + 1;
+    /* the limit belongs to the kernel, which runs of every grid share: it is
+     * set to the most any of them may ask for (a grid that asks for more is
+     * refused here)                                                       */
+    const size_t most = 224 * 1024;
+    PGB_CK(r, cudaFuncSetAttribute(k_sort_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(sort_smem(nk) > most ? sort_smem(nk) : most)));
+    size_t hist = sizeof(int) * nk;
     if (hist > 48 * 1024) PGB_CK(r, cudaFuncSetAttribute(k_sort_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist));
     return 0;
 }
