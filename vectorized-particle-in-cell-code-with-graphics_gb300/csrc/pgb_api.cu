@@ -711,7 +711,7 @@ extern "C" int pgb_collide_electrons(pgb_run* r) {
     int rc = need_particles(r);
     if (rc) return rc;
     if ((rc = set_device_step(r, r->time_step, 1))) return rc;
-    if (pgb_launch_mcc(r, 0) || pgb_launch_scatter(r, 0) || pgb_build_list(r, LIST_ION_EV, 0) ||
+    if (pgb_launch_mcc(r, 0) || pgb_build_list(r, LIST_ION_EV, 0) ||
         pgb_launch_ionize_appends(r, 1, 1))
         return PGB_ERR_CUDA;
     return sync_state(r);
@@ -864,11 +864,6 @@ static int collide_lanes(Lanes& L, int leave_sms, bool ion_step) {
     const bool products = products_stored(r, ion_step);
     if (pgb_launch_mcc(r, leave_sms, !products)) return PGB_ERR_CUDA;
     PROF_MARK(r, 9);
-    /* the field solve beside the collisions ends before the collision test
-     * does (0.11 against 0.15 ms at 513^2): the kernels after the test take
-     * every SM (their blocks queue behind the solve's, which have the
-     * higher priority, when it has not ended)                             */
-    if (pgb_launch_scatter(r, 0)) return PGB_ERR_CUDA;
     PROF_MARK(r, 10);
     if (products && pgb_build_list(r, LIST_ION_EV, 0)) return PGB_ERR_CUDA;
     PROF_MARK(r, 11);

@@ -67,7 +67,6 @@ struct DevState {
                                 step's collisions                                      */
     unsigned int ticket;     /* blocks of a wall kernel that are done            */
     unsigned int pad3;
-    unsigned long long scat_n;   /* scattering events queued by the collision pass */
     long long n_cx;          /* ion slots whose charge exchange was tested before this
                                 step's appends (the rest are tested after them)       */
 };
@@ -307,7 +306,6 @@ int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit = 0)
 int pgb_launch_ionize_appends(pgb_run* r, int store_e, int store_i);
 /* count_events: ds->list_n[LIST_ION_EV] counts the ionization events (from 0) */
 int pgb_launch_mcc(pgb_run* r, int leave_sms, bool count_events = false);
-int pgb_launch_scatter(pgb_run* r, int leave_sms);
 /* tail 0: the ions present (records their count); 1: those appended since;
  * 2: the same in one block, for a tail of a few thousand ions at most     */
 int pgb_launch_cx(pgb_run* r, int tail, int leave_sms);

@@ -10,8 +10,8 @@
  * (particle.cpp:491-510).
  *
  * k_mcc reads each electron (16 B position/velocity, 4 B vz, 4 B id) for
- * the collision test and writes back only the ~5% whose velocity changes;
- * it reads no field, so it runs beside the previous step's field solve.
+ * the collision test, and handles and writes back the ~5% whose velocity
+ * changes; it reads no field, so it runs beside the previous step's field solve.
  * One pass of k_push then reads a particle once (16 B, plus 4 B vz with a
  * magnetic field and 4 B weight), gathers E bilinearly from the FP32 node
  * grid (L2 resident), pushes, deposits the new position into the int64
@@ -44,7 +44,6 @@ struct PushArgs {
     int* tc_out;
     int* tl_ev;                 /* per-tile ionization-event list     */
     int* tc_ev;
-    int count_ev;               /* count the ionization events here (no list is built) */
 };
 
 /* gather (pic.cl:56-92) + push (pic.cl:95-149) of one particle in cell units */
@@ -162,13 +161,17 @@ __device__ __forceinline__ void mcc_ionize(const CollConsts& cc, const float* ne
     }
 }
 
-/* add per-thread event counts (elastic, ionization) with one atomic per warp */
-__device__ __forceinline__ void flush_stats(int (&st)[2], long long* stats) {
+/* add per-thread event counts (elastic, ionization) with one atomic per
+ * warp; the ionizations also to *events, if given                        */
+__device__ __forceinline__ void flush_stats(int (&st)[2], long long* stats, long long* events) {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         int v = st[k];
         for (int d = 16; d; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-        if ((threadIdx.x & 31) == 0 && v) atomicAdd((unsigned long long*)&stats[ST_ELASTIC + k], (unsigned long long)v);
+        if ((threadIdx.x & 31) == 0 && v) {
+            atomicAdd((unsigned long long*)&stats[ST_ELASTIC + k], (unsigned long long)v);
+            if (k == 1 && events) atomicAdd((unsigned long long*)events, (unsigned long long)v);
+        }
     }
 }
 
@@ -380,180 +383,78 @@ __global__ void __launch_bounds__(256) k_deposit(const float4* xv, const float* 
     }
 }
 
-/* e_collisions::collision (e_collisions.cpp:480-597) in two kernels, the
- * first of a step.  They read no field, so they run while the previous
- * step's field solve is still in flight.
- *   k_mcc      the collision test of every electron; the ionizations of
- *              electrons that do not also scatter; the ordered per-tile
- *              list of ionization events; the scattering events (about one
- *              electron in twenty) appended, unordered, to a dense list
- *   k_scatter  one thread per listed event: the scattering, then the
- *              ionization of the parent if it also ionizes
+/* e_collisions::collision (e_collisions.cpp:480-597), the first kernel of a
+ * step: the collision test of every electron, the scatterings (about one
+ * electron in twenty), the ionizations' effect on their parents, and the
+ * ionization events' number or their ordered per-tile list.  It reads no
+ * field, so it runs while the previous step's field solve is in flight.
  * Each event touches only its own electron and draws from that electron's
- * stream, so the order of the scattering list changes nothing.
+ * stream, so the order in which events are handled changes nothing.
  *
- * A block is MCC_GROUPS independent groups of 256 threads, each with its
- * own list scratch and named barrier, each taking one tile at a time.  At
- * 64 registers a thread the block fills an SM's register file, so a grid
- * of sms - k blocks leaves k SMs wholly free: the field solve's one-CTA
- * multigrid (1024 threads) needs an SM of its own.                       */
-#define MCC_GROUPS 4
+ * Every warp works alone, on 128 consecutive slots at a time:
+ *   (1) every electron: the domain test, |v|^2, the Philox draw R and
+ *       mcc_candidate; the candidates (about one in ten at a few eV) go to
+ *       the warp's queue in shared memory;
+ *   (2) whenever 32 candidates wait, one per lane: the cross-sections, the
+ *       exponential and the decisions of mcc_decide; the scatterings go to
+ *       a second queue;
+ *   (3) whenever 32 scatterings wait, one per lane: the electron (read
+ *       again, from L1 or L2) scatters and, if it also ionizes, ionizes.
+ * Bound by instruction issue: one Philox4x32-10 block per electron is
+ * about half of it.  With a tile per 256 threads, queues per tile, five
+ * barriers a tile and the scatterings in a kernel of their own it took 145
+ * + 28 us at 16 Mi electrons.
+ *
+ * At 64 registers a thread a block fills an SM's register file, so a grid
+ * of sms - k blocks leaves k SMs wholly free for the field solve beside it. */
+#define MCC_GROUPS 4                                    /* tiles a block has in work  */
 #define MCC_THREADS (MCC_GROUPS * PGB_PUSH_THREADS)
+#define MCC_WARPS (MCC_THREADS / 32)
+#define MCC_UNIT 128                                    /* slots of a warp at a time  */
 #define MCC_ION_BIT 0x80000000u
-struct MccGroupSmem {
-    int off[PGB_ITEMS][PGB_PUSH_THREADS / 32];    /* ionization events per (item, warp) */
-    int soff[PGB_ITEMS][PGB_PUSH_THREADS / 32];   /* scattering events per (item, warp) */
-    unsigned long long sbase;                      /* the tile's first scattering-list entry */
-    int qn;                                        /* candidates queued                      */
-    float qu2[PGB_TILE];                           /* candidate |v|^2, R and tile position   */
-    float qr[PGB_TILE];
-    unsigned short qi[PGB_TILE];
-    unsigned char ev[PGB_TILE];                    /* decisions by tile position             */
+static_assert(MCC_UNIT * (PGB_PUSH_THREADS / 32) == PGB_TILE, "eight warps share a tile");
+struct MccQueue {
+    float u2[32 + MCC_UNIT], r[32 + MCC_UNIT];   /* candidates: |v|^2, R, slot */
+    int slot[32 + MCC_UNIT];
+    unsigned scat[64];                           /* scatterings: slot | MCC_ION_BIT */
 };
-static_assert(MCC_GROUPS * sizeof(MccGroupSmem) <= 48 * 1024, "static shared memory");
-__device__ __forceinline__ void group_sync(int g) {
-    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(PGB_PUSH_THREADS) : "memory");
-}
-/* A tile in three passes.  (1) Every electron: the domain test, |v|^2,
- * the Philox draw R and mcc_candidate; the candidates (about one in ten
- * at a few eV) are queued.  (2) The queue, one candidate per thread: the
- * cross-sections, the exponential and the decisions of mcc_decide, so
- * that the fits run densely instead of in every warp that holds one
- * candidate.  (3) Every electron takes its decisions back in slot order
- * for the lists.                                                         */
-__global__ void __launch_bounds__(MCC_THREADS, 1) k_mcc(PushArgs a, int* scat) {
-    pgb_pdl_entry();
-    __shared__ MccGroupSmem s_grp[MCC_GROUPS];
-    const int g = threadIdx.x / PGB_PUSH_THREADS, t = threadIdx.x % PGB_PUSH_THREADS;
-    const int lane = t & 31, warp = t >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    MccGroupSmem& S = s_grp[g];
-    const long long n = a.ds->n[0];
-    const int ntiles = (int)((n + PGB_TILE - 1) / PGB_TILE);
-    const unsigned step = (unsigned)a.ds->t;
-    int st_loc[2] = {0, 0};
-    if (t == 0) S.qn = 0;
-    group_sync(g);
-    for (int tile = blockIdx.x * MCC_GROUPS + g; tile < ntiles; tile += gridDim.x * MCC_GROUPS) {
-        const long long base = (long long)tile * PGB_TILE;
-        /* (1) all loads of the thread's items first, then the draws */
-        float4 pa[PGB_ITEMS];
-        float vza[PGB_ITEMS];
-        unsigned int ida[PGB_ITEMS];
-#pragma unroll
-        for (int k = 0; k < PGB_ITEMS; ++k) {
-            long long i = base + k * PGB_PUSH_THREADS + t;
-            pa[k] = make_float4(pos_dead(), 0.0f, 0.0f, 0.0f);
-            vza[k] = 0.0f;
-            ida[k] = 0u;
-            if (i < n) {
-                pa[k] = a.xv[i];
-                vza[k] = a.vz[i];
-                ida[k] = a.id[i];
-            }
-        }
-        unsigned cand = 0;   /* bit k: item k is queued */
-#pragma unroll
-        for (int k = 0; k < PGB_ITEMS; ++k) {
-            float u2 = 0.0f, R = 1.0f;
-            bool c = false;
-            if (!is_dead(pa[k].x) && mcc_draw(a.cc, ida[k], step, a.pc.nx, a.pc.ny, a.pc.ps, pa[k], vza[k], u2, R))
-                c = mcc_candidate(a.cc, u2, R);
-            const unsigned cm = __ballot_sync(0xffffffffu, c);
-            int qb = 0;
-            if (lane == 0 && cm) qb = atomicAdd(&S.qn, __popc(cm));
-            qb = __shfl_sync(0xffffffffu, qb, 0);
-            if (c) {
-                const int q = qb + __popc(cm & lt);
-                S.qu2[q] = u2;
-                S.qr[q] = R;
-                S.qi[q] = (unsigned short)(k * PGB_PUSH_THREADS + t);
-                cand |= 1u << k;
-            }
-        }
-        group_sync(g);
-        /* (2) the queued candidates, densely */
-        {
-            const int qn = S.qn;
-            for (int q = t; q < qn; q += PGB_PUSH_THREADS) S.ev[S.qi[q]] = (unsigned char)mcc_decide(a.cc, S.qu2[q], S.qr[q]);
-        }
-        group_sync(g);
-        /* (3) decisions back in slot order */
-        if (t == 0) S.qn = 0;   /* every thread has read it before the barrier */
-        bool f[PGB_ITEMS], sc[PGB_ITEMS];
-#pragma unroll
-        for (int k = 0; k < PGB_ITEMS; ++k) {
-            const int i = (int)(base + k * PGB_PUSH_THREADS + t);
-            const int ev = (cand >> k) & 1u ? S.ev[k * PGB_PUSH_THREADS + t] : 0;
-            sc[k] = (ev & MCC_SCATTER) != 0;
-            f[k] = (ev & MCC_IONIZE) != 0;
-            st_loc[0] += sc[k] ? 1 : 0;
-            st_loc[1] += f[k] ? 1 : 0;
-            /* an ionization without scattering is applied here (rare: the
-             * electron is read again rather than held through the passes) */
-            if (f[k] && !sc[k]) {
-                float4 p = a.xv[i];
-                float vz = a.vz[i];
-                mcc_ionize(a.cc, a.neut, a.id[i], step, p, vz);
-                a.xv[i] = p;
-                a.vz[i] = vz;
-            }
-        }
-        /* the tile's ionization events in slot order (as tile_masks), and its
-         * scattering events appended to the dense list with one counter
-         * update for the tile (a counter update per warp serialised some
-         * 400k atomics on one address per launch)                        */
-        unsigned m[PGB_ITEMS], ms[PGB_ITEMS];
-#pragma unroll
-        for (int k = 0; k < PGB_ITEMS; ++k) {
-            m[k] = __ballot_sync(0xffffffffu, f[k]);
-            ms[k] = __ballot_sync(0xffffffffu, sc[k]);
-            if (lane == 0) {
-                S.off[k][warp] = __popc(m[k]);
-                S.soff[k][warp] = __popc(ms[k]);
-            }
-        }
-        group_sync(g);
-        /* exclusive scans of the group's 32 (item, warp) counts by its first
-         * warp, in (item, warp) order, which is slot order                */
-        static_assert(PGB_ITEMS * (PGB_PUSH_THREADS / 32) == 32, "one count per lane");
-        if (warp == 0) {
-            int* const io = &S.off[0][0];
-            int* const so = &S.soff[0][0];
-            const int c = io[lane], d = so[lane];
-            int x = c, y = d;
-#pragma unroll
-            for (int dd = 1; dd < 32; dd <<= 1) {
-                const int xu = __shfl_up_sync(0xffffffffu, x, dd), yu = __shfl_up_sync(0xffffffffu, y, dd);
-                if (lane >= dd) { x += xu; y += yu; }
-            }
-            io[lane] = x - c;
-            so[lane] = y - d;
-            if (lane == 31) {
-                a.tc_ev[tile] = x;
-                if (a.count_ev && x) atomicAdd((unsigned long long*)&a.ds->list_n[LIST_ION_EV], (unsigned long long)x);
-                S.sbase = y ? atomicAdd(&a.ds->scat_n, (unsigned long long)y) : 0ull;
-            }
-        }
-        group_sync(g);
-#pragma unroll
-        for (int k = 0; k < PGB_ITEMS; ++k) {
-            const int i = (int)(base + k * PGB_PUSH_THREADS + t);
-            /* the ionization events as the tile's mask words (tile_masks) */
-            if (lane == 0) ((unsigned*)a.tl_ev)[(long long)tile * 32 + k * (PGB_PUSH_THREADS / 32) + warp] = m[k];
-            if (sc[k]) scat[S.sbase + S.soff[k][warp] + __popc(ms[k] & lt)] = (int)((unsigned)i | (f[k] ? MCC_ION_BIT : 0u));
-        }
-        group_sync(g);
+/* one candidate per lane of the first m: decisions; returns the number of
+ * scatterings queued                                                     */
+__device__ __forceinline__ int mcc_candidates(const PushArgs& a, MccQueue& Q, int base, int m, int nscat, unsigned step,
+                                              int (&st)[2], bool list) {
+    const int lane = threadIdx.x & 31;
+    int ev = 0, slot = 0;
+    if (lane < m) {
+        slot = Q.slot[base + lane];
+        ev = mcc_decide(a.cc, Q.u2[base + lane], Q.r[base + lane]);
     }
-    flush_stats(st_loc, a.ds->stats);
+    const bool sc = (ev & MCC_SCATTER) != 0, io = (ev & MCC_IONIZE) != 0;
+    st[0] += sc ? 1 : 0;
+    st[1] += io ? 1 : 0;
+    if (io) {
+        if (list) {
+            /* slot order: word slot/32 of the lists, bit slot%32 (tile_masks) */
+            atomicOr((unsigned*)a.tl_ev + (slot >> 5), 1u << (slot & 31));
+            atomicAdd(a.tc_ev + slot / PGB_TILE, 1);
+        }
+        if (!sc) {
+            float4 p = a.xv[slot];
+            float vz = a.vz[slot];
+            mcc_ionize(a.cc, a.neut, a.id[slot], step, p, vz);
+            a.xv[slot] = p;
+            a.vz[slot] = vz;
+        }
+    }
+    const unsigned ms = __ballot_sync(0xffffffffu, sc);
+    if (sc) Q.scat[nscat + __popc(ms & ((1u << lane) - 1u))] = (unsigned)slot | (io ? MCC_ION_BIT : 0u);
+    __syncwarp();
+    return nscat + __popc(ms);
 }
-
-__global__ void __launch_bounds__(MCC_THREADS, 1) k_scatter(PushArgs a, const int* scat) {
-    pgb_pdl_entry();
-    const long long m = (long long)a.ds->scat_n;
-    const unsigned step = (unsigned)a.ds->t;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < m; r += (long long)gridDim.x * blockDim.x) {
-        const unsigned e = (unsigned)scat[r];
+/* one scattering per lane of the first m */
+__device__ __forceinline__ void mcc_scatterings(const PushArgs& a, const MccQueue& Q, int base, int m, unsigned step) {
+    const int lane = threadIdx.x & 31;
+    if (lane < m) {
+        const unsigned e = Q.scat[base + lane];
         const int slot = (int)(e & ~MCC_ION_BIT);
         float4 p = a.xv[slot];
         float vz = a.vz[slot];
@@ -567,6 +468,69 @@ __global__ void __launch_bounds__(MCC_THREADS, 1) k_scatter(PushArgs a, const in
         a.xv[slot] = p;
         a.vz[slot] = vz;
     }
+    __syncwarp();
+}
+__global__ void __launch_bounds__(MCC_THREADS, 1) k_mcc(PushArgs a, int list) {
+    pgb_pdl_entry();
+    extern __shared__ __align__(16) unsigned char s_mcc[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    MccQueue& Q = reinterpret_cast<MccQueue*>(s_mcc)[warp];
+    const long long n = a.ds->n[0];
+    const int ntiles = (int)((n + PGB_TILE - 1) / PGB_TILE);
+    const unsigned step = (unsigned)a.ds->t;
+    int st_loc[2] = {0, 0};
+    int nc = 0, ns = 0;   /* candidates and scatterings queued */
+    for (int tile = blockIdx.x * MCC_GROUPS + (warp >> 3); tile < ntiles; tile += gridDim.x * MCC_GROUPS) {
+        const int base = tile * PGB_TILE + (warp & 7) * MCC_UNIT;
+        const int left = (int)min((long long)MCC_UNIT, n - base);   /* slots of this unit in use */
+        if (left <= 0 && !list) continue;
+        /* all loads of the lane's items first, then the draws */
+        float4 pa[MCC_UNIT / 32];
+        float vza[MCC_UNIT / 32];
+        unsigned int ida[MCC_UNIT / 32];
+#pragma unroll
+        for (int k = 0; k < MCC_UNIT / 32; ++k) {
+            const int o = k * 32 + lane;
+            pa[k] = make_float4(pos_dead(), 0.0f, 0.0f, 0.0f);
+            vza[k] = 0.0f;
+            ida[k] = 0u;
+            if (o < left) {
+                pa[k] = a.xv[base + o];
+                vza[k] = a.vz[base + o];
+                ida[k] = a.id[base + o];
+            }
+        }
+        if (list && lane < MCC_UNIT / 32) ((unsigned*)a.tl_ev)[(base >> 5) + lane] = 0u;
+#pragma unroll
+        for (int k = 0; k < MCC_UNIT / 32; ++k) {
+            float u2 = 0.0f, R = 1.0f;
+            bool c = false;
+            if (!is_dead(pa[k].x) && mcc_draw(a.cc, ida[k], step, a.pc.nx, a.pc.ny, a.pc.ps, pa[k], vza[k], u2, R))
+                c = mcc_candidate(a.cc, u2, R);
+            const unsigned cm = __ballot_sync(0xffffffffu, c);
+            if (c) {
+                const int q = nc + __popc(cm & lt);
+                Q.u2[q] = u2;
+                Q.r[q] = R;
+                Q.slot[q] = base + k * 32 + lane;
+            }
+            nc += __popc(cm);
+        }
+        __syncwarp();
+        /* the queues from their ends, so that what stays is in place */
+        while (nc >= 32) {
+            nc -= 32;
+            ns = mcc_candidates(a, Q, nc, 32, ns, step, st_loc, list);
+            if (ns >= 32) {
+                ns -= 32;
+                mcc_scatterings(a, Q, ns, 32, step);
+            }
+        }
+    }
+    if (nc) ns = mcc_candidates(a, Q, 0, nc, ns, step, st_loc, list);
+    for (int q = 0; q < ns; q += 32) mcc_scatterings(a, Q, q, min(32, ns - q), step);
+    flush_stats(st_loc, a.ds->stats, list ? nullptr : &a.ds->list_n[LIST_ION_EV]);
 }
 
 /* the last kernel of a step's particle phases moves the step counter on
@@ -1144,7 +1108,6 @@ static PushArgs push_args(pgb_run* r, int s) {
     a.tc_out = r->tile_cnt[s == 0 ? LIST_OUT_E : LIST_OUT_I];
     a.tl_ev = r->tile_list[LIST_ION_EV];
     a.tc_ev = r->tile_cnt[LIST_ION_EV];
-    a.count_ev = 0;
     return a;
 }
 
@@ -1174,31 +1137,18 @@ int pgb_launch_step_advance(pgb_run* r) {
     return 0;
 }
 
-/* leave_sms: SMs the collision kernels leave free (one block fills an SM).
- * Small runs take fewer blocks: one per MCC_GROUPS tiles for k_mcc, one per
- * 16 Ki electrons for k_scatter (about a scattering per thread), from the
- * electron count last read back; both kernels loop grid-stride.
- * The scattering list is the spare dense list (capacity >= electron slots). */
-static int mcc_blocks(pgb_run* r, int leave_sms, long long per_block) {
-    const long long n = std::max<long long>(r->hs->n[0], 0);
-    const long long want = std::max<long long>(1, (n + per_block - 1) / per_block);
-    return (int)std::min<long long>(std::max(1, r->sms - leave_sms), want);
-}
+/* leave_sms: SMs the collision kernel leaves free (one block fills an SM).
+ * Small runs take fewer blocks: one per MCC_GROUPS tiles, from the electron
+ * count last read back; the kernel loops over the tiles.                 */
 int pgb_launch_mcc(pgb_run* r, int leave_sms, bool count_events) {
     PushArgs a = push_args(r, 0);
-    a.count_ev = count_events;
-    const int g = mcc_blocks(r, leave_sms, (long long)MCC_GROUPS * PGB_TILE);
-    PGB_CK(r, cudaMemsetAsync(&r->ds->scat_n, 0, sizeof(unsigned long long), r->stream));
-    PGB_CK(r, pgb_launch_pdl(k_mcc, dim3(g), dim3(MCC_THREADS), 0, r->stream, a, r->list[LIST_SPARE]));
-    r->launches++;
-    PGB_CK(r, cudaGetLastError());
-    return 0;
-}
-
-int pgb_launch_scatter(pgb_run* r, int leave_sms) {
-    PushArgs a = push_args(r, 0);
-    const int g = mcc_blocks(r, leave_sms, 16384);
-    PGB_CK(r, pgb_launch_pdl(k_scatter, dim3(g), dim3(MCC_THREADS), 0, r->stream, a, (const int*)r->list[LIST_SPARE]));
+    const long long n = std::max<long long>(r->hs->n[0], 0), per = (long long)MCC_GROUPS * PGB_TILE;
+    const int g = (int)std::min<long long>(std::max(1, r->sms - leave_sms), std::max<long long>(1, (n + per - 1) / per));
+    const size_t smem = sizeof(MccQueue) * MCC_WARPS;
+    if (!count_events)   /* the list's counts are added up event by event */
+        PGB_CK(r, cudaMemsetAsync(a.tc_ev, 0, sizeof(int) * r->ntiles_cap, r->stream));
+    PGB_CK(r, cudaFuncSetAttribute(k_mcc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PGB_CK(r, pgb_launch_pdl(k_mcc, dim3(g), dim3(MCC_THREADS), smem, r->stream, a, count_events ? 0 : 1));
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;
