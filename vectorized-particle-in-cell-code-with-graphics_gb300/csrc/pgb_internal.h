@@ -22,6 +22,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <cmath>
 #include <string>
 #include "picgb.h"
 
@@ -97,6 +98,24 @@ inline int pgb_pos_shift(int nx, int ny) {
     while ((1 << b) < cells) ++b;
     int ps = 29 - b;
     return ps > 23 ? 23 : (ps < 8 ? 8 : ps);
+}
+
+/* r = 2^ps / d for pos_from_m: its mantissa in the upper 53 bits, and the
+ * shift that leaves the mantissa product in units of 2^-16 less the
+ * exponent of x; no x is in range (the division decides) where r is not a
+ * normal number                                                          */
+struct PosScale {
+    unsigned long long mant;
+    int shift;
+};
+inline PosScale pgb_pos_scale(double d, int ps) {
+    const double r = std::ldexp(1.0 / d, ps);
+    if (!std::isnormal(r) || r < 0.0) return PosScale{0ull, -4096};
+    int e;
+    const double f = std::frexp(r, &e);   /* r = f 2^e, 1/2 <= f < 1 */
+    /* x = m 2^(ex - 1075), r = (f 2^53) 2^(e - 53); the product's upper half
+     * is m f 2^53 2^-42, so |x| r 2^16 = it * 2^(42 + ex - 1075 + e - 53 + 16) */
+    return PosScale{(unsigned long long)std::ldexp(f, 53) << 11, 1070 - e};
 }
 
 struct PushConsts {

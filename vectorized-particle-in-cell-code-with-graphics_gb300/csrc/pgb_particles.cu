@@ -24,6 +24,7 @@
 #include <math.h>
 #include "pgb_internal.h"
 #include "pgb_physics.cuh"
+#include "pgb_deposit.cuh"
 
 /* ------------------------------------------------------------ device state */
 struct PushArgs {
@@ -218,13 +219,6 @@ __device__ __forceinline__ void tile_masks(const bool (&f)[PGB_ITEMS], int tile,
 static_assert(PGB_PIECE_TILES * PGB_TILE <= 4096, "window sums are sized for 4096 particles per piece");
 static_assert((PGB_FIX_SCALE * 1.99 + 1.0) * 4096.0 < 4294967296.0, "window sums must fit 32 bits");
 
-/* round(v) to nearest even for 0 <= v < 2^22, as __float2int_rn: adding
- * 1.5 * 2^23 leaves v's integer part in the low mantissa bits, rounded by
- * the addition itself (1.5 * 2^23 is even, so ties go the same way)      */
-__device__ __forceinline__ unsigned int round_small(float v) {
-    return (unsigned int)__float_as_int(__fadd_rn(v, 12582912.0f)) - 0x4b400000u;
-}
-
 /* deposit into the CTA's shared window when the four nodes fall inside it,
  * else into the global grid.  Caller checks deposit_ok (x, y > 0).       */
 __device__ __forceinline__ void deposit_win(unsigned long long* qacc, unsigned int* win, int ox, int oy, int nx,
@@ -373,14 +367,20 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS) k_flag(const float4* xv, Dev
 }
 
 /* standalone deposit (particle::collect_charge) */
-__global__ void __launch_bounds__(256) k_deposit(const float4* xv, const float* w, DevState* ds, int s, int nx, int ny,
-                                                 int ps, unsigned long long* qacc) {
-    pgb_pdl_entry();
-    const long long n = ds->n[s];
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        float4 p = xv[i];
-        if (deposit_ok(p.x, p.y, nx, ny, ps)) deposit_cell(qacc, nx, ps, p.x, p.y, w[i]);
+struct SlotSource {
+    const float4* xv;
+    const float* w;
+    __device__ __forceinline__ void operator()(long long i, float& x, float& y, float& wt) const {
+        const float4 p = xv[i];
+        x = p.x;
+        y = p.y;
+        wt = w[i];
     }
+};
+__global__ void __launch_bounds__(DEP_THREADS) k_deposit(SlotSource src, DevState* ds, int s, int nx, int ny, int ps,
+                                                         unsigned long long* qacc) {
+    pgb_pdl_entry();
+    deposit_windows(src, ds->n[s], nx, ny, ps, qacc);
 }
 
 /* e_collisions::collision (e_collisions.cpp:480-597), the first kernel of a
@@ -959,13 +959,14 @@ __global__ void k_compact_commit(DevState* ds, int s, const long long* total) {
 
 /* ------------------------------------------------------------ load / dump */
 /* slots [i0, i1) from records aos[6 i ..] */
-__global__ void k_load(Species S, const double* aos, long long i0, long long i1, double dx, double dy, int ps) {
+__global__ void k_load(Species S, const double* aos, long long i0, long long i1, double dx, double dy, PosScale rx, PosScale ry,
+                       int ps) {
     pgb_pdl_entry();
     for (long long i = i0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < i1; i += (long long)gridDim.x * blockDim.x) {
         const double* r = aos + 6 * i;
-        S.xv[i] = make_float4(pos_from_m(r[0], dx, ps), pos_from_m(r[1], dy, ps), (float)r[2], (float)r[3]);
+        S.xv[i] = make_float4(pos_from_m(r[0], dx, rx, ps), pos_from_m(r[1], dy, ry, ps), (float)r[2], (float)r[3]);
         S.vz[i] = (float)r[4];
-        S.w[i] = (float)r[5];
+        S.w[i] = weight_from_double(r[5]);
         S.id[i] = (unsigned int)i;
     }
 }
@@ -1164,7 +1165,9 @@ int pgb_build_list(pgb_run* r, int which, int s, int commit) {
 }
 
 int pgb_launch_deposit(pgb_run* r, int s) {
-    PGB_CK(r, pgb_launch_pdl(k_deposit, dim3(grid_for(r, 8)), dim3(256), 0, r->stream, r->sp[s].xv, r->sp[s].w, r->ds, s, r->nx, r->ny, r->ps, r->qacc[s]));
+    PGB_CK(r, cudaFuncSetAttribute(k_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEP_SMEM));
+    PGB_CK(r, pgb_launch_pdl(k_deposit, dim3(grid_for(r, DEP_BLOCKS_PER_SM)), dim3(DEP_THREADS), DEP_SMEM, r->stream,
+                             SlotSource{r->sp[s].xv, r->sp[s].w}, r->ds, s, r->nx, r->ny, r->ps, r->qacc[s]));
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;
@@ -1238,7 +1241,8 @@ int pgb_launch_compact(pgb_run* r, int s) {
 }
 
 int pgb_launch_load(pgb_run* r, int s, const double* d_aos, long long i0, long long i1) {
-    PGB_CK(r, pgb_launch_pdl(k_load, dim3(grid_for(r, 4)), dim3(256), 0, r->stream, r->sp[s], d_aos, i0, i1, r->dx, r->dy, r->ps));
+    PGB_CK(r, pgb_launch_pdl(k_load, dim3(grid_for(r, 4)), dim3(256), 0, r->stream, r->sp[s], d_aos, i0, i1, r->dx, r->dy,
+                             pgb_pos_scale(r->dx, r->ps), pgb_pos_scale(r->dy, r->ps), r->ps));
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;

@@ -97,6 +97,36 @@ __device__ __forceinline__ float pos_from_cells(double c, int ps) {
     return __int_as_float(__double2int_rn(v));
 }
 __device__ __forceinline__ float pos_from_m(double x, double d, int ps) { return pos_from_cells(x / d, ps); }
+/* The same position in integer arithmetic: FP64 runs at 1.7 lane-operations
+ * per clock and SM, and the division alone is some fifteen of them (loading
+ * 1 Mi records took 75 us, most of it divisions).  The upper 64 bits of the
+ * product of the mantissas of x and r = 2^ps / d, shifted, are |x| r in
+ * units of 2^-16: within 2^-23 (the rounding of r) and one unit (the bits
+ * cut off) of |x|/d 2^ps, so they round to the same integer unless they are
+ * within a unit of a half.  Then, and outside 2^-17 <= |x| r < 2^30 (zero,
+ * NaN, infinite and saturating positions), the division decides.         */
+__device__ __forceinline__ float pos_from_m(double x, double d, PosScale r, int ps) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+    const int s = r.shift - (int)((bits >> 52) & 0x7ff);
+    if ((unsigned)(s - 18) <= 45u) {
+        const unsigned long long m = ((bits << 11) | (1ull << 63));
+        const unsigned long long t = __umul64hi(m, r.mant) >> s;
+        if (((unsigned)t & 0xffffu) - 0x7fffu > 2u) {
+            const int v = (int)((t + 0x8000) >> 16);
+            return __int_as_float((long long)bits < 0 ? -v : v);
+        }
+    }
+    return pos_from_m(x, d, ps);
+}
+/* (float)w; a value that FP32 holds exactly (1, 0.5, ...) needs no FP64
+ * conversion: its mantissa's low 29 bits are 0 and its exponent normal   */
+__device__ __forceinline__ float weight_from_double(double w) {
+    const unsigned hi = (unsigned)__double2hiint(w), lo = (unsigned)__double2loint(w);
+    const unsigned e = (hi >> 20) & 0x7ff;
+    if ((lo & 0x1fffffffu) == 0u && e - 897u < 254u)
+        return __int_as_float((int)((hi & 0x80000000u) | ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29)));
+    return (float)w;
+}
 /* x + d with d in units of 2^-ps of a cell (the push: d = dt*v/DX*2^ps),
  * in 32-bit integers: |x| <= 2^30 and |d| < 2^30 cannot overflow           */
 __device__ __forceinline__ float pos_step(float lane, float d) {

@@ -41,6 +41,7 @@
 #include <string>
 #include "pgb_internal.h"
 #include "pgb_physics.cuh"
+#include "pgb_deposit.cuh"
 
 #define PGB_STATIC_MAX_DEVICES 64
 
@@ -48,6 +49,14 @@
 static __device__ __align__(256) unsigned long long g_static_acc[PGB_STATIC_DEPOSIT_MAX_NODES];
 
 namespace {
+
+/* Windows pay (their zeroing, flush and fewer blocks in flight) where nodes
+ * are shared: from eight records per node and 4096 in all, and from 128 Ki
+ * on any grid.  Measured, straight / through windows: 17^2 nodes, 65 Ki
+ * records 46.8 / 12.0 us; 65^2, 65 Ki 12.7 / 12.6; 129^2, 65 Ki 11.1 / 14.9;
+ * 513^2, 65 Ki 12.8 / 17.7, 6 M in bins 437 / 132 (the latter with the
+ * positions in integer arithmetic on one side only).                     */
+inline bool static_windows(int64_t n, int64_t nodes) { return n >= 4096 && (n >= 8 * nodes || n >= 131072); }
 
 struct DeviceSetup {
     unsigned long long* acc = nullptr;   /* device address of g_static_acc */
@@ -58,6 +67,7 @@ std::mutex g_setup_mu;
 DeviceSetup g_setup[PGB_STATIC_MAX_DEVICES];
 
 __global__ void k_static_clear(unsigned long long* acc, int nodes) {
+    pgb_pdl_entry();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nodes; k += gridDim.x * blockDim.x) acc[k] = 0ull;
 }
 
@@ -65,18 +75,38 @@ __global__ void k_static_clear(unsigned long long* acc, int nodes) {
  * x and y become fixed-point positions exactly as pgb_load_species makes
  * them (pgb_pos_shift of the grid), so the deposit is bit-identical to the
  * run handle's.                                                          */
-__global__ void __launch_bounds__(256) k_static_deposit(const double* aos6, long long n, int nx, int ny, double dx,
-                                                        double dy, int ps, unsigned long long* acc) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const double* r = aos6 + 6 * i;
-        float xl = pos_from_m(r[0], dx, ps), yl = pos_from_m(r[1], dy, ps), w = (float)r[5];
-        if (deposit_ok(xl, yl, nx, ny, ps)) deposit_cell(acc, nx, ps, xl, yl, w);
+struct RecordSource {
+    const double* aos6;
+    double dx, dy;
+    PosScale rx, ry;
+    int ps;
+    __device__ __forceinline__ void operator()(long long i, float& x, float& y, float& w) const {
+        const double* const r = aos6 + 6 * i;
+        x = pos_from_m(r[0], dx, rx, ps);
+        y = pos_from_m(r[1], dy, ry, ps);
+        w = weight_from_double(r[5]);
     }
+};
+/* few records for the grid: one thread each, straight to the accumulator */
+__global__ void __launch_bounds__(256) k_static_deposit_few(RecordSource src, long long n, int nx, int ny,
+                                                            unsigned long long* acc) {
+    pgb_pdl_entry();
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        float x, y, w;
+        src(i, x, y, w);
+        if (deposit_ok(x, y, nx, ny, src.ps)) deposit_cell(acc, nx, src.ps, x, y, w);
+    }
+}
+__global__ void __launch_bounds__(DEP_THREADS) k_static_deposit(RecordSource src, long long n, int nx, int ny,
+                                                                unsigned long long* acc) {
+    pgb_pdl_entry();
+    deposit_windows(src, n, nx, ny, src.ps, acc);
 }
 
 /* q = (sum / PGB_FIX_SCALE * qc/(DX*DY)) * edge factor, the sum being in
- * units of 2^-19 of a unit weight (particle.cpp:829-845)                 */
+ * units of 2^-19 of a unit weight (particle.cpp:829-845)                  */
 __global__ void k_static_finish(const unsigned long long* acc, int nx, int ny, double qcdxdy, double* q) {
+    pgb_pdl_entry();
     const int nodes = nx * ny;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nodes; k += gridDim.x * blockDim.x) {
         int j = k / nx, i = k - j * nx;
@@ -138,14 +168,25 @@ extern "C" int pgb_deposit_static(const double* d_aos6, int64_t n, int32_t nx, i
     cudaStream_t st = (cudaStream_t)stream;
     const int nodes = nx * ny;
     const int gblocks = (nodes + 255) / 256 < s.sms * 4 ? (nodes + 255) / 256 : s.sms * 4;
-    k_static_clear<<<gblocks, 256, 0, st>>>(s.acc, nodes);
-    if (n > 0) {
-        long long want = (n + 255) / 256;
-        int pblocks = want < (long long)s.sms * 8 ? (int)want : s.sms * 8;
-        k_static_deposit<<<pblocks, 256, 0, st>>>(d_aos6, (long long)n, nx, ny, dx, dy, pgb_pos_shift(nx, ny), s.acc);
+    const int ps = pgb_pos_shift(nx, ny);
+    const RecordSource src{d_aos6, dx, dy, pgb_pos_scale(dx, ps), pgb_pos_scale(dy, ps), ps};
+    cudaError_t e = pgb_launch_pdl(k_static_clear, dim3(gblocks), dim3(256), 0, st, s.acc, nodes);
+    if (e != cudaSuccess) return setup_error("pgb_deposit_static: kernel launch", e);
+    if (static_windows(n, nodes)) {
+        /* a block's window is zeroed and flushed once per run of records */
+        const long long want = (n + DEP_CHUNK - 1) / DEP_CHUNK;
+        const int blocks = want < (long long)s.sms * DEP_BLOCKS_PER_SM ? (int)want : s.sms * DEP_BLOCKS_PER_SM;
+        e = cudaFuncSetAttribute(k_static_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEP_SMEM);
+        if (e == cudaSuccess)
+            e = pgb_launch_pdl(k_static_deposit, dim3(blocks), dim3(DEP_THREADS), DEP_SMEM, st, src, (long long)n, nx, ny, s.acc);
+    } else if (n > 0) {
+        e = pgb_launch_pdl(k_static_deposit_few, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, src, (long long)n, nx, ny, s.acc);
     }
-    k_static_finish<<<gblocks, 256, 0, st>>>(s.acc, nx, ny, qc / (dx * dy), d_q);
-    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = pgb_launch_pdl(k_static_finish, dim3(gblocks), dim3(256), 0, st, (const unsigned long long*)s.acc, nx, ny,
+                           qc / (dx * dy), d_q);
+    if (e != cudaSuccess) return setup_error("pgb_deposit_static: kernel launch", e);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return setup_error("pgb_deposit_static: kernel launch", e);
     return 0;
 }
