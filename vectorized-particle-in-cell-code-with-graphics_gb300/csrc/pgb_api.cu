@@ -783,7 +783,7 @@ extern "C" int pgb_poisson(pgb_run* r, int64_t t) {
 
 extern "C" int pgb_efield(pgb_run* r) {
     if (!r) return PGB_ERR_ARG;
-    if (pgb_launch_efield(r, 0)) return PGB_ERR_CUDA;
+    if (pgb_launch_efield(r)) return PGB_ERR_CUDA;
     return sync_state(r);
 }
 
@@ -955,8 +955,7 @@ static int step_fields(pgb_run* r, bool) {
     /* collect_charge edge doubling, grid_rho, grid_potential, grid_electric_field */
     PROF_MARK(r, 5);
     if (pgb_launch_finalize(r, 3, true, true)) return PGB_ERR_CUDA;
-    if (pgb_poisson_solve(r)) return PGB_ERR_CUDA;
-    if (pgb_launch_efield(r, 1)) return PGB_ERR_CUDA;
+    if (pgb_poisson_solve(r, true, true)) return PGB_ERR_CUDA;
     PROF_MARK(r, 6);
     return 0;
 }

@@ -13,15 +13,20 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include "pgb_internal.h"
+#include "pgb_fp64.cuh"
 
 /* ------------------------------------------------ charge, rho, rhs */
+enum { F32_NONE = 0, F32_CHARGE = 1, F32_RHS = 2 };
 struct FinalizeArgs {
     unsigned long long* acc[2];
     double* q[2];
     double* rho;
     double* f;            /* Poisson right-hand side, or null */
+    float* f32;           /* an FP32 right-hand side, by f32_what */
+    int f32_what;         /* F32_CHARGE: -rho/EPSILON on the interior (the walls'
+                             terms are in the wall solutions), F32_RHS: f   */
     int nx, ny;
-    double qcdxdy[2];     /* qc/(DX*DY) per species */
+    double qs[2];         /* qc/(DX*DY) per unit of the accumulators, per species */
     int mask;             /* species whose q is rebuilt from acc */
     int clear;            /* zero acc once read                  */
     double coef;          /* 1/EPSILON */
@@ -37,32 +42,49 @@ __device__ __forceinline__ double edge_factor(int i, int j, int nx, int ny) {
     return (ex ? 2.0 : 1.0) * (ey ? 2.0 : 1.0) * ((ex && ey) ? 2.0 : 1.0);
 }
 
-/* RHS of fields::grid_potential (fields.cpp:184-204) for node (j, i) */
-__device__ __forceinline__ double rhs_node(double rho, int i, int j, const FinalizeArgs& a, double phirx) {
-    double f = -a.coef * rho;
+/* RHS of fields::grid_potential (fields.cpp:184-204) for node (j, i) from
+ * charge = -coef * rho                                                   */
+__device__ __forceinline__ double rhs_node(double charge, int i, int j, const FinalizeArgs& a, double phirx) {
+    double f = charge;
     if (i == 1) f = f - a.phi0x * a.divdxdy;
     if (i == a.nx - 2) f = f - phirx * a.divdxdy;
     if (j == 1) f = f - a.phi0y * a.divdxdy;
     if (j == a.ny - 2) f = f - a.phily * a.divdxdy;
     return f;
 }
+__device__ __forceinline__ void store_rhs(const FinalizeArgs& a, int k, int i, int j, double rho, double phirx) {
+    const double charge = -a.coef * rho;
+    const double f = rhs_node(charge, i, j, a, phirx);
+    a.f[k] = f;
+    if (a.f32_what == F32_RHS) a.f32[k] = f64_to_f32(f);
+    if (a.f32_what == F32_CHARGE)
+        a.f32[k] = (i > 0 && j > 0 && i < a.nx - 1 && j < a.ny - 1) ? f64_to_f32(charge) : 0.0f;
+}
 
+/* The sum is an integer number of 2^-19 of a unit weight and the edge
+ * factor a power of two: q = sum * (qs * factor) rounds once, as
+ * (sum * 2^-19 * qc/(DX*DY)) * factor does.                              */
 __global__ void k_finalize(FinalizeArgs a) {
     pgb_pdl_entry();
     const int G = a.nx * a.ny;
     const double phirx = a.phi_tab[a.ds->tf - a.ds->t_base];
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < G; k += gridDim.x * blockDim.x) {
-        int j = k / a.nx, i = k - j * a.nx;
-        double ef = edge_factor(i, j, a.nx, a.ny);
-        for (int s = 0; s < 2; ++s)
-            if (a.mask & (1 << s)) {
-                double v = (double)(long long)a.acc[s][k] * (1.0 / PGB_FIX_SCALE);
-                if (a.clear) a.acc[s][k] = 0ull;
-                a.q[s][k] = (v * a.qcdxdy[s]) * ef;
-            }
-        double rho = a.q[1][k] + a.q[0][k];
+        const long long v0 = a.mask & 1 ? (long long)a.acc[0][k] : 0, v1 = a.mask & 2 ? (long long)a.acc[1][k] : 0;
+        const int j = k / a.nx, i = k - j * a.nx;
+        double s0 = a.qs[0], s1 = a.qs[1];
+        if (i == 0 || j == 0 || i == a.nx - 1 || j == a.ny - 1) {
+            const double ef = edge_factor(i, j, a.nx, a.ny);
+            s0 = s0 * ef;
+            s1 = s1 * ef;
+        }
+        const double q0 = a.mask & 1 ? i64_to_f64(v0) * s0 : a.q[0][k];
+        const double q1 = a.mask & 2 ? i64_to_f64(v1) * s1 : a.q[1][k];
+        if (a.mask & 1) a.q[0][k] = q0;
+        if (a.mask & 2) a.q[1][k] = q1;
+        if (a.clear) a.acc[0][k] = a.acc[1][k] = 0ull;
+        const double rho = q1 + q0;
         a.rho[k] = rho;
-        if (a.f) a.f[k] = rhs_node(rho, i, j, a, phirx);
+        if (a.f) store_rhs(a, k, i, j, rho, phirx);
     }
 }
 
@@ -72,59 +94,148 @@ __global__ void k_rhs(FinalizeArgs a) {
     const double phirx = a.phi_tab[a.ds->tf - a.ds->t_base];
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < G; k += gridDim.x * blockDim.x) {
         int j = k / a.nx, i = k - j * a.nx;
-        a.f[k] = rhs_node(a.rho[k], i, j, a, phirx);
+        store_rhs(a, k, i, j, a.rho[k], phirx);
     }
 }
 
-/* ------------------------------------------------------- E field */
-/* fields::grid_electric_field (fields.cpp:230-268) in the stride-nx layout
- * of an (nx+1)*(ny+1) buffer; also writes the FP32 {Ex,Ey} copy read by
- * the gather.                                                           */
-__device__ __forceinline__ double ex_interior(const double* phi, int nx, int ny, int j, int i, double twoDX) {
-    if (j < 1 || j > ny - 2 || i < 1 || i > nx - 2) return 0.0;
-    return (phi[j * nx + i - 1] - phi[j * nx + i + 1]) / twoDX;
+/* ------------------------------------------------ potential and E field */
+/* Where the potential of an interior node comes from. */
+struct PhiSource {
+    const double* u;      /* FP64 part, or null */
+    const float* e;       /* FP32 part to add, or null */
+    const double* phi;    /* or the potential itself, walls included */
+};
+struct FieldArgs {
+    PhiSource src;
+    double* phi;          /* written where src.phi is null */
+    double *Ex, *Ey;      /* null: the potential only */
+    float2* exy;
+    int nx, ny;
+    DivBy two_dx;
+    double phi0x, phi0y, phily;
+    const double* phi_tab;
+    DevState* ds;
+    int advance;          /* move the field step counter on */
+};
+/* the potential at node (j, i): fields.cpp:209-219 sets columns first, then
+ * rows overwrite the corners                                             */
+__device__ __forceinline__ double phi_at(const FieldArgs& a, double phirx, int j, int i) {
+    const int k = j * a.nx + i;
+    if (a.src.phi) return a.src.phi[k];
+    if (j == 0) return a.phi0y;
+    if (j == a.ny - 1) return a.phily;
+    if (i == 0) return a.phi0x;
+    if (i == a.nx - 1) return phirx;
+    if (!a.src.e) return a.src.u[k];
+    const double e = f32_to_f64(a.src.e[k]);
+    return a.src.u ? a.src.u[k] + e : e;
 }
-__device__ __forceinline__ double ey_interior(const double* phi, int nx, int ny, int j, int i, double twoDX) {
-    if (j < 1 || j > ny - 2 || i < 1 || i > nx - 2) return 0.0;
-    return (phi[(j - 1) * nx + i] - phi[(j + 1) * nx + i]) / twoDX;
+/* fields::grid_electric_field (fields.cpp:230-268) at interior nodes, 0 on
+ * the walls                                                              */
+__device__ __forceinline__ double ex_interior(const FieldArgs& a, double phirx, int j, int i) {
+    if (j < 1 || j > a.ny - 2 || i < 1 || i > a.nx - 2) return 0.0;
+    return div_const(phi_at(a, phirx, j, i - 1) - phi_at(a, phirx, j, i + 1), a.two_dx);
 }
-__global__ void k_efield(const double* phi, double* Ex, double* Ey, float2* exy, int nx, int ny, double twoDX,
-                         DevState* ds, int advance) {
+__device__ __forceinline__ double ey_interior(const FieldArgs& a, double phirx, int j, int i) {
+    if (j < 1 || j > a.ny - 2 || i < 1 || i > a.nx - 2) return 0.0;
+    return div_const(phi_at(a, phirx, j - 1, i) - phi_at(a, phirx, j + 1, i), a.two_dx);
+}
+/* The end of a field solve in one launch: the last correction's addition,
+ * the walls, E in the stride-nx layout of an (nx+1)*(ny+1) buffer (its
+ * entries past nx*ny stay 0 from the allocation) and the FP32 {Ex,Ey} copy
+ * read by the gather.  A block takes a 32 x 8 tile of nodes and forms each
+ * potential once, in shared memory with a ring around the tile.  At 513^2 the
+ * three kernels that did this took 4.0 + 3.7 + 16.5 us, most of it two FP64
+ * divisions a node.                                                      */
+#define FT_X 32
+#define FT_Y 8
+__global__ void __launch_bounds__(FT_X * FT_Y) k_field(FieldArgs a) {
     pgb_pdl_entry();
-    /* the last kernel of a field solve moves the field step counter on */
-    if (advance && blockIdx.x == 0 && threadIdx.x == 0) ds->tf += 1;
-    const int GE = (nx + 1) * (ny + 1);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < GE; k += gridDim.x * blockDim.x) {
-        double ex = 0.0, ey = 0.0;
-        if (k < nx * ny) {
-            int j = k / nx, i = k - j * nx;
-            if (i == 0) ex = 2.0 * ex_interior(phi, nx, ny, j, 1, twoDX) - ex_interior(phi, nx, ny, j, 2, twoDX);
-            else if (i == nx - 1) ex = 2.0 * ex_interior(phi, nx, ny, j, nx - 2, twoDX) - ex_interior(phi, nx, ny, j, nx - 3, twoDX);
-            else ex = ex_interior(phi, nx, ny, j, i, twoDX);
-            if (j == 0) ey = 2.0 * ey_interior(phi, nx, ny, 1, i, twoDX) - ey_interior(phi, nx, ny, 2, i, twoDX);
-            else if (j == ny - 1) ey = 2.0 * ey_interior(phi, nx, ny, ny - 2, i, twoDX) - ey_interior(phi, nx, ny, ny - 3, i, twoDX);
-            else ey = ey_interior(phi, nx, ny, j, i, twoDX);
+    __shared__ double s[FT_Y + 2][FT_X + 2];
+    const int nx = a.nx, ny = a.ny;
+    const double phirx = a.phi_tab[a.ds->tf - a.ds->t_base];
+    const int i0 = blockIdx.x * FT_X - 1, j0 = blockIdx.y * FT_Y - 1;
+    for (int t = threadIdx.x; t < (FT_Y + 2) * (FT_X + 2); t += FT_X * FT_Y) {
+        const int r = t / (FT_X + 2), c = t - r * (FT_X + 2), j = j0 + r, i = i0 + c;
+        if (j >= 0 && i >= 0 && j < ny && i < nx) s[r][c] = phi_at(a, phirx, j, i);
+    }
+    __syncthreads();
+    const int c = threadIdx.x % FT_X + 1, r = threadIdx.x / FT_X + 1, i = i0 + c, j = j0 + r;
+    if (i < nx && j < ny) {
+        const int k = j * nx + i;
+        if (!a.src.phi) a.phi[k] = s[r][c];
+        if (a.Ex) {
+            double ex, ey;
+            if (i > 0 && j > 0 && i < nx - 1 && j < ny - 1) {
+                ex = div_const(s[r][c - 1] - s[r][c + 1], a.two_dx);
+                ey = div_const(s[r - 1][c] - s[r + 1][c], a.two_dx);
+            } else {
+                if (i == 0) ex = 2.0 * ex_interior(a, phirx, j, 1) - ex_interior(a, phirx, j, 2);
+                else if (i == nx - 1) ex = 2.0 * ex_interior(a, phirx, j, nx - 2) - ex_interior(a, phirx, j, nx - 3);
+                else ex = ex_interior(a, phirx, j, i);
+                if (j == 0) ey = 2.0 * ey_interior(a, phirx, 1, i) - ey_interior(a, phirx, 2, i);
+                else if (j == ny - 1) ey = 2.0 * ey_interior(a, phirx, ny - 2, i) - ey_interior(a, phirx, ny - 3, i);
+                else ey = ey_interior(a, phirx, j, i);
+            }
+            a.Ex[k] = ex;
+            a.Ey[k] = ey;
+            a.exy[k] = make_float2(f64_to_f32(ex), f64_to_f32(ey));
         }
-        Ex[k] = ex;
-        Ey[k] = ey;
-        exy[k] = make_float2((float)ex, (float)ey);
+    }
+    /* the last block to get here moves the field step counter on: every
+     * block has read it by then                                          */
+    if (a.advance) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(&a.ds->ticket_f, 1u) == gridDim.x * gridDim.y - 1) {
+                a.ds->ticket_f = 0u;
+                a.ds->tf += 1;
+            }
+        }
     }
 }
 
-__global__ void k_walls(double* phi, int nx, int ny, double phi0x, const double* phi_tab, const DevState* ds,
-                        double phi0y, double phily) {
+/* ---------------------------------------------- FP64 defect correction */
+/* One update of the FP64 solution, u' = u + e (u' = e where u is null;
+ * FIRST: u' = wc + phi_right(t) wr + e, the walls' solutions and the FP32
+ * solve of the charge term), written to a second buffer so that neighbours
+ * read the old values, and the FP64 defect d = f - L u' of the interior
+ * (zero on the walls) stored as FP32 for the next FP32 correction.  The
+ * walls of u, e and so u' are 0.  A block forms each u' of its 32 x 8 tile
+ * and the ring around it once, in shared memory.  4 u' is exact, so one
+ * fused operation subtracts it from the neighbours' sum as the two separate
+ * ones do.  At 513^2: 17.8 (FIRST) and 12.2 us before, in FP64 operations
+ * of five sums per node.                                                 */
+template <bool FIRST>
+__global__ void __launch_bounds__(FT_X * FT_Y) k_dc_update(const double* __restrict__ u, const double* __restrict__ wc,
+                                                          const double* __restrict__ wr, const double* phi_tab,
+                                                          const DevState* ds, const float* __restrict__ e,
+                                                          double* __restrict__ uout, const double* __restrict__ f,
+                                                          float* __restrict__ d, int n, double h2i) {
     pgb_pdl_entry();
-    const double phirx = phi_tab[ds->tf - ds->t_base];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nx * ny; k += gridDim.x * blockDim.x) {
-        int j = k / nx, i = k - j * nx;
-        /* fields.cpp:209-219: columns first, then rows overwrite the corners */
-        if (j == 0) phi[k] = phi0y;
-        else if (j == ny - 1) phi[k] = phily;
-        else if (i == 0) phi[k] = phi0x;
-        else if (i == nx - 1) phi[k] = phirx;
+    __shared__ double s[FT_Y + 2][FT_X + 2];
+    const double phirx = FIRST ? phi_tab[ds->tf - ds->t_base] : 0.0;
+    const int i0 = blockIdx.y * FT_Y - 1, j0 = blockIdx.x * FT_X - 1;
+    for (int t = threadIdx.x; t < (FT_Y + 2) * (FT_X + 2); t += FT_X * FT_Y) {
+        const int r = t / (FT_X + 2), c = t - r * (FT_X + 2), i = i0 + r, j = j0 + c;
+        if (i >= 0 && j >= 0 && i < n && j < n) {
+            const int k = i * n + j;
+            const double ek = f32_to_f64(e[k]);
+            s[r][c] = FIRST ? (wc[k] + phirx * wr[k]) + ek : u ? u[k] + ek : ek;
+        }
     }
+    __syncthreads();
+    const int c = threadIdx.x % FT_X + 1, r = threadIdx.x / FT_X + 1, i = i0 + r, j = j0 + c;
+    if (i >= n || j >= n) return;
+    const int k = i * n + j;
+    const double x = s[r][c];
+    float v = 0.0f;
+    if (i > 0 && j > 0 && i < n - 1 && j < n - 1)
+        v = f64_to_f32(f[k] - h2i * __fma_rn(-4.0, x, s[r + 1][c] + s[r - 1][c] + s[r][c + 1] + s[r][c - 1]));
+    uout[k] = x;
+    d[k] = v;
 }
-
 /* ====================================================== host side */
 static FinalizeArgs fin_args(pgb_run* r, int mask, bool rhs) {
     FinalizeArgs a;
@@ -132,8 +243,12 @@ static FinalizeArgs fin_args(pgb_run* r, int mask, bool rhs) {
     a.q[0] = r->q[0]; a.q[1] = r->q[1];
     a.rho = r->rho; a.f = rhs ? r->mg_f[r->ng - 1] : nullptr;
     a.nx = r->nx; a.ny = r->ny;
-    a.qcdxdy[0] = r->sp[0].qc / (r->dx * r->dy);
-    a.qcdxdy[1] = r->sp[1].qc / (r->dx * r->dy);
+    for (int s = 0; s < 2; ++s) a.qs[s] = r->sp[s].qc / (r->dx * r->dy) * (1.0 / PGB_FIX_SCALE);
+    /* the FP32 solvers' right-hand side comes with the FP64 one */
+    a.f32 = r->mg32_f[r->ng - 1];
+    a.f32_what = !rhs || r->p.poisson_mode == PGB_POISSON_FMG_REF ? F32_NONE
+                 : r->p.poisson_mode == PGB_POISSON_DST_DC        ? F32_CHARGE
+                                                                  : F32_RHS;
     a.mask = mask;
     a.clear = 0;
     a.coef = 1.0 / 8.854e-12;
@@ -169,121 +284,75 @@ static int blocks_for(long long work) {
     return (int)b;
 }
 
-/* One defect-correction update: u' = u + e in FP64 (u' = e on the first
- * pass, when u is null), written to a second buffer so that neighbours
- * read the old values, and the FP64 defect d = f - L u' of the interior
- * (zero on the walls) stored as FP32 for the next FP32 correction.  The
- * walls of u, e and so u' are 0.                                         */
-__global__ void k_dc_update(const double* __restrict__ u, const float* __restrict__ e, double* __restrict__ uout,
-                            const double* __restrict__ f, float* __restrict__ d, int n, double h2i) {
-    pgb_pdl_entry();
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n * n; k += gridDim.x * blockDim.x) {
-        int i = k / n, j = k - i * n;
-        auto U = [&](int q) { return u ? u[q] + (double)e[q] : (double)e[q]; };
-        double c = U(k), v = 0.0;
-        if (i > 0 && j > 0 && i < n - 1 && j < n - 1)
-            v = f[k] - h2i * (U(k + n) + U(k - n) + U(k + 1) + U(k - 1) - 4.0 * c);
-        uout[k] = c;
-        d[k] = (float)v;
-    }
-}
-/* the last correction: phi = u + e in FP64 (the walls are set after) */
-__global__ void k_dc_final(double* __restrict__ phi, const double* __restrict__ u, const float* __restrict__ e,
-                           int count) {
-    pgb_pdl_entry();
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x)
-        phi[k] = u[k] + (double)e[k];
-}
-/* DST_DC: the FP32 right-hand side of the charge alone, -rho/EPSILON on
- * the interior (the walls' terms are in the wall solutions)             */
-__global__ void k_rho32(float* __restrict__ f32, const double* __restrict__ rho, int n, double coef) {
-    pgb_pdl_entry();
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n * n; k += gridDim.x * blockDim.x) {
-        int i = k / n, j = k - i * n;
-        f32[k] = (i > 0 && j > 0 && i < n - 1 && j < n - 1) ? (float)(-coef * rho[k]) : 0.0f;
-    }
-}
-/* DST_DC's first update: u = wc + phi_right(t) * wr + e (the walls' FP64
- * solutions and the FP32 solve of the charge term), and the FP64 defect
- * d = f - L u of the full right-hand side, as k_dc_update            */
-__global__ void k_dc_first(const double* __restrict__ wc, const double* __restrict__ wr, const double* phi_tab,
-                           const DevState* ds, const float* __restrict__ e, double* __restrict__ uout,
-                           const double* __restrict__ f, float* __restrict__ d, int n, double h2i) {
-    pgb_pdl_entry();
-    const double phirx = phi_tab[ds->tf - ds->t_base];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n * n; k += gridDim.x * blockDim.x) {
-        int i = k / n, j = k - i * n;
-        auto U = [&](int q) { return (wc[q] + phirx * wr[q]) + (double)e[q]; };
-        double c = U(k), v = 0.0;
-        if (i > 0 && j > 0 && i < n - 1 && j < n - 1)
-            v = f[k] - h2i * (U(k + n) + U(k - n) + U(k + 1) + U(k - 1) - 4.0 * c);
-        uout[k] = c;
-        d[k] = (float)v;
-    }
-}
 /* the walls' terms of the right-hand side alone (rhs_node at rho = 0) */
 __global__ void k_wall_rhs(FinalizeArgs a, double phirx) {
     pgb_pdl_entry();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < a.nx * a.ny; k += gridDim.x * blockDim.x) {
         int j = k / a.nx, i = k - j * a.nx;
-        a.f[k] = rhs_node(0.0, i, j, a, phirx);
+        a.f[k] = rhs_node(-0.0, i, j, a, phirx);
     }
 }
 __global__ void k_to32(float* d, const double* s, int count) {
     pgb_pdl_entry();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) d[k] = (float)s[k];
 }
-__global__ void k_to64(double* d, const float* s, int count) {
+/* u + e in FP64 */
+__global__ void k_dc_sum(double* __restrict__ out, const double* __restrict__ u, const float* __restrict__ e, int count) {
     pgb_pdl_entry();
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) d[k] = (double)s[k];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) out[k] = u[k] + (double)e[k];
 }
 
-/* FP64 defect correction around the FP32 sine-transform solve of L u = f64
- * (zero walls), `passes` solves in all; the result goes to out (FP64).
+static dim3 field_grid(int nx, int ny) { return dim3((nx + FT_X - 1) / FT_X, (ny + FT_Y - 1) / FT_Y); }
+
+/* FP64 defect correction around an FP32 solve of L u = f64 (zero walls),
+ * `passes` solves in all.  *out: the parts whose sum is the solution.
+ * The FP32 solve goes from f32 to e32.                                   */
+template <class Solve>
+static int defect_correction(pgb_run* r, const double* f64, float* f32, const float* e32, int passes, Solve solve,
+                             PhiSource* out) {
+    const int n = r->nx;
+    const double h = r->p.xlength / (n - 1), h2i = 1.0 / (h * h);
+    double* ua = const_cast<double*>(out->u);   /* FP64 solution so far (null: 0) */
+    for (int it = 1; it < passes; ++it) {
+        double* const ub = ua == r->dc_u ? r->dc_u2 : r->dc_u;
+        PGB_CK(r, pgb_launch_pdl(k_dc_update<false>, field_grid(n, n), dim3(FT_X * FT_Y), 0, r->stream, (const double*)ua,
+                                 (const double*)nullptr, (const double*)nullptr, (const double*)nullptr,
+                                 (const DevState*)nullptr, out->e, ub, f64, f32, n, h2i));
+        r->launches++;
+        ua = ub;
+        if (solve()) return PGB_ERR_CUDA;
+        *out = PhiSource{ua, e32, nullptr};
+    }
+    return 0;
+}
+
+/* DST_DC.  The FP32 right-hand side is in mg32_f[top].
  * lift: the first approximation is the walls' solution wc + phi_right(t) wr
  * plus the FP32 solve of the charge term alone, which keeps the walls'
  * terms (-phi/(DX DY) next to a wall, a thousand times the charge term at
  * 1 V) out of the FP32 transform, whose rounding they would otherwise
  * spread over every mode; each pass then divides the error by about 1e6
  * instead of about 300.  Otherwise the first solve is of f64 itself.  */
-static int dst_dc(pgb_run* r, const double* f64, double* out, int passes, bool lift) {
-    const int top = r->ng - 1, n = r->nx, G = n * n, gb = blocks_for(G);
-    const double h = r->p.xlength / (n - 1), h2i = 1.0 / (h * h);
+static int dst_dc(pgb_run* r, const double* f64, int passes, bool lift, PhiSource* out) {
+    const int top = r->ng - 1, n = r->nx;
     float* const f32 = r->mg32_f[top];   /* right-hand side, then each defect */
     float* const e32 = r->mg32_u[top];   /* each FP32 solve                   */
-    if (lift) PGB_CK(r, pgb_launch_pdl(k_rho32, dim3(gb), dim3(256), 0, r->stream, f32, (const double*)r->rho, n,
-                                       1.0 / 8.854e-12));
-    else PGB_CK(r, pgb_launch_pdl(k_to32, dim3(gb), dim3(256), 0, r->stream, f32, f64, G));
-    r->launches++;
-    if (pgb_dst_solve(r, f32, e32)) return PGB_ERR_CUDA;
-    if (passes <= 1 && !lift) {
-        PGB_CK(r, pgb_launch_pdl(k_to64, dim3(gb), dim3(256), 0, r->stream, out, (const float*)e32, G));
-        r->launches++;
-        return 0;
-    }
-    double* ua = nullptr;   /* FP64 solution so far */
-    double* ub = passes <= 1 ? out : r->dc_u;
+    auto solve = [&] { return pgb_dst_solve(r, f32, e32); };
+    if (solve()) return PGB_ERR_CUDA;
+    *out = PhiSource{nullptr, e32, nullptr};
     if (lift) {
-        PGB_CK(r, pgb_launch_pdl(k_dc_first, dim3(gb), dim3(256), 0, r->stream, (const double*)r->dst_wc,
-                                 (const double*)r->dst_wr, (const double*)r->phi_tab, (const DevState*)r->ds,
-                                 (const float*)e32, ub, f64, f32, n, h2i));
+        const double h = r->p.xlength / (n - 1), h2i = 1.0 / (h * h);
+        PGB_CK(r, pgb_launch_pdl(k_dc_update<true>, field_grid(n, n), dim3(FT_X * FT_Y), 0, r->stream, (const double*)nullptr,
+                                 (const double*)r->dst_wc, (const double*)r->dst_wr, (const double*)r->phi_tab,
+                                 (const DevState*)r->ds, (const float*)e32, r->dc_u, f64, f32, n, h2i));
         r->launches++;
+        *out = PhiSource{r->dc_u, nullptr, nullptr};
         if (passes <= 1) return 0;
-        ua = ub;
-        ub = r->dc_u2;
-        if (pgb_dst_solve(r, f32, e32)) return PGB_ERR_CUDA;
+        if (solve()) return PGB_ERR_CUDA;
+        out->e = e32;
+        passes--;
     }
-    for (int it = lift ? 2 : 1; it < passes; ++it) {
-        PGB_CK(r, pgb_launch_pdl(k_dc_update, dim3(gb), dim3(256), 0, r->stream, (const double*)ua, (const float*)e32,
-                                 ub, f64, f32, n, h2i));
-        r->launches++;
-        ua = ub;
-        ub = (ub == r->dc_u) ? r->dc_u2 : r->dc_u;
-        if (pgb_dst_solve(r, f32, e32)) return PGB_ERR_CUDA;
-    }
-    PGB_CK(r, pgb_launch_pdl(k_dc_final, dim3(gb), dim3(256), 0, r->stream, out, (const double*)ua, (const float*)e32, G));
-    r->launches++;
-    return 0;
+    return defect_correction(r, f64, f32, e32, passes, solve, out);
 }
 
 /* DST_DC's wall solutions: L u = (the walls' right-hand side terms), the
@@ -295,13 +364,16 @@ static int dst_wall_solutions(pgb_run* r) {
     PGB_CK(r, cudaMalloc(&r->dst_wr, G * sizeof(double)));
     PGB_CK(r, cudaDeviceSynchronize());   /* the setup's memsets ran on the legacy stream */
     double* const f64 = r->mg_w[r->ng - 1];   /* FP64 scratch of the top level */
+    const dim3 gb(blocks_for((long long)G)), tb(256);
     for (int w = 0; w < 2; ++w) {
         FinalizeArgs a = fin_args(r, 0, true);
         a.f = f64;
         if (w == 1) a.phi0x = a.phi0y = a.phily = 0.0;
-        PGB_CK(r, pgb_launch_pdl(k_wall_rhs, dim3(blocks_for((long long)G)), dim3(256), 0, r->stream, a,
-                                 w == 1 ? 1.0 : 0.0));
-        if (dst_dc(r, f64, w == 0 ? r->dst_wc : r->dst_wr, 8, false)) return PGB_ERR_CUDA;
+        PGB_CK(r, pgb_launch_pdl(k_wall_rhs, gb, tb, 0, r->stream, a, w == 1 ? 1.0 : 0.0));
+        PGB_CK(r, pgb_launch_pdl(k_to32, gb, tb, 0, r->stream, r->mg32_f[r->ng - 1], (const double*)f64, (int)G));
+        PhiSource src;
+        if (dst_dc(r, f64, 8, false, &src)) return PGB_ERR_CUDA;
+        PGB_CK(r, pgb_launch_pdl(k_dc_sum, gb, tb, 0, r->stream, w == 0 ? r->dst_wc : r->dst_wr, src.u, src.e, (int)G));
     }
     PGB_CK(r, cudaMemsetAsync(f64, 0, G * sizeof(double), r->stream));   /* the level's walls stay 0 */
     PGB_CK(r, cudaStreamSynchronize(r->stream));
@@ -364,57 +436,45 @@ void pgb_mg_free(pgb_run* r) {
  *            up to FP32 rounding (about 1e-6 of phi): a first solve, then
  *            dc_max_iters - 1 corrections, each dividing the error by
  *            about 1e6.                                                  */
-int pgb_poisson_solve(pgb_run* r) {
-    const int top = r->ng - 1, n = r->nx;
-    const int G = n * n;
-    const int gb = blocks_for(G);
+static int launch_field(pgb_run* r, const PhiSource& src, bool field, bool advance) {
+    FieldArgs a;
+    a.src = src;
+    a.phi = r->phi;
+    a.Ex = field ? r->ex : nullptr;
+    a.Ey = r->ey;
+    a.exy = r->exy;
+    a.nx = r->nx; a.ny = r->ny;
+    a.two_dx = div_by(2.0 * r->dx);
+    a.phi0x = r->p.phi_left; a.phi0y = r->p.phi_bottom; a.phily = r->p.phi_top;
+    a.phi_tab = r->phi_tab; a.ds = r->ds;
+    a.advance = advance;
+    PGB_CK(r, pgb_launch_pdl(k_field, field_grid(r->nx, r->ny), dim3(FT_X * FT_Y), 0, r->stream, a));
+    r->launches++;
+    PGB_CK(r, cudaGetLastError());
+    return 0;
+}
+
+int pgb_poisson_solve(pgb_run* r, bool field, bool advance) {
+    const int top = r->ng - 1;
+    PhiSource src{nullptr, nullptr, nullptr};
     if (r->p.poisson_mode == PGB_POISSON_FMG_REF) {
         if (pgb_mg_fmg64(r)) return PGB_ERR_CUDA;
-        PGB_CK(r, cudaMemcpyAsync(r->phi, r->mg_u[top], sizeof(double) * G, cudaMemcpyDeviceToDevice, r->stream));
+        src.u = r->mg_u[top];
     } else if (r->p.poisson_mode == PGB_POISSON_DST_DC) {
         if (!pgb_dst_ok(r)) return PGB_ERR_CUDA;
-        if (dst_dc(r, r->mg_f[top], r->phi, r->p.dc_max_iters > 1 ? r->p.dc_max_iters : 1, true)) return PGB_ERR_CUDA;
+        if (dst_dc(r, r->mg_f[top], r->p.dc_max_iters > 1 ? r->p.dc_max_iters : 1, true, &src)) return PGB_ERR_CUDA;
     } else {
-        PGB_CK(r, pgb_launch_pdl(k_to32, dim3(gb), dim3(256), 0, r->stream, r->mg32_f[top], (const double*)r->mg_f[top], G));
-        r->launches++;
         if (pgb_mg_fmg32(r)) return PGB_ERR_CUDA;
-        const float* e = r->mg32_u[top];   /* the FMG pass's result        */
+        src.e = r->mg32_u[top];   /* the FMG pass's result */
         const int passes = r->p.poisson_mode == PGB_POISSON_FP32_DC && r->p.dc_max_iters > 1 ? r->p.dc_max_iters : 1;
-        if (passes == 1) {
-            PGB_CK(r, pgb_launch_pdl(k_to64, dim3(gb), dim3(256), 0, r->stream, r->phi, e, G));
-            r->launches++;
-        } else {
-            const double h = r->p.xlength / (n - 1), h2i = 1.0 / (h * h);
-            double* ua = nullptr;        /* FP64 solution so far (null: 0) */
-            double* ub = r->dc_u;
-            for (int it = 1; it < passes; ++it) {
-                /* the defect goes to the level's residual array, its V-cycle
-                 * from 0 to the level's correction array                 */
-                PGB_CK(r, pgb_launch_pdl(k_dc_update, dim3(gb), dim3(256), 0, r->stream, (const double*)ua, e, ub,
-                                         (const double*)r->mg_f[top], r->mg32_r[top], n, h2i));
-                r->launches++;
-                ua = ub;
-                ub = (ub == r->dc_u) ? r->dc_u2 : r->dc_u;
-                if (pgb_mg_vcycle32(r)) return PGB_ERR_CUDA;
-                e = r->mg32_v[top];
-            }
-            PGB_CK(r, pgb_launch_pdl(k_dc_final, dim3(gb), dim3(256), 0, r->stream, r->phi, (const double*)ua, e, G));
-            r->launches++;
-        }
+        /* each defect goes to the level's residual array, its V-cycle from 0
+         * to the level's correction array                                */
+        if (defect_correction(r, r->mg_f[top], r->mg32_r[top], r->mg32_v[top], passes, [&] { return pgb_mg_vcycle32(r); },
+                              &src))
+            return PGB_ERR_CUDA;
     }
-    PGB_CK(r, pgb_launch_pdl(k_walls, dim3(blocks_for((long long)r->nx * r->ny)), dim3(256), 0, r->stream, r->phi, r->nx, r->ny, r->p.phi_left, r->phi_tab,
-                                                                         r->ds, r->p.phi_bottom, r->p.phi_top));
-    r->launches++;
-    PGB_CK(r, cudaGetLastError());
-    return 0;
+    return launch_field(r, src, field, advance);
 }
 
-int pgb_launch_efield(pgb_run* r, int advance) {
-    int GE = (r->nx + 1) * (r->ny + 1);
-    PGB_CK(r, pgb_launch_pdl(k_efield, dim3(blocks_for(GE)), dim3(256), 0, r->stream, r->phi, r->ex, r->ey, r->exy, r->nx, r->ny, 2.0 * r->dx, r->ds, advance));
-    r->launches++;
-    PGB_CK(r, cudaGetLastError());
-    return 0;
-}
-
-
+/* E of the potential in r->phi (the step's field comes with its potential) */
+int pgb_launch_efield(pgb_run* r) { return launch_field(r, PhiSource{nullptr, nullptr, r->phi}, true, false); }

@@ -67,7 +67,7 @@ struct DevState {
                                 potential); trails t while a solve overlaps the next
                                 step's collisions                                      */
     unsigned int ticket;     /* blocks of a wall kernel that are done            */
-    unsigned int pad3;
+    unsigned int ticket_f;   /* the same of k_field                              */
     long long n_cx;          /* ion slots whose charge exchange was tested before this
                                 step's appends (the rest are tested after them)       */
 };
@@ -354,7 +354,8 @@ void pgb_bins(pgb_run* r, int* nbx, int* nby);
 int pgb_launch_reduce(pgb_run* r, int s);
 int pgb_launch_step_advance(pgb_run* r);
 int pgb_launch_graphs(pgb_run* r);
-int pgb_poisson_solve(pgb_run* r);
-int pgb_launch_efield(pgb_run* r, int advance);
+/* the potential, with `field` E too; advance: then ds->tf += 1 */
+int pgb_poisson_solve(pgb_run* r, bool field = false, bool advance = false);
+int pgb_launch_efield(pgb_run* r);
 int pgb_launch_rhs(pgb_run* r);
 int pgb_launch_cross_sections(int which, const double* d_e, long long n, double* d_out, cudaStream_t st);
