@@ -1206,9 +1206,14 @@ static int issue_one_step(pgb_run* r) {
         if ((rc = flush_fields(r)) || (rc = pgb_launch_graphs(r))) return rc;
     }
     r->time_step += 1;
-    /* counters come back asynchronously; the host reads them only to
-     * decide when to compact, which never changes results          */
-    PGB_CK(r, cudaMemcpyAsync(r->hs, r->ds, sizeof(DevState), cudaMemcpyDeviceToHost, r->stream));
+    /* Counters come back asynchronously; the host reads them only to decide
+     * when to compact and, before a sort, whether the storage has to grow,
+     * which never changes results.  A copy between two steps' graphs costs
+     * some 3 us, so only every eighth step, and the one before a sort, has
+     * one.                                                                */
+    const long long t = r->time_step;
+    if (t % 8 == 0 || (r->p.sort_interval > 0 && (t + 1) % r->p.sort_interval == 0))
+        PGB_CK(r, cudaMemcpyAsync(r->hs, r->ds, sizeof(DevState), cudaMemcpyDeviceToHost, r->stream));
     return 0;
 }
 

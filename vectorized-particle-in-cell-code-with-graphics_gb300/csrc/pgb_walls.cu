@@ -431,7 +431,12 @@ __global__ void __launch_bounds__(WALL_CHUNK) k_ewall2(WallArgs a) {
 /* boundary::steadyBoundaryX/Y (boundary.cpp:890-1082): per wall, the r-th
  * outside electron in list order is paired with the r-th outside ion, and
  * both are re-inserted at one random point (plop_particles,
- * boundary.cpp:854-878).  One CTA; lists are a small fraction of N.       */
+ * boundary.cpp:854-878).  A cluster of STEADY_CTAS CTAs, each with a run of
+ * both lists: it counts its outside particles per wall, and the counts of
+ * the CTAs before it give its ranks.  (Unpaired particles stay outside and
+ * stay listed, so the lists grow: at 100 steps of the default preset with
+ * 300k particles one CTA took 85 us of a 324 us step.)                    */
+#define STEADY_CTAS 16
 __device__ __forceinline__ int steady_class(float c, int ncells, int ps) {
     if (pos_lt0(c)) return 1;               /* left / bottom  */
     if (pcell(c, ps) >= ncells) return 2;   /* right / top    */
@@ -456,47 +461,88 @@ __device__ __forceinline__ void block_scan2(int a, int b, int& ea, int& eb, int&
     ta = sa; tb = sb;
     __syncthreads();
 }
+/* every CTA's writes before are seen by every CTA's reads (past L1) after */
+__device__ __forceinline__ void steady_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+/* the wall coordinate of a listed particle, past L1: another CTA of the
+ * cluster may have re-inserted it                                        */
+__device__ __forceinline__ int listed_class(const float4* xv, int slot, int axis, int nc, int ps) {
+    const float2 p = __ldcg(reinterpret_cast<const float2*>(xv + slot));
+    return steady_class(axis == 0 ? p.x : p.y, nc, ps);
+}
 
-__global__ void __launch_bounds__(1024) k_steady(WallArgs a, int* ion_by_rank) {
+/* count: 4 * STEADY_CTAS ints of scratch */
+__global__ void __launch_bounds__(512) k_steady(WallArgs a, int* ion_by_rank, int* count) {
     pgb_pdl_entry();
     const long long me_ = a.ds->list_n[LIST_OUT_E], mi_ = a.ds->list_n[LIST_OUT_I];
-    __shared__ int s_plops;
+    const int cta = blockIdx.x;
+    /* this CTA's runs of the lists */
+    const long long pe = (me_ + STEADY_CTAS - 1) / STEADY_CTAS, pi = (mi_ + STEADY_CTAS - 1) / STEADY_CTAS;
+    const long long e0 = min(pe * cta, me_), e1 = min(e0 + pe, me_), i0 = min(pi * cta, mi_), i1 = min(i0 + pi, mi_);
+    __shared__ int s_cnt[4], s_plops;
     if (threadIdx.x == 0) s_plops = 0;
     for (int axis = 0; axis < 2; ++axis) {
         const int nc = axis == 0 ? a.nx : a.ny;
+        /* ions and electrons of this CTA at the low and the high wall */
+        if (threadIdx.x < 4) s_cnt[threadIdx.x] = 0;
+        __syncthreads();
+        int c4[4] = {0, 0, 0, 0};
+        for (long long k = i0 + threadIdx.x; k < i1; k += blockDim.x) {
+            const int cls = listed_class(a.i.xv, a.list_i[k], axis, nc, a.ps);
+            c4[0] += cls == 1;
+            c4[1] += cls == 2;
+        }
+        for (long long k = e0 + threadIdx.x; k < e1; k += blockDim.x) {
+            const int cls = listed_class(a.e.xv, a.list_e[k], axis, nc, a.ps);
+            c4[2] += cls == 1;
+            c4[3] += cls == 2;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int v = __reduce_add_sync(0xffffffffu, c4[q]);
+            if ((threadIdx.x & 31) == 0 && v) atomicAdd(&s_cnt[q], v);
+        }
+        __syncthreads();
+        if (threadIdx.x < 4) count[4 * cta + threadIdx.x] = s_cnt[threadIdx.x];
+        steady_sync();
+        /* counts before this CTA, and all ions' */
+        int lo_i = 0, hi_i = 0, rlo = 0, rhi = 0, cnt_lo = 0, cnt_hi = 0;
+        for (int c = 0; c < STEADY_CTAS; ++c) {
+            const int4 v = __ldcg(reinterpret_cast<const int4*>(count) + c);
+            if (c < cta) { lo_i += v.x; hi_i += v.y; rlo += v.z; rhi += v.w; }
+            cnt_lo += v.x;
+            cnt_hi += v.y;
+        }
         /* ions: record slots by (class, rank); lo from the front, hi from the back */
-        int cnt_lo = 0, cnt_hi = 0;
-        for (long long b = 0; b < mi_; b += blockDim.x) {
+        for (long long b = i0; b < i1; b += blockDim.x) {
             long long k = b + threadIdx.x;
             int cls = 0, slot = -1;
-            if (k < mi_) {
+            if (k < i1) {
                 slot = a.list_i[k];
-                float4 p = a.i.xv[slot];
-                cls = steady_class(axis == 0 ? p.x : p.y, nc, a.ps);
+                cls = listed_class(a.i.xv, slot, axis, nc, a.ps);
             }
             int ea, eb, ta, tb;
             block_scan2(cls == 1, cls == 2, ea, eb, ta, tb);
-            if (cls == 1) ion_by_rank[cnt_lo + ea] = slot;
-            if (cls == 2) ion_by_rank[mi_ - 1 - (cnt_hi + eb)] = slot;
-            cnt_lo += ta;
-            cnt_hi += tb;
+            if (cls == 1) ion_by_rank[lo_i + ea] = slot;
+            if (cls == 2) ion_by_rank[mi_ - 1 - (hi_i + eb)] = slot;
+            lo_i += ta;
+            hi_i += tb;
         }
-        __syncthreads();
+        steady_sync();
         /* electrons: pair by rank */
-        int rlo = 0, rhi = 0;
-        for (long long b = 0; b < me_; b += blockDim.x) {
+        for (long long b = e0; b < e1; b += blockDim.x) {
             long long k = b + threadIdx.x;
             int cls = 0, slot = -1;
-            if (k < me_) {
+            if (k < e1) {
                 slot = a.list_e[k];
-                float4 p = a.e.xv[slot];
-                cls = steady_class(axis == 0 ? p.x : p.y, nc, a.ps);
+                cls = listed_class(a.e.xv, slot, axis, nc, a.ps);
             }
             int ea, eb, ta, tb;
             block_scan2(cls == 1, cls == 2, ea, eb, ta, tb);
             int partner = -1;
-            if (cls == 1 && rlo + ea < cnt_lo) partner = ion_by_rank[rlo + ea];
-            if (cls == 2 && rhi + eb < cnt_hi) partner = ion_by_rank[mi_ - 1 - (rhi + eb)];
+            if (cls == 1 && rlo + ea < cnt_lo) partner = __ldcg(ion_by_rank + rlo + ea);
+            if (cls == 2 && rhi + eb < cnt_hi) partner = __ldcg(ion_by_rank + mi_ - 1 - (rhi + eb));
             if (partner >= 0) {
                 pgb_stream st;
                 pgb_stream_init(&st, a.seed, a.e.id[slot], (unsigned int)a.ds->t, PGB_STREAM_PLOP, 0);
@@ -508,20 +554,19 @@ __global__ void __launch_bounds__(1024) k_steady(WallArgs a, int* ion_by_rank) {
                 double evz = maxwell_fp64(&st, a.vte), ivz = maxwell_fp64(&st, a.vti);
                 store_particle(a.e, slot, x, y, evx, evy, evz, a.dx, a.dy, a.ps);
                 store_particle(a.i, partner, x, y, ivx, ivy, ivz, a.dx, a.dy, a.ps);
-                float4 q = a.e.xv[slot];
-                maybe_deposit(a.qacc_e, a.nx, a.ny, a.ps, q.x, q.y, a.e.w[slot]);
-                q = a.i.xv[partner];
-                maybe_deposit(a.qacc_i, a.nx, a.ny, a.ps, q.x, q.y, a.i.w[partner]);
+                const float px = pos_from_m(x, a.dx, a.ps), py = pos_from_m(y, a.dy, a.ps);
+                maybe_deposit(a.qacc_e, a.nx, a.ny, a.ps, px, py, a.e.w[slot]);
+                maybe_deposit(a.qacc_i, a.nx, a.ny, a.ps, px, py, a.i.w[partner]);
                 atomicAdd(&s_plops, 1);
             }
             rlo += ta;
             rhi += tb;
         }
-        __syncthreads();
+        steady_sync();
     }
     if (threadIdx.x == 0) {
-        a.ds->stats[ST_PLOP] += s_plops;
-        if (a.advance) pgb_step_end(a.ds);
+        if (s_plops) atomicAdd((unsigned long long*)&a.ds->stats[ST_PLOP], (unsigned long long)s_plops);
+        if (cta == 0 && a.advance) pgb_step_end(a.ds);   /* every CTA has read the step by now */
     }
 }
 
@@ -851,9 +896,22 @@ int pgb_launch_walls(pgb_run* r, int which, bool advance) {
     const dim3 g(r->sms * 4), b(WALL_CHUNK);
     if (r->p.steadystate) {
         if (which == PGB_BOUNDARY_ELECTRONS) {
-            PGB_CK(r, pgb_launch_pdl(k_steady, dim3(1), dim3(1024), 0, r->stream, a, r->aux_i));
+            /* aux_i: ion slots by rank (at most list_cap); aux_j: the counts */
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(STEADY_CTAS);
+            cfg.blockDim = dim3(512);
+            cfg.stream = r->stream;
+            cudaLaunchAttribute attr[2];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            attr[1].id = cudaLaunchAttributeClusterDimension;
+            attr[1].val.clusterDim.x = STEADY_CTAS;
+            attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 2;
+            PGB_CK(r, cudaFuncSetAttribute(k_steady, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            PGB_CK(r, cudaLaunchKernelEx(&cfg, k_steady, a, r->aux_i, r->aux_j));
             r->launches++;
-            PGB_CK(r, cudaGetLastError());
         }
         return 0;
     }
