@@ -883,15 +883,25 @@ static int particles_lanes(Lanes& L, bool ion_step) {
     pgb_run* const r = L.r;
     const size_t G = (size_t)r->nx * r->ny;
     const bool products = products_stored(r, ion_step), inject = r->p.number_to_inject > 0;
+    /* Walls that only remove what reaches them need no list: the push does
+     * it.  Electrons without impact emission (their yield, and with it
+     * reflection and backscatter, is 0 then), ions without theirs.  A
+     * stored product takes its parent's position after the push, so the
+     * parent is kept until then.                                          */
+    const bool emits_e = r->p.e_impact_see != 0, emits_i = r->p.species == PGB_ARGON && r->p.ion_impact_see;
+    const bool absorb_e = !r->p.steadystate && !emits_e && !emits_i && !products,
+               absorb_i = !r->p.steadystate && !emits_i;
     /* where the products' number is entered: with the injection, else with
-     * the wall lists (both come before the walls take new ids)            */
+     * the wall lists, else at the end (all come before the walls take ids) */
     const int commit_e = r->p.have_collisions && !products ? 1 : 0, commit_i = 2 * commit_e;
+    int commit_end = 0;
     /* get_particle_electric_field + move_particles, charge deposit */
     L.electrons();
     PROF_MARK(r, 8);
-    if (pgb_launch_push(r, 0, true)) return PGB_ERR_CUDA;
+    if (pgb_launch_push(r, 0, true, absorb_e)) return PGB_ERR_CUDA;
     PROF_MARK(r, 7);
-    if (pgb_build_list(r, LIST_OUT_E, 0, inject ? 0 : commit_e)) return PGB_ERR_CUDA;
+    if (!absorb_e && pgb_build_list(r, LIST_OUT_E, 0, inject ? 0 : commit_e)) return PGB_ERR_CUDA;
+    if (absorb_e && !inject) commit_end |= commit_e;
     PROF_MARK(r, 1);
     if (products) {
         /* the ionization products join after the push: an ion takes its
@@ -899,7 +909,7 @@ static int particles_lanes(Lanes& L, bool ion_step) {
         if (pgb_launch_ionize_appends(r, r->p.steadystate ? 1 : 0, 1) || L.ions_after_electrons()) return PGB_ERR_CUDA;
     }
     /* inject_more_particles: electrons are pushed as they are created */
-    if (inject && pgb_launch_inject(r, 1, true, commit_e)) return PGB_ERR_CUDA;
+    if (inject && pgb_launch_inject(r, 1, true, commit_e, absorb_e)) return PGB_ERR_CUDA;
     L.ions();
     if (inject && pgb_launch_inject(r, 2, true, commit_i)) return PGB_ERR_CUDA;
     PROF_MARK(r, 2);
@@ -911,27 +921,28 @@ static int particles_lanes(Lanes& L, bool ion_step) {
         const bool few = !r->p.steadystate && r->p.number_to_inject <= 4096;
         if (r->p.have_collisions && appended && pgb_launch_cx(r, few ? 2 : 1, 0)) return PGB_ERR_CUDA;
         PROF_MARK(r, 3);
-        if (pgb_launch_push(r, 1, true)) return PGB_ERR_CUDA;
-        if (pgb_build_list(r, LIST_OUT_I, 1, inject ? 0 : commit_i)) return PGB_ERR_CUDA;
+        if (pgb_launch_push(r, 1, true, absorb_i)) return PGB_ERR_CUDA;
+        if (!absorb_i && pgb_build_list(r, LIST_OUT_I, 1, inject ? 0 : commit_i)) return PGB_ERR_CUDA;
+        if (absorb_i && !inject) commit_end |= commit_i;
         PROF_MARK(r, 4);
+        if (L.join()) return PGB_ERR_CUDA;
+        L.electrons();
         /* electrons emitted by ion impact join after the injected ones */
-        const bool emits = r->p.species == PGB_ARGON && r->p.ion_impact_see;
-        if (emits) {
-            if (L.join()) return PGB_ERR_CUDA;
-            L.electrons();
-        }
-        if (pgb_launch_walls(r, PGB_BOUNDARY_IONS)) return PGB_ERR_CUDA;
-        if (!emits && L.join()) return PGB_ERR_CUDA;
+        if (!absorb_i && pgb_launch_walls(r, PGB_BOUNDARY_IONS)) return PGB_ERR_CUDA;
     } else {
         PROF_MARK(r, 3);
         if (pgb_launch_deposit(r, 1)) return PGB_ERR_CUDA;
         if (r->p.steadystate && (pgb_launch_flag_outside(r, 1) || pgb_build_list(r, LIST_OUT_I, 1))) return PGB_ERR_CUDA;
         PROF_MARK(r, 4);
         if (L.join()) return PGB_ERR_CUDA;
+        L.electrons();
     }
-    L.electrons();
     const bool reduce = !no_reduction(r);
-    if (pgb_launch_walls(r, PGB_BOUNDARY_ELECTRONS, !reduce)) return PGB_ERR_CUDA;
+    if (!absorb_e) {
+        if (pgb_launch_walls(r, PGB_BOUNDARY_ELECTRONS, !reduce, commit_end)) return PGB_ERR_CUDA;
+        commit_end = 0;
+    }
+    if (absorb_e && !reduce) return pgb_launch_step_advance(r, commit_end);
     if (!reduce) return 0;
     /* contain_particle_growth: only when a species can exceed its limit */
     for (int s = 0; s < 2; ++s) {
@@ -948,7 +959,7 @@ static int particles_lanes(Lanes& L, bool ion_step) {
             }
         }
     }
-    return pgb_launch_step_advance(r);
+    return pgb_launch_step_advance(r, commit_end);
 }
 
 static int step_fields(pgb_run* r, bool) {

@@ -303,6 +303,14 @@ inline cudaError_t pgb_launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, si
     } while (0)
 
 #ifdef __CUDACC__
+/* The event count of a step whose ionization products are not stored (see
+ * particles_lanes): the ids that they would have taken, and their removal,
+ * per species.  One thread.                                              */
+__device__ __forceinline__ void ionize_count_commit(DevState* ds, int species_mask) {
+    const long long m = ds->list_n[LIST_ION_EV];
+    if (species_mask & 1) { ds->next_id[0] += (unsigned int)m; ds->stats[ST_ABS_E] += m; }
+    if (species_mask & 2) { ds->next_id[1] += (unsigned int)m; ds->stats[ST_ABS_I] += m; }
+}
 /* end of a step's particle phases: the step counter moves on, and the
  * ionization events are counted from 0 again.  One thread.               */
 __device__ __forceinline__ void pgb_step_end(DevState* ds) {
@@ -313,7 +321,8 @@ __device__ __forceinline__ void pgb_step_end(DevState* ds) {
 
 /* kernels launched from the host side (defined in the .cu files) */
 struct CollConsts;
-int pgb_launch_push(pgb_run* r, int s, bool deposit);
+/* absorb: particles that leave are removed by the push (no wall list) */
+int pgb_launch_push(pgb_run* r, int s, bool deposit, bool absorb = false);
 int pgb_launch_flag_outside(pgb_run* r, int s);
 /* commit: species (1 electrons, 2 ions) whose ionization products, which
  * are not stored, are entered with the list                              */
@@ -321,15 +330,16 @@ int pgb_build_list(pgb_run* r, int which, int species_for_tiles, int commit = 0)
 int pgb_launch_deposit(pgb_run* r, int s);
 /* clear: leave the charge accumulators zero for the next step */
 int pgb_launch_finalize(pgb_run* r, int which_species_mask, bool make_rhs, bool clear = false);
-int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit = 0);
+int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit = 0, bool absorb_e = false);
 int pgb_launch_ionize_appends(pgb_run* r, int store_e, int store_i);
 /* count_events: ds->list_n[LIST_ION_EV] counts the ionization events (from 0) */
 int pgb_launch_mcc(pgb_run* r, int leave_sms, bool count_events = false);
 /* tail 0: the ions present (records their count); 1: those appended since;
  * 2: the same in one block, for a tail of a few thousand ions at most     */
 int pgb_launch_cx(pgb_run* r, int tail, int leave_sms);
-/* advance: the last kernel of the electron (or steady) walls ends the step */
-int pgb_launch_walls(pgb_run* r, int which, bool advance = false);
+/* advance: the last kernel of the electron (or steady) walls ends the step,
+ * after entering the products of the species in commit                   */
+int pgb_launch_walls(pgb_run* r, int which, bool advance = false, int commit = 0);
 int pgb_launch_load(pgb_run* r, int s, const double* d_aos, long long i0, long long i1);
 int pgb_launch_dump_offsets(pgb_run* r, int s);
 int pgb_launch_dump(pgb_run* r, int s, double* d_out, unsigned int* d_ids, long long cap, int t0, int t1);
@@ -352,7 +362,7 @@ int pgb_launch_sort(pgb_run* r, int s);
 int pgb_sort_setup(pgb_run* r);
 void pgb_bins(pgb_run* r, int* nbx, int* nby);
 int pgb_launch_reduce(pgb_run* r, int s);
-int pgb_launch_step_advance(pgb_run* r);
+int pgb_launch_step_advance(pgb_run* r, int commit = 0);
 int pgb_launch_graphs(pgb_run* r);
 /* the potential, with `field` E too; advance: then ds->tf += 1 */
 int pgb_poisson_solve(pgb_run* r, bool field = false, bool advance = false);

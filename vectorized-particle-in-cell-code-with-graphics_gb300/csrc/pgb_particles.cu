@@ -245,9 +245,11 @@ __device__ __forceinline__ void deposit_win(unsigned long long* qacc, unsigned i
     }
 }
 
-template <bool DEP>
+/* ABSORB: a particle that leaves is removed here (and counted), where the
+ * walls would do nothing else with it; else its tile's wall list is made */
+template <bool DEP, bool ABSORB>
 __device__ __forceinline__ void push_tile(const PushArgs& a, const PushConsts& pc, int tile, long long n,
-                                          unsigned int* win, int ox, int oy, int* s_cnt, int& it) {
+                                          unsigned int* win, int ox, int oy, int* s_cnt, int& it, int& gone) {
     const long long base = (long long)tile * PGB_TILE;
     bool f[PGB_ITEMS];
     /* all loads of the thread's items first, so that they are in flight
@@ -273,19 +275,23 @@ __device__ __forceinline__ void push_tile(const PushArgs& a, const PushConsts& p
         if (is_dead(p[k].x)) continue;
         bool moved;
         gather_push_one(pc, a.exy, p[k], vz[k], moved);
-        if (moved) a.xv[i] = p[k];
-        if (pc.bfield && moved) a.vz[i] = vz[k];
         if (DEP && deposit_ok(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps))
             deposit_win(a.qacc, win, ox, oy, pc.nx, pc.ps, p[k].x, p[k].y, w[k]);
         f[k] = pc.steady ? outside_steady(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps)
                          : outside_absorbing(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps);
+        if (ABSORB && f[k]) {
+            p[k].x = pos_dead();
+            gone++;
+        }
+        if (moved || (ABSORB && f[k])) a.xv[i] = p[k];
+        if (pc.bfield && moved) a.vz[i] = vz[k];
     }
-    tile_masks(f, tile, (unsigned*)a.tl_out, a.tc_out, s_cnt, it);
+    if (!ABSORB) tile_masks(f, tile, (unsigned*)a.tl_out, a.tc_out, s_cnt, it);
 }
 
 /* Work items: the bin pieces of the last sort (tiles of one bin, deposited
  * through a shared window), then every tile after the sorted region.     */
-template <bool DEP>
+template <bool DEP, bool ABSORB>
 __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
     pgb_pdl_entry();
     __shared__ unsigned int s_win[WIN_NODES];
@@ -296,7 +302,7 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
     const int nitems = npieces + (ntiles > tile0 ? ntiles - tile0 : 0);
     const PushConsts pc = a.pc;
     __shared__ int s_cnt[2];
-    int it = 0;
+    int it = 0, gone = 0;
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
     /* the window starts zeroed; each flush leaves it zeroed again */
     if (DEP && npieces > 0)
@@ -313,7 +319,7 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
                 oy = (pc4.z / a.nbx) * PGB_BIN - PGB_HALO;
             }
             for (int t = pc4.x; t < pc4.x + pc4.y && t < ntiles; ++t)
-                push_tile<DEP>(a, pc, t, n, win, ox, oy, s_cnt, it);
+                push_tile<DEP, ABSORB>(a, pc, t, n, win, ox, oy, s_cnt, it, gone);
             if (win) {
                 __syncthreads();
                 /* a warp per window row, a lane per node: add the non-zero
@@ -335,7 +341,14 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
                 __syncthreads();
             }
         } else {
-            push_tile<DEP>(a, pc, tile0 + (item - npieces), n, nullptr, 0, 0, s_cnt, it);
+            push_tile<DEP, ABSORB>(a, pc, tile0 + (item - npieces), n, nullptr, 0, 0, s_cnt, it, gone);
+        }
+    }
+    if (ABSORB) {
+        gone = __reduce_add_sync(0xffffffffu, gone);
+        if ((threadIdx.x & 31) == 0 && gone) {
+            atomicAdd((unsigned long long*)&a.ds->dead[a.s], (unsigned long long)gone);
+            atomicAdd((unsigned long long*)&a.ds->stats[a.s == 0 ? ST_ABS_E : ST_ABS_I], (unsigned long long)gone);
         }
     }
 }
@@ -534,9 +547,11 @@ __global__ void __launch_bounds__(MCC_THREADS, 1) k_mcc(PushArgs a, int list) {
 }
 
 /* the last kernel of a step's particle phases moves the step counter on
- * (where the wall kernels do not, see pgb_launch_walls)                  */
-__global__ void k_step_advance(DevState* ds) {
+ * (where the wall kernels do not, see pgb_launch_walls); commit: species
+ * whose uncounted ionization products it enters                          */
+__global__ void k_step_advance(DevState* ds, int commit) {
     pgb_pdl_entry();
+    if (commit) ionize_count_commit(ds, commit);
     pgb_step_end(ds);
 }
 
@@ -598,15 +613,6 @@ __global__ void __launch_bounds__(1024) k_scan_small(const int* cnt, int* off, c
     const long long m = n_ptr ? (*n_ptr + PGB_TILE - 1) / PGB_TILE : m_const;
     long long t = block_excl_scan(cnt, off, m, 0);
     if (threadIdx.x == 0) *total = t;
-}
-
-/* The event count of a step whose ionization products are not stored (see
- * step_particles): the ids that they would have taken, and their removal,
- * per species.  One thread.                                              */
-__device__ __forceinline__ void ionize_count_commit(DevState* ds, int species_mask) {
-    const long long m = ds->list_n[LIST_ION_EV];
-    if (species_mask & 1) { ds->next_id[0] += (unsigned int)m; ds->stats[ST_ABS_E] += m; }
-    if (species_mask & 2) { ds->next_id[1] += (unsigned int)m; ds->stats[ST_ABS_I] += m; }
 }
 
 /* Per-tile lists (32 mask words a tile, see tile_masks) to one dense list
@@ -705,6 +711,7 @@ struct InjectArgs {
     const float2* exy;
     unsigned long long* qacc_e;
     int push_e;                  /* push the new electrons (inside pgb_step) */
+    int absorb_e;                /* ... and remove those that leave          */
     int species_mask;            /* 1 = electrons, 2 = ions                  */
     int* list_out_e;             /* append outside electrons (ordered)       */
     long long list_cap;
@@ -733,6 +740,12 @@ __device__ __forceinline__ bool inject_one(const InjectArgs& a, int s, int jj, l
         /* weight 0: the deposit adds nothing (particle.cpp:497) */
         out = a.pce.steady ? outside_steady(p.x, p.y, a.pce.nx, a.pce.ny, a.pce.ps)
                            : outside_absorbing(p.x, p.y, a.pce.nx, a.pce.ny, a.pce.ps);
+        if (out && a.absorb_e) {
+            p.x = pos_dead();
+            atomicAdd((unsigned long long*)&a.ds->dead[0], 1ull);
+            atomicAdd((unsigned long long*)&a.ds->stats[ST_ABS_E], 1ull);
+            out = false;   /* joins no list */
+        }
     }
     S.xv[slot] = p;
     S.vz[slot] = vz;
@@ -1112,10 +1125,10 @@ static PushArgs push_args(pgb_run* r, int s) {
     return a;
 }
 
-int pgb_launch_push(pgb_run* r, int s, bool deposit) {
+int pgb_launch_push(pgb_run* r, int s, bool deposit, bool absorb) {
     PushArgs a = push_args(r, s);
     int g = grid_for(r, r->tune_push_per_sm);
-    void (*kp)(PushArgs) = deposit ? k_push<true> : k_push<false>;
+    void (*kp)(PushArgs) = !deposit ? k_push<false, false> : absorb ? k_push<true, true> : k_push<true, false>;
     PGB_CK(r, pgb_launch_pdl(kp, dim3(g), dim3(PGB_PUSH_THREADS), 0, r->stream, a));
     r->launches++;
     PGB_CK(r, cudaGetLastError());
@@ -1132,8 +1145,8 @@ int pgb_launch_flag_outside(pgb_run* r, int s) {
 }
 
 
-int pgb_launch_step_advance(pgb_run* r) {
-    PGB_CK(r, pgb_launch_pdl(k_step_advance, dim3(1), dim3(1), 0, r->stream, r->ds));
+int pgb_launch_step_advance(pgb_run* r, int commit) {
+    PGB_CK(r, pgb_launch_pdl(k_step_advance, dim3(1), dim3(1), 0, r->stream, r->ds, commit));
     r->launches++;
     return 0;
 }
@@ -1173,13 +1186,13 @@ int pgb_launch_deposit(pgb_run* r, int s) {
     return 0;
 }
 
-int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit) {
+int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit, bool absorb_e) {
     InjectArgs a;
     a.e = r->sp[0]; a.i = r->sp[1]; a.ds = r->ds; a.k = r->p.number_to_inject;
     a.dx = r->dx; a.dy = r->dy; a.xlength = r->p.xlength; a.ylength = r->p.ylength;
     a.seed = r->p.seed;
     a.pce = push_consts(r, 0); a.exy = r->exy; a.qacc_e = r->qacc[0];
-    a.push_e = push_e; a.species_mask = species_mask;
+    a.push_e = push_e; a.absorb_e = absorb_e; a.species_mask = species_mask;
     a.list_out_e = r->list[LIST_OUT_E]; a.list_cap = r->list_cap;
     a.flag = r->inject_flag;
     if (a.k <= 0) return 0;

@@ -36,7 +36,7 @@ struct WallArgs {
     const int* list_i;
     int* aux;                  /* per list entry: secondary count  */
     int* csum;                 /* per WALL_CHUNK entries: their sum */
-    int advance;               /* the last block ends the step     */
+    int advance, commit;       /* the last block ends the step (pgb_launch_walls) */
     unsigned long long* qacc_e;
     unsigned long long* qacc_i;
     int nx, ny;
@@ -177,6 +177,7 @@ __device__ __forceinline__ void wall_commit(const WallArgs& a, long long m, int 
     ds->next_id[0] += (unsigned int)t;
     if (which == 0) { ds->stats[ST_ABS_I] += m; ds->dead[1] += m; }
     ds->stats[which == 0 ? ST_ISEE_EM : ST_SEE_EM] += t;
+    if (a.commit) ionize_count_commit(ds, a.commit);
     if (a.advance) pgb_step_end(ds);
 }
 
@@ -877,7 +878,7 @@ static WallArgs wall_args(pgb_run* r) {
     WallArgs a;
     a.e = r->sp[0]; a.i = r->sp[1]; a.ds = r->ds;
     a.list_e = r->list[LIST_OUT_E]; a.list_i = r->list[LIST_OUT_I];
-    a.aux = r->aux_i; a.csum = r->aux_j; a.advance = 0;
+    a.aux = r->aux_i; a.csum = r->aux_j; a.advance = a.commit = 0;
     a.qacc_e = r->qacc[0]; a.qacc_i = r->qacc[1];
     a.nx = r->nx; a.ny = r->ny; a.ps = r->ps; a.dx = r->dx; a.dy = r->dy; a.dt = r->p.dt;
     a.me = r->p.electron_mass; a.mi = r->p.ion_mass;
@@ -890,9 +891,10 @@ static WallArgs wall_args(pgb_run* r) {
     return a;
 }
 
-int pgb_launch_walls(pgb_run* r, int which, bool advance) {
+int pgb_launch_walls(pgb_run* r, int which, bool advance, int commit) {
     WallArgs a = wall_args(r);
     a.advance = advance && which == PGB_BOUNDARY_ELECTRONS;
+    a.commit = commit;
     const dim3 g(r->sms * 4), b(WALL_CHUNK);
     if (r->p.steadystate) {
         if (which == PGB_BOUNDARY_ELECTRONS) {
