@@ -589,6 +589,7 @@ __global__ void __launch_bounds__(512) k_steady(WallArgs a, int* ion_by_rank, in
  * sum can reach 2^32.                                                     */
 #define CX_TILE PGB_CX_TILE
 #define CX_AHEAD 8
+#define CX_GROUPS 8
 #define CX_ONE (1ll << 40)
 static_assert((long long)CX_TILE << 20 <= (1ll << 31), "32-bit halves of the tile sums must not overflow");
 
@@ -752,30 +753,44 @@ __global__ void __launch_bounds__(256) k_cx_walk(CxArgs a) {
             for (int w = lane; w < (ntiles + 63) / 64; w += 32) mrow[w] = 0ull;
         return;
     }
-    for (int t0 = 0; t0 < ntiles; t0 += 32) {
-        int t = t0 + lane;
-        long long s = (t < ntiles && ((mrow[t >> 6] >> (t & 63)) & 1ull)) ? row[t] : 0;
-        /* inclusive prefix over the 32 tiles */
-        long long ps = s;
-        for (int d = 1; d < 32; d <<= 1) {
-            long long y = __shfl_up_sync(0xffffffffu, ps, d);
-            if (lane >= d) ps += y;
+    /* CX_GROUPS groups of 32 tile sums are in flight together (one group at
+     * a time, 2048 tiles were a chain of 64 pairs of loads, 23 us)        */
+    int next;
+    for (int t0 = 0; t0 < ntiles; t0 = next) {
+        long long sums[CX_GROUPS];
+#pragma unroll
+        for (int u = 0; u < CX_GROUPS; ++u) {
+            const int t = t0 + 32 * u + lane;
+            sums[u] = (t < ntiles && ((mrow[t >> 6] >> (t & 63)) & 1ull)) ? row[t] : 0;
         }
-        unsigned cross = __ballot_sync(0xffffffffu, acc + ps > CX_ONE);
-        if (!cross) {
-            acc += __shfl_sync(0xffffffffu, ps, 31);
-            continue;
+        next = t0 + 32 * CX_GROUPS;
+        int tt = -1;   /* the first tile that can fire */
+#pragma unroll
+        for (int u = 0; u < CX_GROUPS; ++u) {
+            if (tt >= 0 || !__any_sync(0xffffffffu, sums[u] != 0)) continue;
+            /* inclusive prefix over the 32 tiles */
+            long long ps = sums[u];
+            for (int d = 1; d < 32; d <<= 1) {
+                long long y = __shfl_up_sync(0xffffffffu, ps, d);
+                if (lane >= d) ps += y;
+            }
+            const unsigned cross = __ballot_sync(0xffffffffu, acc + ps > CX_ONE);
+            if (!cross) {
+                acc += __shfl_sync(0xffffffffu, ps, 31);
+                continue;
+            }
+            /* tiles before the first crossing cannot fire */
+            const int first = __ffs(cross) - 1;
+            const long long before = __shfl_sync(0xffffffffu, ps, first ? first - 1 : 0);
+            if (first) acc += before;
+            tt = t0 + 32 * u + first;
         }
-        /* tiles before the first crossing cannot fire */
-        int first = __ffs(cross) - 1;
-        long long before = first ? __shfl_sync(0xffffffffu, ps, first - 1) : 0;
-        acc += before;
-        /* scan tile t0+first element by element, then continue after it.
+        if (tt < 0) continue;
+        /* scan tile tt element by element, then continue after it.
          * The ions of CX_AHEAD batches are in flight together: one batch at
          * a time, a tile was a chain of 64 loads, 25-50 us for a whole step
          * in which any column crosses (argon, 257^2, 4 Mi ions: charge
          * exchange 119 us a step), while the GPU held one warp per column */
-        int tt = t0 + first;
         for (int b = 0; b < CX_TILE; b += 32 * CX_AHEAD) {
             float4 p[CX_AHEAD];
             float vz[CX_AHEAD];
@@ -809,8 +824,7 @@ __global__ void __launch_bounds__(256) k_cx_walk(CxArgs a) {
                 }
             }
         }
-        /* resume with the tiles after tt */
-        t0 = tt + 1 - 32;
+        next = tt + 1;   /* resume with the tiles after tt */
     }
     __syncwarp();
     for (int w = lane; w < (ntiles + 63) / 64; w += 32) mrow[w] = 0ull;
