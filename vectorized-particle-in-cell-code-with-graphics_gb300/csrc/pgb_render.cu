@@ -13,20 +13,17 @@
  *     int, at least 1 (graphics.cpp:421-452), and plots the particles with
  *     |vx|, |vy| below it (graphics.cpp:499-503);
  *   - a point is 2 x 2 pixels (glPointSize(2), graphics.cpp:483).  Points
- *     mark a one-byte-per-pixel layer (1 electrons, 2 ions; the ion pass
- *     runs second and overwrites), storing only where the byte changes:
- *     dense plasma puts tens of points on a pixel, and unconditional
- *     stores to the same lines serialise.  k_rd_resolve turns the layer
- *     into colours, one thread per pixel.
- *   - Blocks take 1024-particle tiles in a scrambled order (tile t * P mod
+ *     set bits of a one-bit-per-pixel layer per species (see rd_mark);
+ *     k_rd_resolve turns the layers into colours, ions over electrons.
+ *   - Blocks take 4096-particle tiles in a scrambled order (tile t * P mod
  *     ntiles, P a prime above any tile count): spatially sorted particles
- *     would otherwise put every block in flight on the same few bins, and
- *     so on the same few lines of the layer.
+ *     would otherwise put the blocks in flight on the same few words.
  * Field plots (k_rd_field, one thread per pixel): the pixel's grid
  * coordinate picks a cell; the cell's quad is inset by a tenth of a cell,
  * and its colour is the ramp of drawField (graphics.cpp:303-356) applied to
  * |mean of the four corners / max|.  The maximum comes from k_rd_fmax, an
- * order-independent max over the field (NaN values ignored).
+ * order-independent max over the field (NaN values ignored), the corners'
+ * values from k_rd_nodes.
  *
  * The unit is compiled with --fmad=false so that every pixel and colour
  * equals the oracle's C restatement of the same rules bit for bit.
@@ -77,11 +74,13 @@ struct PointArgs {
     uint32_t seed;
     const unsigned int* vmax;   /* phase: bits of max |vx|, |vy| */
     unsigned int* vmax_out;     /* k_rd_vmax */
-    unsigned char* layer;       /* one byte per pixel */
-    unsigned char mark;         /* 1 electrons, 2 ions */
+    unsigned int* layer;        /* one bit per pixel */
+    int words;                  /* of the layer */
+    int shared;                 /* the layer fits in shared memory */
 };
 
-#define RD_TILE 1024
+#define RD_TILE 4096
+#define RD_THREADS 1024
 #define RD_SCRAMBLE 2147483647ull   /* 2^31-1, prime and above any tile count (at most 2^21):
                                       t -> t * P mod ntiles is a permutation */
 
@@ -89,33 +88,43 @@ __device__ __forceinline__ long long rd_tile(long long t, long long ntiles) {
     return (long long)(((unsigned long long)t * RD_SCRAMBLE) % (unsigned long long)ntiles);
 }
 
+/* p.x, p.y: the position in FP32 cells (NaN for a NaN position) */
 __device__ __forceinline__ bool rd_candidate(const PointArgs& a, long long i, long long nlive, float4& p) {
-    p = a.xv[i];
     if (is_dead(p.x)) return false;
-    /* the position in FP32 cells (NaN for a NaN position) */
     p.x = pos_cellsf(p.x, a.ps);
     p.y = pos_cellsf(p.y, a.ps);
     if (!(p.x > 0.0f && p.x < (float)(a.nx - 1) && p.y > 0.0f && p.y < (float)(a.ny - 1))) return false;
+    if (a.max_points <= 0 || nlive <= a.max_points) return true;
     return rd_keep(a.id[i], a.seed, nlive, a.max_points);
 }
+/* f(i, particle) for the block's tiles; a thread's items load together */
+template <class F>
+__device__ __forceinline__ void rd_particles(const PointArgs& a, long long n, F f) {
+    const long long ntiles = (n + RD_TILE - 1) / RD_TILE;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const long long base = rd_tile(t, ntiles) * RD_TILE;
+        float4 p[RD_TILE / RD_THREADS];
+#pragma unroll
+        for (int q = 0; q < RD_TILE / RD_THREADS; ++q) {
+            const long long i = base + q * RD_THREADS + threadIdx.x;
+            p[q] = i < n ? a.xv[i] : make_float4(pos_dead(), 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int q = 0; q < RD_TILE / RD_THREADS; ++q) f(base + q * RD_THREADS + threadIdx.x, p[q]);
+    }
+}
 
-__global__ void __launch_bounds__(256) k_rd_vmax(PointArgs a) {
+__global__ void __launch_bounds__(RD_THREADS) k_rd_vmax(PointArgs a) {
     const long long n = a.ds->n[a.s], nlive = n - a.ds->dead[a.s];
     unsigned int mx = 0u, my = 0u;
-    const long long ntiles = (n + RD_TILE - 1) / RD_TILE;
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x)
-    for (long long i = rd_tile(t, ntiles) * RD_TILE + threadIdx.x, e = min(n, rd_tile(t, ntiles) * RD_TILE + RD_TILE);
-         i < e; i += blockDim.x) {
-        float4 p;
-        if (!rd_candidate(a, i, nlive, p)) continue;
+    rd_particles(a, n, [&](long long i, float4 p) {
+        if (!rd_candidate(a, i, nlive, p)) return;
         const float ax = fabsf(p.z), ay = fabsf(p.w);
         if (ax == ax) mx = max(mx, __float_as_uint(ax));   /* non-negative floats order as their bits */
         if (ay == ay) my = max(my, __float_as_uint(ay));
-    }
-    for (int d = 16; d; d >>= 1) {
-        mx = max(mx, __shfl_down_sync(0xffffffffu, mx, d));
-        my = max(my, __shfl_down_sync(0xffffffffu, my, d));
-    }
+    });
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    my = __reduce_max_sync(0xffffffffu, my);
     if ((threadIdx.x & 31) == 0) {
         if (mx) atomicMax(&a.vmax_out[0], mx);
         if (my) atomicMax(&a.vmax_out[1], my);
@@ -129,28 +138,54 @@ __device__ __forceinline__ int rd_vscale(unsigned int bits) {
     return m < 1 ? 1 : m;
 }
 
-__device__ __forceinline__ void rd_splat(const PointArgs& a, int px, int py) {
-    for (int dy = 0; dy < 2; ++dy)
-        for (int dx = 0; dx < 2; ++dx) {
-            const int x = px + dx, y = py - dy;
-            if (x < 0 || x >= a.width || y < 0 || y >= a.height) continue;
-            unsigned char* q = a.layer + (long long)y * a.width + x;
-            if (*q != a.mark) *q = a.mark;   /* a racing store writes the same byte */
-        }
+/* The pixels that points cover are bits: a block marks them in its own copy
+ * of the layer in shared memory (an image of 1.6 M pixels fits) and adds
+ * that to the layer at its end; a larger image is marked in the layer
+ * itself.  Marks are only set, in any order, so the image does not depend on
+ * it; a bit already seen set needs no atomic.  With a byte per pixel in
+ * global memory, read and stored by every point, the X-Y frame of 3 M
+ * particles at 768^2 took 2 x 160 us.                                     */
+__device__ __forceinline__ void rd_mark(unsigned int* w, unsigned int m) {
+    if ((*(volatile unsigned int*)w & m) != m) atomicOr(w, m);
 }
-
-/* layer byte -> colour: 0 black, 1 electron colour, 2 ion colour */
-__global__ void k_rd_resolve(const unsigned char* layer, long long npx, Rgb c1, Rgb c2, unsigned char* img) {
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < npx; k += (long long)gridDim.x * blockDim.x) {
-        const unsigned char m = layer[k];
-        const Rgb c = m == 1 ? c1 : (m == 2 ? c2 : Rgb{0, 0, 0});
-        img[3 * k] = c.r;
-        img[3 * k + 1] = c.g;
-        img[3 * k + 2] = c.b;
+/* a 2 x 2 point with its lower left pixel at (px, py) */
+__device__ __forceinline__ void rd_splat(const PointArgs& a, unsigned int* layer, int px, int py) {
+    const int cols = px + 1 < a.width ? 2 : 1;
+    for (int dy = 0; dy < 2; ++dy) {
+        const int y = py - dy;
+        if (y < 0) continue;
+        const unsigned int k = (unsigned int)y * a.width + px, b = k & 31;
+        const unsigned int m = cols == 2 ? 3u : 1u;
+        rd_mark(layer + (k >> 5), m << b);
+        if (cols == 2 && b == 31) rd_mark(layer + (k >> 5) + 1, 1u);
     }
 }
 
-__global__ void __launch_bounds__(256) k_rd_points(PointArgs a) {
+/* layer bits -> colours: c2 over c1 over black; four pixels a thread */
+__global__ void k_rd_resolve(const unsigned int* l1, const unsigned int* l2, long long npx, Rgb c1, Rgb c2,
+                             unsigned char* img) {
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; 4 * q < npx; q += (long long)gridDim.x * blockDim.x) {
+        const long long k = 4 * q;
+        const unsigned int b1 = (l1 ? l1[k >> 5] : 0u) >> (k & 31), b2 = (l2 ? l2[k >> 5] : 0u) >> (k & 31);
+        unsigned char v[12];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const Rgb c = (b2 >> j) & 1u ? c2 : (b1 >> j) & 1u ? c1 : Rgb{0, 0, 0};
+            v[3 * j] = c.r; v[3 * j + 1] = c.g; v[3 * j + 2] = c.b;
+        }
+        if (k + 4 <= npx) {
+            unsigned int* const o = reinterpret_cast<unsigned int*>(img + 3 * k);
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                o[j] = v[4 * j] | (unsigned)v[4 * j + 1] << 8 | (unsigned)v[4 * j + 2] << 16 | (unsigned)v[4 * j + 3] << 24;
+        } else {
+            for (int j = 0; j < 3 * (int)(npx - k); ++j) img[3 * k + j] = v[j];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(RD_THREADS) k_rd_points(PointArgs a) {
+    extern __shared__ unsigned int s_layer[];
     const long long n = a.ds->n[a.s], nlive = n - a.ds->dead[a.s];
     int mvx = 1, mvy = 1;
     if (a.phase) {
@@ -158,15 +193,16 @@ __global__ void __launch_bounds__(256) k_rd_points(PointArgs a) {
         mvy = rd_vscale(a.vmax[1]);
     }
     const float W = (float)a.width, H = (float)a.height;
-    const long long ntiles = (n + RD_TILE - 1) / RD_TILE;
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x)
-    for (long long i = rd_tile(t, ntiles) * RD_TILE + threadIdx.x, e = min(n, rd_tile(t, ntiles) * RD_TILE + RD_TILE);
-         i < e; i += blockDim.x) {
-        float4 p;
-        if (!rd_candidate(a, i, nlive, p)) continue;
+    unsigned int* const layer = a.shared ? s_layer : a.layer;
+    if (a.shared) {
+        for (int k = threadIdx.x; k < a.words; k += RD_THREADS) s_layer[k] = 0u;
+        __syncthreads();
+    }
+    rd_particles(a, n, [&](long long i, float4 p) {
+        if (!rd_candidate(a, i, nlive, p)) return;
         float fx, fy;
         if (a.phase) {
-            if (!(fabsf(p.z) < (float)mvx && fabsf(p.w) < (float)mvy)) continue;
+            if (!(fabsf(p.z) < (float)mvx && fabsf(p.w) < (float)mvy)) return;
             fx = (p.z / (float)mvx + 1.0f) * 0.5f;
             fy = (p.w / (float)mvy + 1.0f) * 0.5f;
         } else {
@@ -176,7 +212,14 @@ __global__ void __launch_bounds__(256) k_rd_points(PointArgs a) {
         int px = (int)(fx * W), py = a.height - 1 - (int)(fy * H);
         px = px < 0 ? 0 : (px > a.width - 1 ? a.width - 1 : px);
         py = py < 0 ? 0 : (py > a.height - 1 ? a.height - 1 : py);
-        rd_splat(a, px, py);
+        rd_splat(a, layer, px, py);
+    });
+    if (a.shared) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < a.words; k += RD_THREADS) {
+            const unsigned int v = s_layer[k];
+            if (v && (a.layer[k] & v) != v) atomicOr(a.layer + k, v);
+        }
     }
 }
 
@@ -227,27 +270,30 @@ __device__ __forceinline__ void rd_ramp(float zAv, float (&c)[3]) {
     for (int k = 0; k < 3; ++k) c[k] = c_ramp[b][k] * (1.0f - alpha) + c_ramp[b + 1][k] * alpha;   /* glm::mix */
 }
 
-__global__ void k_rd_field(const double* src, double div, int n, int grid_start, const unsigned long long* fmax_key,
-                           int width, int height, unsigned char* img) {
+/* the plotted value of each node, (float)(src / div / max): once per node,
+ * not four times per pixel (FP64 divisions; 105 us of a 768^2 frame)       */
+__global__ void k_rd_nodes(const double* src, double div, int count, const unsigned long long* fmax_key, float* z) {
     double fmax = fabs(rd_unkey(*fmax_key));
     if (*fmax_key == 0ull || !(fmax >= 1.0)) fmax = 1.0;   /* if (fieldMax < 1.0) fieldMax = 1.0 */
-    const long long npx = (long long)width * height;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < npx; k += (long long)gridDim.x * blockDim.x) {
-        const int px = (int)(k % width), py = (int)(k / width);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x)
+        z[k] = (float)(src[k] / div / fmax);
+}
+__global__ void k_rd_field(const float* z, int n, int grid_start, int width, int height, unsigned char* img) {
+    const unsigned int npx = (unsigned int)width * (unsigned int)height;
+    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < npx; k += gridDim.x * blockDim.x) {
+        const int py = (int)(k / (unsigned)width), px = (int)(k - (unsigned)py * (unsigned)width);
         const float u = ((float)px + 0.5f) * (float)(n - 1) / (float)width;
         const float v = ((float)(height - 1 - py) + 0.5f) * (float)(n - 1) / (float)height;
         const int i = (int)u, j = (int)v;
         const float fu = u - (float)i, fv = v - (float)j;
-        unsigned char* q = img + 3 * k;
+        unsigned char* q = img + 3ull * k;
         if (i < grid_start || i >= n - grid_start - 1 || j < grid_start || j >= n - grid_start - 1 || fu < 0.1f ||
             fu > 0.9f || fv < 0.1f || fv > 0.9f) {
             q[0] = q[1] = q[2] = 0;
             continue;
         }
-        const float z0 = (float)(src[(long long)(j + 1) * n + i] / div / fmax);
-        const float z1 = (float)(src[(long long)(j + 1) * n + i + 1] / div / fmax);
-        const float z2 = (float)(src[(long long)j * n + i + 1] / div / fmax);
-        const float z3 = (float)(src[(long long)j * n + i] / div / fmax);
+        const float z0 = z[(long long)(j + 1) * n + i], z1 = z[(long long)(j + 1) * n + i + 1];
+        const float z2 = z[(long long)j * n + i + 1], z3 = z[(long long)j * n + i];
         const float zAv = (float)fabs((double)(z0 + z1 + z2 + z3) / 4.0);
         float c[3];
         rd_ramp(zAv, c);
@@ -276,16 +322,20 @@ extern "C" int pgb_render(pgb_run* r, int plot, int32_t width, int32_t height, i
     if (cap < bytes) return rd_fail(r, PGB_ERR_ARG, "pgb_render: rgb buffer smaller than width*height*3");
     if (plot <= PGB_PLOT_ION_VX_VY && (r->sp[0].cap == 0 || r->sp[1].cap == 0))
         return rd_fail(r, PGB_ERR_STATE, "pgb_render: load both species first");
-    if (4 * npx > r->rd_cap) {   /* RGB image, then the point layer */
+    /* the RGB image, then a bit layer per species or the nodes' values */
+    const long long words = (npx + 31) / 32 + 1, nodes = (long long)r->nx * r->ny;
+    const long long img_bytes = (bytes + 255) & ~255ll;
+    const long long need = img_bytes + std::max<long long>(8 * words, 4 * nodes);
+    if (need > r->rd_cap) {
         PGB_CK(r, cudaStreamSynchronize(r->stream));
         cudaFree(r->rd_img);
         r->rd_img = nullptr;
         r->rd_cap = 0;
-        if (cudaMalloc(&r->rd_img, (size_t)(4 * npx)) != cudaSuccess) {
+        if (cudaMalloc(&r->rd_img, (size_t)need) != cudaSuccess) {
             cudaGetLastError();
             return rd_fail(r, PGB_ERR_NOMEM, "pgb_render: image allocation failed");
         }
-        r->rd_cap = 4 * npx;
+        r->rd_cap = need;
     }
     if (!r->rd_scratch) {
         if (cudaMalloc(&r->rd_scratch, 16) != cudaSuccess) {
@@ -296,35 +346,39 @@ extern "C" int pgb_render(pgb_run* r, int plot, int32_t width, int32_t height, i
     unsigned char* img = (unsigned char*)r->rd_img;
     PGB_CK(r, cudaMemsetAsync(r->rd_scratch, 0, 16, r->stream));
     if (plot <= PGB_PLOT_ION_VX_VY) {
-        unsigned char* layer = img + bytes;
-        PGB_CK(r, cudaMemsetAsync(layer, 0, (size_t)npx, r->stream));
+        unsigned int* const layers = (unsigned int*)(img + img_bytes);
+        PGB_CK(r, cudaMemsetAsync(layers, 0, (size_t)(8 * words), r->stream));
         PointArgs a;
         a.ds = r->ds; a.nx = r->nx; a.ny = r->ny; a.ps = r->ps; a.width = width; a.height = height;
-        a.max_points = max_points; a.seed = seed; a.layer = layer;
+        a.max_points = max_points; a.seed = seed;
+        a.words = (int)words;
         a.vmax = (const unsigned int*)r->rd_scratch;
         a.vmax_out = (unsigned int*)r->rd_scratch;
-        const int blocks = r->sms * 8;
+        const size_t most = 200 * 1024;
+        a.shared = 4 * words <= (long long)most;
+        const size_t smem = a.shared ? (size_t)(4 * words) : 0;
+        PGB_CK(r, cudaFuncSetAttribute(k_rd_points, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+        const int blocks = r->sms * (smem > 100 * 1024 ? 1 : 2);
         if (plot == PGB_PLOT_PARTICLE_XY) {
             a.phase = 0;
             for (int s = 0; s < 2; ++s) {   /* electrons, then ions on top (graphics.cpp:560-606) */
                 a.s = s; a.xv = r->sp[s].xv; a.id = r->sp[s].id;
-                a.mark = (unsigned char)(s + 1);
-                k_rd_points<<<blocks, 256, 0, r->stream>>>(a);
+                a.layer = layers + s * words;
+                k_rd_points<<<blocks, RD_THREADS, smem, r->stream>>>(a);
                 r->launches++;
             }
         } else {
             const int s = plot == PGB_PLOT_ELECTRON_VX_VY ? 0 : 1;   /* lime / hot pink, graphics.cpp:692, 696 */
             a.phase = 1; a.s = s; a.xv = r->sp[s].xv; a.id = r->sp[s].id;
-            a.mark = (unsigned char)(s + 1);
-            k_rd_vmax<<<blocks, 256, 0, r->stream>>>(a);
-            k_rd_points<<<blocks, 256, 0, r->stream>>>(a);
+            a.layer = layers + s * words;
+            k_rd_vmax<<<r->sms * 2, RD_THREADS, 0, r->stream>>>(a);
+            k_rd_points<<<blocks, RD_THREADS, smem, r->stream>>>(a);
             r->launches += 2;
         }
-        const int rb = (int)std::min<long long>((npx + 255) / 256, (long long)r->sms * 16);
-        k_rd_resolve<<<rb, 256, 0, r->stream>>>(layer, npx, kLime, kHotPink, img);
+        const int rb = (int)std::min<long long>((npx + 1023) / 1024, (long long)r->sms * 16);
+        k_rd_resolve<<<rb, 256, 0, r->stream>>>(layers, layers + words, npx, kLime, kHotPink, img);
         r->launches++;
     } else {
-        const int nodes = r->nx * r->ny;
         const double* src = nullptr;
         double div = 1.0;
         int grid_start = 0;
@@ -342,10 +396,13 @@ extern "C" int pgb_render(pgb_run* r, int plot, int32_t width, int32_t height, i
         }
         if (averaged) div = (double)r->gr.g.no_graph_steps;
         unsigned long long* key = (unsigned long long*)r->rd_scratch;
-        k_rd_fmax<<<std::min((nodes + 255) / 256, r->sms * 4), 256, 0, r->stream>>>(src, div, nodes, key);
+        float* const z = (float*)(img + img_bytes);
+        const int nb = (int)std::min<long long>((nodes + 255) / 256, (long long)r->sms * 8);
+        k_rd_fmax<<<std::min(nb, r->sms * 4), 256, 0, r->stream>>>(src, div, (int)nodes, key);
+        k_rd_nodes<<<nb, 256, 0, r->stream>>>(src, div, (int)nodes, key, z);
         const int pb = (int)std::min<long long>((npx + 255) / 256, (long long)r->sms * 16);
-        k_rd_field<<<pb, 256, 0, r->stream>>>(src, div, r->nx, grid_start, key, width, height, img);
-        r->launches += 2;
+        k_rd_field<<<pb, 256, 0, r->stream>>>(z, r->nx, grid_start, width, height, img);
+        r->launches += 3;
     }
     PGB_CK(r, cudaGetLastError());
     PGB_CK(r, cudaMemcpyAsync(rgb, img, (size_t)bytes, cudaMemcpyDeviceToHost, r->stream));
