@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(512) k_steady(WallArgs a, int* ion_by_rank, in
  * A probability is at most 2^40, so with 2048 ions a tile neither 32-bit
  * sum can reach 2^32.                                                     */
 #define CX_TILE PGB_CX_TILE
-#define CX_AHEAD 8
+#define CX_AHEAD 32
 #define CX_GROUPS 8
 #define CX_ONE (1ll << 40)
 static_assert((long long)CX_TILE << 20 <= (1ll << 31), "32-bit halves of the tile sums must not overflow");
@@ -728,10 +728,13 @@ __global__ void __launch_bounds__(256) k_cx_tiles(CxArgs a) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_cx_walk(CxArgs a) {
+#define CX_WALK_WARPS 4
+__global__ void __launch_bounds__(32 * CX_WALK_WARPS) k_cx_walk(CxArgs a) {
     pgb_pdl_entry();
+    __shared__ unsigned short s_ions[CX_WALK_WARPS][CX_TILE];
     const int lane = threadIdx.x & 31;
-    const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int col = blockIdx.x * CX_WALK_WARPS + (threadIdx.x >> 5);
+    unsigned short* const ions = s_ions[threadIdx.x >> 5];
     long long i0, n;
     cx_range(a, i0, n);
     /* the tail pass starts where this one ends (k_cx_tiles has read n) */
@@ -786,44 +789,59 @@ __global__ void __launch_bounds__(256) k_cx_walk(CxArgs a) {
             tt = t0 + 32 * u + first;
         }
         if (tt < 0) continue;
-        /* scan tile tt element by element, then continue after it.
-         * The ions of CX_AHEAD batches are in flight together: one batch at
-         * a time, a tile was a chain of 64 loads, 25-50 us for a whole step
-         * in which any column crosses (argon, 257^2, 4 Mi ions: charge
-         * exchange 119 us a step), while the GPU held one warp per column */
+        /* Scan tile tt ion by ion, then continue after it.  First the tile's
+         * ions of this column, in slot order (a sorted tile holds some 64 of
+         * 2048), found from their x alone with 32 loads in flight per lane;
+         * then their probabilities, 32 at a time.  Evaluating where they were
+         * found, one or two lanes of a warp at a time, took 41 us a tile.   */
+        const long long base = i0 + (long long)tt * CX_TILE;
+        int m = 0;
         for (int b = 0; b < CX_TILE; b += 32 * CX_AHEAD) {
-            float4 p[CX_AHEAD];
-            float vz[CX_AHEAD];
+            float x[CX_AHEAD];
 #pragma unroll
             for (int q = 0; q < CX_AHEAD; ++q) {
-                const long long i = i0 + (long long)tt * CX_TILE + b + 32 * q + lane;
-                p[q] = make_float4(pos_dead(), 0.f, 0.f, 0.f);
-                vz[q] = 0.f;
-                if (i < n) {
-                    p[q] = a.i.xv[i];
-                    vz[q] = a.i.vz[i];
-                }
+                const long long i = base + b + 32 * q + lane;
+                x[q] = i < n ? a.i.xv[i].x : pos_dead();
             }
 #pragma unroll
             for (int q = 0; q < CX_AHEAD; ++q) {
-                int c = -1;
-                long long pf = 0;
                 /* a dead or NaN position's cell index is no column */
-                if (pcell(p[q].x, a.ps) == col) pf = cx_prob_fixed(a, p[q], vz[q], c);
-                unsigned match = __ballot_sync(0xffffffffu, c == col && pf > 0);
-                while (match) {
-                    int l = __ffs(match) - 1;
-                    match &= match - 1;
-                    long long v = __shfl_sync(0xffffffffu, pf, l);
-                    acc += v;
-                    if (acc > CX_ONE) {
-                        acc = 0;
-                        if (lane == l) cx_exchange(a, i0 + (long long)tt * CX_TILE + b + 32 * q + lane);
-                        fired++;
-                    }
-                }
+                const bool hit = pcell(x[q], a.ps) == col;
+                const unsigned mask = __ballot_sync(0xffffffffu, hit);
+                if (hit) ions[m + __popc(mask & ((1u << lane) - 1u))] = (unsigned short)(b + 32 * q + lane);
+                m += __popc(mask);
             }
         }
+        __syncwarp();
+        for (int j = 0; j < m; j += 32) {
+            long long i = 0, v = 0;
+            if (j + lane < m) {
+                int c;
+                i = base + ions[j + lane];
+                v = cx_prob_fixed(a, a.i.xv[i], a.i.vz[i], c);
+                if (v < 0) v = 0;
+            }
+            /* the first lane that takes the column above 1 fires, the column
+             * restarts from 0 after it                                     */
+            for (;;) {
+                long long ps = v;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const long long y = __shfl_up_sync(0xffffffffu, ps, d);
+                    if (lane >= d) ps += y;
+                }
+                const unsigned cross = __ballot_sync(0xffffffffu, v > 0 && acc + ps > CX_ONE);
+                if (!cross) {
+                    acc += __shfl_sync(0xffffffffu, ps, 31);
+                    break;
+                }
+                const int f = __ffs(cross) - 1;
+                if (lane == f) cx_exchange(a, i);
+                if (lane <= f) v = 0;
+                acc = 0;
+                fired++;
+            }
+        }
+        __syncwarp();
         next = tt + 1;   /* resume with the tiles after tt */
     }
     __syncwarp();
@@ -967,8 +985,7 @@ int pgb_launch_cx(pgb_run* r, int tail, int leave_sms) {
     const int sms = r->sms - leave_sms > 8 ? r->sms - leave_sms : 8;
     PGB_CK(r, pgb_launch_pdl(k_cx_tiles, dim3(sms * 4), dim3(256), 2 * sizeof(unsigned int) * r->nx, r->stream, a));
     r->launches++;
-    int warps = 8;
-    PGB_CK(r, pgb_launch_pdl(k_cx_walk, dim3((r->nx + warps - 1) / warps), dim3(warps * 32), 0, r->stream, a));
+    PGB_CK(r, pgb_launch_pdl(k_cx_walk, dim3((r->nx + CX_WALK_WARPS - 1) / CX_WALK_WARPS), dim3(32 * CX_WALK_WARPS), 0, r->stream, a));
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;
