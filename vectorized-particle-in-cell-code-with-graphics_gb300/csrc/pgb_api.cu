@@ -374,7 +374,6 @@ extern "C" int pgb_create(const pgb_params* p, pgb_run** out) {
     ok = ok && cudaMalloc(&r->inject_flag, sizeof(int) * (p->number_to_inject + 1)) == cudaSuccess;
     ok = ok && cudaMalloc(&r->phi_tab, sizeof(double) * r->phi_tab_cap) == cudaSuccess;
     ok = ok && cudaMallocHost(&r->phi_host, sizeof(double) * r->phi_tab_cap) == cudaSuccess;
-    ok = ok && cudaMallocHost(&r->t_host, sizeof(long long) * 2) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&r->phi_ev, cudaEventDisableTiming) == cudaSuccess;
     if (ok) r->phi_ev_ok = true;
     int ng = 0, nn = r->nx;
@@ -437,7 +436,6 @@ extern "C" int pgb_destroy(pgb_run* r) {
     drop_graphs(r);
     cudaFree(r->phi_tab);
     if (r->phi_host) cudaFreeHost(r->phi_host);
-    if (r->t_host) cudaFreeHost(r->t_host);
     if (r->phi_ev_ok) cudaEventDestroy(r->phi_ev);
     cudaFree(r->inject_flag);
     free_species(r->sp[0]);
@@ -516,18 +514,13 @@ extern "C" int pgb_load_species(pgb_run* r, int s, const double* aos6, int64_t n
                  cudaEventRecord(ev, r->copy_stream) == cudaSuccess &&
                  cudaStreamWaitEvent(r->stream, ev, 0) == cudaSuccess && pgb_launch_load(r, s, r->d_stage, c, e) == 0;
         }
-        if (!ok || cudaStreamSynchronize(r->stream) != cudaSuccess)
-            return fail(r, PGB_ERR_CUDA, "pgb_load_species: upload failed");
+        if (!ok) return fail(r, PGB_ERR_CUDA, "pgb_load_species: upload failed");
     }
     r->hs->n[s] = n;
     r->hs->dead[s] = 0;
     r->hs->next_id[s] = (unsigned)n;
-    PGB_CK(r, cudaMemcpyAsync(&r->ds->n[s], &r->hs->n[s], sizeof(long long), cudaMemcpyHostToDevice, r->stream));
-    PGB_CK(r, cudaMemcpyAsync(&r->ds->dead[s], &r->hs->dead[s], sizeof(long long), cudaMemcpyHostToDevice, r->stream));
-    PGB_CK(r, cudaMemcpyAsync(&r->ds->next_id[s], &r->hs->next_id[s], sizeof(unsigned), cudaMemcpyHostToDevice, r->stream));
-    PGB_CK(r, cudaMemsetAsync(&r->ds->n_pieces[s], 0, sizeof(int), r->stream));
-    PGB_CK(r, cudaMemsetAsync(&r->ds->sorted_tiles[s], 0, sizeof(long long), r->stream));
-    PGB_CK(r, cudaStreamSynchronize(r->stream));
+    if (pgb_launch_load_commit(r, s, n)) return PGB_ERR_CUDA;
+    if (cudaStreamSynchronize(r->stream) != cudaSuccess) return fail(r, PGB_ERR_CUDA, "pgb_load_species: upload failed");
     return 0;
 }
 
@@ -583,13 +576,13 @@ extern "C" int pgb_dump_species(pgb_run* r, int s, double* aos6, int64_t cap, in
      * chunk c (copy stream) overlaps the packing of chunk c+1 (run stream) */
     const long long n = r->hs->n[s];
     const int ntiles = (int)((n + PGB_TILE - 1) / PGB_TILE);
-    std::vector<int> toff((size_t)ntiles);
-    if (pgb_launch_dump_offsets(r, s) ||
-        cudaMemcpyAsync(toff.data(), r->aux_j, sizeof(int) * (size_t)ntiles, cudaMemcpyDeviceToHost, r->stream) != cudaSuccess ||
-        cudaStreamSynchronize(r->stream) != cudaSuccess)
-        return fail(r, PGB_ERR_CUDA, "pgb_dump_species: offsets failed");
     const int per = PGB_COPY_CHUNK / PGB_TILE;
-    bool ok = true;
+    std::vector<int> toff((size_t)ntiles);   /* read where a later chunk starts */
+    bool ok = pgb_launch_dump_offsets(r, s) == 0;
+    if (ok && ntiles > per)
+        ok = cudaMemcpyAsync(toff.data(), r->aux_j, sizeof(int) * (size_t)ntiles, cudaMemcpyDeviceToHost, r->stream) == cudaSuccess &&
+             cudaStreamSynchronize(r->stream) == cudaSuccess;
+    if (!ok) return fail(r, PGB_ERR_CUDA, "pgb_dump_species: offsets failed");
     for (int t0 = 0, k = 0; ok && t0 < ntiles; t0 += per, ++k) {
         const int t1 = std::min(ntiles, t0 + per);
         const long long a = std::min<long long>(toff[t0], m), b = std::min<long long>(t1 < ntiles ? toff[t1] : live, m);
@@ -655,16 +648,15 @@ static int need_particles(pgb_run* r) {
  * reference does                                                         */
 static int set_device_step(pgb_run* r, int64_t t0, int n) {
     if (n > r->phi_tab_cap) return fail(r, PGB_ERR_ARG, "step table too small");
-    /* the pinned staging is reused once its previous upload has left */
-    PGB_CK(r, cudaEventSynchronize(r->phi_ev));
-    for (int k = 0; k < n; ++k) r->phi_host[k] = r->p.phi_right * cos(r->p.phi_period * (double)(t0 + k));
-    r->t_host[0] = (long long)t0;
-    PGB_CK(r, cudaMemcpyAsync(r->phi_tab, r->phi_host, sizeof(double) * n, cudaMemcpyHostToDevice, r->stream));
-    PGB_CK(r, cudaMemcpyAsync(&r->ds->t, r->t_host, sizeof(long long), cudaMemcpyHostToDevice, r->stream));
-    PGB_CK(r, cudaMemcpyAsync(&r->ds->t_base, r->t_host, sizeof(long long), cudaMemcpyHostToDevice, r->stream));
-    PGB_CK(r, cudaMemcpyAsync(&r->ds->tf, r->t_host, sizeof(long long), cudaMemcpyHostToDevice, r->stream));
-    PGB_CK(r, cudaEventRecord(r->phi_ev, r->stream));
-    return 0;
+    const double phi0 = r->p.phi_right * cos(r->p.phi_period * (double)t0);
+    if (n > 1) {
+        /* the pinned staging is reused once its previous upload has left */
+        PGB_CK(r, cudaEventSynchronize(r->phi_ev));
+        for (int k = 0; k < n; ++k) r->phi_host[k] = r->p.phi_right * cos(r->p.phi_period * (double)(t0 + k));
+        PGB_CK(r, cudaMemcpyAsync(r->phi_tab, r->phi_host, sizeof(double) * n, cudaMemcpyHostToDevice, r->stream));
+        PGB_CK(r, cudaEventRecord(r->phi_ev, r->stream));
+    }
+    return pgb_launch_set_step(r, (long long)t0, phi0, n <= 1);
 }
 
 /* ---------------------------------------------------- phase entry points */

@@ -180,9 +180,8 @@ struct pgb_run {
     double* neut64[2] = {nullptr, nullptr};
     double* prob_cx = nullptr;             /* per-column CX accumulator       */
     double* phi_tab = nullptr;             /* right-wall potential per step   */
-    double* phi_host = nullptr;            /* pinned: the table and the step number on their way */
-    long long* t_host = nullptr;
-    cudaEvent_t phi_ev;                    /* recorded after their upload     */
+    double* phi_host = nullptr;            /* pinned: the table on its way    */
+    cudaEvent_t phi_ev;                    /* recorded after its upload       */
     bool phi_ev_ok = false;
     long long phi_tab_cap = 0;
     /* CUDA graphs of one step, keyed by (ion step, buffer orientation e, i) */
@@ -341,6 +340,8 @@ int pgb_launch_cx(pgb_run* r, int tail, int leave_sms);
  * after entering the products of the species in commit                   */
 int pgb_launch_walls(pgb_run* r, int which, bool advance = false, int commit = 0);
 int pgb_launch_load(pgb_run* r, int s, const double* d_aos, long long i0, long long i1);
+int pgb_launch_load_commit(pgb_run* r, int s, long long n);
+int pgb_launch_set_step(pgb_run* r, long long t, double phi, bool one);
 int pgb_launch_dump_offsets(pgb_run* r, int s);
 int pgb_launch_dump(pgb_run* r, int s, double* d_out, unsigned int* d_ids, long long cap, int t0, int t1);
 int pgb_mg_setup(pgb_run* r);

@@ -25,6 +25,7 @@
 #include "pgb_internal.h"
 #include "pgb_physics.cuh"
 #include "pgb_deposit.cuh"
+#include "pgb_fp64.cuh"
 
 /* ------------------------------------------------------------ device state */
 struct PushArgs {
@@ -988,44 +989,73 @@ __global__ void k_load(Species S, const double* aos, long long i0, long long i1,
 /* tiles [t0, t1) of the live-slot order */
 /* out (6 doubles per particle) and ids (the particle's id) are each
  * written when not null                                                  */
-__global__ void __launch_bounds__(PGB_PUSH_THREADS) k_dump(Species S, DevState* ds, int s, const int* toff, double dx,
-                                                           double dy, int ps, double* out, unsigned int* ids,
-                                                           long long cap, int t0, int t1) {
+__global__ void __launch_bounds__(PGB_PUSH_THREADS) k_dump(Species S, DevState* ds, int s, const int* toff, double ux,
+                                                           double uy, double* out, unsigned int* ids, long long cap,
+                                                           int t0, int t1) {
     pgb_pdl_entry();
     const long long n = ds->n[s];
     const int ntiles = min(t1, (int)((n + PGB_TILE - 1) / PGB_TILE));
-    __shared__ int s_off[PGB_ITEMS][PGB_PUSH_THREADS / 32];
+    __shared__ int s_off[PGB_ITEMS * (PGB_PUSH_THREADS / 32)];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int tile = t0 + blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        float4 p[PGB_ITEMS];
         bool f[PGB_ITEMS];
         unsigned m[PGB_ITEMS];
+#pragma unroll
         for (int k = 0; k < PGB_ITEMS; ++k) {
             long long i = (long long)tile * PGB_TILE + k * PGB_PUSH_THREADS + threadIdx.x;
-            f[k] = (i < n) && !is_dead(S.xv[i].x);
+            p[k] = i < n ? S.xv[i] : make_float4(pos_dead(), 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < PGB_ITEMS; ++k) {
+            f[k] = !is_dead(p[k].x);
             m[k] = __ballot_sync(0xffffffffu, f[k]);
-            if (lane == 0) s_off[k][warp] = __popc(m[k]);
+            if (lane == 0) s_off[k * (PGB_PUSH_THREADS / 32) + warp] = __popc(m[k]);
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            int acc = toff[tile];
-            for (int k = 0; k < PGB_ITEMS; ++k)
-                for (int w = 0; w < PGB_PUSH_THREADS / 32; ++w) { int c = s_off[k][w]; s_off[k][w] = acc; acc += c; }
+        if (warp == 0) {   /* 32 (item, warp) counts, a lane each */
+            const int c = s_off[lane];
+            int x = c;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += y;
+            }
+            s_off[lane] = toff[tile] + x - c;
         }
         __syncthreads();
+#pragma unroll
         for (int k = 0; k < PGB_ITEMS; ++k)
             if (f[k]) {
                 long long i = (long long)tile * PGB_TILE + k * PGB_PUSH_THREADS + threadIdx.x;
-                long long pos = s_off[k][warp] + __popc(m[k] & ((1u << lane) - 1u));
+                long long pos = s_off[k * (PGB_PUSH_THREADS / 32) + warp] + __popc(m[k] & ((1u << lane) - 1u));
                 if (pos < cap && out) {
-                    float4 p = S.xv[i];
-                    double* o = out + 6 * pos;
-                    o[0] = pos_m(p.x, ps, dx); o[1] = pos_m(p.y, ps, dy);
-                    o[2] = p.z; o[3] = p.w; o[4] = S.vz[i]; o[5] = S.w[i];
+                    double2* const o = reinterpret_cast<double2*>(out + 6 * pos);   /* 48 B a record, 16-byte aligned */
+                    o[0] = make_double2(pos_m(p[k].x, ux), pos_m(p[k].y, uy));
+                    o[1] = make_double2(f32_to_f64(p[k].z), f32_to_f64(p[k].w));
+                    o[2] = make_double2(f32_to_f64(S.vz[i]), f32_to_f64(S.w[i]));
                 }
                 if (pos < cap && ids) ids[pos] = S.id[i];
             }
         __syncthreads();
     }
+}
+
+/* after a load: the species' counts; its slots are in no bin order */
+__global__ void k_load_commit(DevState* ds, int s, long long n) {
+    pgb_pdl_entry();
+    ds->n[s] = n;
+    ds->dead[s] = 0;
+    ds->next_id[s] = (unsigned int)n;
+    ds->n_pieces[s] = 0;
+    ds->sorted_tiles[s] = 0;
+}
+/* the step counters, and the right-wall potential of the first step where
+ * there is only one (else the table is copied)                           */
+__global__ void k_set_step(DevState* ds, long long t, double* phi_tab, double phi, int one) {
+    pgb_pdl_entry();
+    ds->t = ds->t_base = ds->tf = t;
+    if (one) phi_tab[0] = phi;
 }
 
 /* ====================================================== host launchers */
@@ -1236,7 +1266,6 @@ int pgb_launch_compact(pgb_run* r, int s) {
     Species& S = r->sp[s];
     int* tc = r->tile_cnt[LIST_SPARE];
     int* toff = r->aux_j;
-    PGB_CK(r, cudaMemsetAsync(tc, 0, sizeof(int) * r->ntiles_cap, r->stream));
     PGB_CK(r, pgb_launch_pdl(k_alive_count, dim3(grid_for(r, 8)), dim3(PGB_PUSH_THREADS), 0, r->stream, S.xv, r->ds, s, tc));
     r->launches++;
     PGB_CK(r, pgb_launch_pdl(k_scan_small, dim3(1), dim3(1024), 0, r->stream, tc, toff, &r->ds->n[s], 0, &r->ds->list_n[LIST_SPARE]));
@@ -1261,10 +1290,20 @@ int pgb_launch_load(pgb_run* r, int s, const double* d_aos, long long i0, long l
     return 0;
 }
 
+int pgb_launch_load_commit(pgb_run* r, int s, long long n) {
+    PGB_CK(r, pgb_launch_pdl(k_load_commit, dim3(1), dim3(1), 0, r->stream, r->ds, s, n));
+    r->launches++;
+    return 0;
+}
+int pgb_launch_set_step(pgb_run* r, long long t, double phi, bool one) {
+    PGB_CK(r, pgb_launch_pdl(k_set_step, dim3(1), dim3(1), 0, r->stream, r->ds, t, r->phi_tab, phi, one ? 1 : 0));
+    r->launches++;
+    return 0;
+}
+
 /* live-slot offsets per tile (into r->aux_j) for pgb_launch_dump */
 int pgb_launch_dump_offsets(pgb_run* r, int s) {
     int* tc = r->tile_cnt[LIST_SPARE];
-    PGB_CK(r, cudaMemsetAsync(tc, 0, sizeof(int) * r->ntiles_cap, r->stream));
     PGB_CK(r, pgb_launch_pdl(k_alive_count, dim3(grid_for(r, 8)), dim3(PGB_PUSH_THREADS), 0, r->stream, r->sp[s].xv, r->ds, s, tc));
     r->launches++;
     PGB_CK(r, pgb_launch_pdl(k_scan_small, dim3(1), dim3(1024), 0, r->stream, tc, r->aux_j, &r->ds->n[s], 0, &r->ds->list_n[LIST_SPARE]));
@@ -1274,8 +1313,8 @@ int pgb_launch_dump_offsets(pgb_run* r, int s) {
 }
 
 int pgb_launch_dump(pgb_run* r, int s, double* d_out, unsigned int* d_ids, long long cap, int t0, int t1) {
-    PGB_CK(r, pgb_launch_pdl(k_dump, dim3(grid_for(r, 8)), dim3(PGB_PUSH_THREADS), 0, r->stream, r->sp[s], r->ds, s, r->aux_j, r->dx, r->dy, r->ps, d_out,
-                             d_ids, cap, t0, t1));
+    PGB_CK(r, pgb_launch_pdl(k_dump, dim3(grid_for(r, 8)), dim3(PGB_PUSH_THREADS), 0, r->stream, r->sp[s], r->ds, s, (const int*)r->aux_j, ldexp(r->dx, -r->ps),
+                             ldexp(r->dy, -r->ps), d_out, d_ids, cap, t0, t1));
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;

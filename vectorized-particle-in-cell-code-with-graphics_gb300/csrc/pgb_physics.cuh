@@ -12,6 +12,7 @@
 #include <stdint.h>
 #include "pgb_internal.h"
 #include "pgb_rng.h"
+#include "pgb_fp64.cuh"
 
 #define PGB_PI 3.141592654
 #define PGB_CHARGE 1.602177e-19
@@ -84,6 +85,11 @@ __device__ __forceinline__ double pos_cells(float lane, int ps) {
     return x == PGB_POS_NAN ? __longlong_as_double(0x7ff8000000000000ll) : ldexp((double)x, -ps);
 }
 __device__ __forceinline__ double pos_m(float lane, int ps, double d) { return pos_cells(lane, ps) * d; }
+/* the same in metres with u = d 2^-ps: x u rounds once, as (x 2^-ps) d does */
+__device__ __forceinline__ double pos_m(float lane, double u) {
+    const int x = __float_as_int(lane);
+    return x == PGB_POS_NAN ? __longlong_as_double(0x7ff8000000000000ll) : i64_to_f64(x) * u;
+}
 /* FP32 cells, for plots and histograms                                   */
 __device__ __forceinline__ float pos_cellsf(float lane, int ps) {
     const int x = __float_as_int(lane);
