@@ -290,6 +290,40 @@ __device__ __forceinline__ void push_tile(const PushArgs& a, const PushConsts& p
     if (!ABSORB) tile_masks(f, tile, (unsigned*)a.tl_out, a.tc_out, s_cnt, it);
 }
 
+/* The window's non-zero sums to the grid, zeroed for the next piece.  A warp
+ * per row; a lane takes columns lane and lane + 32, whose places in the
+ * grid and whether they lie inside it are the same in every row.  (With
+ * addresses and four bounds formed per node, the flush was 17% of the
+ * push's instructions.)                                                  */
+static_assert(PGB_WIN > 32 && PGB_WIN <= 64, "two columns a lane");
+__device__ __forceinline__ void flush_window(unsigned long long* qacc, unsigned int* win, int ox, int oy, int nx, int ny) {
+    const int lane = threadIdx.x & 31;
+    const bool in0 = (unsigned)(ox + lane) < (unsigned)nx;
+    const bool two = lane < PGB_WIN - 32, in1 = two && (unsigned)(ox + lane + 32) < (unsigned)nx;
+    int ry = threadIdx.x >> 5;
+    unsigned int* w = win + ry * PGB_WIN + lane;
+    unsigned long long* q = qacc + (long long)(oy + ry) * nx + ox + lane;   /* used inside the grid only */
+    const long long dq = (long long)(PGB_PUSH_THREADS / 32) * nx;
+#pragma unroll
+    for (int k = 0; k < (PGB_WIN + PGB_PUSH_THREADS / 32 - 1) / (PGB_PUSH_THREADS / 32); ++k) {
+        if (ry < PGB_WIN) {
+            const unsigned int v0 = w[0], v1 = two ? w[32] : 0u;
+            const bool in = (unsigned)(oy + ry) < (unsigned)ny;
+            if (v0) {
+                w[0] = 0u;
+                if (in && in0) atomicAdd(q, (unsigned long long)v0);
+            }
+            if (v1) {
+                w[32] = 0u;
+                if (in && in1) atomicAdd(q + 32, (unsigned long long)v1);
+            }
+        }
+        ry += PGB_PUSH_THREADS / 32;
+        w += PGB_PUSH_THREADS / 32 * PGB_WIN;
+        q += dq;
+    }
+}
+
 /* Work items: the bin pieces of the last sort (tiles of one bin, deposited
  * through a shared window), then every tile after the sorted region.     */
 template <bool DEP, bool ABSORB>
@@ -323,22 +357,7 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
                 push_tile<DEP, ABSORB>(a, pc, t, n, win, ox, oy, s_cnt, it, gone);
             if (win) {
                 __syncthreads();
-                /* a warp per window row, a lane per node: add the non-zero
-                 * sums to the grid and zero them for the next piece        */
-                const int lane = threadIdx.x & 31;
-                for (int ry = threadIdx.x >> 5; ry < PGB_WIN; ry += PGB_PUSH_THREADS / 32) {
-                    const int gy = oy + ry;
-                    unsigned long long* qrow = a.qacc + (long long)gy * pc.nx;
-                    for (int rx = lane; rx < PGB_WIN; rx += 32) {
-                        const unsigned int v = s_win[ry * PGB_WIN + rx];
-                        if (v) {
-                            s_win[ry * PGB_WIN + rx] = 0u;
-                            const int gx = ox + rx;
-                            if (gx >= 0 && gy >= 0 && gx < pc.nx && gy < pc.ny)
-                                atomicAdd(qrow + gx, (unsigned long long)v);
-                        }
-                    }
-                }
+                flush_window(a.qacc, s_win, ox, oy, pc.nx, pc.ny);
                 __syncthreads();
             }
         } else {
