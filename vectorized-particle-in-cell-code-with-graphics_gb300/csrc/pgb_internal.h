@@ -68,6 +68,8 @@ struct DevState {
                                 step's collisions                                      */
     unsigned int ticket;     /* blocks of a wall kernel that are done            */
     unsigned int ticket_f;   /* the same of k_field                              */
+    int work[2];             /* items of the push taken, per species; 0 between launches */
+    int work_done[2];        /* blocks of the push that are done                 */
     long long n_cx;          /* ion slots whose charge exchange was tested before this
                                 step's appends (the rest are tested after them)       */
 };

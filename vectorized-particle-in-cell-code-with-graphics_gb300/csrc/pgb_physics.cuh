@@ -74,9 +74,10 @@ __device__ __forceinline__ bool pos_lt0(float lane) {
     return x < 0 && x != PGB_POS_NAN;
 }
 /* x/DX - (int)(x/DX) for x >= 0, exact: the ps fraction bits placed in the
- * mantissa of 1.0 (ps <= 23), minus 1                                     */
+ * mantissa of 1.0 (ps <= 23; the cell's bits are shifted out above it),
+ * minus 1                                                                 */
 __device__ __forceinline__ float pfrac(float lane, int ps) {
-    const unsigned m = ((unsigned)__float_as_int(lane) & ((1u << ps) - 1u)) << (23 - ps);
+    const unsigned m = ((unsigned)__float_as_int(lane) << (23 - ps)) & 0x7fffffu;
     return __int_as_float(0x3f800000 | (int)m) - 1.0f;
 }
 /* the position in cells (exact in FP64) and in metres                    */

@@ -383,7 +383,7 @@ int pgb_launch_sort(pgb_run* r, int s) {
     a.nbins = a.nbx * a.nby;
     a.counts = r->sort_counts; a.offs = r->sort_offs; a.key_total = r->sort_key_total;
     a.key_start = r->sort_key_start; a.pieces = r->pieces[s];
-    a.want_pieces = 4 * r->sms;
+    a.want_pieces = 2 * r->sms;
     const int nk = a.nbins + 1;
     PGB_CK(r, pgb_launch_pdl(k_sort_count, dim3(r->sms * 4), dim3(512), sizeof(int) * nk, r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_sort_scan_keys, dim3((nk + 31) / 32), dim3(1024), 0, r->stream, a));
