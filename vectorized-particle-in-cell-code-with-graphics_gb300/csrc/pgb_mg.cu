@@ -24,9 +24,9 @@
  *   n <= 17 (FP64), 33 (FP32)   one CTA, every level in shared memory
  *   up to n = 129   a cluster of 16 CTAs in the same launch, a band of rows
  *                   per CTA with the halo that makes one exchange (through
- *                   L2, a cluster barrier of 380 clocks) enough for
- *                   smoothing, residual and restriction, and one for
- *                   correction and smoothing
+ *                   the CTAs' shared memory, a cluster barrier of 400
+ *                   clocks) enough for smoothing, residual and restriction,
+ *                   and one for correction and smoothing
  *   n >= 257        two launches per level and V-cycle (the same two tile
  *                   functions on 16 x 32 tiles)
  */
@@ -259,9 +259,9 @@ __device__ __forceinline__ void sm_walls(int t) {
     if (t >= 0 && t < n) u[t] = u[(n - 1) * n + t] = u[t * n] = u[t * n + n - 1] = (T)0;
     if constexpr (L > 0) sm_walls<T, L - 1, TOP>(t - n);
 }
-/* F of level L (and G) from a global right-hand side with the same nodes */
-template <class T, int L>
-__device__ __forceinline__ void sm_load_f(const T* gf, const MgConst<T>& mc, bool red) {
+/* F of level L (and G) from get(i, j) of its interior */
+template <class T, int L, class Get>
+__device__ __forceinline__ void sm_load_f(Get get, const MgConst<T>& mc, bool red) {
     using A = Arr<T, L, true>;
     constexpr int n = sm_n(L), W = 2 << L, trips = (W * W + Cfg<T>::THREADS - 1) / Cfg<T>::THREADS;
     const T h2 = mc.h2[L];
@@ -269,7 +269,7 @@ __device__ __forceinline__ void sm_load_f(const T* gf, const MgConst<T>& mc, boo
 #pragma unroll
     for (int q = 0; q < trips; ++q) {
         const int t = threadIdx.x + q * Cfg<T>::THREADS, i = t >> (L + 1), j = t & (W - 1);
-        v[q] = (i > 0 && j > 0 && i < W) ? __ldcg(gf + i * n + j) : (T)0;
+        v[q] = (i > 0 && j > 0 && i < W) ? get(i, j) : (T)0;
     }
     sm_walls<T, L, true>(threadIdx.x);
     if constexpr (L > 0) sm_walls<T, L - 1, false>((int)threadIdx.x - Cfg<T>::THREADS / 2);
@@ -336,22 +336,20 @@ struct SmF<T, 0> {
         if (threadIdx.x < Team<0>::size) SmV<T, 0, true, FROM_U>::run(mc);
     }
 };
-/* full multigrid at level L, right-hand side f, into u (one CTA) */
+/* full multigrid at level L, right-hand side f (one CTA) */
 template <class T, int L>
-__device__ __forceinline__ void sm_fmg(const T* f, T* u, const MgConst<T>& mc) {
-    sm_load_f<T, L>(f, mc, false);
+__device__ __forceinline__ void sm_fmg(const T* f, const MgConst<T>& mc) {
+    sm_load_f<T, L>([f](int i, int j) { return __ldcg(f + i * sm_n(L) + j); }, mc, false);
     SmF<T, L>::restrict_all(mc);
     SmF<T, L>::solve(mc);
     __syncthreads();
-    sm_store_u<T, L>(u);
 }
-/* one V-cycle from 0 at level L, right-hand side f, into u (one CTA) */
+/* one V-cycle from 0 at level L, right-hand side f (one CTA) */
 template <class T, int L>
-__device__ __forceinline__ void sm_vcycle0(const T* f, T* u, const MgConst<T>& mc) {
-    sm_load_f<T, L>(f, mc, true);
+__device__ __forceinline__ void sm_vcycle0(const T* f, const MgConst<T>& mc) {
+    sm_load_f<T, L>([f](int i, int j) { return __ldcg(f + i * sm_n(L) + j); }, mc, true);
     if (threadIdx.x < Team<L>::size) SmV<T, L, true, FROM_ZERO>::run(mc);
     __syncthreads();
-    sm_store_u<T, L>(u);
 }
 
 /* ------------------------------------------------------------- tiles */
@@ -544,29 +542,49 @@ struct MgPtrs {
     MgConst<T> c;
 };
 
-/* every CTA's global writes before are seen by every CTA's reads after */
+/* every CTA's writes before are seen by every CTA's reads after */
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 __device__ __forceinline__ int cluster_rank() {
     unsigned r;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return (int)r;
 }
+/* *p as CTA `rank` of the cluster holds it in its shared memory */
+__device__ __forceinline__ unsigned remote_addr(const void* p, int rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ double remote(const double* p, int rank) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote_addr(p, rank)));
+    return v;
+}
+__device__ __forceinline__ float remote(const float* p, int rank) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote_addr(p, rank)));
+    return v;
+}
 
 /* The band of a CTA on level L: coarse rows ic0 = 1 + M rank ... and their
  * fine rows 2 ic0 - 1 ..., whole rows, with the halo that makes the
  * smoothing, the residual, the restriction and, later, the correction and
- * its smoothing local.  It stays in shared memory from the way down to the
- * way up; only the restricted residual, the coarse correction and the
- * result go through global memory (L2).                                  */
+ * its smoothing local.  Between the levels, and from one V-cycle to the
+ * next, a CTA reads the rows it needs from the shared memory of the CTAs
+ * that own them: a cluster barrier costs 400 clocks when only shared memory
+ * was written before it, 2000 when global stores were.                   */
 template <class T, int L>
 struct Band {
     static constexpr int n = sm_n(L), N = 1 << L, M = N / CL_CTAS;
     static constexpr int UR = 2 * M + 8;   /* u: rows 2 ic0 - 5 ...       */
     static constexpr int GR = 2 * M + 6;   /* g: rows 2 ic0 - 4 ...       */
     static constexpr int FR = 2 * M + 1;   /* f, residual: rows 2 ic0 - 1 ... */
-    static constexpr int WORDS = (UR + GR + 2 * FR) * n;
+    static constexpr int WORDS = (UR + GR + 2 * FR) * n + M * sm_n(L - 1);
     static constexpr int BASE = Sm<T>::WORDS + [] {
         if constexpr (L > Cfg<T>::TOP + 1) return Band<T, L - 1>::END;
         else return 0;
@@ -576,7 +594,32 @@ struct Band {
     static __device__ __forceinline__ T* g() { return u() + UR * n; }
     static __device__ __forceinline__ T* f() { return g() + GR * n; }
     static __device__ __forceinline__ T* res() { return f() + FR * n; }
+    static __device__ __forceinline__ T* rc() { return res() + FR * n; }   /* restricted residual: coarse rows ic0 ... */
+    /* u at fine row i (not a wall) from its owner */
+    static __device__ __forceinline__ T owner_u(int i, int j) {
+        const int o = (i - 1) / (2 * M);
+        return remote(u() + (i - 2 * M * o + 3) * n + j, o);
+    }
+    /* the restricted residual at coarse row i (interior) from its owner */
+    static __device__ __forceinline__ T owner_rc(int i, int j) {
+        const int o = (i - 1) / M;
+        return remote(rc() + (i - 1 - M * o) * sm_n(L - 1) + j, o);
+    }
 };
+/* u of level L at row i (any), column j: from the level's bands, or from the
+ * first CTA                                                              */
+template <class T, int L>
+__device__ __forceinline__ T cluster_u(int i, int j) {
+    if constexpr (L > Cfg<T>::TOP) return i > 0 && i < sm_n(L) - 1 ? Band<T, L>::owner_u(i, j) : (T)0;
+    else return remote(Arr<T, L, true>::u() + i * sm_n(L) + j, 0);
+}
+/* the sum of the two coarse values whose mean is the interpolation at black
+ * point (i, j) of level L (black_pair)                                   */
+template <class T, int L>
+__device__ __forceinline__ T coarse_pair(int i, int j) {
+    if (j & 1) return cluster_u<T, L - 1>(i >> 1, (j + 1) >> 1) + cluster_u<T, L - 1>(i >> 1, (j - 1) >> 1);
+    return cluster_u<T, L - 1>((i + 1) >> 1, j >> 1) + cluster_u<T, L - 1>((i - 1) >> 1, j >> 1);
+}
 /* one colour on `rows` band rows from row i0: a row has N slots */
 template <class T, int L>
 __device__ __forceinline__ void band_sweep(int color, int i0, int rows, int iu) {
@@ -594,23 +637,30 @@ __device__ __forceinline__ void band_sweep(int color, int i0, int rows, int iu) 
     }
     __syncthreads();
 }
-/* V-cycle of level L.  u, f: the level's arrays; uc: the coarser solution
- * (FROM_COARSE).                                                         */
-template <class T, int L, int START>
-__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* u, const T* f, const T* uc);
-template <class T, int L>
+template <class T, int L, int START, bool ABOVE>
+__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, const T* gf);
+/* one V-cycle from 0 at level L on the residual restricted from level L+1
+ * (ABOVE) or on r[L]                                                     */
+template <class T, int L, bool ABOVE>
 struct ClLower {
     static __device__ __forceinline__ void run(const MgPtrs<T>& p) {
         if constexpr (L > Cfg<T>::TOP) {
-            cl_vcycle<T, L, FROM_ZERO>(p, p.v[L], p.r[L], nullptr);
+            cl_vcycle<T, L, FROM_ZERO, ABOVE>(p, p.r[L]);
         } else {
-            if (cluster_rank() == 0) sm_vcycle0<T, L>(p.r[L], p.v[L], p.c);
+            if (cluster_rank() == 0) {
+                sm_load_f<T, L>([](int i, int j) { return Band<T, L + 1>::owner_rc(i, j); }, p.c, true);
+                if (threadIdx.x < Team<L>::size) SmV<T, L, true, FROM_ZERO>::run(p.c);
+                __syncthreads();
+            }
             cluster_sync();
         }
     }
 };
-template <class T, int L, int START>
-__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* gu, const T* gf, const T* uc) {
+/* V-cycle of level L.  ABOVE: the right-hand side is what level L+1
+ * restricted; else it is gf (global), read on the first of two V-cycles and
+ * kept for the second (FROM_U).  The result stays in the bands.          */
+template <class T, int L, int START, bool ABOVE>
+__device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, const T* gf) {
     using B = Band<T, L>;
     constexpr int n = B::n, N = B::N, M = B::M, nc = sm_n(L - 1), TH = Cfg<T>::THREADS;
     const int ic0 = 1 + M * cluster_rank(), iu = 2 * ic0 - 5;
@@ -619,40 +669,50 @@ __device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* gu, const T* gf
     T* const sg = B::g();
     T* const sf = B::f();
     T* const sr = B::res();
-    /* the walls, then the black points from their source (a correction: 0) */
-    for (int t = threadIdx.x; t < B::UR; t += TH) su[t * n] = su[t * n + n - 1] = (T)0;
+    if constexpr (START == FROM_U) {
+        /* the halo's black points from their owners; the others are here */
+        constexpr int halo = B::UR - 2 * M;
+#pragma unroll
+        for (int t = threadIdx.x; t < halo << L; t += TH) {
+            const int h = t >> L, a = h < 4 ? h : h + 2 * M, i = iu + a, j = 1 + (i & 1) + 2 * (t & (N - 1));
+            if (i > 0 && i < n - 1 && j < n - 1) su[a * n + j] = B::owner_u(i, j);
+        }
+    } else {
+        /* the walls, then the black points from their source (a correction: 0) */
+        for (int t = threadIdx.x; t < B::UR; t += TH) su[t * n] = su[t * n + n - 1] = (T)0;
 #pragma unroll 4
-    for (int t = threadIdx.x; t < B::UR << L; t += TH) {
-        const int a = t >> L, i = iu + a, c = 2 * (t & (N - 1)) + 1, j = c + (i & 1);
-        T v = (T)0;
-        if (START != FROM_ZERO && i > 0 && i < n - 1 && j < n - 1) {
-            if (START == FROM_U) v = __ldcg(gu + i * n + j);
-            else {
-                int k1, k0;
-                black_pair(i, j, nc, k1, k0);
-                v = down_pow2<1>(__ldcg(uc + k1) + __ldcg(uc + k0));
+        for (int t = threadIdx.x; t < B::UR << L; t += TH) {
+            const int a = t >> L, i = iu + a, c = 2 * (t & (N - 1)) + 1, j = c + (i & 1);
+            T v = (T)0;
+            if (START == FROM_COARSE && i > 0 && i < n - 1 && j < n - 1) v = down_pow2<1>(coarse_pair<T, L>(i, j));
+            if (j < n - 1) su[a * n + j] = v;
+            /* a wall row's red points are read as 0 too */
+            const int jr = c + ((i + 1) & 1);
+            if ((i <= 0 || i >= n - 1) && jr < n - 1) su[a * n + jr] = (T)0;
+        }
+        /* g on the red region, f where residuals are taken; a correction's
+         * red points start from g                                        */
+#pragma unroll 4
+        for (int t = threadIdx.x; t < B::GR << (L + 1); t += TH) {
+            const int a = t >> (L + 1), j = t & (2 * N - 1), i = iu + 1 + a;
+            if (i > 0 && i < n - 1 && j > 0) {
+                T v;
+                if constexpr (ABOVE) v = Band<T, L + 1>::owner_rc(i, j);
+                else v = __ldcg(gf + i * n + j);
+                const T g = h2 * v;
+                sg[a * n + j] = g;
+                const int b = a - 3;
+                if (b >= 0 && b < B::FR) sf[b * n + j] = v;
+                if (START == FROM_ZERO && ((i + j) & 1) == 0) su[(a + 1) * n + j] = red_from_zero(g);
             }
         }
-        if (j < n - 1) su[a * n + j] = v;
-        /* a wall row's red points are read as 0 too */
-        const int jr = c + ((i + 1) & 1);
-        if ((i <= 0 || i >= n - 1) && jr < n - 1) su[a * n + jr] = (T)0;
     }
-    /* g on the red region, f where residuals are taken; a correction's red
-     * points start from g                                                */
-#pragma unroll 4
-    for (int t = threadIdx.x; t < B::GR << (L + 1); t += TH) {
-        const int a = t >> (L + 1), j = t & (2 * N - 1), i = iu + 1 + a;
-        if (i > 0 && i < n - 1 && j > 0) {
-            const T v = __ldcg(gf + i * n + j), g = h2 * v;
-            sg[a * n + j] = g;
-            const int b = a - 3;
-            if (b >= 0 && b < B::FR) sf[b * n + j] = v;
-            if (START == FROM_ZERO && ((i + j) & 1) == 0) su[(a + 1) * n + j] = red_from_zero(g);
-        }
-    }
+    /* a neighbour may still be reading this band's black points (FROM_U):
+     * they change in the black sweep                                     */
+    if (START == FROM_U) cluster_arrive();
     __syncthreads();
     if (START != FROM_ZERO) band_sweep<T, L>(0, iu + 1, B::GR, iu);
+    if (START == FROM_U) cluster_wait();
     band_sweep<T, L>(1, iu + 2, B::GR - 2, iu);
     /* residuals: even rows 2 ic0 ... whole, odd rows at even columns */
 #pragma unroll 2
@@ -667,35 +727,39 @@ __device__ __forceinline__ void cl_vcycle(const MgPtrs<T>& p, T* gu, const T* gf
         }
     }
     __syncthreads();
+    T* const rc = B::rc();
     for (int t = threadIdx.x; t < M << L; t += TH) {
         const int a = t >> L, jc = t & (N - 1), ic = ic0 + a;
         if (jc > 0 && ic < nc - 1) {
             const T* const r = sr + (2 * a + 1) * n + 2 * jc;
-            p.r[L - 1][ic * nc + jc] = half_weight(r[0], r[n], r[-n], r[1], r[-1]);
+            rc[a * nc + jc] = half_weight(r[0], r[n], r[-n], r[1], r[-1]);
         }
     }
     cluster_sync();
-    ClLower<T, L - 1>::run(p);
+    ClLower<T, L - 1, true>::run(p);
     /* the correction of the black points, then a sweep */
-    const T* const vc = p.v[L - 1];
 #pragma unroll 4
     for (int t = threadIdx.x; t < (2 * M + 4) << L; t += TH) {
         const int a = t >> L, i = iu + 2 + a, j = 1 + (i & 1) + 2 * (t & (N - 1));
         if (i > 0 && i < n - 1 && j < n - 1) {
-            int k1, k0;
-            black_pair(i, j, nc, k1, k0);
             T& x = su[(a + 2) * n + j];
-            x = fma_t((T)0.5, __ldcg(vc + k1) + __ldcg(vc + k0), x);
+            x = fma_t((T)0.5, coarse_pair<T, L>(i, j), x);
         }
     }
     __syncthreads();
     band_sweep<T, L>(0, iu + 3, 2 * M + 2, iu);
     band_sweep<T, L>(1, iu + 4, 2 * M, iu);
-    for (int t = threadIdx.x; t < (2 * M) << (L + 1); t += TH) {
-        const int a = t >> (L + 1), j = t & (2 * N - 1), i = iu + 4 + a;
-        if (j > 0 && i < n - 1) gu[i * n + j] = su[(a + 4) * n + j];
-    }
     cluster_sync();
+}
+/* the bands' own rows to global memory */
+template <class T, int L>
+__device__ __forceinline__ void cl_store(T* gu) {
+    using B = Band<T, L>;
+    const int i0 = 2 * B::M * cluster_rank() + 1;   /* band row 4 */
+    for (int t = threadIdx.x; t < (2 * B::M) << (L + 1); t += Cfg<T>::THREADS) {
+        const int a = t >> (L + 1), j = t & (2 * B::N - 1), i = i0 + a;
+        if (j > 0 && i < B::n - 1) gu[i * B::n + j] = B::u()[(a + 4) * B::n + j];
+    }
 }
 /* right-hand side of level L from level L+1, shared out */
 template <class T, int L>
@@ -716,10 +780,13 @@ struct ClF {
         if constexpr (L > Cfg<T>::TOP) {
             cl_restrict<T, L - 1>(p);
             ClF<T, L - 1>::run(p);
-            cl_vcycle<T, L, FROM_COARSE>(p, p.u[L], p.f[L], p.u[L - 1]);
-            cl_vcycle<T, L, FROM_U>(p, p.u[L], p.f[L], nullptr);
+            cl_vcycle<T, L, FROM_COARSE, false>(p, p.f[L]);
+            cl_vcycle<T, L, FROM_U, false>(p, p.f[L]);
         } else {
-            if (cluster_rank() == 0) sm_fmg<T, L>(p.f[L], p.u[L], p.c);
+            if (cluster_rank() == 0) {
+                sm_fmg<T, L>(p.f[L], p.c);
+                __syncthreads();
+            }
             cluster_sync();
         }
     }
@@ -733,10 +800,12 @@ __global__ void __launch_bounds__(Cfg<T>::THREADS) k_mg_levels(const __grid_cons
     pgb_pdl_entry();
     if constexpr (J > Cfg<T>::TOP) {
         if constexpr (FMG) ClF<T, J>::run(p);
-        else ClLower<T, J>::run(p);
+        else ClLower<T, J, false>::run(p);
+        cl_store<T, J>(FMG ? p.u[J] : p.v[J]);
     } else {
-        if constexpr (FMG) sm_fmg<T, J>(p.f[J], p.u[J], p.c);
-        else sm_vcycle0<T, J>(p.r[J], p.v[J], p.c);
+        if constexpr (FMG) sm_fmg<T, J>(p.f[J], p.c);
+        else sm_vcycle0<T, J>(p.r[J], p.c);
+        sm_store_u<T, J>(FMG ? p.u[J] : p.v[J]);
     }
 }
 
