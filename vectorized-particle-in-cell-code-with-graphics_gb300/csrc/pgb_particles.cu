@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
     const int npieces = a.ds->n_pieces[a.s];
     const int tile0 = (int)a.ds->sorted_tiles[a.s];
     const int nitems = npieces + (ntiles > tile0 ? ntiles - tile0 : 0);
+    if ((int)blockIdx.x >= nitems) return;   /* small runs: no item for this block */
     const PushConsts pc = a.pc;
     __shared__ int s_cnt[2];
     int it = 0, gone = 0;
