@@ -26,9 +26,10 @@
  *   k_dst_columns  pairs of k: transform over i, division by the
  *                  eigenvalue, inverse transform over l
  *   k_dst_back     row pairs: inverse transform over k, written to u
- * Each CTA runs one radix-2 FFT of length M in shared memory (in-place,
- * decimation in time from a bit-reversed load), twiddles from a table made
- * in FP64 on the host.
+ * Each CTA runs FFTs of length M in shared memory: radix-2 butterflies,
+ * decimation in time, one or two stages at a time in registers, twiddles
+ * from a table made in FP64 on the host.  How many stages a pass takes does
+ * not change a value.
  */
 #include <cuda_runtime.h>
 #include <math.h>
@@ -45,137 +46,210 @@ struct DstArgs {
     float scale;         /* -(2/N)^2 h^2                                 */
 };
 
-__device__ __forceinline__ int bitrev(int q, int logM) { return (int)(__brev((unsigned)q) >> (32 - logM)); }
-
-/* stage the twiddles, then an in-place FFT of z (already bit-reversed) */
-__device__ __forceinline__ void fft_inplace(float2* z, const float2* stw, int M, int logM) {
-    for (int st = 0; st < logM; ++st) {
-        const int h = 1 << st;
-        for (int b = threadIdx.x; b < (M >> 1); b += blockDim.x) {
-            const int pos = b & (h - 1);
-            const int i0 = ((b >> st) << (st + 1)) + pos, i1 = i0 + h;
-            const float2 w = stw[pos << (logM - 1 - st)];
-            const float2 a = z[i0], c = z[i1];
-            const float2 tt = make_float2(w.x * c.x - w.y * c.y, w.x * c.y + w.y * c.x);
-            z[i0] = make_float2(a.x + tt.x, a.y + tt.y);
-            z[i1] = make_float2(a.x - tt.x, a.y - tt.y);
-        }
-        __syncthreads();
-    }
+/* Where element i of an FFT buffer, or of the twiddles, lies: bits 0-3 (a
+ * bank of 8 bytes) exclusive-or bits 4 and up, folded so that the strided
+ * accesses of the passes (elements M/16, 16 or 4 apart, twiddles a power of
+ * two apart) spread over the banks.  Linear over GF(2): for i and
+ * j without a common bit, slot(i + j) = slot(i) ^ slot(j).               */
+__device__ __forceinline__ int slot(int i) {
+    const int s = i >> 4;
+    return i ^ ((((s & 3) << 2) ^ (s >> 2) ^ (s >> 6)) & 15);
 }
 
-/* odd extension of the pair (a_q, b_q), q = 1..N-1, into z in bit-reversed
- * order; get(q) returns (a_q, b_q)                                       */
-template <class G>
-__device__ __forceinline__ void load_odd(float2* z, int N, int logM, G get) {
-    const int M = 2 * N;
-    for (int q = threadIdx.x; q < M; q += blockDim.x) {
-        float2 v = make_float2(0.0f, 0.0f);
-        if (q > 0 && q < N) v = get(q);
-        else if (q > N) {
-            v = get(M - q);
-            v.x = -v.x;
-            v.y = -v.y;
+/* stages s .. s + R - 1 on the 2^R elements pos + j 2^s of one thread */
+template <int R>
+__device__ __forceinline__ void fft_stages(float2 (&v)[1 << R], const float2* stw, int pos, int s, int logM) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+#pragma unroll
+        for (int m = 0; m < (1 << q); ++m) {
+            const float2 w = stw[slot((pos + (m << s)) << (logM - 1 - s - q))];
+#pragma unroll
+            for (int p = m; p < (1 << R); p += 2 << q) {
+                const float2 a = v[p], c = v[p + (1 << q)];
+                const float2 tt = make_float2(w.x * c.x - w.y * c.y, w.x * c.y + w.y * c.x);
+                v[p] = make_float2(a.x + tt.x, a.y + tt.y);
+                v[p + (1 << q)] = make_float2(a.x - tt.x, a.y - tt.y);
+            }
         }
-        z[bitrev(q, logM)] = v;
     }
+}
+/* one pass of R stages over z; the last one hands Z_k, k < M/2, to put */
+template <int R, class P>
+__device__ __forceinline__ void fft_pass(float2* z, const float2* stw, int s, int logM, P put) {
+    const bool last = s + R == logM;
+    for (int t = threadIdx.x; t < 1 << (logM - R); t += blockDim.x) {
+        const int pos = t & ((1 << s) - 1), base = ((t >> s) << (s + R)) + pos, b = slot(base);
+        float2 v[1 << R];
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j) v[j] = z[b ^ slot(j << s)];
+        fft_stages<R>(v, stw, pos, s, logM);
+        if (last) {
+#pragma unroll
+            for (int j = 0; j < (1 << R) / 2; ++j) put(base + (j << s), v[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < (1 << R); ++j) z[b ^ slot(j << s)] = v[j];
+        }
+    }
+    __syncthreads();
+}
+/* FFT of length M = 2^logM of the odd extension of the pair (a_q, b_q) =
+ * get(q), q = 1..N-1: radix-2 butterflies, decimation in time, R stages at
+ * a time in registers; put(k, Z_k) for k < N.  The first pass takes its
+ * elements (t, t + M/2^R, ... in order, as the bit reversal wants them)
+ * straight from get.                                                     */
+template <int R, class G, class P>
+__device__ __forceinline__ void fft_odd(float2* z, const float2* stw, int N, int logM, G get, P put) {
+    const int M = 2 * N;
+    for (int t = threadIdx.x; t < M >> R; t += blockDim.x) {
+        float2 v[1 << R];
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j) {
+            const int q = t + (int)(__brev((unsigned)j) >> (32 - R)) * (M >> R);
+            v[j] = make_float2(0.0f, 0.0f);
+            if (q > 0 && q < N) v[j] = get(q);
+            else if (q > N) {
+                const float2 x = get(M - q);
+                v[j] = make_float2(-x.x, -x.y);
+            }
+        }
+        fft_stages<R>(v, stw, 0, 0, logM);
+        const int b = slot((int)(((unsigned long long)__brev((unsigned)t) << (logM - R)) >> 32) << R);
+#pragma unroll
+        for (int j = 0; j < (1 << R); ++j) z[b ^ slot(j)] = v[j];
+    }
+    __syncthreads();
+    int s = R;
+    for (; s + R < logM; s += R) fft_pass<R>(z, stw, s, logM, put);
+    if (logM - s == R) fft_pass<R>(z, stw, s, logM, put);
+    else fft_pass<1>(z, stw, s, logM, put);
 }
 
 __device__ __forceinline__ float2* dst_smem(float2*& stw, int M) {
     extern __shared__ __align__(16) float2 smem[];
     stw = smem;              /* M/2 twiddles */
-    return smem + M / 2;     /* then the FFT buffer(s) */
+    return smem + M / 2;     /* then the FFT buffer, M, and N coefficients */
 }
 
 __device__ __forceinline__ void stage_twiddles(float2* stw, const float2* tw, int M) {
-    for (int q = threadIdx.x; q < M / 2; q += blockDim.x) stw[q] = tw[q];
+    for (int q = threadIdx.x; q < M / 2; q += blockDim.x) stw[slot(q)] = tw[q];
 }
 
 /* row pair p: rows i0 = 2p+1 and i0+1 (the wall row n-1 reads as 0) */
+template <int R>
 __global__ void k_dst_rows(DstArgs a) {
-    pgb_pdl_entry();
     const int N = a.N, M = 2 * N, n = a.n;
     float2* stw;
     float2* z = dst_smem(stw, M);
-    stage_twiddles(stw, a.tw, M);
+    stage_twiddles(stw, a.tw, M);   /* the run's own table: no kernel before writes it */
+    pgb_pdl_entry();
+    __syncthreads();
     const int i0 = 2 * blockIdx.x + 1, i1 = i0 + 1;
     const float* ra = a.f + (size_t)i0 * n;
     const float* rb = i1 <= n - 2 ? a.f + (size_t)i1 * n : nullptr;
-    load_odd(z, N, a.logM, [&](int j) { return make_float2(ra[j], rb ? rb[j] : 0.0f); });
-    __syncthreads();
-    fft_inplace(z, stw, M, a.logM);
     /* S_a,k = -Im Z_k / 2 (row i0), S_b,k = Re Z_k / 2 (row i1); for the
      * wall row an exact 0, not the rounding of row i0 that Re Z_k holds  */
-    for (int k = 1 + threadIdx.x; k < N; k += blockDim.x) {
-        const float2 Z = z[k];
-        *reinterpret_cast<float2*>(a.t + (size_t)(k - 1) * N + (i0 - 1)) = make_float2(-0.5f * Z.y, rb ? 0.5f * Z.x : 0.0f);
-    }
+    fft_odd<R>(z, stw, N, a.logM, [&](int j) { return make_float2(ra[j], rb ? rb[j] : 0.0f); },
+               [&](int k, float2 Z) {
+                   if (k > 0)
+                       *reinterpret_cast<float2*>(a.t + (size_t)(k - 1) * N + (i0 - 1)) =
+                           make_float2(-0.5f * Z.y, rb ? 0.5f * Z.x : 0.0f);
+               });
 }
 
 /* pair q of frequencies k0 = 2q+1, k1 = k0+1 (k1 = N reads as 0, not written) */
+template <int R>
 __global__ void k_dst_columns(DstArgs a) {
-    pgb_pdl_entry();
     const int N = a.N, M = 2 * N;
     float2* stw;
     float2* z = dst_smem(stw, M);
-    float2* z2 = z + M;
+    float2* const coef = z + M;
     stage_twiddles(stw, a.tw, M);
+    pgb_pdl_entry();
+    __syncthreads();
     const int k0 = 2 * blockIdx.x + 1, k1 = k0 + 1;
     float* const ta = a.t + (size_t)(k0 - 1) * N;
     float* const tb = k1 <= N - 1 ? a.t + (size_t)(k1 - 1) * N : nullptr;
-    load_odd(z, N, a.logM, [&](int i) { return make_float2(ta[i - 1], tb ? tb[i - 1] : 0.0f); });
-    __syncthreads();
-    fft_inplace(z, stw, M, a.logM);
-    /* the solution's coefficients, then their odd extension over l */
     const float sa = a.s[k0], sb = a.s[k1 < N ? k1 : 1];
-    load_odd(z2, N, a.logM, [&](int l) {
-        const float2 Z = z[l];
-        const float sl = a.s[l];
-        return make_float2((-0.5f * Z.y) * a.scale / (sa + sl), tb ? (0.5f * Z.x) * a.scale / (sb + sl) : 0.0f);
-    });
-    __syncthreads();
-    fft_inplace(z2, stw, M, a.logM);
-    for (int i = 1 + threadIdx.x; i < N; i += blockDim.x) {
-        const float2 Z = z2[i];
-        ta[i - 1] = -0.5f * Z.y;
-        if (tb) tb[i - 1] = 0.5f * Z.x;
-    }
+    /* the solution's coefficients, then the transform of those over l */
+    fft_odd<R>(z, stw, N, a.logM, [&](int i) { return make_float2(ta[i - 1], tb ? tb[i - 1] : 0.0f); },
+               [&](int l, float2 Z) {
+                   if (l == 0) return;
+                   const float sl = a.s[l];
+                   coef[l] = make_float2((-0.5f * Z.y) * a.scale / (sa + sl), tb ? (0.5f * Z.x) * a.scale / (sb + sl) : 0.0f);
+               });
+    fft_odd<R>(z, stw, N, a.logM, [&](int l) { return coef[l]; },
+               [&](int i, float2 Z) {
+                   if (i == 0) return;
+                   ta[i - 1] = -0.5f * Z.y;
+                   if (tb) tb[i - 1] = 0.5f * Z.x;
+               });
 }
 
 /* row pair p: u rows i0 = 2p+1 and i0+1 from t's columns i0-1 and i0 */
+template <int R>
 __global__ void k_dst_back(DstArgs a) {
-    pgb_pdl_entry();
     const int N = a.N, M = 2 * N, n = a.n;
     float2* stw;
     float2* z = dst_smem(stw, M);
     stage_twiddles(stw, a.tw, M);
+    pgb_pdl_entry();
+    __syncthreads();
     const int i0 = 2 * blockIdx.x + 1, i1 = i0 + 1;
     /* the wall row's slot (column N-1 of t) is never written by the column
      * pass: read it as 0, or its values would leak into row i0 through the
      * rounding of the shared transform                                    */
     const bool wall = i1 > n - 2;
-    load_odd(z, N, a.logM, [&](int k) {
-        const float2 v = *reinterpret_cast<const float2*>(a.t + (size_t)(k - 1) * N + (i0 - 1));
-        return make_float2(v.x, wall ? 0.0f : v.y);
-    });
-    __syncthreads();
-    fft_inplace(z, stw, M, a.logM);
     float* const ua = a.u + (size_t)i0 * n;
     float* const ub = a.u + (size_t)i1 * n;   /* i1 <= n-1: the top wall row is written 0 */
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        float va = 0.0f, vb = 0.0f;
-        if (j > 0 && j < n - 1) {
-            const float2 Z = z[j];
-            va = -0.5f * Z.y;
-            vb = i1 <= n - 2 ? 0.5f * Z.x : 0.0f;
-        }
-        ua[j] = va;
-        ub[j] = vb;
-        if (blockIdx.x == 0) a.u[j] = 0.0f;   /* the bottom wall row */
-    }
+    fft_odd<R>(z, stw, N, a.logM,
+               [&](int k) {
+                   const float2 v = *reinterpret_cast<const float2*>(a.t + (size_t)(k - 1) * N + (i0 - 1));
+                   return make_float2(v.x, wall ? 0.0f : v.y);
+               },
+               [&](int j, float2 Z) {
+                   ua[j] = j > 0 ? -0.5f * Z.y : 0.0f;
+                   ub[j] = j > 0 && !wall ? 0.5f * Z.x : 0.0f;
+                   if (blockIdx.x == 0) a.u[j] = 0.0f;   /* the bottom wall row */
+                   if (j == 0) {                         /* the right walls */
+                       ua[N] = ub[N] = 0.0f;
+                       if (blockIdx.x == 0) a.u[N] = 0.0f;
+                   }
+               });
 }
 
-static int dst_threads(int M) { return M / 2 < 32 ? 32 : (M / 2 > 512 ? 512 : M / 2); }
+static int dst_threads(int per) { return per < 32 ? 32 : (per > 512 ? 512 : per); }
+
+template <int R>
+static int dst_attributes(pgb_run* r, int smem) {
+    PGB_CK(r, cudaFuncSetAttribute(k_dst_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    PGB_CK(r, cudaFuncSetAttribute(k_dst_columns<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    PGB_CK(r, cudaFuncSetAttribute(k_dst_back<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return 0;
+}
+template <int R>
+static int dst_launch(pgb_run* r, const DstArgs& a) {
+    const int M = 2 * a.N;
+    const dim3 th(dst_threads(M >> R)), blocks(a.N / 2);
+    const size_t sm1 = sizeof(float2) * (M / 2 + M), sm2 = sm1 + sizeof(float2) * a.N;
+    PGB_CK(r, pgb_launch_pdl(k_dst_rows<R>, blocks, th, sm1, r->stream, a));
+    PGB_CK(r, pgb_launch_pdl(k_dst_columns<R>, blocks, th, sm2, r->stream, a));
+    PGB_CK(r, pgb_launch_pdl(k_dst_back<R>, blocks, th, sm1, r->stream, a));
+    r->launches += 3;
+    PGB_CK(r, cudaGetLastError());
+    return 0;
+}
+/* Stages per pass: one point pair a thread is the shorter chain where the
+ * kernels are launch and latency, two stages in registers halve the traffic
+ * with shared memory and the barriers where they are not.  A pass of the
+ * solver (three kernels and the FP64 update), R = 1 / 2 / 3, and before
+ * (radix-2 in place from a bit-reversed store, up to 16-way bank conflicts
+ * on it and on the twiddles): 65 nodes 10.2 / 11.9 / 14.4 (10.9) us,
+ * 129 12.1 / 13.3 / 18.1 (12.8), 257 14.6 / 14.9 / 19.7 (16.1),
+ * 513 28.7 / 23.3 / 25.6 (34.5).  At 257 other kernels run beside it, so
+ * there the one with fewer instructions.                                 */
+static bool dst_two_stages(int M) { return M >= 512; }
 
 int pgb_dst_setup(pgb_run* r) {
     const int n = r->nx, N = n - 1;
@@ -197,11 +271,7 @@ int pgb_dst_setup(pgb_run* r) {
     PGB_CK(r, cudaMemcpy(r->dst_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
     PGB_CK(r, cudaMemcpy(r->dst_s, s.data(), sizeof(float) * s.size(), cudaMemcpyHostToDevice));
     const int smem = (int)(sizeof(float2) * (M / 2 + 2 * M));
-    if (smem > 48 * 1024) {
-        PGB_CK(r, cudaFuncSetAttribute(k_dst_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        PGB_CK(r, cudaFuncSetAttribute(k_dst_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        PGB_CK(r, cudaFuncSetAttribute(k_dst_back, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    }
+    if (smem > 48 * 1024 && dst_attributes<2>(r, smem)) return PGB_ERR_CUDA;
     return 0;
 }
 
@@ -227,12 +297,5 @@ int pgb_dst_solve(pgb_run* r, const float* f, float* u) {
     while ((1 << a.logM) < M) a.logM++;
     const double h = r->p.xlength / (double)a.N;
     a.scale = (float)(-(2.0 / a.N) * (2.0 / a.N) * h * h);
-    const int th = dst_threads(M), blocks = a.N / 2;
-    const size_t sm1 = sizeof(float2) * (M / 2 + M), sm2 = sizeof(float2) * (M / 2 + 2 * M);
-    PGB_CK(r, pgb_launch_pdl(k_dst_rows, dim3(blocks), dim3(th), sm1, r->stream, a));
-    PGB_CK(r, pgb_launch_pdl(k_dst_columns, dim3(blocks), dim3(th), sm2, r->stream, a));
-    PGB_CK(r, pgb_launch_pdl(k_dst_back, dim3(blocks), dim3(th), sm1, r->stream, a));
-    r->launches += 3;
-    PGB_CK(r, cudaGetLastError());
-    return 0;
+    return dst_two_stages(M) ? dst_launch<2>(r, a) : dst_launch<1>(r, a);
 }
