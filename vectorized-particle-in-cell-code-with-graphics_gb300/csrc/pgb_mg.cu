@@ -22,13 +22,13 @@
  *
  * Who works on a level (Cfg):
  *   n <= 17 (FP64), 33 (FP32)   one CTA, every level in shared memory
- *   up to n = 129   a cluster of 16 CTAs in the same launch, a band of rows
+ *   up to n = 65 (FP64), 129 (FP32)
+ *                   a cluster of 16 CTAs in the same launch, a band of rows
  *                   per CTA with the halo that makes one exchange (through
  *                   the CTAs' shared memory, a cluster barrier of 400
  *                   clocks) enough for smoothing, residual and restriction,
  *                   and one for correction and smoothing
- *   n >= 257        two launches per level and V-cycle (the same two tile
- *                   functions on 16 x 32 tiles)
+ *   above           two launches per level and V-cycle on tiles
  */
 #include <cuda_runtime.h>
 #include <math.h>
@@ -106,15 +106,19 @@ struct MgConst {
 __host__ __device__ constexpr int sm_n(int l) { return (2 << l) + 1; }
 __host__ __device__ constexpr int sm_below(int l) { return l == 0 ? 0 : sm_below(l - 1) + sm_n(l - 1) * sm_n(l - 1); }
 
-/* the finest level that one CTA solves, and the threads of a CTA.  FP64:
- * 17 nodes (a level of 33 nodes takes 7.3 us in one CTA, bound by its FP64
- * pipe, and 2.9 us on the cluster); FP32: 33 nodes (1.0 us in one CTA)   */
+/* TOP: the finest level that one CTA solves.  FP64: 17 nodes (a level of 33
+ * nodes takes 7.3 us in one CTA, bound by its FP64 pipe, and 2.9 us on the
+ * cluster); FP32: 33 nodes (1.0 us in one CTA).  CL: the finest that the
+ * cluster solves.  FP64: 65 nodes, as 129 keep the FP64 pipes of 16 SMs busy
+ * (a visit 15 us, two tile launches 10; the whole solve at 129^2, 257^2 and
+ * 513^2 152, 225 and 342 us on the cluster, 139, 204 and 313 in tiles);
+ * FP32: 129 (a visit 3.7 us, less than two launches).                    */
 template <class T>
 struct Cfg;
 template <>
-struct Cfg<double> { static constexpr int TOP = 3, THREADS = 256; };
+struct Cfg<double> { static constexpr int TOP = 3, CL = 5, THREADS = 256; };
 template <>
-struct Cfg<float> { static constexpr int TOP = 4, THREADS = 512; };
+struct Cfg<float> { static constexpr int TOP = 4, CL = 6, THREADS = 512; };
 
 /* ----------------------------------------------------- levels in one CTA */
 /* shared image: U, F, G = h^2 F of levels 0..TOP (a V-cycle's top), V, R,
@@ -499,21 +503,18 @@ __device__ __forceinline__ void tile_up(const T* w, const T* vc, const T* f, T* 
     __syncthreads();
 }
 
-/* ------------------------------------ levels on the whole GPU (n >= 257) */
-#define MG_M 8
-#define MG_N 16
+/* ------------------------------------------ levels on the whole GPU */
 #define MG_THREADS 256
-template <class T, int START>
+template <class T, int M, int N, int START>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_down(const T* u, const T* uc, const T* f, T* w, T* rc, int n, T h2,
                                                         T h2i) {
     pgb_pdl_entry();
-    tile_down<T, MG_M, MG_N, START, MG_THREADS>(u, uc, f, w, rc, n, 1 + MG_M * blockIdx.y, 1 + MG_N * blockIdx.x, h2,
-                                               h2i);
+    tile_down<T, M, N, START, MG_THREADS>(u, uc, f, w, rc, n, 1 + M * blockIdx.y, 1 + N * blockIdx.x, h2, h2i);
 }
-template <class T>
+template <class T, int M, int N>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_up(const T* w, const T* vc, const T* f, T* u, int n, T h2) {
     pgb_pdl_entry();
-    tile_up<T, MG_M, MG_N, MG_THREADS>(w, vc, f, u, n, 1 + MG_M * blockIdx.y, 1 + MG_N * blockIdx.x, h2);
+    tile_up<T, M, N, MG_THREADS>(w, vc, f, u, n, 1 + M * blockIdx.y, 1 + N * blockIdx.x, h2);
 }
 /* right-hand side of the coarser level (interior) */
 template <class T>
@@ -529,7 +530,7 @@ __global__ void k_mg_restrict(T* fc, const T* ff, int nc) {
     }
 }
 
-/* ------------------------------------------- levels in one launch (n <= 129) */
+/* ------------------------------------------- levels in one launch */
 constexpr int CL_CTAS = 16;
 /* level arrays in global memory */
 template <class T>
@@ -810,14 +811,13 @@ __global__ void __launch_bounds__(Cfg<T>::THREADS) k_mg_levels(const __grid_cons
 }
 
 /* ====================================================== host side */
-constexpr int CL_TOP = 6;   /* the finest level of k_mg_levels (129 nodes) */
 template <class T, int J>
 constexpr size_t levels_smem() {
     if constexpr (J > Cfg<T>::TOP) return sizeof(T) * (Sm<T>::WORDS + Band<T, J>::END);
     else return sizeof(T) * Sm<T>::WORDS;
 }
-template <class T>
-constexpr size_t tile_smem() { return sizeof(T) * Tile<MG_M, MG_N>::WORDS; }
+template <class T, int M, int N>
+constexpr size_t tile_smem() { return sizeof(T) * Tile<M, N>::WORDS; }
 
 template <class T>
 MgConst<T> mg_const(const pgb_run* r) {
@@ -888,8 +888,8 @@ int levels_launch(pgb_run* r, int J) {
         case 3: return levels_go<T, 3, FMG>(r);
         case 4: return levels_go<T, 4, FMG>(r);
         case 5: return levels_go<T, 5, FMG>(r);
-        default: return levels_go<T, 6, FMG>(r);
     }
+    return levels_go<T, Cfg<T>::CL, FMG>(r);
 }
 template <class T>
 int mg_attrs(pgb_run* r) {
@@ -898,48 +898,62 @@ int mg_attrs(pgb_run* r) {
     PGB_CK(r, (levels_attr<T, 3, true>()));
     PGB_CK(r, (levels_attr<T, 4, true>()));
     PGB_CK(r, (levels_attr<T, 5, true>()));
-    PGB_CK(r, (levels_attr<T, 6, true>()));
+    PGB_CK(r, (levels_attr<T, Cfg<T>::CL, true>()));
     PGB_CK(r, (levels_attr<T, 1, false>()));
     PGB_CK(r, (levels_attr<T, 2, false>()));
     PGB_CK(r, (levels_attr<T, 3, false>()));
     PGB_CK(r, (levels_attr<T, 4, false>()));
     PGB_CK(r, (levels_attr<T, 5, false>()));
-    PGB_CK(r, (levels_attr<T, 6, false>()));
+    PGB_CK(r, (levels_attr<T, Cfg<T>::CL, false>()));
     return 0;
 }
-static_assert(tile_smem<double>() <= 48 * 1024, "the tile kernels use no more than the default shared memory");
+static_assert(tile_smem<double, 8, 8>() <= 48 * 1024, "the tile kernels use no more than the default shared memory");
 
-/* V-cycle at level j > CL_TOP (mglin.cpp:176-196): u -> w -> u.  A level
- * has one V-cycle in flight at a time, so one spare buffer w serves.     */
+/* V-cycle at level j > CL (mglin.cpp:176-196): u -> w -> u.  A level has
+ * one V-cycle in flight at a time, so one spare buffer w serves.         */
 template <class T, int START>
-int vcycle(pgb_run* r, const MgPtrs<T>& p, int j, T* u, const T* f, const T* uc) {
+int vcycle(pgb_run* r, const MgPtrs<T>& p, int j, T* u, const T* f, const T* uc);
+template <class T, int M, int N, int START>
+int vcycle_tiles(pgb_run* r, const MgPtrs<T>& p, int j, T* u, const T* f, const T* uc) {
     const int n = r->mg_n[j], nc = r->mg_n[j - 1];
-    const dim3 grid((nc - 2 + MG_N - 1) / MG_N, (nc - 2 + MG_M - 1) / MG_M);
-    PGB_CK(r, pgb_launch_pdl(k_mg_down<T, START>, grid, dim3(MG_THREADS), tile_smem<T>(), r->stream, (const T*)u, uc, f,
-                             p.w[j], p.r[j - 1], n, p.c.h2[j], p.c.h2i[j]));
+    const dim3 grid((nc - 2 + N - 1) / N, (nc - 2 + M - 1) / M);
+    PGB_CK(r, pgb_launch_pdl(k_mg_down<T, M, N, START>, grid, dim3(MG_THREADS), tile_smem<T, M, N>(), r->stream, (const T*)u,
+                             uc, f, p.w[j], p.r[j - 1], n, p.c.h2[j], p.c.h2i[j]));
     r->launches++;
-    if (j - 1 > CL_TOP) {
+    if (j - 1 > Cfg<T>::CL) {
         if (vcycle<T, FROM_ZERO>(r, p, j - 1, p.v[j - 1], p.r[j - 1], nullptr)) return PGB_ERR_CUDA;
     } else if (levels_launch<T, false>(r, j - 1)) {
         return PGB_ERR_CUDA;
     }
-    PGB_CK(r, pgb_launch_pdl(k_mg_up<T>, grid, dim3(MG_THREADS), tile_smem<T>(), r->stream, (const T*)p.w[j],
+    PGB_CK(r, pgb_launch_pdl(k_mg_up<T, M, N>, grid, dim3(MG_THREADS), tile_smem<T, M, N>(), r->stream, (const T*)p.w[j],
                              (const T*)p.v[j - 1], f, u, n, p.c.h2[j]));
     r->launches++;
     return 0;
 }
+/* Tiles of 8 x 8 coarse points, 256 of them at 257^2: with 8 x 16, half as
+ * many, a block was alone on its SM with its load latencies and barriers
+ * (FMG_REF / ten passes of FP32_DC at 257^2 206.6 / 291.8 us, with 8 x 8
+ * 203.1 / 278.2; at 513^2 317.7 / 445.9 and 312.0 / 425.7).  4 x 8 at 129
+ * nodes (FP64 only), where 8 x 8 are 64 tiles (142.6 and 139.9 us).      */
+template <class T, int START>
+int vcycle(pgb_run* r, const MgPtrs<T>& p, int j, T* u, const T* f, const T* uc) {
+    if constexpr (Cfg<T>::CL < 6)
+        if (j == 6) return vcycle_tiles<T, 4, 8, START>(r, p, j, u, f, uc);
+    return vcycle_tiles<T, 8, 8, START>(r, p, j, u, f, uc);
+}
 
 template <class T>
 int fmg(pgb_run* r) {
+    constexpr int CL = Cfg<T>::CL;
     const int ng = r->ng;
     const MgPtrs<T> p = mg_ptrs<T>(r);
-    for (int j = ng - 2; j >= CL_TOP; --j) {
+    for (int j = ng - 2; j >= CL; --j) {
         const int nc = r->mg_n[j], blocks = (nc * nc + 255) / 256;
         PGB_CK(r, pgb_launch_pdl(k_mg_restrict<T>, dim3(blocks), dim3(256), 0, r->stream, p.f[j], (const T*)p.f[j + 1], nc));
         r->launches++;
     }
-    if (levels_launch<T, true>(r, ng - 1 < CL_TOP ? ng - 1 : CL_TOP)) return PGB_ERR_CUDA;
-    for (int j = CL_TOP + 1; j < ng; ++j) {
+    if (levels_launch<T, true>(r, ng - 1 < CL ? ng - 1 : CL)) return PGB_ERR_CUDA;
+    for (int j = CL + 1; j < ng; ++j) {
         if (vcycle<T, FROM_COARSE>(r, p, j, p.u[j], p.f[j], p.u[j - 1])) return PGB_ERR_CUDA;
         if (vcycle<T, FROM_U>(r, p, j, p.u[j], p.f[j], nullptr)) return PGB_ERR_CUDA;
     }
@@ -955,7 +969,7 @@ int pgb_mg_fmg32(pgb_run* r) { return fmg<float>(r); }
 int pgb_mg_vcycle32(pgb_run* r) {
     const MgPtrs<float> p = mg_ptrs<float>(r);
     const int top = r->ng - 1;
-    const int rc = top > CL_TOP ? vcycle<float, FROM_ZERO>(r, p, top, p.v[top], p.r[top], nullptr)
+    const int rc = top > Cfg<float>::CL ? vcycle<float, FROM_ZERO>(r, p, top, p.v[top], p.r[top], nullptr)
                                 : levels_launch<float, false>(r, top);
     if (rc) return rc;
     PGB_CK(r, cudaGetLastError());
