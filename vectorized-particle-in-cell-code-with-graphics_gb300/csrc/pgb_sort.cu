@@ -105,35 +105,53 @@ __device__ __forceinline__ long long block_excl_scan_ll(long long v, long long* 
     return before + x - v;
 }
 
-/* per key: exclusive scan over the chunks.  A CTA takes 32 keys (a lane
- * each), a warp a run of chunks: sums, a scan over the warps, offsets.   */
-__global__ void __launch_bounds__(1024) k_sort_scan_keys(SortArgs a) {
+/* per key: exclusive scan over the chunks.  A CTA takes eight keys (a
+ * sector of each chunk's row) and splits the chunks into 128 runs, a run and
+ * key per thread: sums, a warp's scan over the runs per key, offsets.  (With
+ * 32 keys and 32 runs per CTA the 257 keys of 513^2 were 9 CTAs: 30 us for
+ * 16 Mi particles, now 15.)                                              */
+#define SCAN_KEYS 8
+#define SCAN_RUNS 128
+__global__ void __launch_bounds__(SCAN_KEYS * SCAN_RUNS) k_sort_scan_keys(SortArgs a) {
     pgb_pdl_entry();
-    __shared__ int s_sum[32][33];
+    __shared__ int s_sum[SCAN_KEYS][SCAN_RUNS + 1];
     const long long n = a.ds->n[a.s];
     const int nch = (int)((n + SORT_CHUNK - 1) / SORT_CHUNK), nk = a.nbins + 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int key = blockIdx.x * 32 + lane;
-    const int per = (nch + 31) / 32, c0 = min(warp * per, nch), c1 = min(c0 + per, nch);
+    const int sub = threadIdx.x % SCAN_KEYS, run = threadIdx.x / SCAN_KEYS;
+    const int key = blockIdx.x * SCAN_KEYS + sub;
+    const int per = (nch + SCAN_RUNS - 1) / SCAN_RUNS, c0 = min(run * per, nch), c1 = min(c0 + per, nch);
     int sum = 0;
     if (key < nk) {
 #pragma unroll 8
         for (int c = c0; c < c1; ++c) sum += a.counts[(long long)c * nk + key];
     }
-    s_sum[warp][lane] = sum;
+    s_sum[sub][run] = sum;
     __syncthreads();
-    if (warp == 0) {
-        int acc = 0;
-        for (int w = 0; w < 32; ++w) {
-            const int v = s_sum[w][lane];
-            s_sum[w][lane] = acc;
-            acc += v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < SCAN_KEYS) {
+        int* const v = s_sum[warp] + lane * (SCAN_RUNS / 32);
+        int t = 0;
+#pragma unroll
+        for (int q = 0; q < SCAN_RUNS / 32; ++q) t += v[q];
+        int x = t;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
         }
-        if (key < nk) a.key_total[key] = acc;
+        const int k = blockIdx.x * SCAN_KEYS + warp;
+        if (lane == 31 && k < nk) a.key_total[k] = x;
+        x -= t;
+#pragma unroll
+        for (int q = 0; q < SCAN_RUNS / 32; ++q) {
+            const int c = v[q];
+            v[q] = x;
+            x += c;
+        }
     }
     __syncthreads();
     if (key >= nk) return;
-    int acc = s_sum[warp][lane];
+    int acc = s_sum[sub][run];
 #pragma unroll 8
     for (int c = c0; c < c1; ++c) {
         const int v = a.counts[(long long)c * nk + key];
@@ -207,7 +225,11 @@ __global__ void __launch_bounds__(1024) k_sort_scan_bins(SortArgs a) {
  * running count of its key plus the lanes of the same key before it; the
  * warps' counts are then scanned per key and the keys over the chunk, which
  * gives each particle its place in the sorted chunk.  The particles go
- * there in shared memory and leave from there, bin after bin.            */
+ * there in shared memory and leave from there, bin after bin.
+ * What bounds it is the latency of shared memory (the counts are a chain
+ * from item to item) and of the loads, so two CTAs share an SM: at 123
+ * registers a thread one filled it, and a 16 Mi sort's scatter took 313 us,
+ * now 224 (0.94 GB, 4.2 TB/s).                                           */
 #define SORT_THREADS 512
 #define SORT_WARPS (SORT_THREADS / 32)
 #define SORT_ITEMS (SORT_CHUNK / SORT_THREADS)
@@ -218,7 +240,7 @@ static size_t sort_smem(int nkeys) {
     const size_t w = ((size_t)nkeys * SORT_WARPS * sizeof(unsigned short) + 15) & ~(size_t)15;
     return SORT_CHUNK * (sizeof(float4) + sizeof(unsigned short)) + w + (size_t)nkeys * sizeof(long long);
 }
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SortArgs a) {
+__global__ void __launch_bounds__(SORT_THREADS, 2) k_sort_scatter(SortArgs a) {
     pgb_pdl_entry();
     extern __shared__ __align__(16) unsigned char s_raw[];
     const int nk = a.nbins + 1;
@@ -270,12 +292,10 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SortArgs a) {
         for (int b = 0; b < nk; b += SORT_THREADS) {
             const int k = b + threadIdx.x;
             int tot = 0;
-            if (k < nk)
-                for (int w = 0; w < SORT_WARPS; ++w) {
-                    const int v = s_cnt[w * nk + k];
-                    s_cnt[w * nk + k] = (unsigned short)tot;
-                    tot += v;
-                }
+            if (k < nk) {
+#pragma unroll
+                for (int w = 0; w < SORT_WARPS; ++w) tot += s_cnt[w * nk + k];
+            }
             int x = tot;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -292,7 +312,13 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(SortArgs a) {
             }
             const int start = carry + before + x - tot;   /* of key k in the sorted chunk */
             if (k < nk) {
-                for (int w = 0; w < SORT_WARPS; ++w) s_cnt[w * nk + k] = (unsigned short)(s_cnt[w * nk + k] + start);
+                int acc = start;
+#pragma unroll
+                for (int w = 0; w < SORT_WARPS; ++w) {
+                    const int v = s_cnt[w * nk + k];
+                    s_cnt[w * nk + k] = (unsigned short)acc;
+                    acc += v;
+                }
                 s_dst[k] = a.key_start[k] + a.offs[(long long)c * nk + k] - start;
             }
             carry += all;
@@ -386,7 +412,7 @@ int pgb_launch_sort(pgb_run* r, int s) {
     a.want_pieces = 2 * r->sms;
     const int nk = a.nbins + 1;
     PGB_CK(r, pgb_launch_pdl(k_sort_count, dim3(r->sms * 4), dim3(512), sizeof(int) * nk, r->stream, a));
-    PGB_CK(r, pgb_launch_pdl(k_sort_scan_keys, dim3((nk + 31) / 32), dim3(1024), 0, r->stream, a));
+    PGB_CK(r, pgb_launch_pdl(k_sort_scan_keys, dim3((nk + SCAN_KEYS - 1) / SCAN_KEYS), dim3(SCAN_KEYS * SCAN_RUNS), 0, r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_sort_scan_bins, dim3(1), dim3(1024), 0, r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_sort_scatter, dim3(r->sms * 2), dim3(SORT_THREADS), sort_smem(nk), r->stream, a));
     PGB_CK(r, pgb_launch_pdl(k_sort_pad, dim3(r->sms), dim3(256), 0, r->stream, a));
