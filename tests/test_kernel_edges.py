@@ -226,6 +226,41 @@ def test_absorbing_push_equals_the_calls(inject, ratio, n):
         assert n < 3000 or ca["absorbed_e"] > 0
 
 
+@pytest.mark.parametrize("nodes,n,steady,magnetic", [
+    (5, 400, "NO", 0.0), (17, 16 * 289 - 1, "NO", 0.0), (17, 16 * 289, "YES", 0.02), (17, 1500001, "NO", 0.0),
+    (65, 16 * 4225, "NO", 0.02), (129, 16 * 16641, "YES", 0.0), (129, 400003, "NO", 0.0), (257, 1100003, "NO", 0.0)])
+def test_unsorted_push_through_the_whole_grid_equals_the_calls(nodes, n, steady, magnetic):
+    """A run without sort deposits through windows of the whole grid from 16
+    particles a node; gather_push and deposit, call by call, take other
+    kernels.  Weights of every kind, sums that wrap 32 bits on the smallest
+    grids, injection on the way."""
+    p = picgb.make_params(X_NO_OF_CELLS=nodes, STEADYSTATE=steady, MAGNETIC_FIELD=magnetic, RAND_SEED=2, POISSON="DST_DC",
+                          DC_MAX_ITERS=2, NUMBER_TO_INJECT=0 if steady == "YES" else 17)
+    state = plasma(p, n, nodes + n, lo=0.0, hi=1.0)
+    for a in state:
+        a[:, 5] = np.random.default_rng(n).choice([1.0, 1.0, 1.98, 0.25, 2.5, 0.0, -0.5], n)
+    with loaded(p, state) as a, loaded(p, state) as b:
+        a.initial_boundary()
+        b.initial_boundary()
+        for t in range(3):
+            a.step(1)
+            b.set_time_step(t)
+            b.inject()
+            b.gather_push(0)
+            b.gather_push(1)
+            b.boundary(picgb.PGB_BOUNDARY_IONS)
+            b.boundary(picgb.PGB_BOUNDARY_ELECTRONS)
+            if steady == "NO":
+                b.contain_growth(0)
+                b.contain_growth(1)
+            b.deposit(1)
+            b.deposit(0)
+            b.grid_rho()
+            b.poisson(t)
+            b.efield()
+            assert_same(end_state(a), end_state(b), t)
+
+
 @pytest.mark.parametrize("nodes,n", [(33, 6001), (129, 300007)])
 def test_push_items_do_not_depend_on_the_launch(nodes, n):
     """More items than blocks, and blocks without an item: any grid of the

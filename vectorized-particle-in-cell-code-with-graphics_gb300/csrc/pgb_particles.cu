@@ -97,7 +97,7 @@ __device__ __forceinline__ void gather_push_one(const PushConsts& pc, const floa
 #define MCC_SCATTER 1
 #define MCC_IONIZE 2
 /* |v|^2 with its roundings spelled out: the collision test and the
- * scattering kernel must derive the same energy from the same velocity */
+ * scatterings must derive the same energy from the same velocity        */
 __device__ __forceinline__ float speed2(const float4& p, float vz) {
     return __fmaf_rn(vz, vz, __fmaf_rn(p.w, p.w, __fmul_rn(p.z, p.z)));
 }
@@ -189,7 +189,7 @@ __device__ __forceinline__ void flush_stats(int (&st)[2], long long* stats, long
  * tile*TILE + k*THREADS + t, so word k*warps + w of the tile (the ballot of
  * warp w's item k) holds its slots in slot order, and the words in order
  * are the tile's list.  The tile's count goes through a shared counter:
- * one barrier per tile, and no scan (k_gather_lists expands the words).
+ * one barrier per tile, and no scan (k_build_list expands the words).
  * s_cnt: two shared counters, zero at the kernel's start, used by turns
  * (it counts the calls of the block), so that a block's next tile can
  * count while thread 0 reads and clears this one's after the barrier.   */
@@ -255,9 +255,25 @@ __device__ __forceinline__ void deposit_win(unsigned long long* qacc, unsigned i
     }
 }
 
+/* the same into a window of the whole grid, whose sums may wrap: pgb_deposit.cuh */
+__device__ __forceinline__ void deposit_whole(unsigned long long* qacc, unsigned int* win, int nx, int ny, int ps,
+                                              float xs, float ys, float w) {
+    if ((unsigned)__float_as_int(w) >= (unsigned)__float_as_int(WIN_MAX_WEIGHT)) {
+        deposit_cell(qacc, nx, ps, xs, ys, w);
+        return;
+    }
+    const DepWindow W{win, 0, 0, nx, ny, true};
+    const int k = (pbits(ys) >> ps) * nx + (pbits(xs) >> ps);
+    const float wj = pfrac(xs, ps), wk = pfrac(ys, ps), wS = w * PGB_FIX_SCALE_F;
+    dep_add(W, qacc, nx, k, (1.0f - wj) * (1.0f - wk), wS);
+    dep_add(W, qacc, nx, k + 1, wj * (1.0f - wk), wS);
+    dep_add(W, qacc, nx, k + nx, wk * (1.0f - wj), wS);
+    dep_add(W, qacc, nx, k + nx + 1, wj * wk, wS);
+}
+
 /* ABSORB: a particle that leaves is removed here (and counted), where the
  * walls would do nothing else with it; else its tile's wall list is made */
-template <bool DEP, bool ABSORB>
+template <bool DEP, bool ABSORB, bool WHOLE>
 __device__ __forceinline__ void push_tile(const PushArgs& a, const PushConsts& pc, int tile, long long n,
                                           unsigned int* win, int ox, int oy, int* s_cnt, int& it, int& gone) {
     const long long base = (long long)tile * PGB_TILE;
@@ -289,7 +305,8 @@ __device__ __forceinline__ void push_tile(const PushArgs& a, const PushConsts& p
         gather_push_one(pc, a.exy, p[k], vz[k], moved);
         /* inside the deposit region it is outside no wall */
         if (deposit_ok(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps)) {
-            if (DEP) deposit_win(a.qacc, win, ox, oy, pc.nx, pc.ps, p[k].x, p[k].y, w[k]);
+            if (DEP && WHOLE) deposit_whole(a.qacc, win, pc.nx, pc.ny, pc.ps, p[k].x, p[k].y, w[k]);
+            else if (DEP) deposit_win(a.qacc, win, ox, oy, pc.nx, pc.ps, p[k].x, p[k].y, w[k]);
         } else {
             f[k] = pc.steady ? outside_steady(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps)
                              : outside_absorbing(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps);
@@ -340,11 +357,13 @@ __device__ __forceinline__ void flush_window(unsigned long long* qacc, unsigned 
 }
 
 /* Work items: the bin pieces of the last sort (tiles of one bin, deposited
- * through a shared window), then every tile after the sorted region.     */
-template <bool DEP, bool ABSORB>
-__global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
+ * through a shared window), then every tile after the sorted region.
+ * WHOLE: one window of the whole grid per block, flushed at its end.     */
+template <bool DEP, bool ABSORB, bool WHOLE>
+__global__ void __launch_bounds__(PGB_PUSH_THREADS, WHOLE ? 2 : 4) k_push(PushArgs a) {
     pgb_pdl_entry();
-    __shared__ unsigned int s_win[WIN_NODES];
+    __shared__ unsigned int s_win[WHOLE ? 1 : WIN_NODES];
+    extern __shared__ __align__(16) unsigned int s_grid[];   /* WHOLE */
     const long long n = a.ds->n[a.s];
     const int ntiles = (int)((n + PGB_TILE - 1) / PGB_TILE);
     const int npieces = a.ds->n_pieces[a.s];
@@ -356,7 +375,9 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
     int it = 0, gone = 0;
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
     /* the window starts zeroed; each flush leaves it zeroed again */
-    if (DEP && npieces > 0)
+    if (WHOLE)
+        for (int k = threadIdx.x; k < pc.nx * pc.ny; k += blockDim.x) s_grid[k] = 0u;
+    else if (DEP && npieces > 0)
         for (int k = threadIdx.x; k < WIN_NODES; k += blockDim.x) s_win[k] = 0u;
     __syncthreads();
     /* A block's first item is its own; where there are more items than
@@ -372,24 +393,34 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, 4) k_push(PushArgs a) {
             int4 pc4 = a.pieces[item];
             unsigned int* win = nullptr;
             int ox = 0, oy = 0;
-            if (DEP && pc4.z >= 0) {
+            if (WHOLE) {
+                win = s_grid;
+            } else if (DEP && pc4.z >= 0) {
                 win = s_win;
                 ox = (pc4.z % a.nbx) * PGB_BIN - PGB_HALO;
                 oy = (pc4.z / a.nbx) * PGB_BIN - PGB_HALO;
             }
             for (int t = pc4.x; t < pc4.x + pc4.y && t < ntiles; ++t)
-                push_tile<DEP, ABSORB>(a, pc, t, n, win, ox, oy, s_cnt, it, gone);
-            if (win) {
+                push_tile<DEP, ABSORB, WHOLE>(a, pc, t, n, win, ox, oy, s_cnt, it, gone);
+            if (!WHOLE && win) {
                 __syncthreads();
                 flush_window(a.qacc, s_win, ox, oy, pc.nx, pc.ny);
                 __syncthreads();
             }
         } else {
-            push_tile<DEP, ABSORB>(a, pc, tile0 + (item - npieces), n, nullptr, 0, 0, s_cnt, it, gone);
+            push_tile<DEP, ABSORB, WHOLE>(a, pc, tile0 + (item - npieces), n, WHOLE ? s_grid : nullptr, 0, 0, s_cnt, it, gone);
         }
         if (!more) break;
         __syncthreads();   /* the next item is there, and the other word is free */
         item = s_item[turn];
+    }
+    if (WHOLE) {
+        __syncthreads();
+        for (int row = threadIdx.x >> 5; row < pc.ny; row += PGB_PUSH_THREADS / 32)
+            for (int c = threadIdx.x & 31; c < pc.nx; c += 32) {
+                const unsigned int v = s_grid[row * pc.nx + c];
+                if (v) atomicAdd(a.qacc + (long long)row * pc.nx + c, (unsigned long long)v);
+            }
     }
     /* the last block to get here puts the counter back */
     if (more && threadIdx.x == 0 && atomicAdd(&a.ds->work_done[a.s], 1) == (int)gridDim.x - 1) {
@@ -1206,11 +1237,30 @@ static PushArgs push_args(pgb_run* r, int s) {
     return a;
 }
 
+/* Whether a push deposits through a window of the whole grid: runs that do
+ * not sort (a sorted one's pieces have small windows), on grids of which a
+ * window fits, from 16 particles a node, where one block per SM (two, if
+ * the window leaves room) still adds fewer times to L2 than the particles
+ * themselves would.  Both ways add the same integers.  A step of an argon
+ * run without sort, straight / window: 17^2 nodes, 1 Mi particles a species
+ * 934 / 54 us; 33^2, 300 K 93 / 41; 65^2, 60 K 37 / 35, 300 K 59 / 46, 4 M
+ * 467 / 164; 129^2, 150 K 42 / 43, 300 K 53 / 52, 1 M 114 / 85, 4 M 385 /
+ * 242.  The count is the host's latest; it is no part of the result.      */
+static bool push_whole(const pgb_run* r, int s) {
+    const long long nodes = (long long)r->nx * r->ny;
+    return r->p.sort_interval == 0 && nodes <= DEP_NODES && r->hs->n[s] >= 16 * nodes;
+}
 int pgb_launch_push(pgb_run* r, int s, bool deposit, bool absorb) {
     PushArgs a = push_args(r, s);
-    int g = grid_for(r, r->tune_push_per_sm);
-    void (*kp)(PushArgs) = !deposit ? k_push<false, false> : absorb ? k_push<true, true> : k_push<true, false>;
-    PGB_CK(r, pgb_launch_pdl(kp, dim3(g), dim3(PGB_PUSH_THREADS), 0, r->stream, a));
+    if (deposit && push_whole(r, s)) {
+        void (*kp)(PushArgs) = absorb ? k_push<true, true, true> : k_push<true, false, true>;
+        const size_t smem = sizeof(unsigned int) * r->nx * r->ny;
+        PGB_CK(r, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEP_SMEM));
+        PGB_CK(r, pgb_launch_pdl(kp, dim3(grid_for(r, smem > 48 * 1024 ? 1 : 2)), dim3(PGB_PUSH_THREADS), smem, r->stream, a));
+    } else {
+        void (*kp)(PushArgs) = !deposit ? k_push<false, false, false> : absorb ? k_push<true, true, false> : k_push<true, false, false>;
+        PGB_CK(r, pgb_launch_pdl(kp, dim3(grid_for(r, r->tune_push_per_sm)), dim3(PGB_PUSH_THREADS), 0, r->stream, a));
+    }
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;
