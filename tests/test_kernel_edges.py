@@ -230,9 +230,9 @@ def test_absorbing_push_equals_the_calls(inject, ratio, n):
     (5, 400, "NO", 0.0), (17, 16 * 289 - 1, "NO", 0.0), (17, 16 * 289, "YES", 0.02), (17, 1500001, "NO", 0.0),
     (65, 16 * 4225, "NO", 0.02), (129, 16 * 16641, "YES", 0.0), (129, 400003, "NO", 0.0), (257, 1100003, "NO", 0.0)])
 def test_unsorted_push_through_the_whole_grid_equals_the_calls(nodes, n, steady, magnetic):
-    """A run without sort deposits through windows of the whole grid from 16
-    particles a node; gather_push and deposit, call by call, take other
-    kernels.  Weights of every kind, sums that wrap 32 bits on the smallest
+    """A run without sort deposits through windows of the whole grid up to 65
+    nodes a side and from 16 particles a node, else two lanes to a particle;
+    gather_push and deposit, call by call, take other kernels.  Weights of every kind, sums that wrap 32 bits on the smallest
     grids, injection on the way."""
     p = picgb.make_params(X_NO_OF_CELLS=nodes, STEADYSTATE=steady, MAGNETIC_FIELD=magnetic, RAND_SEED=2, POISSON="DST_DC",
                           DC_MAX_ITERS=2, NUMBER_TO_INJECT=0 if steady == "YES" else 17)

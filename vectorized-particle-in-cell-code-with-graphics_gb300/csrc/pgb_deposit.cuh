@@ -64,6 +64,39 @@ __device__ __forceinline__ void dep_add(const DepWindow& W, unsigned long long* 
     }
 }
 
+/* The deposits of a warp's particles (`ok` ones) straight to the grid, two
+ * lanes to a particle: a lane adds to one column's two nodes of its own
+ * particle and of its neighbour's, so that the two nodes of a row, which
+ * mostly share a sector, go to L2 as one request (all 32 lanes call it).
+ * With four adds of its own per lane, unsorted argon runs took per step:
+ * 257^2 nodes, 300 K particles a species 55 us, now 49, 4 M 308, now 243;
+ * 513^2, 8 M 550, now 466.                                               */
+__device__ __forceinline__ void deposit_pairs(unsigned long long* qacc, int nx, int ps, bool ok, float xs, float ys,
+                                              float w) {
+    if (ok && !(w >= 0.0f && w < 1.99f)) {
+        deposit_cell(qacc, nx, ps, xs, ys, w);
+        ok = false;
+    }
+    const bool odd = threadIdx.x & 1;
+    const float wj = pfrac(xs, ps), wk = pfrac(ys, ps), wS = w * PGB_FIX_SCALE_F;
+    const unsigned v0 = round_small(__fmul_rn((1.0f - wj) * (1.0f - wk), wS)), v1 = round_small(__fmul_rn(wj * (1.0f - wk), wS));
+    const unsigned v2 = round_small(__fmul_rn(wk * (1.0f - wj), wS)), v3 = round_small(__fmul_rn(wj * wk, wS));
+    const int k = ok ? (pbits(ys) >> ps) * nx + (pbits(xs) >> ps) : -1;
+    const int ko = __shfl_xor_sync(0xffffffffu, k, 1);
+    const unsigned a = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1), b = __shfl_xor_sync(0xffffffffu, odd ? v2 : v3, 1);
+    /* even lanes take the left column, odd lanes the right one */
+    unsigned long long* const q = qacc + (odd ? 1 : 0);
+    const int ke = odd ? ko : k, kd = odd ? k : ko;   /* the even and the odd lane's particle */
+    if (ke >= 0) {
+        atomicAdd(q + ke, (unsigned long long)(odd ? a : v0));
+        atomicAdd(q + ke + nx, (unsigned long long)(odd ? b : v2));
+    }
+    if (kd >= 0) {
+        atomicAdd(q + kd, (unsigned long long)(odd ? v1 : a));
+        atomicAdd(q + kd + nx, (unsigned long long)(odd ? v3 : b));
+    }
+}
+
 /* All particles i in [0, n) of src, which returns a particle's fixed-point
  * position lanes and weight (a dead one where it has none).  Blocks of
  * DEP_THREADS; a block takes a run of consecutive particles.             */
@@ -136,13 +169,14 @@ __device__ __forceinline__ void deposit_windows(const Src& src, long long n, int
                 if (W.live) dep_zero(W);
             }
         }
+        if (!W.live) {
+#pragma unroll
+            for (int q = 0; q < DEP_ITEMS; ++q) deposit_pairs(acc, nx, ps, ok[q], x[q], y[q], w[q]);
+            continue;
+        }
 #pragma unroll
         for (int q = 0; q < DEP_ITEMS; ++q) {
             if (!ok[q]) continue;
-            if (!W.live) {
-                deposit_cell(acc, nx, ps, x[q], y[q], w[q]);
-                continue;
-            }
             const int k = ((pbits(y[q]) >> ps) - W.oy) * W.nx + (pbits(x[q]) >> ps) - W.ox;
             const float wj = pfrac(x[q], ps), wk = pfrac(y[q], ps), wS = w[q] * PGB_FIX_SCALE_F;
             dep_add(W, acc, nx, k, (1.0f - wj) * (1.0f - wk), wS);

@@ -235,7 +235,7 @@ __device__ __forceinline__ void deposit_win(unsigned long long* qacc, unsigned i
     const int jp = pbits(xs) >> ps, kp = pbits(ys) >> ps;
     const int lx = jp - ox, ly = kp - oy;
     /* 0 <= w < WIN_MAX_WEIGHT: such floats order as their bits, others' are above */
-    if (win && (unsigned)lx < (unsigned)(PGB_WIN - 1) && (unsigned)ly < (unsigned)(PGB_WIN - 1) &&
+    if ((unsigned)lx < (unsigned)(PGB_WIN - 1) && (unsigned)ly < (unsigned)(PGB_WIN - 1) &&
         (unsigned)__float_as_int(w) < (unsigned)__float_as_int(WIN_MAX_WEIGHT)) {
         float wj = pfrac(xs, ps), wk = pfrac(ys, ps);
         float a4 = (1.0f - wj) * (1.0f - wk), a3 = wj * (1.0f - wk);
@@ -299,25 +299,29 @@ __device__ __forceinline__ void push_tile(const PushArgs& a, const PushConsts& p
 #pragma unroll
     for (int k = 0; k < PGB_ITEMS; ++k) {
         f[k] = false;
+        bool straight = false;   /* deposits straight to the grid */
         const int o = k * PGB_PUSH_THREADS + threadIdx.x;
-        if (is_dead(p[k].x)) continue;
-        bool moved;
-        gather_push_one(pc, a.exy, p[k], vz[k], moved);
-        /* inside the deposit region it is outside no wall */
-        if (deposit_ok(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps)) {
-            if (DEP && WHOLE) deposit_whole(a.qacc, win, pc.nx, pc.ny, pc.ps, p[k].x, p[k].y, w[k]);
-            else if (DEP) deposit_win(a.qacc, win, ox, oy, pc.nx, pc.ps, p[k].x, p[k].y, w[k]);
-        } else {
-            f[k] = pc.steady ? outside_steady(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps)
-                             : outside_absorbing(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps);
-            if (ABSORB && f[k]) {
-                p[k].x = pos_dead();
-                gone++;
-                moved = true;
+        if (!is_dead(p[k].x)) {
+            bool moved;
+            gather_push_one(pc, a.exy, p[k], vz[k], moved);
+            /* inside the deposit region it is outside no wall */
+            if (deposit_ok(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps)) {
+                if (DEP && WHOLE) deposit_whole(a.qacc, win, pc.nx, pc.ny, pc.ps, p[k].x, p[k].y, w[k]);
+                else if (DEP && win) deposit_win(a.qacc, win, ox, oy, pc.nx, pc.ps, p[k].x, p[k].y, w[k]);
+                else straight = true;
+            } else {
+                f[k] = pc.steady ? outside_steady(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps)
+                                 : outside_absorbing(p[k].x, p[k].y, pc.nx, pc.ny, pc.ps);
+                if (ABSORB && f[k]) {
+                    p[k].x = pos_dead();
+                    gone++;
+                    moved = true;
+                }
             }
+            if (moved) xv[o] = p[k];
+            if (pc.bfield && moved) a.vz[base + o] = vz[k];
         }
-        if (moved) xv[o] = p[k];
-        if (pc.bfield && moved) a.vz[base + o] = vz[k];
+        if (DEP && !WHOLE && !win) deposit_pairs(a.qacc, pc.nx, pc.ps, straight, p[k].x, p[k].y, w[k]);
     }
     if (!ABSORB) tile_masks(f, tile, (unsigned*)a.tl_out, a.tc_out, s_cnt, it);
 }
@@ -1238,25 +1242,24 @@ static PushArgs push_args(pgb_run* r, int s) {
 }
 
 /* Whether a push deposits through a window of the whole grid: runs that do
- * not sort (a sorted one's pieces have small windows), on grids of which a
- * window fits, from 16 particles a node, where one block per SM (two, if
- * the window leaves room) still adds fewer times to L2 than the particles
- * themselves would.  Both ways add the same integers.  A step of an argon
- * run without sort, straight / window: 17^2 nodes, 1 Mi particles a species
- * 934 / 54 us; 33^2, 300 K 93 / 41; 65^2, 60 K 37 / 35, 300 K 59 / 46, 4 M
- * 467 / 164; 129^2, 150 K 42 / 43, 300 K 53 / 52, 1 M 114 / 85, 4 M 385 /
- * 242.  The count is the host's latest; it is no part of the result.      */
+ * not sort (a sorted one's pieces have small windows), on grids of which
+ * two windows fit on an SM beside L1 (65 nodes a side), from 16 particles a
+ * node.  Both ways add the same integers.  A step of an argon run without
+ * sort, straight (deposit_pairs) / window: 17^2 nodes, 1 M particles a
+ * species 648 / 54 us; 33^2, 30 K 33 / 33, 300 K 68 / 41; 65^2, 60 K 35 / 35,
+ * 150 K 39 / 37, 1 M 91 / 62, 4 M 307 / 163.  129^2, with one window per SM:
+ * 300 K 45 / 52, 1 M 83 / 85, 4 M 256 / 243.  The count is the host's latest;
+ * it is no part of the result.                                            */
 static bool push_whole(const pgb_run* r, int s) {
     const long long nodes = (long long)r->nx * r->ny;
-    return r->p.sort_interval == 0 && nodes <= DEP_NODES && r->hs->n[s] >= 16 * nodes;
+    return r->p.sort_interval == 0 && nodes * 4 <= 48 * 1024 && r->hs->n[s] >= 16 * nodes;
 }
 int pgb_launch_push(pgb_run* r, int s, bool deposit, bool absorb) {
     PushArgs a = push_args(r, s);
     if (deposit && push_whole(r, s)) {
         void (*kp)(PushArgs) = absorb ? k_push<true, true, true> : k_push<true, false, true>;
         const size_t smem = sizeof(unsigned int) * r->nx * r->ny;
-        PGB_CK(r, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEP_SMEM));
-        PGB_CK(r, pgb_launch_pdl(kp, dim3(grid_for(r, smem > 48 * 1024 ? 1 : 2)), dim3(PGB_PUSH_THREADS), smem, r->stream, a));
+        PGB_CK(r, pgb_launch_pdl(kp, dim3(grid_for(r, 2)), dim3(PGB_PUSH_THREADS), smem, r->stream, a));
     } else {
         void (*kp)(PushArgs) = !deposit ? k_push<false, false, false> : absorb ? k_push<true, true, false> : k_push<true, false, false>;
         PGB_CK(r, pgb_launch_pdl(kp, dim3(grid_for(r, r->tune_push_per_sm)), dim3(PGB_PUSH_THREADS), 0, r->stream, a));

@@ -54,8 +54,9 @@ namespace {
  * are shared: from eight records per node and 4096 in all, and from 128 Ki
  * on any grid.  Measured, straight / through windows: 17^2 nodes, 65 Ki
  * records 46.8 / 12.0 us; 65^2, 65 Ki 12.7 / 12.6; 129^2, 65 Ki 11.1 / 14.9;
- * 513^2, 65 Ki 12.8 / 17.7, 6 M in bins 437 / 132 (the latter with the
- * positions in integer arithmetic on one side only).                     */
+ * 513^2, 65 Ki 12.8 / 17.7.  Straight with a division per position: 513^2,
+ * 150 K 25.6, now 15.9, 6 M in random order 437, now 164, in bins 437, now
+ * 115.                                                                   */
 inline bool static_windows(int64_t n, int64_t nodes) { return n >= 4096 && (n >= 8 * nodes || n >= 131072); }
 
 struct DeviceSetup {
@@ -91,11 +92,10 @@ struct RecordSource {
 __global__ void __launch_bounds__(256) k_static_deposit_few(RecordSource src, long long n, int nx, int ny,
                                                             unsigned long long* acc) {
     pgb_pdl_entry();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        float x, y, w;
-        src(i, x, y, w);
-        if (deposit_ok(x, y, nx, ny, src.ps)) deposit_cell(acc, nx, src.ps, x, y, w);
-    }
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    float x = pos_dead(), y = pos_dead(), w = 0.0f;
+    if (i < n) src(i, x, y, w);
+    deposit_pairs(acc, nx, src.ps, deposit_ok(x, y, nx, ny, src.ps), x, y, w);
 }
 __global__ void __launch_bounds__(DEP_THREADS) k_static_deposit(RecordSource src, long long n, int nx, int ny,
                                                                 unsigned long long* acc) {
