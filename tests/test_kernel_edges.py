@@ -195,6 +195,23 @@ def test_converged_modes_at_every_depth(mode, n, bound):
             assert np.max(np.abs(a - b)) <= bound * np.max(np.abs(b)), grid
 
 
+@pytest.mark.parametrize("n", [513, 1025])
+def test_two_converged_solvers_agree_on_large_grids(n):
+    """The sine transforms against the multigrid's tiles (1025 nodes are the
+    most that a run takes): both are the discrete solution, up to FP64
+    rounding of the residual, 2e-16 n^2 / pi^2 of phi = 2e-11 at 1025; bound
+    1e-9."""
+    rho = 1e-6 * np.random.default_rng(n).standard_normal((n, n))
+    phi = []
+    for mode, passes in (("DST_DC", 3), ("FP32_DC", 28)):
+        p = picgb.make_params(X_NO_OF_CELLS=n, POISSON=mode, DC_MAX_ITERS=passes, DC_TOLERANCE=0.0, PHI_RIGHT=1.5)
+        with picgb.Run(p) as r:
+            r.set_rho(rho)
+            r.poisson(0)
+            phi.append(r.get_grid("phi"))
+    assert np.max(np.abs(phi[0] - phi[1])) <= 1e-9 * np.max(np.abs(phi[1]))
+
+
 # -------------------------------------------------------------------- steps
 @pytest.mark.parametrize("inject,ratio,n", [(0, 1.0, 1), (1, 2.0, 257), (40, 1.0, 5000), (4096, 2.0, 3000), (4097, 1.0, 3000)])
 def test_absorbing_push_equals_the_calls(inject, ratio, n):
