@@ -58,13 +58,15 @@ __device__ __forceinline__ uint32_t rd_hash(uint32_t id, uint32_t seed) {
     return x;
 }
 
-/* in the sample: all particles when max_points <= 0 or n <= max_points,
- * else hash < max_points/n of the 32-bit range                          */
-__device__ __forceinline__ bool rd_keep(uint32_t id, uint32_t seed, long long nlive, int max_points) {
-    if (max_points <= 0 || nlive <= max_points) return true;
-    const unsigned long long thresh = (unsigned long long)((double)max_points / (double)nlive * 4294967296.0);
-    return (unsigned long long)rd_hash(id, seed) < thresh;
-}
+/* the sample: all particles when max_points <= 0 or n <= max_points, else
+ * those with hash < max_points/n of the 32-bit range                     */
+struct RdSample {
+    bool all;
+    unsigned long long thresh;
+    __device__ __forceinline__ RdSample(int max_points, long long nlive)
+        : all(max_points <= 0 || nlive <= max_points),
+          thresh(all ? 0ull : (unsigned long long)((double)max_points / (double)nlive * 4294967296.0)) {}
+};
 
 struct PointArgs {
     const float4* xv;
@@ -89,36 +91,47 @@ __device__ __forceinline__ long long rd_tile(long long t, long long ntiles) {
 }
 
 /* p.x, p.y: the position in FP32 cells (NaN for a NaN position) */
-__device__ __forceinline__ bool rd_candidate(const PointArgs& a, long long i, long long nlive, float4& p) {
+__device__ __forceinline__ bool rd_candidate(const PointArgs& a, float4& p) {
     if (is_dead(p.x)) return false;
     p.x = pos_cellsf(p.x, a.ps);
     p.y = pos_cellsf(p.y, a.ps);
-    if (!(p.x > 0.0f && p.x < (float)(a.nx - 1) && p.y > 0.0f && p.y < (float)(a.ny - 1))) return false;
-    if (a.max_points <= 0 || nlive <= a.max_points) return true;
-    return rd_keep(a.id[i], a.seed, nlive, a.max_points);
+    return p.x > 0.0f && p.x < (float)(a.nx - 1) && p.y > 0.0f && p.y < (float)(a.ny - 1);
 }
-/* f(i, particle) for the block's tiles; a thread's items load together */
+/* f(particle) for the sampled slots of the block's tiles; a thread's items
+ * load together.  A sample is decided by the ids alone (4 B a slot), and
+ * only its particles are read: 5000 of 2 x 16 M drawn at 1024^2 pixels took
+ * 240 us when the ids were read after the positions, now 141 (all 253).  */
 template <class F>
-__device__ __forceinline__ void rd_particles(const PointArgs& a, long long n, F f) {
+__device__ __forceinline__ void rd_particles(const PointArgs& a, long long n, long long nlive, F f) {
     const long long ntiles = (n + RD_TILE - 1) / RD_TILE;
+    const RdSample smp(a.max_points, nlive);
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const long long base = rd_tile(t, ntiles) * RD_TILE;
         float4 p[RD_TILE / RD_THREADS];
+        unsigned int id[RD_TILE / RD_THREADS];
+        if (!smp.all) {
+#pragma unroll
+            for (int q = 0; q < RD_TILE / RD_THREADS; ++q) {
+                const long long i = base + q * RD_THREADS + threadIdx.x;
+                id[q] = i < n ? a.id[i] : 0u;
+            }
+        }
 #pragma unroll
         for (int q = 0; q < RD_TILE / RD_THREADS; ++q) {
             const long long i = base + q * RD_THREADS + threadIdx.x;
-            p[q] = i < n ? a.xv[i] : make_float4(pos_dead(), 0.0f, 0.0f, 0.0f);
+            const bool keep = i < n && (smp.all || (unsigned long long)rd_hash(id[q], a.seed) < smp.thresh);
+            p[q] = keep ? a.xv[i] : make_float4(pos_dead(), 0.0f, 0.0f, 0.0f);
         }
 #pragma unroll
-        for (int q = 0; q < RD_TILE / RD_THREADS; ++q) f(base + q * RD_THREADS + threadIdx.x, p[q]);
+        for (int q = 0; q < RD_TILE / RD_THREADS; ++q) f(p[q]);
     }
 }
 
 __global__ void __launch_bounds__(RD_THREADS) k_rd_vmax(PointArgs a) {
     const long long n = a.ds->n[a.s], nlive = n - a.ds->dead[a.s];
     unsigned int mx = 0u, my = 0u;
-    rd_particles(a, n, [&](long long i, float4 p) {
-        if (!rd_candidate(a, i, nlive, p)) return;
+    rd_particles(a, n, nlive, [&](float4 p) {
+        if (!rd_candidate(a, p)) return;
         const float ax = fabsf(p.z), ay = fabsf(p.w);
         if (ax == ax) mx = max(mx, __float_as_uint(ax));   /* non-negative floats order as their bits */
         if (ay == ay) my = max(my, __float_as_uint(ay));
@@ -198,8 +211,8 @@ __global__ void __launch_bounds__(RD_THREADS) k_rd_points(PointArgs a) {
         for (int k = threadIdx.x; k < a.words; k += RD_THREADS) s_layer[k] = 0u;
         __syncthreads();
     }
-    rd_particles(a, n, [&](long long i, float4 p) {
-        if (!rd_candidate(a, i, nlive, p)) return;
+    rd_particles(a, n, nlive, [&](float4 p) {
+        if (!rd_candidate(a, p)) return;
         float fx, fy;
         if (a.phase) {
             if (!(fabsf(p.z) < (float)mvx && fabsf(p.w) < (float)mvy)) return;
