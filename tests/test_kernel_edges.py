@@ -85,9 +85,9 @@ def deposit_reference(a, n, d, qc):
 
 
 @pytest.mark.parametrize("nodes,n,order", [
-    (17, 1, "random"), (17, 4095, "random"), (17, 4096, "random"), (33, 8711, "random"), (33, 8712, "random"),
-    (65, 2048 * 17 + 1, "binned"), (129, 131071, "random"), (129, 133128, "random"), (257, 131071, "binned"),
-    (257, 131072, "binned"), (257, 131073, "random"), (513, 200003, "binned"), (513, 200003, "random"),
+    (17, 1, "random"), (17, 8191, "random"), (17, 8192, "random"), (33, 17423, "random"), (33, 17424, "random"),
+    (65, 2048 * 33 + 1, "binned"), (129, 266255, "random"), (129, 266256, "random"), (257, 1056784, "binned"),
+    (257, 1056785, "random"), (513, 200003, "binned"), (513, 200003, "random"),
     (17, 2000003, "one node")])
 def test_deposit_windows_add_the_exact_integers(lib, nodes, n, order):
     """pgb_deposit_static and pgb_deposit on both sides of the rule that picks

@@ -25,6 +25,16 @@
 #define DEP_SMEM (DEP_NODES * sizeof(unsigned int))
 #define DEP_BLOCKS_PER_SM 3
 
+/* Windows pay for their zeroing, their flush and fewer blocks in flight from
+ * 16 particles a node (8192 in all): straight (deposit_pairs) / windows, the
+ * kernel alone, 17^2 nodes, 5000 particles 4.0 / 5.5 us, 20 K 9.6 / 5.6;
+ * 65^2, 50 K 4.8 / 7.2, 131 K 7.5 / 7.4, 1 M 34 / 12; 129^2, 300 K 9.8 / 11.6,
+ * 1 M 27 / 18.  On larger grids they pay if the particles come binned, which
+ * the caller of a large deposit mostly has them: records, 257^2, 1 M 23 / 29
+ * in random order and 27 / 21 in bins, 6 M 119 / 163 and 226 / 104; 513^2,
+ * 2.5 M 48 / 68 and 55 / 58, 6 M 102 / 159 and 158 / 113.                 */
+inline bool deposit_through_windows(int64_t n, int64_t nodes) { return n >= 8192 && n >= 16 * nodes; }
+
 struct DepWindow {
     unsigned int* w;
     int ox, oy, nx, ny;   /* first node, nodes a row, rows */

@@ -387,8 +387,9 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, WHOLE ? 2 : 4) k_push(PushAr
     /* A block's first item is its own; where there are more items than
      * blocks, the others come from a counter: a fixed share of the pieces
      * left the SMs between 75 and 117% of their mean work (4 Mi electrons at
-     * 513^2).  The next item is fetched while the present one is in work.  */
-    const bool more = nitems > (int)gridDim.x;
+     * 513^2).  The next item is fetched while the present one is in work.
+     * Without pieces the items are single tiles, alike, and shared out.    */
+    const bool more = npieces > 0 && nitems > (int)gridDim.x;
     __shared__ int s_item[2];
     int turn = 0;
     for (int item = blockIdx.x; item < nitems; turn ^= 1) {
@@ -414,7 +415,10 @@ __global__ void __launch_bounds__(PGB_PUSH_THREADS, WHOLE ? 2 : 4) k_push(PushAr
         } else {
             push_tile<DEP, ABSORB, WHOLE>(a, pc, tile0 + (item - npieces), n, WHOLE ? s_grid : nullptr, 0, 0, s_cnt, it, gone);
         }
-        if (!more) break;
+        if (!more) {
+            item += gridDim.x;
+            continue;
+        }
         __syncthreads();   /* the next item is there, and the other word is free */
         item = s_item[turn];
     }
@@ -477,6 +481,18 @@ struct SlotSource {
         wt = w[i];
     }
 };
+/* few particles for the grid: a thread each, straight to the accumulator */
+__global__ void __launch_bounds__(256) k_deposit_few(SlotSource src, const DevState* ds, int s, int nx, int ny, int ps,
+                                                     unsigned long long* qacc) {
+    pgb_pdl_entry();
+    const long long n = ds->n[s];
+    for (long long base = blockIdx.x * 256ll; base < n; base += gridDim.x * 256ll) {
+        const long long i = base + threadIdx.x;
+        float x = pos_dead(), y = pos_dead(), w = 0.0f;
+        if (i < n) src(i, x, y, w);
+        deposit_pairs(qacc, nx, ps, deposit_ok(x, y, nx, ny, ps), x, y, w);
+    }
+}
 __global__ void __launch_bounds__(DEP_THREADS) k_deposit(SlotSource src, DevState* ds, int s, int nx, int ny, int ps,
                                                          unsigned long long* qacc) {
     pgb_pdl_entry();
@@ -1312,9 +1328,17 @@ int pgb_build_list(pgb_run* r, int which, int s, int commit) {
 }
 
 int pgb_launch_deposit(pgb_run* r, int s) {
-    PGB_CK(r, cudaFuncSetAttribute(k_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEP_SMEM));
-    PGB_CK(r, pgb_launch_pdl(k_deposit, dim3(grid_for(r, DEP_BLOCKS_PER_SM)), dim3(DEP_THREADS), DEP_SMEM, r->stream,
-                             SlotSource{r->sp[s].xv, r->sp[s].w}, r->ds, s, r->nx, r->ny, r->ps, r->qacc[s]));
+    const SlotSource src{r->sp[s].xv, r->sp[s].w};
+    const long long n = r->hs->n[s];   /* the host's latest count: it picks the kernel, no result */
+    if (deposit_through_windows(n, (long long)r->nx * r->ny)) {
+        PGB_CK(r, cudaFuncSetAttribute(k_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEP_SMEM));
+        PGB_CK(r, pgb_launch_pdl(k_deposit, dim3(grid_for(r, DEP_BLOCKS_PER_SM)), dim3(DEP_THREADS), DEP_SMEM, r->stream,
+                                 src, r->ds, s, r->nx, r->ny, r->ps, r->qacc[s]));
+    } else {
+        const long long blocks = std::min<long long>(std::max<long long>((n + 255) / 256, 1), grid_for(r, 8));
+        PGB_CK(r, pgb_launch_pdl(k_deposit_few, dim3((unsigned)blocks), dim3(256), 0, r->stream, src, (const DevState*)r->ds,
+                                 s, r->nx, r->ny, r->ps, r->qacc[s]));
+    }
     r->launches++;
     PGB_CK(r, cudaGetLastError());
     return 0;

@@ -50,15 +50,6 @@ static __device__ __align__(256) unsigned long long g_static_acc[PGB_STATIC_DEPO
 
 namespace {
 
-/* Windows pay (their zeroing, flush and fewer blocks in flight) where nodes
- * are shared: from eight records per node and 4096 in all, and from 128 Ki
- * on any grid.  Measured, straight / through windows: 17^2 nodes, 65 Ki
- * records 46.8 / 12.0 us; 65^2, 65 Ki 12.7 / 12.6; 129^2, 65 Ki 11.1 / 14.9;
- * 513^2, 65 Ki 12.8 / 17.7.  Straight with a division per position: 513^2,
- * 150 K 25.6, now 15.9, 6 M in random order 437, now 164, in bins 437, now
- * 115.                                                                   */
-inline bool static_windows(int64_t n, int64_t nodes) { return n >= 4096 && (n >= 8 * nodes || n >= 131072); }
-
 struct DeviceSetup {
     unsigned long long* acc = nullptr;   /* device address of g_static_acc */
     int sms = 0;
@@ -172,7 +163,7 @@ extern "C" int pgb_deposit_static(const double* d_aos6, int64_t n, int32_t nx, i
     const RecordSource src{d_aos6, dx, dy, pgb_pos_scale(dx, ps), pgb_pos_scale(dy, ps), ps};
     cudaError_t e = pgb_launch_pdl(k_static_clear, dim3(gblocks), dim3(256), 0, st, s.acc, nodes);
     if (e != cudaSuccess) return setup_error("pgb_deposit_static: kernel launch", e);
-    if (static_windows(n, nodes)) {
+    if (deposit_through_windows(n, nodes)) {
         /* a block's window is zeroed and flushed once per run of records */
         const long long want = (n + DEP_CHUNK - 1) / DEP_CHUNK;
         const int blocks = want < (long long)s.sms * DEP_BLOCKS_PER_SM ? (int)want : s.sms * DEP_BLOCKS_PER_SM;
