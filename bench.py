@@ -53,7 +53,7 @@ GRID_NODES = 513
 # library records around each kernel in a profiled pass).  B = 0 in this
 # workload, so the push neither reads nor writes vz.
 ELECTRON_KERNELS = {
-    "k_mcc": {"desc": "k_mcc (electron collision test, ionization list, scattering list)", "prof": "ms_collide_e",
+    "k_mcc": {"desc": "k_mcc (electron collision tests, scatterings, ionization words)", "prof": "ms_collide_e",
               "alg_bytes": 24, "bytes_note": "read x, y, vx, vy, vz, id (24 B); the ~5% of events write back"},
     "k_push_e": {"desc": "k_push<DEP> (electrons: gather, push, deposit, wall list)", "prof": "ms_push_e_kernel",
                  "alg_bytes": 36, "bytes_note": "read x, y, vx, vy, w (20 B); write x, y, vx, vy (16 B)"},

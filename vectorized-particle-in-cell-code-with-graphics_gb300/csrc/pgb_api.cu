@@ -2,14 +2,13 @@
  * C ABI of libpicgb (include/picgb.h): run handles, particle I/O and the
  * host-side sequencing of the per-step kernels.
  *
- * pgb_step follows pic::pic_run's loop body (pic.cpp:1069-1250) on one CUDA
- * stream without host synchronisation inside a step:
- *   electron collisions + gather + push + deposit + wall list   (one kernel)
- *   ionization products, injection (+ push of the injected electrons)
- *   [ion step] charge exchange, ion gather + push + deposit + wall list,
- *              ion walls, electron walls
- *   [other steps] ion deposit, electron walls
- *   charge -> rho -> Poisson right-hand side, full multigrid, E
+ * pgb_step follows pic::pic_run's loop body (pic.cpp:1069-1250) without
+ * host synchronisation inside a step (its parts and streams: Lanes, below):
+ *   electron collisions; [ion step] charge exchange
+ *   electron gather + push + deposit, ionization products, injection
+ *   [ion step] ion gather + push + deposit, ion walls; else ion deposit
+ *   electron walls
+ *   charge -> rho -> Poisson right-hand side, Poisson solve, E
  * The per-phase entry points run the same kernels one reference call at a
  * time.
  */
