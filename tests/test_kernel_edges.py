@@ -213,7 +213,7 @@ def test_two_converged_solvers_agree_on_large_grids(n):
 
 
 # -------------------------------------------------------------------- steps
-@pytest.mark.parametrize("inject,ratio,n", [(0, 1.0, 1), (1, 2.0, 257), (40, 1.0, 5000), (4096, 2.0, 3000), (4097, 1.0, 3000)])
+@pytest.mark.parametrize("inject,ratio,n", [(0, 1.0, 1), (1, 2.0, 257), (40, 1.0, 5000), (256, 2.0, 3000), (257, 1.0, 3000), (4500, 2.0, 3000)])
 def test_absorbing_push_equals_the_calls(inject, ratio, n):
     """pgb_step removes particles at absorbing walls in the push; the same
     step call by call builds lists for the walls.  Injection on both sides of
@@ -319,6 +319,37 @@ def test_sorts_of_different_grids_in_turn():
         r.close()
 
 
+@pytest.mark.parametrize("inject", [256, 257, 4096, 6000])
+def test_injected_electrons_join_the_wall_list_in_order(inject):
+    """Walls that emit take the new electrons that left from the list's end, in
+    slot order, and give the secondaries slots and ids by that order: one
+    step against the same step call by call, on both sides of the injection's
+    one-block size.  A time step of several cells puts many outside."""
+    p = picgb.make_params(X_NO_OF_CELLS=17, STEADYSTATE="NO", NUMBER_TO_INJECT=inject, DT_SCALE=40.0, TEMPERATURE=30.0,
+                          E_IMPACT_SEE="YES", REFLECTION="YES", BACKSCATTER="YES", RAND_SEED=9)
+    state = plasma(p, 2000, 4, temp_e=200.0)
+    with loaded(p, state) as a, loaded(p, state) as b:
+        a.initial_boundary()
+        b.initial_boundary()
+        for t in range(2):
+            a.step(1)
+            b.set_time_step(t)
+            b.inject()
+            b.gather_push(0)
+            b.gather_push(1)
+            b.boundary(picgb.PGB_BOUNDARY_IONS)
+            b.boundary(picgb.PGB_BOUNDARY_ELECTRONS)
+            b.deposit(1)
+            b.deposit(0)
+            b.grid_rho()
+            b.poisson(t)
+            b.efield()
+            assert_same(end_state(a), end_state(b), t)
+        ca, cb = a.counters(), b.counters()
+        assert {k: ca[k] for k in ca if k != "step"} == {k: cb[k] for k in cb if k != "step"}
+        assert ca["absorbed_e"] > 50
+
+
 # -------------------------------------------------------------------- walls
 @pytest.mark.parametrize("ne,ni", [(1, 1), (3, 0), (8191, 8193), (20011, 9000), (500, 30000)])
 def test_steady_walls_with_long_lists(ne, ni):
@@ -356,8 +387,9 @@ def test_steady_walls_with_long_lists(ne, ni):
                 assert np.max(np.abs(a[:, 2:5] - b[:, 2:5])) <= 1e-4 * vt
 
 
-@pytest.mark.parametrize("species,see", [("ARGON", "NO"), ("ARGON", "YES"), ("HYDROGEN", "YES")])
-def test_collisions_and_walls_in_full_queues(species, see):
+@pytest.mark.parametrize("species,see,inject", [("ARGON", "NO", 33), ("ARGON", "NO", 300), ("ARGON", "YES", 300),
+                                                ("HYDROGEN", "YES", 33)])
+def test_collisions_and_walls_in_full_queues(species, see, inject):
     """A gas so dense that most electrons collide each step, and hot particles
     that reach the walls in long lists: event counts agree with the oracle to
     1% + 2 (decisions within FP32 rounding of their threshold)."""
@@ -365,7 +397,7 @@ def test_collisions_and_walls_in_full_queues(species, see):
                           SPECIES=species, ION_MASS_AMU=1.0 if species == "HYDROGEN" else 39.948, THRESHOLD=15.75 if
                           species == "ARGON" else 13.6, SIGMA="ENERGY_DEPENDENT", SIGMA_ELASTIC="ENERGY_DEPENDENT",
                           SIGMA_IONIZATION="ENERGY_DEPENDENT", E_IMPACT_SEE=see, REFLECTION=see, BACKSCATTER=see,
-                          NUMBER_TO_INJECT=33, DTI_RATIO=2.0, SORT_INTERVAL=2)
+                          NUMBER_TO_INJECT=inject, DTI_RATIO=2.0, SORT_INTERVAL=2)
     state = plasma(p, 30011, 8, temp_e=60.0, temp_i=30.0, lo=0.0, hi=1.0)
     o = orc.Oracle(p, rng=orc.ORC_RNG_PHILOX, order=orc.ORC_ORDER_STABLE)
     with loaded(p, state) as r:

@@ -872,10 +872,12 @@ __global__ void k_inject(InjectArgs a) {
  * INJECT_BLOCK_MAX: the ids of the step's uncounted ionization products
  * first (commit), the particles, then the counts and the wall list.  Two
  * launches and the products' commit kernel in one (6.4 + 4.2 + 2.3 us ->
- * 6.5 us, ncu); each thread's work is a chain of some 2 us, so more than
- * four rounds of 1024 are better spread over blocks (k_inject).          */
-#define INJECT_BLOCK_MAX 4096
-__global__ void __launch_bounds__(1024) k_inject_block(InjectArgs a, int s, int commit) {
+ * 6.5 us, ncu).  More particles are better spread over blocks (k_inject):
+ * each one's draws and divisions keep an SM's FP64 pipe busy.  A step with
+ * one block / spread: 10 injected 70.5 / 72.0 us, 200 74.9 / 73.9, 600 84.6
+ * / 75.6, 1000 102 / 79, 4000 183 / 83.                                   */
+#define INJECT_BLOCK_MAX 256
+__global__ void __launch_bounds__(INJECT_BLOCK_MAX) k_inject_block(InjectArgs a, int s, int commit) {
     pgb_pdl_entry();
     __shared__ unsigned s_out[INJECT_BLOCK_MAX / 32];
     if (commit && threadIdx.x == 0) ionize_count_commit(a.ds, commit);
@@ -907,28 +909,47 @@ __global__ void __launch_bounds__(1024) k_inject_block(InjectArgs a, int s, int 
     a.ds->stats[s == 0 ? ST_INJ_E : ST_INJ_I] += k;
 }
 
-/* after k_inject: counts, ids, and the wall list entries of new electrons */
-__global__ void k_inject_commit(InjectArgs a) {
+/* after k_inject: counts, ids, and the wall list entries of new electrons in
+ * slot order, 1024 flags at a time (one thread took 261 us for 5000)      */
+__global__ void __launch_bounds__(1024) k_inject_commit(InjectArgs a) {
     pgb_pdl_entry();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ int s_cnt[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int s = 0; s < 2; ++s) {
         if (!(a.species_mask & (1 << s))) continue;
         const Species& S = s == 0 ? a.e : a.i;
-        long long n0 = a.ds->n[s];
+        const long long n0 = a.ds->n[s];
         int k = a.k;
         if (n0 + k > S.cap) k = (int)(S.cap - n0 > 0 ? S.cap - n0 : 0);
-        if (s == 0 && a.push_e) {
-            for (int j = 0; j < k; ++j)
-                if (a.flag[j]) {
-                    long long pos = a.ds->list_n[LIST_OUT_E];
-                    if (pos < a.list_cap) { a.list_out_e[pos] = (int)(n0 + j); a.ds->list_n[LIST_OUT_E] = pos + 1; }
-                    else a.ds->err |= ERR_LIST;
-                    a.flag[j] = 0;
+        if (s == 0 && a.push_e && !a.absorb_e) {
+            long long pos = a.ds->list_n[LIST_OUT_E];
+            for (int base = 0; base < k; base += 1024) {
+                const int j = base + threadIdx.x;
+                const bool f = j < k && a.flag[j];
+                const unsigned m = __ballot_sync(0xffffffffu, f);
+                if (lane == 0) s_cnt[warp] = __popc(m);
+                __syncthreads();
+                int before = __popc(m & ((1u << lane) - 1u)), all = 0;
+                for (int w = 0; w < 32; ++w) {
+                    if (w < warp) before += s_cnt[w];
+                    all += s_cnt[w];
                 }
+                if (f) {
+                    a.flag[j] = 0;
+                    if (pos + before < a.list_cap) a.list_out_e[pos + before] = (int)(n0 + j);
+                    else atomicOr(&a.ds->err, ERR_LIST);
+                }
+                pos += all;
+                __syncthreads();
+            }
+            if (threadIdx.x == 0) a.ds->list_n[LIST_OUT_E] = pos < a.list_cap ? pos : a.list_cap;
         }
-        a.ds->n[s] = n0 + k;
-        a.ds->next_id[s] += (unsigned int)k;
-        a.ds->stats[s == 0 ? ST_INJ_E : ST_INJ_I] += k;
+        __syncthreads();   /* every thread has read the counts */
+        if (threadIdx.x == 0) {
+            a.ds->n[s] = n0 + k;
+            a.ds->next_id[s] += (unsigned int)k;
+            a.ds->stats[s == 0 ? ST_INJ_E : ST_INJ_I] += k;
+        }
     }
 }
 
@@ -1355,7 +1376,7 @@ int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit, boo
     a.flag = r->inject_flag;
     if (a.k <= 0) return 0;
     if (a.k <= INJECT_BLOCK_MAX) {
-        const int threads = std::min(1024, (a.k + 31) & ~31);
+        const int threads = (a.k + 31) & ~31;
         for (int s = 0; s < 2; ++s)
             if (species_mask & (1 << s)) {
                 PGB_CK(r, pgb_launch_pdl(k_inject_block, dim3(1), dim3(threads), 0, r->stream, a, s, commit & (1 << s)));
@@ -1370,7 +1391,7 @@ int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit, boo
         r->launches++;
     }
     PGB_CK(r, pgb_launch_pdl(k_inject, dim3((tot + 127) / 128), dim3(128), 0, r->stream, a));
-    PGB_CK(r, pgb_launch_pdl(k_inject_commit, dim3(1), dim3(32), 0, r->stream, a));
+    PGB_CK(r, pgb_launch_pdl(k_inject_commit, dim3(1), dim3(1024), 0, r->stream, a));
     r->launches += 2;
     PGB_CK(r, cudaGetLastError());
     return 0;
