@@ -340,13 +340,14 @@ extern "C" int pgb_create(const pgb_params* p, pgb_run** out) {
      * kernels get SMs ahead of queued blocks of the other two.            */
     {
         int prio_lo = 0, prio_hi = 0;
-        cudaEvent_t* const evs[5] = {&r->ev_fork, &r->ev_join, &r->ev_i0, &r->ev_i1, &r->ev_e0};
+        cudaEvent_t* const evs[] = {&r->ev_fork, &r->ev_join, &r->ev_i0, &r->ev_i1, &r->ev_i2, &r->ev_e0};
+        const int all = sizeof evs / sizeof evs[0];
         int made = 0;
         if (cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) == cudaSuccess &&
             cudaStreamCreateWithPriority(&r->side, cudaStreamNonBlocking, prio_hi) == cudaSuccess &&
             cudaStreamCreateWithFlags(&r->ion, cudaStreamNonBlocking) == cudaSuccess)
-            while (made < 5 && cudaEventCreateWithFlags(evs[made], cudaEventDisableTiming) == cudaSuccess) ++made;
-        r->side_ok = made == 5;
+            while (made < all && cudaEventCreateWithFlags(evs[made], cudaEventDisableTiming) == cudaSuccess) ++made;
+        r->side_ok = made == all;
         if (!r->side_ok) {
             for (int k = 0; k < made; ++k) cudaEventDestroy(*evs[k]);
             if (r->side) cudaStreamDestroy(r->side);
@@ -459,7 +460,7 @@ extern "C" int pgb_destroy(pgb_run* r) {
     if (r->copy_ev_ok)
         for (int k = 0; k < PGB_COPY_EVENTS; ++k) cudaEventDestroy(r->copy_ev[k]);
     if (r->side_ok)
-        for (cudaEvent_t e : {r->ev_fork, r->ev_join, r->ev_i0, r->ev_i1, r->ev_e0}) cudaEventDestroy(e);
+        for (cudaEvent_t e : {r->ev_fork, r->ev_join, r->ev_i0, r->ev_i1, r->ev_i2, r->ev_e0}) cudaEventDestroy(e);
     if (r->side) cudaStreamDestroy(r->side);
     if (r->ion) cudaStreamDestroy(r->ion);
     if (r->copy_stream) cudaStreamDestroy(r->copy_stream);
@@ -818,8 +819,9 @@ static int clear_charge(pgb_run* r) {
  *
  * Within A and B the electrons and the ions meet in few places: ionization
  * products that are stored (appended to both species, ions at their parent
- * electron's new position), electrons emitted by ion impact (appended
- * before the electron walls'), and the end of the step.  Everything else
+ * electron's new position, after A's charge exchange of the ions before
+ * them), electrons emitted by ion impact (appended before the electron
+ * walls'), and the end of the step.  Everything else
  * touches one species' particles, counters, lists and charge, so the ions'
  * kernels run on a stream of their own beside the electrons' (Lanes), with
  * an event at each of those places: the short kernels between the large
@@ -841,6 +843,7 @@ struct Lanes {
     int fork() { return order(e, i, r->ev_i0); }
     int join() { return order(i, e, r->ev_i1); }
     int ions_after_electrons() { return order(e, i, r->ev_e0); }
+    int electrons_after_ions() { return order(i, e, r->ev_i2); }
 };
 /* the ionization products are stored (so the event list is read) only with
  * steady-state walls or off ion steps: absorbing walls remove them in the
@@ -896,7 +899,9 @@ static int particles_lanes(Lanes& L, bool ion_step) {
     PROF_MARK(r, 1);
     if (products) {
         /* the ionization products join after the push: an ion takes its
-         * parent electron's new position                                */
+         * parent electron's new position; and after A's charge exchange,
+         * which is for the ions that were there before                  */
+        if (ion_step && L.electrons_after_ions()) return PGB_ERR_CUDA;
         if (pgb_launch_ionize_appends(r, r->p.steadystate ? 1 : 0, 1) || L.ions_after_electrons()) return PGB_ERR_CUDA;
     }
     /* inject_more_particles: electrons are pushed as they are created */

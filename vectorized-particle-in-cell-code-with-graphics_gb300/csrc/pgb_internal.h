@@ -210,7 +210,7 @@ struct pgb_run {
     cudaStream_t side = nullptr;
     cudaStream_t ion = nullptr;            /* the ions' kernels, beside the electrons' */
     cudaEvent_t ev_fork, ev_join;
-    cudaEvent_t ev_i0, ev_i1, ev_e0;       /* between the electrons' and the ions' kernels */
+    cudaEvent_t ev_i0, ev_i1, ev_i2, ev_e0;   /* between the electrons' and the ions' kernels */
     bool side_ok = false;
     float* cx_p = nullptr;                 /* per-ion CX probability          */
     float* cx_tile_sum = nullptr;          /* [column][tile] (int64)          */
