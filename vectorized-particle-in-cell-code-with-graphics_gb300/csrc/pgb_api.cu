@@ -781,7 +781,8 @@ extern "C" int pgb_efield(pgb_run* r) {
 
 /* -------------------------------------------------------------- pgb_step */
 /* a step starts from zero charge accumulators and leaves them zero; the
- * phase-by-phase calls leave their charge in them                        */
+ * phase-by-phase calls, and a step that ends in an error, leave their charge
+ * in them                                                                */
 static int clear_charge(pgb_run* r) {
     if (!r->charge_dirty) return 0;
     const size_t G = (size_t)r->nx * r->ny;
@@ -814,7 +815,7 @@ static int clear_charge(pgb_run* r) {
  *                    ds->tf += 1
  * Run in this order they are the reference's step.  The collisions of step
  * t+1 need the particles after step t's walls, not step t's fields, so the
- * pipelined path (issue_one_step) runs them while step t's field solve is
+ * pipelined path (queue_step) runs them while step t's field solve is
  * still in flight on the run's side stream.
  *
  * Within A and B the electrons and the ions meet in few places: ionization
@@ -1134,7 +1135,7 @@ static int launch_merged(pgb_run* r, bool ion_step) {
     return 0;
 }
 
-static int issue_one_step(pgb_run* r) {
+static int queue_step(pgb_run* r) {
     Range range("step");
     int rc;
     const bool pipe = pipelined(r);
@@ -1222,6 +1223,12 @@ static int issue_one_step(pgb_run* r) {
     if (t % 8 == 0 || (r->p.sort_interval > 0 && (t + 1) % r->p.sort_interval == 0))
         PGB_CK(r, cudaMemcpyAsync(r->hs, r->ds, sizeof(DevState), cudaMemcpyDeviceToHost, r->stream));
     return 0;
+}
+
+static int issue_one_step(pgb_run* r) {
+    const int rc = queue_step(r);
+    if (rc) r->charge_dirty = true;   /* it may have ended before its field solve */
+    return rc;
 }
 
 extern "C" int pgb_step(pgb_run* r, int32_t nsteps) {

@@ -1173,12 +1173,14 @@ __global__ void k_load_commit(DevState* ds, int s, long long n) {
     ds->n_pieces[s] = 0;
     ds->sorted_tiles[s] = 0;
 }
-/* the step counters, and the right-wall potential of the first step where
- * there is only one (else the table is copied)                           */
+/* the step counters, the right-wall potential of the first step where there
+ * is only one (else the table is copied), and the ionization events counted
+ * from 0 (a step that ended in an error leaves its count)                */
 __global__ void k_set_step(DevState* ds, long long t, double* phi_tab, double phi, int one) {
     pgb_pdl_entry();
     ds->t = ds->t_base = ds->tf = t;
     if (one) phi_tab[0] = phi;
+    ds->list_n[LIST_ION_EV] = 0;
 }
 
 /* ====================================================== host launchers */
