@@ -105,7 +105,8 @@ inline int pgb_pos_shift(int nx, int ny) {
 /* r = 2^ps / d for pos_from_m: its mantissa in the upper 53 bits, and the
  * shift that leaves the mantissa product in units of 2^-16 less the
  * exponent of x; no x is in range (the division decides) where r is not a
- * normal number                                                          */
+ * normal number, or so large that the exponent field 0 (x zero or subnormal,
+ * whose mantissa has no leading 1) would be                              */
 struct PosScale {
     unsigned long long mant;
     int shift;
@@ -115,6 +116,7 @@ inline PosScale pgb_pos_scale(double d, int ps) {
     if (!std::isnormal(r) || r < 0.0) return PosScale{0ull, -4096};
     int e;
     const double f = std::frexp(r, &e);   /* r = f 2^e, 1/2 <= f < 1 */
+    if (e > 1006) return PosScale{0ull, -4096};   /* up to 1006 the shift at exponent field 0 is above 63 */
     /* x = m 2^(ex - 1075), r = (f 2^53) 2^(e - 53); the product's upper half
      * is m f 2^53 2^-42, so |x| r 2^16 = it * 2^(42 + ex - 1075 + e - 53 + 16) */
     return PosScale{(unsigned long long)std::ldexp(f, 53) << 11, 1070 - e};
