@@ -900,7 +900,7 @@ __global__ void __launch_bounds__(INJECT_BLOCK_MAX) k_inject_block(InjectArgs a,
             for (unsigned m = s_out[w]; m; m &= m - 1) {
                 const int j = 32 * w + __ffs(m) - 1;
                 if (pos < a.list_cap) a.list_out_e[pos++] = (int)(n0 + j);
-                else a.ds->err |= ERR_LIST;
+                else atomicOr(&a.ds->err, ERR_LIST);   /* the ions' injection may report beside it */
             }
         a.ds->list_n[LIST_OUT_E] = pos;
     }
@@ -995,7 +995,7 @@ __global__ void k_ionize_append(IonizeAppendArgs a) {
                 a.i.w[s2] = a.e.w[slot];
                 a.i.id[s2] = idi0 + (unsigned int)r;
             } else {
-                a.ds->err |= ERR_CAP_I;
+                atomicOr(&a.ds->err, ERR_CAP_I);
             }
         }
         if (a.store_e) {
@@ -1007,7 +1007,7 @@ __global__ void k_ionize_append(IonizeAppendArgs a) {
                 a.e.w[s2] = a.e.w[slot];
                 a.e.id[s2] = ide0 + (unsigned int)r;
             } else {
-                a.ds->err |= ERR_CAP_E;
+                atomicOr(&a.ds->err, ERR_CAP_E);
             }
         }
     }
