@@ -1125,6 +1125,17 @@ static bool host_work_due(pgb_run* r) {
     return false;
 }
 
+/* a species whose slots, by counts up to eight steps old, may reach its
+ * capacity in the next eight steps                                       */
+static bool near_capacity(const pgb_run* r) {
+    const long long pad = sort_pad_slots(&r->p);
+    for (int s = 0; s < 2; ++s) {
+        const long long n = r->hs->n[s], grow = std::max<long long>(n - pad, 0) / 4 + 16ll * r->p.number_to_inject;
+        if (n + grow > r->sp[s].cap) return true;
+    }
+    return false;
+}
+
 /* The pipelined step as one graph launch, captured once per key
  * (step_merged).  0: launched; 1: not available, use the separate graphs. */
 static int launch_merged(pgb_run* r, bool ion_step) {
@@ -1218,9 +1229,10 @@ static int queue_step(pgb_run* r) {
      * when to compact and, before a sort, whether the storage has to grow,
      * which never changes results.  A copy between two steps' graphs costs
      * some 3 us, so only every eighth step, and the one before a sort, has
-     * one.                                                                */
+     * one; each step where a species comes near its capacity, which only a
+     * compaction or a growth in time keeps it below.                      */
     const long long t = r->time_step;
-    if (t % 8 == 0 || (r->p.sort_interval > 0 && (t + 1) % r->p.sort_interval == 0))
+    if (t % 8 == 0 || (r->p.sort_interval > 0 && (t + 1) % r->p.sort_interval == 0) || near_capacity(r))
         PGB_CK(r, cudaMemcpyAsync(r->hs, r->ds, sizeof(DevState), cudaMemcpyDeviceToHost, r->stream));
     return 0;
 }
