@@ -1,0 +1,64 @@
+"""Step graphs follow the particle counts.
+
+A captured step keeps the kernel variants and grids of its capture.  A handle
+with its storage reserved that first steps a few particles and is then loaded
+with many must step those as a new handle does: the same state, and in the
+same time (a factor of 2 allowed; grids made for 500 particles take more than
+five times as long for two million).
+"""
+import time
+
+import numpy as np
+import pytest
+
+import picgb
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(p, n, seed):
+    rng = np.random.default_rng(seed)
+    out = []
+    for m, t in ((picgb.ELECTRON_MASS, 2.0), (p.ion_mass, 0.03)):
+        a = np.empty((n, 6))
+        a[:, :2] = rng.uniform(0.02, 0.98, (n, 2)) * p.xlength
+        a[:, 2:5] = rng.normal(0.0, np.sqrt(t * picgb.CHARGE / m), (n, 3))
+        a[:, 5] = 1.0
+        out.append(a)
+    return out
+
+
+def _steps(r, state):
+    for s in (0, 1):
+        r.load_particles(s, state[s])
+    r.set_time_step(0)
+    r.set_rho(np.zeros((65, 65)))   # no field of the particles before
+    r.poisson(0)
+    r.efield()
+    r.step(12)
+    t = time.perf_counter()
+    r.step(20)
+    t = time.perf_counter() - t
+    return [r.get_particles(s) for s in (0, 1)] + [r.get_grid(k) for k in ("q_e", "q_i", "phi")], t
+
+
+@pytest.mark.parametrize("collisions,dti,sort", [(True, 2.0, 0), (True, 2.0, 8), (False, 2.0, 0)])
+def test_many_particles_after_few_step_as_in_a_new_handle(collisions, dti, sort):
+    n = 2000003
+    p = picgb.make_params(X_NO_OF_CELLS=65, STEADYSTATE="NO", HAVE_COLLISIONS=collisions, GAS_PRESSURE_TORR=0.01,
+                          SIGMA_ELASTIC="ENERGY_DEPENDENT", SIGMA_IONIZATION="ENERGY_DEPENDENT", POISSON="DST_DC",
+                          DC_MAX_ITERS=2, DTI_RATIO=dti, SORT_INTERVAL=sort, SIZE_TO_CHECK=2**31 - 1,
+                          CAPACITY_E=3 * n, CAPACITY_I=3 * n, E_MACROPARTICLE_SIZE=100.0, ION_MACROPARTICLE_SIZE=100.0)
+    few, many = _state(p, 500, 1), _state(p, n, 2)
+    with picgb.Run(p) as r:
+        want, t_new = _steps(r, many)
+    with picgb.Run(p) as r:
+        _steps(r, few)
+        got, t = _steps(r, many)
+        back, _ = _steps(r, few)
+    with picgb.Run(p) as r:
+        want_few, _ = _steps(r, few)
+    for a, b in ((got, want), (back, want_few)):
+        for k, (x, y) in enumerate(zip(a, b)):
+            assert np.array_equal(x, y, equal_nan=True), k
+    assert t < 2.0 * t_new, (t, t_new)

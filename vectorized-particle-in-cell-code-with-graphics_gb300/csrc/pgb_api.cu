@@ -1047,6 +1047,38 @@ static void drop_graphs(pgb_run* r) {
         if (r->graph_m[k]) { cudaGraphExecDestroy(r->graph_m[k]); r->graph_m[k] = nullptr; }
     }
     if (r->graph_f) { cudaGraphExecDestroy(r->graph_f); r->graph_f = nullptr; }
+    r->graphs_made = false;
+    r->graph_steps_less = 0;
+}
+
+/* A captured step keeps the kernel variants and grids that the counts of its
+ * capture chose (push_whole, pgb_launch_mcc, pgb_launch_deposit): right for
+ * any count, but made for those.  A step of one million particles a species,
+ * 65^2 nodes, argon: 0.98 ms in the graphs of 2000 particles, 0.074 in its
+ * own; one of 2000 in the graphs of one million 0.048, in its own 0.045; new
+ * graphs cost 0.1 to 0.6 ms.  So they are made anew at once where a count
+ * has more than doubled, and after GRAPH_PATIENCE steps, in which the gain
+ * may pay for them, where one has more than halved.  (A sort pads a species
+ * by up to `pad` slots, which a load takes away: that is no halving.)      */
+#define GRAPH_PATIENCE 200
+static bool counts_left_graphs(pgb_run* r) {
+    if (!r->graphs_made) return false;
+    const long long pad = sort_pad_slots(&r->p), few = 1024;
+    bool less = false;
+    for (int s = 0; s < 2; ++s) {
+        const long long n = r->hs->n[s], made = r->graph_n[s];
+        if (n > 2 * std::max(made, few)) return true;
+        less = less || made > 2 * std::max(n + pad, few);
+    }
+    r->graph_steps_less = less ? r->graph_steps_less + 1 : 0;
+    return r->graph_steps_less > GRAPH_PATIENCE;
+}
+/* drop the graphs, once what is queued of them has run */
+static int renew_graphs(pgb_run* r) {
+    for (cudaStream_t st : {r->stream, r->side, r->ion})
+        if (st) PGB_CK(r, cudaStreamSynchronize(st));
+    drop_graphs(r);
+    return 0;
 }
 
 /* graphs are usable when no step needs a host decision: no profiling and
@@ -1058,6 +1090,7 @@ static bool graphs_ok(pgb_run* r) {
 /* capture fn(r, ion_step) as a graph; -1 if the launches cannot be captured */
 static int capture(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGraphExec_t* out, long long* nl) {
     cudaGraph_t g = nullptr;
+    const long long n0[2] = {r->hs->n[0], r->hs->n[1]};   /* the counts may come back meanwhile */
     PGB_CK(r, cudaStreamBeginCapture(r->stream, cudaStreamCaptureModeThreadLocal));
     long long l0 = r->launches;
     int rc = fn(r, ion_step);
@@ -1070,6 +1103,10 @@ static int capture(pgb_run* r, int (*fn)(pgb_run*, bool), bool ion_step, cudaGra
     }
     *nl = r->launches - l0;
     r->launches = l0;
+    if (!r->graphs_made) {
+        for (int s = 0; s < 2; ++s) r->graph_n[s] = n0[s];
+        r->graphs_made = true;
+    }
     e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
@@ -1149,6 +1186,7 @@ static int launch_merged(pgb_run* r, bool ion_step) {
 static int queue_step(pgb_run* r) {
     Range range("step");
     int rc;
+    if (counts_left_graphs(r) && (rc = renew_graphs(r))) return rc;
     const bool pipe = pipelined(r);
     bool forked = false, merged = false;
     if (pipe && r->fields_pending && !host_work_due(r)) {

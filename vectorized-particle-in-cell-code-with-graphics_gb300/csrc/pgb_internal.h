@@ -202,6 +202,9 @@ struct pgb_run {
      * then B -- one launch for a step that needs no host decision         */
     cudaGraphExec_t graph_m[8] = {};
     long long graph_m_launches[8] = {};
+    bool graphs_made = false;              /* any of them, by the counts graph_n */
+    long long graph_n[2] = {0, 0};
+    int graph_steps_less = 0;              /* steps since a count was less than half of graph_n */
     /* launch shapes (pgb_set_launch_config, pgb_autotune): they change no
      * result.  push grid = SMs x tune_push_per_sm; the collision kernels
      * beside a field solve leave it tune_field_sms SMs                   */
