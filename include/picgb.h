@@ -148,8 +148,8 @@ typedef struct pgb_profile {
     int64_t slots_e, slots_i;      /* particle slots swept by the push kernels     */
     int64_t launches;              /* kernel launches issued since pgb_create      */
     double ms_push_e_kernel;       /* the electron push kernel alone (in ms_push_e) */
-    double ms_collide_e;           /* the electron collision kernel alone (in ms_push_e)   */
-    double ms_scatter_e;           /* the gap after it: it does the scatterings too         */
+    double ms_collide_e;           /* the electron collision kernel, with its scatterings (in ms_push_e) */
+    double ms_scatter_e;           /* 0: no kernel of their own (the field keeps the layout)  */
 } pgb_profile;
 
 typedef struct pgb_run pgb_run;

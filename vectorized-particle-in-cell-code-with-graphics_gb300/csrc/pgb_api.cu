@@ -456,7 +456,7 @@ extern "C" int pgb_destroy(pgb_run* r) {
     cudaFree(r->rd_img);
     cudaFree(r->rd_scratch);
     if (r->prof_ev_ok)
-        for (int k = 0; k < 13; ++k) cudaEventDestroy(r->prof_ev[k]);
+        for (int k = 0; k < PGB_PROF_EVENTS; ++k) cudaEventDestroy(r->prof_ev[k]);
     if (r->copy_ev_ok)
         for (int k = 0; k < PGB_COPY_EVENTS; ++k) cudaEventDestroy(r->copy_ev[k]);
     if (r->side_ok)
@@ -859,13 +859,12 @@ static int collide_lanes(Lanes& L, int leave_sms, bool ion_step) {
     const bool products = products_stored(r, ion_step);
     if (pgb_launch_mcc(r, leave_sms, !products)) return PGB_ERR_CUDA;
     PROF_MARK(r, 9);
-    PROF_MARK(r, 10);
     if (products && pgb_build_list(r, LIST_ION_EV, 0)) return PGB_ERR_CUDA;
-    PROF_MARK(r, 11);
+    PROF_MARK(r, 10);
     L.ions();
     if (ion_step && pgb_launch_cx(r, 0, 0)) return PGB_ERR_CUDA;
     L.electrons();
-    PROF_MARK(r, 12);
+    PROF_MARK(r, 11);
     return 0;
 }
 
@@ -1026,9 +1025,7 @@ static int profile_collect(pgb_run* r) {
     if (r->p.have_collisions) {
         PGB_CK(r, cudaEventElapsedTime(&mk, r->prof_ev[0], r->prof_ev[9]));
         r->prof.ms_collide_e += mk;
-        PGB_CK(r, cudaEventElapsedTime(&mk, r->prof_ev[9], r->prof_ev[10]));
-        r->prof.ms_scatter_e += mk;
-        PGB_CK(r, cudaEventElapsedTime(&mk, r->prof_ev[11], r->prof_ev[12]));
+        PGB_CK(r, cudaEventElapsedTime(&mk, r->prof_ev[10], r->prof_ev[11]));
         r->prof.ms_collide_ions += mk;
     }
     r->prof.ms_walls += ms[1] + ms[4];
@@ -1493,7 +1490,7 @@ extern "C" int pgb_autotune(pgb_run* r, int32_t steps, pgb_launch_config* best, 
 extern "C" int pgb_set_profiling(pgb_run* r, int on) {
     if (!r) return PGB_ERR_ARG;
     if (on && !r->prof_ev_ok) {
-        for (int k = 0; k < 13; ++k) PGB_CK(r, cudaEventCreate(&r->prof_ev[k]));
+        for (int k = 0; k < PGB_PROF_EVENTS; ++k) PGB_CK(r, cudaEventCreate(&r->prof_ev[k]));
         r->prof_ev_ok = true;
     }
     memset(&r->prof, 0, sizeof(r->prof));

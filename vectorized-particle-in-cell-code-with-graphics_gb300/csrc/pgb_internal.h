@@ -40,6 +40,7 @@
 #define PGB_SORT_CHUNK 4096    /* slots per chunk of the bin sort passes      */
 #define PGB_COPY_CHUNK (1 << 20)   /* particles per host-copy chunk of load/dump */
 #define PGB_COPY_EVENTS 32
+#define PGB_PROF_EVENTS 12     /* section marks of a profiled step               */
 
 enum { ST_ABS_E = 0, ST_ABS_I, ST_PLOP, ST_REFL, ST_BACK, ST_SEE_EV, ST_SEE_EM, ST_ISEE_EM,
        ST_ELASTIC, ST_IONIZE, ST_CX, ST_INJ_E, ST_INJ_I, ST_RED_E, ST_RED_I, ST_COUNT };
@@ -265,7 +266,7 @@ struct pgb_run {
     int fault_alloc = 0, alloc_events = 0;
     int prof_on = 0;
     pgb_profile prof;
-    cudaEvent_t prof_ev[13];
+    cudaEvent_t prof_ev[PGB_PROF_EVENTS];
     bool prof_ev_ok = false;
 };
 
