@@ -731,7 +731,7 @@ extern "C" int pgb_collide_ions(pgb_run* r) {
     int rc = need_particles(r);
     if (rc) return rc;
     if ((rc = set_device_step(r, r->time_step, 1))) return rc;
-    if (pgb_launch_cx(r, 0, 0)) return PGB_ERR_CUDA;
+    if (pgb_launch_cx(r, 0)) return PGB_ERR_CUDA;
     return sync_state(r);
 }
 
@@ -862,7 +862,7 @@ static int collide_lanes(Lanes& L, int leave_sms, bool ion_step) {
     if (products && pgb_build_list(r, LIST_ION_EV, 0)) return PGB_ERR_CUDA;
     PROF_MARK(r, 10);
     L.ions();
-    if (ion_step && pgb_launch_cx(r, 0, 0)) return PGB_ERR_CUDA;
+    if (ion_step && pgb_launch_cx(r, 0)) return PGB_ERR_CUDA;
     L.electrons();
     PROF_MARK(r, 11);
     return 0;
@@ -915,7 +915,7 @@ static int particles_lanes(Lanes& L, bool ion_step) {
          * ionization products of an ion step are not stored), one block  */
         const bool appended = inject || r->p.steadystate;
         const bool few = !r->p.steadystate && r->p.number_to_inject <= 4096;
-        if (r->p.have_collisions && appended && pgb_launch_cx(r, few ? 2 : 1, 0)) return PGB_ERR_CUDA;
+        if (r->p.have_collisions && appended && pgb_launch_cx(r, few ? 2 : 1)) return PGB_ERR_CUDA;
         PROF_MARK(r, 3);
         if (pgb_launch_push(r, 1, true, absorb_i)) return PGB_ERR_CUDA;
         if (!absorb_i && pgb_build_list(r, LIST_OUT_I, 1, inject ? 0 : commit_i)) return PGB_ERR_CUDA;

@@ -276,15 +276,16 @@ bool pgb_cuda_ok(pgb_run* r, cudaError_t e, const char* what);
 void pgb_set_unbound_error(const std::string& msg);
 /* Programmatic dependent launch.  A kernel launched with pgb_launch_pdl may
  * be launched while the previous kernel on its stream finishes: as that
- * kernel's blocks exit, the next one's are scheduled.  Its first statement
- * is pgb_pdl_entry(), whose griddepcontrol.wait blocks until the previous
- * kernel has completed and its writes are visible.  No memory is touched
- * before it, so results are those of plain launches; what it saves is the
- * launch gap.  No kernel triggers its dependents early: blocks parked at
- * the wait would hold SM slots that other runs' streams need when many
- * runs share the GPU (pgb_step_batch), which cost those a third of their
- * throughput.  On a kernel launched without the attribute the wait does
- * nothing.                                                                */
+ * kernel's blocks exit, the next one's are scheduled.  It starts with
+ * pgb_pdl_entry(), whose griddepcontrol.wait blocks until the previous
+ * kernel has completed and its writes are visible.  Nothing that a run
+ * changes is read and nothing in global memory is written before it (the
+ * sine transforms load their twiddles, which only pgb_create writes), so
+ * results are those of plain launches; what it saves is the launch gap.
+ * No kernel triggers its dependents early: blocks parked at the wait would
+ * hold SM slots that other runs' streams need when many runs share the GPU
+ * (pgb_step_batch), which cost those a third of their throughput.  On a
+ * kernel launched without the attribute the wait does nothing.            */
 #ifdef __CUDACC__
 __device__ __forceinline__ void pgb_pdl_entry() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... KArgs, typename... Args>
@@ -343,7 +344,7 @@ int pgb_launch_ionize_appends(pgb_run* r, int store_e, int store_i);
 int pgb_launch_mcc(pgb_run* r, int leave_sms, bool count_events = false);
 /* tail 0: the ions present (records their count); 1: those appended since;
  * 2: the same in one block, for a tail of a few thousand ions at most     */
-int pgb_launch_cx(pgb_run* r, int tail, int leave_sms);
+int pgb_launch_cx(pgb_run* r, int tail);
 /* advance: the last kernel of the electron (or steady) walls ends the step,
  * after entering the products of the species in commit                   */
 int pgb_launch_walls(pgb_run* r, int which, bool advance = false, int commit = 0);

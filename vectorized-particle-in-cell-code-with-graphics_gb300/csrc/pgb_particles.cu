@@ -812,7 +812,6 @@ struct InjectArgs {
     uint64_t seed;
     PushConsts pce;
     const float2* exy;
-    unsigned long long* qacc_e;
     int push_e;                  /* push the new electrons (inside pgb_step) */
     int absorb_e;                /* ... and remove those that leave          */
     int species_mask;            /* 1 = electrons, 2 = ions                  */
@@ -1372,7 +1371,7 @@ int pgb_launch_inject(pgb_run* r, int species_mask, bool push_e, int commit, boo
     a.e = r->sp[0]; a.i = r->sp[1]; a.ds = r->ds; a.k = r->p.number_to_inject;
     a.dx = r->dx; a.dy = r->dy; a.xlength = r->p.xlength; a.ylength = r->p.ylength;
     a.seed = r->p.seed;
-    a.pce = push_consts(r, 0); a.exy = r->exy; a.qacc_e = r->qacc[0];
+    a.pce = push_consts(r, 0); a.exy = r->exy;
     a.push_e = push_e; a.absorb_e = absorb_e; a.species_mask = species_mask;
     a.list_out_e = r->list[LIST_OUT_E]; a.list_cap = r->list_cap;
     a.flag = r->inject_flag;

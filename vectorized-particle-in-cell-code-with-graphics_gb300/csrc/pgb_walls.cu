@@ -962,7 +962,7 @@ int pgb_launch_walls(pgb_run* r, int which, bool advance, int commit) {
     return 0;
 }
 
-int pgb_launch_cx(pgb_run* r, int tail, int leave_sms) {
+int pgb_launch_cx(pgb_run* r, int tail) {
     CxArgs a;
     a.tail = tail ? 1 : 0;
     a.i = r->sp[1]; a.ds = r->ds; a.nx = r->nx; a.ny = r->ny; a.ps = r->ps;
@@ -982,8 +982,7 @@ int pgb_launch_cx(pgb_run* r, int tail, int leave_sms) {
         PGB_CK(r, cudaGetLastError());
         return 0;
     }
-    const int sms = r->sms - leave_sms > 8 ? r->sms - leave_sms : 8;
-    PGB_CK(r, pgb_launch_pdl(k_cx_tiles, dim3(sms * 4), dim3(256), 2 * sizeof(unsigned int) * r->nx, r->stream, a));
+    PGB_CK(r, pgb_launch_pdl(k_cx_tiles, dim3(r->sms * 4), dim3(256), 2 * sizeof(unsigned int) * r->nx, r->stream, a));
     r->launches++;
     PGB_CK(r, pgb_launch_pdl(k_cx_walk, dim3((r->nx + CX_WALK_WARPS - 1) / CX_WALK_WARPS), dim3(32 * CX_WALK_WARPS), 0, r->stream, a));
     r->launches++;
