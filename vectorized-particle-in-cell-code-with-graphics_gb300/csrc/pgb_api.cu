@@ -1159,6 +1159,28 @@ static bool host_work_due(pgb_run* r) {
     return false;
 }
 
+/* The slots a species may have now: its count when last read back, the
+ * injection of the steps queued since, and the padding of a sort since.
+ * The host may be many steps ahead of the GPU, and a count from the start of
+ * the queue alone would not show that a compaction or a growth is due.    */
+static long long slots_by_now(const pgb_run* r, int s, bool* stale) {
+    const long long seen = *(volatile const long long*)&r->hs->steps;   /* before n: the copy may land meanwhile */
+    const long long n = *(volatile const long long*)&r->hs->n[s], inject = r->p.number_to_inject;
+    *stale = inject > 0 && r->steps > seen;
+    if (!*stale) return n;
+    return n + (r->steps - seen) * inject + (seen <= r->sorted_at[s] ? sort_pad_slots(&r->p) : 0);
+}
+/* runs without sort: the counts themselves, where this step's injection may
+ * not fit before a compaction                                             */
+static int settle_counts(pgb_run* r) {
+    if (r->p.sort_interval > 0) return 0;
+    for (int s = 0; s < 2; ++s) {
+        bool stale;
+        if (slots_by_now(r, s, &stale) + r->p.number_to_inject > r->sp[s].cap && stale) return sync_state(r);
+    }
+    return 0;
+}
+
 /* a species whose slots, by counts up to eight steps old, may reach its
  * capacity in the next eight steps                                       */
 static bool near_capacity(const pgb_run* r) {
@@ -1183,6 +1205,7 @@ static int launch_merged(pgb_run* r, bool ion_step) {
 static int queue_step(pgb_run* r) {
     Range range("step");
     int rc;
+    if ((rc = settle_counts(r))) return rc;
     if (counts_left_graphs(r) && (rc = renew_graphs(r))) return rc;
     const bool pipe = pipelined(r);
     bool forked = false, merged = false;
@@ -1216,9 +1239,11 @@ static int queue_step(pgb_run* r) {
         for (int s = 0; s < 2; ++s)
             if (r->time_step % ((long long)r->p.sort_interval * (s ? PGB_ION_SORT_FACTOR : 1)) == 0) {
                 /* the padded layout needs n + pad slots; grow first if the
-                 * (lazily read) count comes near the capacity              */
+                 * count comes near the capacity                            */
                 const long long pad = sort_pad_slots(&r->p);
-                if (r->hs->n[s] + r->hs->n[s] / 8 + pad > r->sp[s].cap) {
+                bool stale;
+                const long long now = slots_by_now(r, s, &stale);
+                if (now + now / 8 + pad > r->sp[s].cap) {
                     if ((rc = sync_state(r))) return rc;
                     const long long need = 2 * r->hs->n[s] + 65536 + pad;   /* > n + n/8 + pad */
                     if (r->hs->n[s] + r->hs->n[s] / 8 + pad > r->sp[s].cap &&
@@ -1226,6 +1251,7 @@ static int queue_step(pgb_run* r) {
                         return rc;
                 }
                 if (pgb_launch_sort(r, s)) return PGB_ERR_CUDA;
+                r->sorted_at[s] = r->steps;
                 r->orient[s] ^= 1;
             }
     } else {
@@ -1260,6 +1286,7 @@ static int queue_step(pgb_run* r) {
         if ((rc = flush_fields(r)) || (rc = pgb_launch_graphs(r))) return rc;
     }
     r->time_step += 1;
+    r->steps += 1;
     /* Counters come back asynchronously; the host reads them only to decide
      * when to compact and, before a sort, whether the storage has to grow,
      * which never changes results.  A copy between two steps' graphs costs
@@ -1274,7 +1301,13 @@ static int queue_step(pgb_run* r) {
 
 static int issue_one_step(pgb_run* r) {
     const int rc = queue_step(r);
-    if (rc) r->charge_dirty = true;   /* it may have ended before its field solve */
+    if (rc) {
+        /* the step may have ended before its field solve, the solve of the
+         * step before be pending or on the side stream                    */
+        flush_fields(r);
+        if (r->side) cudaStreamSynchronize(r->side);
+        r->charge_dirty = true;
+    }
     return rc;
 }
 
@@ -1348,7 +1381,10 @@ extern "C" int pgb_step_batch(pgb_run* const* runs, int32_t nruns, int32_t nstep
         for (int k = 0; k < chunk; ++k)
             for (int a = 0; a < nruns; ++a) {
                 int rc = issue_one_step(runs[a]);
-                if (rc) return rc;
+                if (rc) {
+                    for (int b = 0; b < nruns; ++b) flush_fields(runs[b]);   /* of the steps that did run */
+                    return rc;
+                }
             }
         for (int a = 0; a < nruns; ++a) {
             int rc = flush_fields(runs[a]);

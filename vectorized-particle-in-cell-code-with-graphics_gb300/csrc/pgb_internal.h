@@ -71,6 +71,7 @@ struct DevState {
     unsigned int ticket_f;   /* the same of k_field                              */
     int work[2];             /* items of the push taken, per species; 0 between launches */
     int work_done[2];        /* blocks of the push that are done                 */
+    long long steps;         /* steps run since pgb_create                       */
     long long n_cx;          /* ion slots whose charge exchange was tested before this
                                 step's appends (the rest are tested after them)       */
 };
@@ -212,6 +213,8 @@ struct pgb_run {
     int tune_push_per_sm = 8;
     int tune_field_sms = 32;
     bool fields_pending = false;           /* last step's field solve not yet issued */
+    int64_t steps = 0;                     /* steps queued since pgb_create (ds->steps: run) */
+    int64_t sorted_at[2] = {-1, -1};       /* ... when a species was last sorted       */
     bool charge_dirty = true;              /* the charge accumulators may not be zero  */
     cudaStream_t side = nullptr;
     cudaStream_t ion = nullptr;            /* the ions' kernels, beside the electrons' */
@@ -323,6 +326,7 @@ __device__ __forceinline__ void ionize_count_commit(DevState* ds, int species_ma
  * ionization events are counted from 0 again.  One thread.               */
 __device__ __forceinline__ void pgb_step_end(DevState* ds) {
     ds->t += 1;
+    ds->steps += 1;
     ds->list_n[LIST_ION_EV] = 0;
 }
 #endif
