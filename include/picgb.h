@@ -208,9 +208,10 @@ PGB_API int pgb_initial_boundary(pgb_run* run);
 PGB_API int pgb_step(pgb_run* run, int32_t nsteps);
 
 /* pgb_step without waiting: the steps are queued on the run's stream and
- * the call returns (no reference counterpart); it waits for queued steps
- * only where the storage has to grow or the counts call for new graphs.  pgb_query tells when the
- * run is idle again; pgb_sync waits for it.  Reads of the run's particles,
+ * the call returns (no reference counterpart).  It waits for queued steps
+ * only where the storage may have to be compacted or to grow, or where the
+ * particle counts call for new step graphs.  pgb_query tells when the run
+ * is idle again; pgb_sync waits for it.  Reads of the run's particles,
  * grids or counters wait for the queued steps themselves.               */
 PGB_API int pgb_step_async(pgb_run* run, int32_t nsteps);
 /* *idle = 1 when no work of the run is queued; device errors of finished
